@@ -9,6 +9,7 @@ them. Weights are N(0, 0.02), activations N(0, 1), biases N(0, 0.01), made from 
     prepare(case, seed)   inputs, weights and output buffers
     run(state)            one pass; returns the outputs as torch views of the library's buffers
     work(case)            bytes and floating-point operations one pass cannot do without
+    exact(case, seed)     the outputs in float64, without the library's code
     tolerance(case)       how far another correct implementation of the same precision may be off
 """
 from __future__ import annotations
@@ -353,6 +354,136 @@ def work(case):
         m, d, n = c["m"], c["hidden"], c["ffn"]
         b, f = c["layers"] * (_q(4 * d, d) + 2 * _q(n, d)) + 6 * m * d, c["layers"] * 2 * m * d * (4 * d + 2 * n)
     return {"bytes": b, "flops": f}
+
+
+# ---- the same results in 64 bits, without the library ------------------------------------------------------------------------
+_E2M1 = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0]
+
+
+def _bf16(x):
+    return x.to(torch.bfloat16).double()
+
+
+def _nvfp4(x, g):
+    """What the NVFP4 copy of a bf16 matrix stands for, without the per-tensor scale g: code times block scale, in float64.
+    The format's own operations are 32-bit ones: scale = e4m3(max * (1 / (6 g))), code = e2m1(x * (1 / (scale * g)))."""
+    one, out = torch.ones((), device=x.device), torch.empty(x.shape, dtype=torch.float64, device=x.device)
+    g = one * g
+    mid = torch.tensor([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], device=x.device)
+    values = torch.tensor(_E2M1, dtype=torch.float64, device=x.device)
+    for i in range(0, x.shape[0], 2048):
+        b = x[i:i + 2048].float().reshape(-1, 16)
+        s = (b.abs().amax(1, keepdim=True) * (one / (6.0 * g))).clamp(max=448.0).to(torch.float8_e4m3fn).float()
+        y = b * torch.where(s > 0, one / (s * g), 0.0)
+        a = y.abs()
+        code = torch.bucketize(a, mid)  # a tie stays in the lower interval ...
+        for t in (1, 3, 5):  # ... and goes up where the lower code is odd
+            code = torch.where(a == mid[t], t + 1, code)
+        out[i:i + 2048] = (torch.copysign(values[code], y.double()) * s.double()).reshape(-1, x.shape[1])
+    return out
+
+
+def _gelu64(v):
+    return 0.5 * v * (1.0 + torch.tanh(math.sqrt(2.0 / math.pi) * (v + 0.044715 * v ** 3)))
+
+
+class _Draws:
+    """The numbers prepare() draws, in its order."""
+
+    def __init__(self, seed):
+        self.gen = torch.Generator(device="cuda:0")
+        self.gen.manual_seed(int(seed))
+
+    randn = _State.randn
+
+    def tensor(self, values):
+        return values.to(torch.bfloat16).double()
+
+    def weight(self, n, k):
+        """(code times block scale, per-tensor scale, bias)"""
+        w = (self.randn(n, k) * 0.02).to(torch.bfloat16)
+        g = float(w.float().abs().max() / 2688.0)
+        return _nvfp4(w, g), g, self.tensor(self.randn(n) * 0.01)
+
+
+def _linear64(a, g_a, w, act=0):
+    v = (a @ w[0].T) * (g_a * w[1]) + w[2]
+    return _gelu64(v) if act else v
+
+
+def _attention64(q, k, v, heads, kv_heads):
+    out = torch.empty_like(q)
+    for h in range(heads):
+        j = h * kv_heads // heads
+        cols, kv = slice(h * HEAD, (h + 1) * HEAD), slice(j * HEAD, (j + 1) * HEAD)
+        for i in range(0, q.shape[0], 4096):
+            s = q[i:i + 4096, cols] @ k[:, kv].T * HEAD ** -0.5
+            out[i:i + 4096, cols] = torch.softmax(s, 1) @ v[:, kv]
+    return out
+
+
+def _f32(g):
+    return float(np.float32(g))
+
+
+def exact(case, seed):
+    """run()'s outputs in float64; what the path stores in bf16 or NVFP4 between two kernels is rounded to that format."""
+    c, d = case, _Draws(seed)
+    if c["kind"] == "linear":
+        m, n, k = c["m"], c["n"], c["k"]
+        w = d.weight(n, k)
+        x = d.randn(m, k)
+        g = _f32(_scale_of(x.abs().max()))
+        v = _linear64(d.tensor(x), 1.0, w, c["act"]) if c["dense"] else _linear64(_nvfp4(x.to(torch.bfloat16), g), g, w, c["act"])
+        if c["swiglu"]:
+            v = v[:, 0::2] * torch.sigmoid(v[:, 0::2]) * v[:, 1::2]
+        if c["gate"]:
+            gate = d.tensor(d.randn(n) * 0.5)
+            v = d.tensor(d.randn(m, n)) + gate * v
+        return v
+    if c["kind"] == "ffn":
+        m, k, ffn = c["m"], c["k"], c["ffn"]
+        up, down = d.weight(ffn, k), d.weight(k, ffn)
+        x = d.randn(m, k)
+        g_x, g_h = _f32(_scale_of(x.abs().max())), _f32(_scale_of(5.5 * 0.02 * math.sqrt(k)))
+        a, out = _nvfp4(x.to(torch.bfloat16), g_x), torch.empty(m, k, dtype=torch.float64, device=x.device)
+        for i in range(0, m, 8192):
+            h = _linear64(a[i:i + 8192], g_x, up, 1).to(torch.bfloat16)
+            out[i:i + 8192] = _linear64(_nvfp4(h, g_h), g_h, down)
+        return out
+    if c["kind"] == "block":
+        m, dim, ffn = c["m"], c["hidden"], c["ffn"]
+        w_qkv, w_out, w_up, w_down = (d.weight(n, k) for n, k in ((3 * dim, dim), (dim, dim), (ffn, dim), (dim, ffn)))
+        x = d.tensor(d.randn(m, dim))
+        mod = [[d.tensor(d.randn(dim) * s) for s in (0.2, 0.3, 0.1)] for _ in (0, 1)]
+        s_lin = 0.02 * math.sqrt(dim)
+        g_x, g_up = _f32(_scale_of(7.0)), _f32(_scale_of(5.5 * s_lin))
+        g_at = _f32(_scale_of(5.5 * s_lin * math.sqrt(0.2 ** 2 + min(1.0, math.exp(min(s_lin ** 4, 3.0)) / m))))
+
+        def normed(v, shift, scale):
+            n = (v - v.mean(1, keepdim=True)) / torch.sqrt(v.var(1, unbiased=False, keepdim=True) + 1e-6)
+            return _nvfp4((n * (1.0 + scale) + shift).to(torch.bfloat16), g_x)
+
+        qkv = _bf16(_linear64(normed(x, mod[0][0], mod[0][1]), g_x, w_qkv))
+        at = _attention64(qkv[:, :dim], qkv[:, dim:2 * dim], qkv[:, 2 * dim:], dim // HEAD, dim // HEAD)
+        h1 = x + mod[0][2] * _linear64(_nvfp4(at.to(torch.bfloat16), g_at), g_at, w_out)
+        up = _linear64(normed(_bf16(h1), mod[1][0], mod[1][1]), g_x, w_up, 1)
+        return h1, _bf16(h1) + mod[1][2] * _linear64(_nvfp4(up.to(torch.bfloat16), g_up), g_up, w_down)
+    if c["kind"] == "sdpa":
+        b, s_q, s_k, hq, hk = c["b"], c["s_q"], c["s_k"], c["heads"], c["kv_heads"]
+        q, k, v = (d.tensor(d.randn(b * s, h * HEAD)) for s, h in ((s_q, hq), (s_k, hk), (s_k, hk)))
+        return torch.cat([_attention64(q[i * s_q:(i + 1) * s_q], k[i * s_k:(i + 1) * s_k], v[i * s_k:(i + 1) * s_k], hq, hk) for i in range(b)])
+    if c["kind"] == "stack":
+        dim, ffn, m = c["hidden"], c["ffn"], c["m"]
+        shapes = ((3 * dim, dim), (dim, dim), (ffn, dim), (dim, ffn))
+        for _ in range(c["layers"]):  # only the last layer's weights reach the result: every layer starts from the auxiliary input
+            w = [d.weight(n, k) for n, k in shapes]
+        d.randn(m, dim)
+        g, v = _f32(_scale_of(5.5)), d.randn(m, dim)
+        for wj, act in zip(w[1:], (0, 1, 0)):
+            v = _linear64(_nvfp4(v.to(torch.bfloat16), g), g, wj, act)
+        return v
+    return None  # codes, scales and bytes: the same everywhere
 
 
 # Measured against a float64 evaluation of the same contract (dequantised operands, exact softmax, tanh and GELU; every tensor
