@@ -402,7 +402,7 @@ class _Draws:
     def weight(self, n, k):
         """(code times block scale, per-tensor scale, bias)"""
         w = (self.randn(n, k) * 0.02).to(torch.bfloat16)
-        g = float(w.float().abs().max() / 2688.0)
+        g = float(np.float32(float(w.float().abs().max())) / np.float32(2688.0))  # a true f32 division: one unit in the last place decides ties
         return _nvfp4(w, g), g, self.tensor(self.randn(n) * 0.01)
 
 
