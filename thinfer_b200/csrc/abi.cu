@@ -501,6 +501,7 @@ int32_t tnf_create(int32_t device, uint64_t vram_budget_bytes, tnf_ctx** out) {
   TNF_CUDA(cudaStreamCreateWithFlags(&ctx->readback, cudaStreamNonBlocking), "cudaStreamCreate");
   TNF_CUDA(cudaMalloc(&ctx->dwords, 256 + 16384), "cudaMalloc(status words)");
   TNF_CUDA(cudaMemset(ctx->dwords, 0, 256 + 16384), "cudaMemset(status words)");
+  TNF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ctx->scale_host), tnf_ctx::kScaleSlots * sizeof(float), cudaHostAllocMapped), "cudaHostAlloc(scale words)");
   *out = ctx;
   return TNF_OK;
 }
@@ -523,6 +524,7 @@ int32_t tnf_destroy(tnf_ctx* ctx) {
     if (ctx->stage_done[i]) cudaEventDestroy(ctx->stage_done[i]);
   }
   cudaFree(ctx->dwords);
+  cudaFreeHost(ctx->scale_host);
   cudaStreamDestroy(ctx->compute);
   cudaStreamDestroy(ctx->copy);
   cudaStreamDestroy(ctx->readback);
@@ -856,12 +858,12 @@ int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint
   uint8_t* s = resolve(ctx, scales, uint64_t(n) * (k / 16), "scales", &st);
   if (!s) return st;
   float* g = reinterpret_cast<float*>(ctx->dwords + 2);
-  TNF_CUDA(launch_amax(src, src_dtype, uint64_t(n) * k, ctx->dwords + 1, ctx->compute), "amax launch");
-  TNF_CUDA(launch_global_scale(ctx->dwords + 1, g, ctx->compute), "global scale launch");
+  float* host_g = global_scale ? ctx->scale_host + ctx->scale_next.fetch_add(1) % tnf_ctx::kScaleSlots : nullptr;
+  TNF_CUDA(launch_amax_scale(src, src_dtype, uint64_t(n) * k, ctx->dwords + 1, host_g, ctx->compute), "amax launch");
   TNF_CUDA(launch_quantize(src, src_dtype, n, k, g, 0.0f, c, s, false, ctx->compute), "weight quantise launch");
   if (global_scale) {
-    TNF_CUDA(cudaMemcpyAsync(global_scale, g, 4, cudaMemcpyDeviceToHost, ctx->compute), "global scale read");
     TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_quantize_weight sync");
+    *global_scale = *static_cast<volatile float*>(host_g);
   }
   return TNF_OK;
 }
@@ -884,18 +886,18 @@ int32_t tnf_prepare_scales(tnf_ctx* ctx, tnf_buf scales_canonical, uint32_t rows
 static int32_t quantize_act_impl(tnf_ctx* ctx, const uint8_t* a, uint32_t m, uint32_t k, float g, bool device_layout,
                                  uint8_t* codes, uint8_t* scales, float* g_used) {
   const float* g_ptr = nullptr;
+  float* host_g = nullptr;
   if (!(g > 0.0f)) {
-    float* gd = reinterpret_cast<float*>(ctx->dwords + 2);
-    TNF_CUDA(launch_amax(a, TNF_DTYPE_BF16, uint64_t(m) * k, ctx->dwords + 1, ctx->compute), "amax launch");
-    TNF_CUDA(launch_global_scale(ctx->dwords + 1, gd, ctx->compute), "global scale launch");
-    g_ptr = gd;
+    if (g_used) host_g = ctx->scale_host + ctx->scale_next.fetch_add(1) % tnf_ctx::kScaleSlots;
+    TNF_CUDA(launch_amax_scale(a, TNF_DTYPE_BF16, uint64_t(m) * k, ctx->dwords + 1, host_g, ctx->compute), "amax launch");
+    g_ptr = reinterpret_cast<float*>(ctx->dwords + 2);
   }
   TNF_CUDA(launch_quantize(a, TNF_DTYPE_BF16, m, k, g_ptr, g, codes, scales, device_layout, ctx->compute),
            "activation quantise launch");
   if (g_used) {
     if (g_ptr) {
-      TNF_CUDA(cudaMemcpyAsync(g_used, g_ptr, 4, cudaMemcpyDeviceToHost, ctx->compute), "global scale read");
       TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_quantize_act sync");
+      *g_used = *static_cast<volatile float*>(host_g);
     } else {
       *g_used = g;
     }

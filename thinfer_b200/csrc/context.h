@@ -1,6 +1,7 @@
 // The per-device context behind the C ABI: buffer table with category accounting, streams,
 // scratch, tensor-map cache, pinned host arenas, upload events. Internal to the library.
 #pragma once
+#include <atomic>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -68,8 +69,13 @@ struct tnf_ctx {
   uint32_t scratch_m = 0, scratch_k = 0;  // shape the scratch was last filled for (0 = never)
   uint64_t wide_id = 0, wide_bytes = 0;   // bf16 image of NVFP4 activations for the mixed arm (workspace category)
   long long wait_limit_cycles = tnf::kDefaultWaitLimitCycles;  // bound of every device-side mbarrier wait
-  // small device words: [0] kernel status, [1] amax bits, [2] global scale (f32)
+  // small device words: [0] kernel status, [1..4] amax bits, scale g, 1/(6g), block counter of amax_scale_kernel
   uint32_t* dwords = nullptr;
+  // Scales the device reports to a waiting host call: a mapped pinned word per call, taken in turn, so that calls of
+  // several threads do not read each other's.
+  static constexpr uint32_t kScaleSlots = 64;
+  float* scale_host = nullptr;
+  std::atomic<uint32_t> scale_next{0};
   std::map<tnf::MapSpec, CUtensorMap> maps;
   // fused-scatter peer windows (opened CUDA IPC mappings), index 0 unused
   static constexpr int kPeerSets = 4;

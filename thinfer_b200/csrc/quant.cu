@@ -17,28 +17,59 @@
 
 namespace tnf {
 
-// ---- absolute maximum -----------------------------------------------------------------------
+// ---- absolute maximum and per-tensor scale ----------------------------------------------------
+// One launch: every block takes the maximum of its share and adds it to words[0]; the block that finishes last turns
+// the result into the scale amax / (6 * 448) (1.0 for an all-zero tensor) and leaves words[0] and the block counter at
+// zero for the next launch on the stream. HBM-bound: a thread has four 16-byte loads in flight, 2048 threads per SM;
+// bf16 maxima are taken on packed pairs (exact, NaNs dropped as fmaxf drops them).
+// words: {amax bits, scale g, 1/(6g), blocks done}; host_g (mapped host memory, may be null) receives g as well.
+constexpr uint32_t kAmaxThreads = 512, kAmaxLoads = 4;
 template <typename T>
-__global__ void amax_kernel(const T* __restrict__ x, uint64_t n, uint32_t* __restrict__ out_bits) {
+__global__ void __launch_bounds__(kAmaxThreads, 4)
+    amax_scale_kernel(const uint4* __restrict__ x, uint64_t n_vec, uint32_t* __restrict__ words, float* host_g) {
+  __shared__ float part[kAmaxThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with programmatic dependent launch: see internal.h
   float m = 0.0f;
-  uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-    float v;
-    if constexpr (sizeof(T) == 2) v = __bfloat162float(x[i]);
-    else v = x[i];
-    m = fmaxf(m, fabsf(v));
+  __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
+  auto take = [&](const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (sizeof(T) == 2) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+      else m = fmaxf(m, fabsf(__uint_as_float(w[i])));
+    }
+  };
+  const uint64_t stride = uint64_t(gridDim.x) * kAmaxThreads;
+  uint64_t i = uint64_t(blockIdx.x) * kAmaxThreads + threadIdx.x;
+  for (; i + (kAmaxLoads - 1) * stride < n_vec; i += kAmaxLoads * stride) {
+    uint4 v[kAmaxLoads];
+#pragma unroll
+    for (uint32_t j = 0; j < kAmaxLoads; ++j) v[j] = __ldg(x + i + j * stride);
+#pragma unroll
+    for (uint32_t j = 0; j < kAmaxLoads; ++j) take(v[j]);
   }
+  for (; i < n_vec; i += stride) take(__ldg(x + i));
+  if constexpr (sizeof(T) == 2) m = fmaxf(m, fmaxf(__low2float(m2), __high2float(m2)));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_uint(m));  // non-negative floats order as uints
-}
-
-// amax bits -> per-tensor scale amax/(6*448), 1.0 for an all-zero tensor.
-__global__ void global_scale_kernel(const uint32_t* amax_bits, float* g) {
-  float a = __uint_as_float(*amax_bits);
-  float gv = a > 0.0f ? __fdiv_rn(a, 2688.0f) : 1.0f;
-  g[0] = gv;
-  g[1] = __fdiv_rn(1.0f, __fmul_rn(6.0f, gv));  // 1/(6g), shared by every block
+  if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (uint32_t j = 1; j < kAmaxThreads / 32; ++j) m = fmaxf(m, part[j]);
+  atomicMax(words, __float_as_uint(m));  // non-negative floats order as uints
+  __threadfence();
+  if (atomicInc(words + 3, gridDim.x - 1u) != gridDim.x - 1u) return;  // wraps to 0 on the last block
+  __threadfence();
+  const float a = __uint_as_float(atomicExch(words, 0u));
+  const float gv = a > 0.0f ? __fdiv_rn(a, 2688.0f) : 1.0f;
+  words[1] = __float_as_uint(gv);
+  words[2] = __float_as_uint(__fdiv_rn(1.0f, __fmul_rn(6.0f, gv)));  // 1/(6g), shared by every block
+  if (host_g) {
+    *reinterpret_cast<volatile float*>(host_g) = gv;
+    __threadfence_system();
+  }
 }
 
 // ---- block quantiser --------------------------------------------------------------------------
@@ -187,19 +218,12 @@ cudaError_t launch_dequant_dense(const uint8_t* codes, const uint8_t* scales_dev
   return cudaGetLastError();
 }
 
-cudaError_t launch_amax(const void* x, int dtype, uint64_t n, uint32_t* amax_bits, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(amax_bits, 0, 4, s);
-  if (e != cudaSuccess) return e;
-  int blocks = int(std::min<uint64_t>((n + 1023) / 1024, 148ull * 8));
-  if (blocks < 1) blocks = 1;
-  if (dtype == 1) amax_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)x, n, amax_bits);
-  else amax_kernel<float><<<blocks, 256, 0, s>>>((const float*)x, n, amax_bits);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_global_scale(const uint32_t* amax_bits, float* g, cudaStream_t s) {
-  global_scale_kernel<<<1, 1, 0, s>>>(amax_bits, g);
-  return cudaGetLastError();
+cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, cudaStream_t s) {
+  const uint64_t n_vec = n / (dtype == 1 ? 8 : 4);  // rows are whole 32-element groups
+  const unsigned blocks = unsigned(std::min<uint64_t>(std::max<uint64_t>(1, (n_vec + kAmaxThreads * kAmaxLoads - 1) / (kAmaxThreads * kAmaxLoads)), 148ull * 4));
+  const uint4* v = static_cast<const uint4*>(x);
+  return dtype == 1 ? launch_pdl(amax_scale_kernel<__nv_bfloat16>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g)
+                    : launch_pdl(amax_scale_kernel<float>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g);
 }
 
 cudaError_t launch_quantize(const void* src, int dtype, uint32_t rows, uint32_t k, const float* g_ptr, float g_val,
