@@ -1,0 +1,73 @@
+"""Attention with more query tiles than half the SMs: CTAs of 256 query rows (one softmax group per 128), the tiles left over
+for a last wave as two 128-row CTAs whose groups share the keys. Against the restated reference, same tolerance and reason as
+test_sdpa_gpu.py (bf16 probabilities in the second product, bf16 inputs and outputs)."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import dev_scales_to_canonical, rel_fro
+from test_sdpa_gpu import TOL, _inputs, _run
+
+pytestmark = pytest.mark.gpu
+SCALE = float(1.0 / np.sqrt(128.0))
+
+
+@pytest.mark.parametrize("b,s_q,s_k,h_q,h_kv,spread", [
+    (1, 300, 200, 80, 80, 1.0),    # 148 whole tiles (every second one with 44 rows: one group), 12 as two key-sharing CTAs (the second empty)
+    (2, 520, 330, 30, 10, 1.0),    # three tiles a sequence, the last with 8 rows; grouped heads; two batches
+    (1, 129, 700, 100, 100, 1.0),  # the second group has one row
+    (1, 100, 17, 100, 50, 1.0),    # one group, one ragged key tile
+    (1, 256, 1024, 76, 76, 6.0),   # peaked rows: the running output of both groups is rescaled from tile to tile
+])
+def test_rows_mode_matches_reference_recurrence(backend, b, s_q, s_k, h_q, h_kv, spread):
+    q, k, v = _inputs(b, s_q, s_k, h_q, h_kv, 31 * s_q + s_k, spread)
+    got = O.bf16_to_f32(_run(backend, q, k, v, SCALE))
+    want = O.bf16_to_f32(O.ref_sdpa(q, k, v, SCALE))
+    assert not np.isnan(got).any()
+    for bi in range(b):  # per head: an error in one CTA's tile must not hide in the norm over all of them
+        for h in range(h_q):
+            assert rel_fro(got[bi, :, h], want[bi, :, h]) <= 1.25 * TOL, (bi, h)
+    assert rel_fro(got, want) <= TOL
+
+
+@pytest.mark.parametrize("s_q,heads", [(130, 1), (256, 80)])  # keys mode, rows mode
+@pytest.mark.parametrize("jumps", [
+    {127: 400.0},                             # the first tile's last key decides the reference maximum
+    {128: 12.0, 256 + 95: 24.0},              # just past the limit, in the keys whose sum is checked
+    {128 + 96: 12.0, 256 + 127: 24.0},        # ... in the last 32 keys, whose maximum is checked
+    {130: 300.0, 300: 600.0, 511: 900.0},     # probabilities would overflow f32 against the older maximum
+    {5: 900.0},                               # everything after the first tile underflows to zero
+])
+def test_scores_that_jump(backend, s_q, heads, jumps):
+    """Score of key j (exp2 domain) = jumps[j], small noise elsewhere, the same for every row."""
+    s_k, d = 520, 128
+    rng = np.random.default_rng(7)
+    k = np.zeros((1, s_k, heads, d), np.float32)
+    k[..., 0] = rng.uniform(-1, 1, (1, s_k, heads))
+    for j, x in jumps.items():
+        k[:, j, :, 0] = x
+    q = np.zeros((1, s_q, heads, d), np.float32)
+    q[..., 0] = np.log(2.0) / SCALE
+    v = rng.standard_normal((1, s_k, heads, d)).astype(np.float32)
+    q, k, v = (O.f32_to_bf16(t) for t in (q, k, v))
+    got, want = O.bf16_to_f32(_run(backend, q, k, v, SCALE)), O.bf16_to_f32(O.ref_sdpa(q, k, v, SCALE))
+    assert not np.isnan(got).any() and rel_fro(got, want) <= TOL
+
+
+def test_rows_mode_fused_output_quantisation(backend):
+    be, (s, heads) = backend, (300, 80)
+    cols = heads * 128
+    q, k, v = _inputs(1, s, s, heads, heads, 512)
+    plain = _run(be, q, k, v, SCALE).reshape(s, cols)
+    g = O.global_scale(O.amax_bf16(plain))
+    qb, kb, vb = be.upload(q), be.upload(k), be.upload(v)
+    want_c, want_s = O.quantize_act(plain, g)
+    want_dev = O.scales_to_device_layout(want_s)
+    codes, scales = be.allocate(s * cols // 2), be.upload(np.full(want_dev.size, 0x7F, np.uint8))
+    be.scope().sdpa(qb, kb, vb, None, 1, s, s, heads, heads, SCALE, out_nvfp4=(codes, scales, g))
+    be.submit(30000)
+    assert np.array_equal(be.read_buffer(codes).reshape(s, cols // 2), want_c)
+    dev = be.read_buffer(scales)
+    assert np.array_equal(dev_scales_to_canonical(dev, s, cols), want_s) and np.array_equal(dev, want_dev)
+    for buf in (qb, kb, vb, codes, scales):
+        be.free(buf)

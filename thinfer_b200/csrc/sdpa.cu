@@ -2,34 +2,28 @@
 // call site thinfer-models/src/qwen_image/dit.rs:618-655: full attention over [txt ++ img], has_mask = 0, D = 128):
 // out = softmax(Q K^T * scale) V per (batch, head), bf16 in and out, f32 softmax statistics and accumulation.
 //
-// One CTA per (128 query rows, head, batch); flash-attention tiling over 128-key tiles, both products on the tensor
-// cores (tcgen05.mma kind::f16); scores, probabilities and the running output live in TMEM:
-//   columns   0-127  S: the score buffer (f32); a thread takes its row into registers at once, so one buffer serves
-//                    both softmax groups in turn
-//           128-255  P_0, P_1: the groups' probability buffers (bf16 pairs, 64 columns each)
-//           256-319  Q (bf16 pairs), copied from shared memory once
-//           384-511  O: the one running output (f32) both groups' products accumulate into
-//   Both products read their A operand (Q, P) from tensor memory: neither costs shared-memory bandwidth in the loop.
-//   warps 0, 10 TMA: the Q tile once, then K tiles (warp 0) and V tiles (warp 10) into two-stage rings ([128 rows x
-//               64 bf16] boxes with 128-byte swizzle straight out of the [B, S, H, D] tensors: a head is a 256-byte
-//               column window);
-//   warp 1      one elected thread issues S = Q K_j^T (K the K-major B operand, 8 MMAs of K = 16) as soon as the previous
-//               tile's score rows have been taken into registers, and O += P_g V_j in tile order, with V as it lies in
-//               memory (keys x d: an MN-major B operand, no transpose pass);
-//   warps 2-9   two softmax groups of four warps, one query row per thread (TMEM lane = row); the key tiles alternate
-//               between them, so that one group's exponentials run under the other's TMEM traffic and waits. The
-//               reference maximum m of a row is ONE chain through all tiles: the thread of tile j takes m_{j-1} from
-//               the other group's thread of the same row (shared memory, an mbarrier per lane quarter and tile
-//               parity), decides m_j -- it only moves when the tile's row maximum exceeds it by more than 8 in the
-//               exp2 domain, so probabilities stay below 256 -- and publishes it before its expensive part. Only when m
-//               moves is O rescaled (tcgen05.ld / mul / tcgen05.st by the thread that moved it, once the previous
-//               product has completed); both threads of the row scale their partial sums. Then
-//               p = exp2(s * scale * log2e - m), summed in f32, goes as bf16 pairs into P_g with tcgen05.st. At the
-//               end the two partial sums are joined and each group writes half of the columns of O / l.
-// Why this shape: a 128 x 128 x 16 MMA with both operands in shared memory reads 8 KB in its 64 cycles, all of an SM's
-// 128 B/clk (measured: 119 cycles), and the TMA's writes of K and V come on top. With Q and P in tensor memory a key
-// tile moves 128 KB through shared memory instead of 224 KB; with one O and one S instead of one per group there are
-// TMEM columns for them.
+// Flash-attention tiling, 128 query rows x 128 keys a tile, both products on the tensor cores (tcgen05.mma kind::f16),
+// scores, probabilities and running outputs in TMEM, TWO softmax groups per CTA with nothing between them: each has a score
+// tile S_g, a running output O_g and a reference maximum of its own, so that one group's exponentials run under the
+// other's two products. A CTA's work is one of two shapes:
+//   rows mode   256 query rows of one (head, batch): group g has rows 128g .. 128g+127 and all key tiles
+//   keys mode   128 query rows: group g has the key tiles of parity g; the two outputs are joined at the end
+// Rows mode reads K and V once for 256 rows; keys mode halves a CTA's time, which fills the chip when there are few rows
+// and shortens the last wave (see the rule at the launch).
+//   TMEM columns 0-127 S_0, 128-255 S_1 (f32), 256-383 O_0, 384-511 O_1 (f32). P_g (bf16 pairs, 64 columns) takes the place
+//   of S_g: a thread has its score row in registers before it writes the first probability.
+//   warp 0      TMA: the Q tiles once, then K tiles into a two-stage ring ([128 rows x 64 bf16] boxes with 128-byte swizzle
+//               straight out of the [B, S, H, D] tensors: a head is a 256-byte column window); warp 2 the same for V;
+//   warp 1      one elected thread issues, for the groups in turn, O_g += P_g V_j and at once S_g = Q_g K_j'^T of the
+//               group's next tile. The tensor pipe runs them in order: S_g may overwrite P_g without a wait, and a finished
+//               S_g says that O_g is complete as well. Q, K: shared memory, K-major; P: tensor memory; V as it lies in
+//               memory (keys x d: an MN-major B operand, no transpose pass). O_g += P_g V starts when 96 of the tile's
+//               128 probabilities are written;
+//   warps 4-11  the softmax groups, one query row per thread (TMEM lane = row): the row's scores to registers in one round
+//               trip, p = exp2(s * scale * log2e - m), f32 row sum, bf16 pairs to P_g. m is the row maximum of the group's
+//               first tile. Later tiles have no pass over the scores for their maximum: the row sum of the first 96 keys (and
+//               the maximum of the last 32) tells whether a probability can have passed 2^10; only then, before anything is
+//               written, is the maximum taken, m moved, O_g rescaled (tcgen05.ld / mul / tcgen05.st) and the tile redone.
 // The reference's kernel is the same recurrence one key at a time in f32 (m' = max(m, s); o = o * exp(m - m') +
 // exp(s - m') v; l likewise); here it runs a tile at a time, p is rounded to bf16 for the tensor cores, and exp is
 // exp2 with the scale folded in: the result agrees with the f32 recurrence to bf16 rounding (tests: relative
@@ -51,19 +45,17 @@
 namespace tnf {
 
 namespace at {
-constexpr int kThreads = 352;          // Q/K loader, MMA issuer, two softmax groups of four warps, V loader
+constexpr int kThreads = 384;          // Q/K loader, MMA issuer, V loader, a spare warp, two softmax groups of four warps
 constexpr uint32_t kD = 128;           // head dimension
-constexpr uint32_t kRows = 128;        // query rows per CTA, keys per tile
+constexpr uint32_t kRows = 128;        // query rows per group, keys per tile
 constexpr uint32_t kSub = 128 * 128;   // one [128 rows x 64 bf16] swizzled box: 16 KB
 constexpr uint32_t kTile = 2 * kSub;   // [128 x 128] bf16
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kSCol = 0;          // the score buffer (f32, 128 columns): a thread takes its row to registers at once, so one
-                                       // buffer serves both groups in turn
-constexpr uint32_t kPCol = 128;        // the groups' probability buffers (bf16 pairs) at columns 128 and 192
-constexpr uint32_t kQCol = 256;        // the Q tile (bf16 pairs, 64 columns): the A operand of every score MMA
-constexpr uint32_t kOCol = 384;        // the running output
-constexpr float kLazy = 8.0f;          // the reference maximum moves only when the row maximum exceeds it by this much
-constexpr uint32_t kSmemBytes = 1024 + 5 * kTile + 512 + 512 + 2048;  // Q | K x 2 | V x 2 | barriers | quantiser table | row statistics
+constexpr uint32_t kOCol = 256;        // O_g at kOCol + 128 g; S_g (and P_g in its first 64 columns) at 128 g
+constexpr uint32_t kSplitK = 6;        // P V starts when kSplitK * 16 probabilities of every row are written
+constexpr float kLazy = 10.0f;         // m moves when a score may exceed it by more than this (exp2 domain) ...
+constexpr float kLazySum = 1024.0f;    // ... which a sum of probabilities above 2^kLazy shows
+constexpr uint32_t kSmemBytes = 1024 + 6 * kTile + 512 + 512 + 2048;  // Q x 2 | K x 2 | V x 2 | barriers | quantiser table | row statistics
 }  // namespace at
 
 struct SdpaParams {
@@ -75,7 +67,9 @@ struct SdpaParams {
   uint32_t* status;
   long long wait_limit;
   uint32_t s_q, s_k, h_q, h_kv;
-  float scale_log2;  // scale * log2(e)
+  uint32_t q_tiles;     // 256-row query tiles per (head, batch)
+  uint32_t full_items;  // query tiles (over all heads and batches) that run in rows mode; each later one as two keys-mode CTAs
+  float scale_log2;     // scale * log2(e)
 };
 
 // MN-major operand, 128-byte swizzle: rows of 128 bytes hold 64 consecutive MN elements of one K index, 8-row (K)
@@ -146,12 +140,6 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// Two non-negative finite f32 -> bf16 pair by integer arithmetic (add half an ulp of bf16, keep the high halves: round
-// to nearest, ties up): the hardware conversion shares the special-function pipe with exp2, which is this kernel's
-// bottleneck, and a tie is one value in 65536.
-__device__ __forceinline__ uint32_t pack_bf16x2_pos(float lo, float hi) {
-  return __byte_perm(__float_as_uint(lo) + 0x8000u, __float_as_uint(hi) + 0x8000u, 0x7632);
-}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -165,23 +153,33 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t sQ = smem_base, sK = sQ + kTile, sV = sK + 2 * kTile, sBar = sV + 2 * kTile;
+  const uint32_t sQ = smem_base, sK = sQ + 2 * kTile, sV = sK + 2 * kTile, sBar = sV + 2 * kTile;
   const uint32_t q_full = sBar, k_full = sBar + 8, k_empty = sBar + 24, v_full = sBar + 40, v_empty = sBar + 56;
-  const uint32_t s_full = sBar + 72, p_full = sBar + 88, pv_done = sBar + 104, s_free = sBar + 120;
-  const uint32_t chain_bar = sBar + 136;  // [4 lane quarters][2 tile parities]: "m of tile j is published", 32 arrivals
-  const uint32_t q_ready = sBar + 200;    // Q has been copied to tensor memory (128 arrivals)
-  const uint32_t tmem_holder = sBar + 208;
+  const uint32_t s_full = sBar + 72, p_part = sBar + 88, p_full = sBar + 104, o_full = sBar + 120;
+  const uint32_t tmem_holder = sBar + 136;
   volatile uint32_t* tmem_holder_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder - smem_base));
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder + 8u - smem_base));
   float* inv_d_lut = reinterpret_cast<float*>(smem_gen + (sBar + 512u - smem_base));  // the activation quantiser's table
-  float* m_chain = reinterpret_cast<float*>(smem_gen + (sBar + 1024u - smem_base));   // [2 tile parities][128 rows]
-  float* l_part = m_chain + 256;                                                       // [2 groups][128 rows]
+  float* m_part = reinterpret_cast<float*>(smem_gen + (sBar + 1024u - smem_base));    // keys mode: [2 groups][128 rows]
+  float* l_part = m_part + 256;
 
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-  const uint32_t qt = blockIdx.x, hq = blockIdx.y, bb = blockIdx.z;
+  // the warp index as a warp-uniform value: the role branches and the MMA descriptors then live in uniform registers
+  // (score MMAs alone: 593 cycles a tile against 617)
+  const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;
+  // this CTA's work: query tile `item` (256 rows of one head and batch), or 128 rows of it
+  const bool keys_mode = blockIdx.x >= p.full_items;
+  const uint32_t over = keys_mode ? blockIdx.x - p.full_items : 0u;
+  const uint32_t item = keys_mode ? p.full_items + (over >> 1) : blockIdx.x;
+  const uint32_t hb = item / p.q_tiles, qt = item - hb * p.q_tiles;
+  const uint32_t bb = hb / p.h_q, hq = hb - bb * p.h_q;
   const uint32_t hkv = (hq * p.h_kv) / p.h_q;
-  const uint32_t q_row0 = bb * p.s_q + qt * kRows, k_row0 = bb * p.s_k;
-  const uint32_t tiles = (p.s_k + kRows - 1u) / kRows;
+  const uint32_t q_first = qt * 256u + (over & 1u) * kRows;  // first query row within the sequence
+  const uint32_t q_row0 = bb * p.s_q + q_first, k_row0 = bb * p.s_k;
+  const bool work = q_first < p.s_q;                                       // the second half of a ragged tile may be empty
+  const uint32_t groups = keys_mode || q_first + kRows < p.s_q ? 2u : 1u;  // rows mode: group 1 may have no rows
+  const uint32_t tiles = work ? (p.s_k + kRows - 1u) / kRows : 0u;
+  const uint32_t units = keys_mode ? tiles : tiles * groups;           // (key tile, group) pairs in the order the MMAs are issued
+  const uint32_t last_valid = p.s_k - ((p.s_k - 1u) / kRows) * kRows;  // keys of the last tile
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
   if (tid == 0) {
@@ -192,12 +190,10 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       mbar_init(v_full + 8 * i, 1);
       mbar_init(v_empty + 8 * i, 1);
       mbar_init(s_full + 8 * i, 1);
-      mbar_init(p_full + 8 * i, 128);
-      mbar_init(pv_done + 8 * i, 1);
-      mbar_init(s_free + 8 * i, 128);
+      mbar_init(p_part + 8 * i, 4);  // a group's four warps
+      mbar_init(p_full + 8 * i, 4);
+      mbar_init(o_full + 8 * i, 1);
     }
-    for (uint32_t i = 0; i < 8; ++i) mbar_init(chain_bar + 8 * i, 32);
-    mbar_init(q_ready, 128);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tensormap(&map_q);
@@ -212,128 +208,122 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder_gen;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();
   pdl_wait();  // Q, K and V are the previous kernels' outputs
 
-  // Key tile j belongs to group g = j % 2 and is the group's use = j / 2; it travels through ring stage g, score
-  // buffer g, probability tile g and output g.
+  // Key tile j travels through ring stage j % 2 of K and V.
   if (warp == 0) {
     // ---------------- Q and K loader ----------------
-    if (elect_one()) {
-      mbar_arrive_expect_tx(q_full, kTile);
-      tma_load_2d(sQ, &map_q, q_full, int32_t(hq * kD), int32_t(q_row0));
-      tma_load_2d(sQ + kSub, &map_q, q_full, int32_t(hq * kD + 64), int32_t(q_row0));
+    if (work && elect_one()) {
+      const uint32_t q_tiles = keys_mode ? 1u : groups;
+      mbar_arrive_expect_tx(q_full, q_tiles * kTile);
+      for (uint32_t g = 0; g < q_tiles; ++g) {
+        tma_load_2d(sQ + g * kTile, &map_q, q_full, int32_t(hq * kD), int32_t(q_row0 + g * kRows));
+        tma_load_2d(sQ + g * kTile + kSub, &map_q, q_full, int32_t(hq * kD + 64), int32_t(q_row0 + g * kRows));
+      }
     }
     __syncwarp();
     for (uint32_t j = 0; j < tiles; ++j) {
-      const uint32_t g = j & 1u, use = j >> 1;
-      if (use > 0 && !mbar_wait_warp(k_empty + 8 * g, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
+      const uint32_t st = j & 1u, use = j >> 1;
+      if (use > 0 && !mbar_wait_warp(k_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
       if (elect_one()) {
-        mbar_arrive_expect_tx(k_full + 8 * g, kTile);
-        tma_load_2d(sK + g * kTile, &map_k, k_full + 8 * g, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
-        tma_load_2d(sK + g * kTile + kSub, &map_k, k_full + 8 * g, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
+        mbar_arrive_expect_tx(k_full + 8 * st, kTile);
+        tma_load_2d(sK + st * kTile, &map_k, k_full + 8 * st, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
+        tma_load_2d(sK + st * kTile + kSub, &map_k, k_full + 8 * st, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
       }
       __syncwarp();
     }
-  } else if (warp == 10) {
+  } else if (warp == 2) {
     // ---------------- V loader (its ring frees later than K's: a warp of its own, so that K never waits behind V) ----------------
     for (uint32_t j = 0; j < tiles; ++j) {
-      const uint32_t g = j & 1u, use = j >> 1;
-      if (use > 0 && !mbar_wait_warp(v_empty + 8 * g, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
+      const uint32_t st = j & 1u, use = j >> 1;
+      if (use > 0 && !mbar_wait_warp(v_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
       if (elect_one()) {
-        mbar_arrive_expect_tx(v_full + 8 * g, kTile);
-        tma_load_2d(sV + g * kTile, &map_v, v_full + 8 * g, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
-        tma_load_2d(sV + g * kTile + kSub, &map_v, v_full + 8 * g, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
+        mbar_arrive_expect_tx(v_full + 8 * st, kTile);
+        tma_load_2d(sV + st * kTile, &map_v, v_full + 8 * st, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
+        tma_load_2d(sV + st * kTile + kSub, &map_v, v_full + 8 * st, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
       }
       __syncwarp();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    constexpr uint32_t idesc_qk = make_idesc_bf16(kRows, kRows);               // A and B K-major
-    constexpr uint32_t idesc_pv = make_idesc_bf16(kRows, kD) | (1u << 16);     // B (V) MN-major
-    bool ok = mbar_wait_warp(q_ready, 0, abort_flag, kStatusMmaTimeout, wait_limit);
-    // S = Q K_j^T into the ONE score buffer, Q from tensor memory: with Q and K both in shared memory a 128 x 128 x 16
-    // MMA needs 8 KB per 64 cycles, all of the SM's shared-memory bandwidth, and measured 119 cycles. Issued as soon as
-    // the previous tile's scores have been taken into registers (that tile belongs to the other group) and K_j has
-    // landed; the barriers alternate by tile parity although the buffer does not, so that no wait ever looks at a barrier
-    // two phases behind.
-    auto issue_s = [&](uint32_t j) -> bool {
-      const uint32_t g = j & 1u, use = j >> 1;
-      if (!mbar_wait_warp(k_full + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) return false;
-      if (j > 0 && !mbar_wait_warp(s_free + 8 * ((j - 1u) & 1u), ((j - 1u) >> 1) & 1u, abort_flag, kStatusAccEmptyTimeout, wait_limit)) return false;
+    constexpr uint32_t idesc_qk = make_idesc_bf16(kRows, kRows);            // A and B K-major
+    constexpr uint32_t idesc_pv = make_idesc_bf16(kRows, kD) | (1u << 16);  // B (V) MN-major
+    // descriptor words of the first tile; the loops only add to the low word's start address
+    const uint64_t k_desc = make_desc_sw128(sK), v_desc = make_desc_mn_sw128(sV, kSub);
+    const uint32_t k_hi = uint32_t(k_desc >> 32), v_hi = uint32_t(v_desc >> 32);
+    const uint32_t q_lo0 = uint32_t(make_desc_sw128(sQ)), k_lo0 = uint32_t(k_desc), v_lo0 = uint32_t(v_desc);
+    const bool by_rows2 = !keys_mode && groups == 2u;
+    // unit u = (key tile, group)
+    auto tile_of = [&](uint32_t u) { return by_rows2 ? u >> 1 : u; };
+    auto group_of = [&](uint32_t u) { return groups == 2u ? u & 1u : 0u; };
+    auto wait_k = [&](uint32_t u) -> bool {
+      const uint32_t j = tile_of(u);
+      return mbar_wait_warp(k_full + 8 * (j & 1u), (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
+    };
+    auto issue_s = [&](uint32_t u) {  // one elected lane
+      const uint32_t g = group_of(u), st = tile_of(u) & 1u;
+      const uint32_t q_lo = q_lo0 + (keys_mode ? 0u : g) * (kTile >> 4), k_lo = k_lo0 + st * (kTile >> 4);
+#pragma unroll
+      for (uint32_t kk = 0; kk < 8; ++kk) {
+        const uint32_t off = ((kk >> 2) * kSub + (kk & 3u) * 32u) >> 4;
+        tc_mma_bf16(tmem_base + g * 128u, (uint64_t(k_hi) << 32) | (q_lo + off), (uint64_t(k_hi) << 32) | (k_lo + off), idesc_qk, kk != 0u);
+      }
+      tc_commit(s_full + 8 * g);
+      if (keys_mode || g + 1u == groups) tc_commit(k_empty + 8 * st);  // the tile's last reader
+    };
+    bool ok = work && mbar_wait_warp(q_full, 0, abort_flag, kStatusMmaTimeout, wait_limit);
+    for (uint32_t u = 0; u < groups && u < units && ok; ++u) {
+      ok = wait_k(u);
+      tc_fence_after();
+      if (ok && elect_one()) issue_s(u);
+      __syncwarp();
+    }
+    for (uint32_t u = 0; u < units && ok; ++u) {
+      const uint32_t g = group_of(u), j = tile_of(u), st = j & 1u;
+      const uint32_t use = keys_mode ? u >> 1 : j;
+      const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
+      const bool next = u + groups < units;
+      const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
+      // the loads are long done: their waits (about 100 cycles each even then) come before the ones on the critical path
+      if (!mbar_wait_warp(v_full + 8 * st, (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
+      if (next && !wait_k(u + groups)) break;
+      if (!mbar_wait_warp(p_part + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
-        for (uint32_t kk = 0; kk < 8; ++kk) {
-          const uint32_t off = (kk >> 2) * kSub + (kk & 3u) * 32u;
-          tc_mma_bf16_ts(tmem_base + kSCol, tmem_base + kQCol + kk * 8u, make_desc_sw128(sK + g * kTile + off), idesc_qk, kk != 0u);
-        }
-        tc_commit(s_full + 8 * g);
-        tc_commit(k_empty + 8 * g);
+        for (uint32_t kk = 0; kk < kSplitK; ++kk)  // P's packed columns 8kk.. in TMEM, V rows 16kk..
+          if (kk < k_steps)
+            tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, (use | kk) != 0u);
       }
       __syncwarp();
-      return true;
-    };
-    if (ok) ok = issue_s(0);
-    if (ok && tiles > 1) ok = issue_s(1);
-    for (uint32_t j = 0; j < tiles && ok; ++j) {
-      const uint32_t g = j & 1u, use = j >> 1;
-      if (j + 2 < tiles && !issue_s(j + 2)) break;
       if (!mbar_wait_warp(p_full + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
-      if (!mbar_wait_warp(v_full + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
-        for (uint32_t kk = 0; kk < 8; ++kk)  // 16 keys each: P's packed columns 8kk.. in TMEM, V rows 16kk..
-          tc_mma_bf16_ts(tmem_base + kOCol, tmem_base + kPCol + g * 64u + kk * 8u, make_desc_mn_sw128(sV + g * kTile + kk * 2048u, kSub),
-                         idesc_pv, (j | kk) != 0u);
-        tc_commit(pv_done + 8 * g);
-        tc_commit(v_empty + 8 * g);
+        for (uint32_t kk = kSplitK; kk < 8; ++kk)
+          if (kk < k_steps)
+            tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, 1u);
+        if (keys_mode || g + 1u == groups) tc_commit(v_empty + 8 * st);
+        if (next) issue_s(u + groups);
+        else tc_commit(o_full + 8 * g);  // the group's last product
       }
       __syncwarp();
     }
-  } else {
+  } else if (warp >= 4) {
     // ---------------- softmax: two groups, one query row per thread ----------------
-    const uint32_t g = (warp - 2u) >> 2, quarter = warp & 3u, row = quarter * 32u + lane;
+    const uint32_t g = (warp - 4u) >> 2, quarter = warp & 3u, row = quarter * 32u + lane;
     const uint32_t lane_addr = tmem_base + ((quarter * 32u) << 16);
-    const uint32_t s_addr = lane_addr + kSCol, p_addr = lane_addr + kPCol + g * 64u, o_addr = lane_addr + kOCol;
-    float m_known = -INFINITY, l = 0.0f;  // l is this group's partial row sum, relative to m_known
+    const uint32_t s_addr = lane_addr + g * 128u, o_addr = lane_addr + kOCol + g * 128u;
+    float m_ref = -INFINITY, l = 0.0f;
     bool ok = true;
     uint32_t s0[32], s1[32], s2[32], s3[32];
     uint32_t use = 0;
-    if (g == 0) {
-      // Q goes from shared to tensor memory once: as the A operand of the score MMAs it then costs no shared-memory
-      // bandwidth. A thread undoes the 128-byte swizzle of its row: chunk c sits at position c ^ (row % 8).
-      ok = mbar_wait_warp(q_full, 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
-      if (ok) {
-        const uint8_t* qrow = smem_gen + (sQ - smem_base) + row * 128u;
-#pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) {
-          const uint4 a = *reinterpret_cast<const uint4*>(qrow + ((c ^ (row & 7u)) << 4));
-          const uint4 b = *reinterpret_cast<const uint4*>(qrow + kSub + ((c ^ (row & 7u)) << 4));
-          s0[c * 4] = a.x; s0[c * 4 + 1] = a.y; s0[c * 4 + 2] = a.z; s0[c * 4 + 3] = a.w;
-          s1[c * 4] = b.x; s1[c * 4 + 1] = b.y; s1[c * 4 + 2] = b.z; s1[c * 4 + 3] = b.w;
-        }
-        tmem_st_32x32b_x32(lane_addr + kQCol, s0);
-        tmem_st_32x32b_x32(lane_addr + kQCol + 32u, s1);
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(q_ready);
-      }
-    }
-    // m_{j}: published by the thread of tile j for the thread of tile j + 1 (the same row, the other group)
-    auto chain_wait = [&](uint32_t j) -> bool {
-      return mbar_wait_warp(chain_bar + 8 * (quarter * 2u + (j & 1u)), (j >> 1) & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
-    };
-    auto adopt = [&](float m_new) {  // bring the partial sum to a new reference maximum
-      if (m_new != m_known) {
-        l *= ex2(m_known - m_new);  // m_known = -inf only while l = 0: ex2(-inf) = 0
-        m_known = m_new;
-      }
-    };
-    for (uint32_t j = g; j < tiles && ok; j += 2, ++use) {
-      const uint32_t valid = min(kRows, p.s_k - j * kRows);  // keys of this tile that exist
+    const uint32_t j_step = keys_mode ? 2u : 1u;
+    for (uint32_t j = keys_mode ? g : 0u; j < tiles && g < groups; j += j_step, ++use) {
+      const uint32_t valid = j + 1u == tiles ? last_valid : kRows;  // keys of this tile that exist
+      // S_g complete; the pipe ran O_g += P_g V of the tile before in front of it, so O_g is complete too
       if (!mbar_wait_warp(s_full + 8 * g, use & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
         ok = false;
         break;
@@ -345,12 +335,9 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       tmem_ld_32x32b_x32(s_addr + 64u, s2);
       tmem_ld_32x32b_x32(s_addr + 96u, s3);
       tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(s_free + 8 * g);  // the score buffer can take the group's next tile
-      float mx = -INFINITY;
-      auto row_max = [&](const uint32_t(&c)[32], uint32_t c4) {
+      auto chunk_max = [&](const uint32_t(&c)[32], uint32_t c4) -> float {
+        float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
         if (valid >= (c4 + 1u) * 32u) {
-          float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {  // three-input maxima: 16 instructions for 32 values
             a = max3(a, __uint_as_float(c[i]), __uint_as_float(c[i + 1]));
@@ -358,70 +345,17 @@ __global__ void __launch_bounds__(at::kThreads, 1)
             d = max3(d, __uint_as_float(c[i + 4]), __uint_as_float(c[i + 5]));
             e = max3(e, __uint_as_float(c[i + 6]), __uint_as_float(c[i + 7]));
           }
-          mx = fmaxf(mx, fmaxf(fmaxf(a, b), fmaxf(d, e)));
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (c4 * 32u + uint32_t(i) < valid) mx = fmaxf(mx, __uint_as_float(c[i]));
+            if (c4 * 32u + uint32_t(i) < valid) a = fmaxf(a, __uint_as_float(c[i]));
         }
+        return fmaxf(fmaxf(a, b), fmaxf(d, e));
       };
-      row_max(s0, 0);
-      row_max(s1, 1);
-      row_max(s2, 2);
-      row_max(s3, 3);
-      mx *= p.scale_log2;  // scale > 0: the maximum commutes with it
-      // the chain: take m_{j-1}, decide m_j, publish it at once (the other group's next tile waits for nothing else)
-      float alpha = 1.0f;
-      if (j == 0) {
-        m_known = mx;
-      } else {
-        if (!chain_wait(j - 1u)) {
-          ok = false;
-          break;
-        }
-        adopt(m_chain[((j - 1u) & 1u) * 128u + row]);
-        if (mx > m_known + kLazy) {
-          alpha = ex2(m_known - mx);
-          l *= alpha;
-          m_known = mx;
-        }
-      }
-      m_chain[(j & 1u) * 128u + row] = m_known;
-      mbar_arrive(chain_bar + 8 * (quarter * 2u + (j & 1u)));
-      // A parity wait is only meaningful on a barrier that is at most one phase behind the awaited one. The group's own
-      // previous product (tile j-2) is therefore awaited first -- it also frees the probability buffer --: its completion
-      // implies tile j-3's, which puts the other group's barrier one phase before tile j-1's, awaited below.
-      if (use > 0) {
-        if (!mbar_wait_warp(pv_done + 8 * g, (use - 1u) & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
-          ok = false;
-          break;
-        }
-      }
-      if (j > 0 && __any_sync(0xFFFFFFFFu, alpha != 1.0f)) {
-        // rare (the maximum jumped by more than 2^8): O is rescaled once every earlier product has completed (the pipe
-        // runs them in order, so tile j-1's completion covers them all). This tile's product is issued only after this
-        // thread's arrival below, and the next tile's after it.
-        const uint32_t pj = j - 1u;
-        if (!mbar_wait_warp(pv_done + 8 * (pj & 1u), (pj >> 1) & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        uint32_t o8[8];
-#pragma unroll 1
-        for (uint32_t c = 0; c < kD; c += 8u) {
-          tmem_ld_32x32b_x8(o_addr + c, o8);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
-          tmem_st_32x32b_x8(o_addr + c, o8);
-        }
-      }
-      // p = exp2(s * scale_log2 - m), row sum in f32, P as bf16 pairs into the group's probability buffer
-      const float neg_m = -m_known;
-      const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(neg_m, neg_m);
-      uint64_t l01 = pack2(0.0f, 0.0f), l23 = l01;
-      auto emit = [&](uint32_t(&c)[32], uint32_t c4) {
+      uint64_t l01, l23;
+      // p = exp2(s * scale_log2 - m) of 32 keys: row sum in f32, P as bf16 pairs (two per 32-bit column, key 2i in the low half)
+      auto exps = [&](uint32_t(&c)[32], uint32_t c4, uint32_t(&w)[16]) {
+        const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(-m_ref, -m_ref);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {  // the scale and the shift for two scores in one packed FMA
           float x0, x1;
@@ -439,52 +373,118 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           l01 = add2(l01, pack2u(c[i], c[i + 1]));
           l23 = add2(l23, pack2u(c[i + 2], c[i + 3]));
         }
-        uint32_t w[16];  // two probabilities per 32-bit column, key 2i in the low half
 #pragma unroll
-        for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2_pos(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
-        tmem_st_32x32b_x16(p_addr + c4 * 16u, w);
+        for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
       };
-      emit(s0, 0);
-      emit(s1, 1);
-      emit(s2, 2);
-      emit(s3, 3);
-      {
-        float l0, l1, l2, l3;
-        unpack2(l01, l0, l1);
-        unpack2(l23, l2, l3);
-        l += (l0 + l1) + (l2 + l3);
+      auto sum4 = [&]() -> float {
+        float a, b, c, d;
+        unpack2(l01, a, b);
+        unpack2(l23, c, d);
+        return (a + b) + (c + d);
+      };
+      uint32_t w0[16], w1[16], w2[16];
+      const float top3 = chunk_max(s3, 3) * p.scale_log2;  // scale > 0: the maximum commutes with it
+      bool bad = use == 0;     // this row's m has to be taken from the scores
+      bool redo = use == 0;    // ... or some row's of this warp
+#pragma unroll 1
+      while (true) {
+        if (redo) {
+          const float mx = fmaxf(fmaxf(fmaxf(chunk_max(s0, 0), chunk_max(s1, 1)), chunk_max(s2, 2)) * p.scale_log2, top3);
+          float alpha = 1.0f;
+          if (bad && mx > m_ref) {
+            alpha = ex2(m_ref - mx);
+            l *= alpha;
+            m_ref = mx;
+          }
+          if (use > 0) {  // O_g is rescaled before this tile's product, which waits for the arrivals below
+            uint32_t o8[8];
+#pragma unroll 1
+            for (uint32_t c = 0; c < kD; c += 8u) {
+              tmem_ld_32x32b_x8(o_addr + c, o8);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
+              tmem_st_32x32b_x8(o_addr + c, o8);
+            }
+          }
+        }
+        l01 = l23 = pack2(0.0f, 0.0f);
+        exps(s0, 0, w0);
+        exps(s1, 1, w1);
+        exps(s2, 2, w2);
+        if (redo) break;
+        bad = !(sum4() <= kLazySum) || !(top3 - m_ref <= kLazy);  // NaN counts as too large
+        redo = __any_sync(0xFFFFFFFFu, bad);
+        if (!redo) break;
+        tmem_ld_32x32b_x32(s_addr, s0);  // rare: the scores again (nothing has been written over them yet)
+        tmem_ld_32x32b_x32(s_addr + 32u, s1);
+        tmem_ld_32x32b_x32(s_addr + 64u, s2);
+        tmem_ld_wait();
       }
+      tmem_st_32x32b_x16(s_addr, w0);
+      tmem_st_32x32b_x16(s_addr + 16u, w1);
+      tmem_st_32x32b_x16(s_addr + 32u, w2);
       tmem_st_wait();
       tc_fence_before();  // this thread's TMEM reads and writes are ordered before the arrival below
-      mbar_arrive(p_full + 8 * g);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_part + 8 * g);
+      exps(s3, 3, w0);
+      tmem_st_32x32b_x16(s_addr + 48u, w0);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full + 8 * g);
+      l += sum4();
     }
-    // ---------------- O / (l_0 + l_1) -> global: each group half of the columns ----------------
-    const uint32_t last = tiles - 1u;
-    if (ok && (last & 1u) != g) {  // the last tile was the other group's: its m is the final one
-      ok = chain_wait(last);
-      if (ok) adopt(m_chain[(last & 1u) * 128u + row]);
+    // ---------------- O / l -> global ----------------
+    // rows mode: a group stores its own rows, all columns. Keys mode: group g stores columns 64g .. 64g+63 of the joint rows,
+    // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
+    if (ok && use > 0) ok = mbar_wait_warp(o_full + 8 * g, 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
+    float f_own = 1.0f / l, f_other = 0.0f;
+    const bool other = keys_mode && (g == 0 ? tiles > 1u : tiles > 0u);  // the other group has seen a tile
+    if (keys_mode) {
+      m_part[g * 128u + row] = m_ref;
+      l_part[g * 128u + row] = l;
+      asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight softmax warps; every one of them gets here, whatever happened
+      if (other) {
+        if (ok) ok = mbar_wait_warp(o_full + 8 * (g ^ 1u), 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
+        const float m_o = m_part[(g ^ 1u) * 128u + row], l_o = l_part[(g ^ 1u) * 128u + row];
+        const float m = use > 0 ? fmaxf(m_ref, m_o) : m_o;
+        const float e_own = use > 0 ? ex2(m_ref - m) : 0.0f, e_other = ex2(m_o - m);
+        const float inv = 1.0f / (use > 0 ? l * e_own + l_o * e_other : l_o * e_other);
+        f_own = e_own * inv;
+        f_other = e_other * inv;
+      }
     }
-    // the group's own last product first (one phase ahead of what it has seen), then the very last one if it is the
-    // other group's: the same rule about parity waits
-    if (ok && use > 0) ok = mbar_wait_warp(pv_done + 8 * g, (use - 1u) & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
-    if (ok && (last & 1u) != g) ok = mbar_wait_warp(pv_done + 8 * (last & 1u), (last >> 1) & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
-    l_part[g * 128u + row] = l;
-    asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight softmax warps; every one of them gets here, whatever happened
     tc_fence_after();
-    if (ok && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
-      const float inv = 1.0f / (l + l_part[(g ^ 1u) * 128u + row]);
-      const bool store = qt * kRows + row < p.s_q;
-      const uint64_t grow = uint64_t(q_row0) + row;  // row of the [b * s_q, h_q * 128] matrix
-      uint16_t* dst = p.out ? p.out + (grow * p.h_q + hq) * kD + g * 64u : nullptr;  // group g writes columns 64g .. 64g+63
-      uint32_t sc4 = 0;  // the four block scales of this thread's 64 columns: one word of the scale layout
+    if (ok && work && g < groups && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
+      const uint32_t q_in_seq = q_first + (keys_mode ? 0u : g * kRows) + row;
+      const bool store = q_in_seq < p.s_q;
+      const uint64_t grow = uint64_t(bb) * p.s_q + q_in_seq;  // row of the [b * s_q, h_q * 128] matrix
+      uint16_t* dst = p.out ? p.out + (grow * p.h_q + hq) * kD : nullptr;
+      const uint32_t c_first = keys_mode ? g * 2u : 0u, c_end = keys_mode ? g * 2u + 2u : 4u;  // 32-column chunks
+      uint32_t sc4 = 0;  // the four block scales of 64 columns: one word of the scale layout
 #pragma unroll 1
-      for (uint32_t c2 = 0; c2 < 2; ++c2) {
-        tmem_ld_32x32b_x32(o_addr + g * 64u + c2 * 32u, s0);
-        tmem_ld_wait();
+      for (uint32_t c2 = c_first; c2 < c_end; ++c2) {
+        if (use > 0) {
+          tmem_ld_32x32b_x32(o_addr + c2 * 32u, s0);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(__uint_as_float(s0[i]) * f_own);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) s0[i] = 0u;
+        }
+        if (other) {
+          tmem_ld_32x32b_x32(lane_addr + kOCol + (g ^ 1u) * 128u + c2 * 32u, s1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), f_other, __uint_as_float(s0[i])));
+        }
         if (store) {
           uint32_t w[16];  // 32 columns as bf16 pairs
 #pragma unroll
-          for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(s0[2 * i]) * inv, __uint_as_float(s0[2 * i + 1]) * inv);
+          for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(s0[2 * i]), __uint_as_float(s0[2 * i + 1]));
           if (dst) {
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
@@ -494,25 +494,27 @@ __global__ void __launch_bounds__(at::kThreads, 1)
             // the out-projection's activation quantiser, on the bf16-rounded values: two 16-column blocks per 32 columns,
             // 8 code bytes each; the same bits tnf_quantize_act makes of the bf16 output
             uint32_t codes[4];
+            if ((c2 & 1u) == 0u) sc4 = 0;
 #pragma unroll
             for (uint32_t blk = 0; blk < 2; ++blk) {
               const uint32_t w8[8] = {w[blk * 8], w[blk * 8 + 1], w[blk * 8 + 2], w[blk * 8 + 3], w[blk * 8 + 4], w[blk * 8 + 5], w[blk * 8 + 6], w[blk * 8 + 7]};
               const uint32_t sc = quant_block16_bf16(w8, inv_d_lut, p.q_inv_t, codes[blk * 2], codes[blk * 2 + 1]);
-              sc4 |= sc << (8u * (c2 * 2u + blk));
+              sc4 |= sc << (8u * ((c2 & 1u) * 2u + blk));
             }
-            *reinterpret_cast<uint4*>(p.q_codes + grow * (uint64_t(p.h_q) * 64u) + hq * 64u + g * 32u + c2 * 16u) =
+            *reinterpret_cast<uint4*>(p.q_codes + grow * (uint64_t(p.h_q) * 64u) + hq * 64u + c2 * 16u) =
                 make_uint4(codes[0], codes[1], codes[2], codes[3]);
+            // blocks hq*8 + 4 * half .. +3 of the row: one 4-byte word of atom hq*2 + half (the launcher has cleared the padding)
+            if (c2 & 1u)
+              *reinterpret_cast<uint32_t*>(p.q_scales + ((grow >> 7) * p.q_k_atoms + hq * 2u + (c2 >> 1)) * 512u + (grow & 31u) * 16u + ((grow & 127u) >> 5) * 4u) = sc4;
           }
         }
-      }
-      if (p.q_scales && store) {
-        // blocks hq*8 + g*4 .. +3 of the row: one 4-byte word of atom hq*2 + g (the launcher has cleared the padding)
-        *reinterpret_cast<uint32_t*>(p.q_scales + ((grow >> 7) * p.q_k_atoms + hq * 2u + g) * 512u + (grow & 31u) * 16u + ((grow & 127u) >> 5) * 4u) = sc4;
       }
     }
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0u)
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // let copies and MMAs in flight retire
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
   if (tid == 0 && *abort_flag != 0u) atomicCAS(p.status, 0u, *abort_flag);
 }
@@ -606,8 +608,19 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     cudaError_t e = cudaFuncSetAttribute(sdpa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
   }
-  cudaError_t e = launch_pdl(sdpa_kernel, dim3((a->s_q + 127u) / 128u, a->h_q, a->b), dim3(at::kThreads), at::kSmemBytes, ctx->compute,
-                             mq, mk, mv, p);
+  // One CTA per SM. Whole waves run in rows mode. The query tiles left over for a last wave run as two keys-mode CTAs each
+  // when every one of those then finds an SM of its own: half the time instead of a whole one on half the chip. With fewer
+  // tiles than half the SMs, that is all of them.
+  p.q_tiles = (a->s_q + 255u) / 256u;
+  const uint64_t items = uint64_t(p.q_tiles) * a->h_q * a->b;
+  const uint64_t sms = uint64_t(ctx->sm_count), tail = items % sms;
+  const uint64_t full = 2 * tail <= sms ? items - tail : items;
+  if (full + 2 * (items - full) > 0x7FFFFFFFull) {
+    set_error("tnf_sdpa: problem too large for the grid (%llu query tiles)", (unsigned long long)items);
+    return TNF_ERR_INVALID_ARGUMENT;
+  }
+  p.full_items = uint32_t(full);
+  cudaError_t e = launch_pdl(sdpa_kernel, dim3(uint32_t(full + 2 * (items - full))), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
   if (e != cudaSuccess) return cuda_fail(e, "sdpa launch");
   return TNF_OK;
 }
