@@ -130,11 +130,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -280,15 +275,20 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       if (ok && elect_one()) issue_s(u);
       __syncwarp();
     }
+    auto wait_v = [&](uint32_t u) -> bool {
+      const uint32_t j = tile_of(u);
+      return mbar_wait_warp(v_full + 8 * (j & 1u), (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
+    };
+    // Waits take about 100 cycles each even when their phase is long over: those for the loads of the NEXT unit stand where
+    // this warp is idle, between the two parts of a unit's P V, not on the way from a finished P to the next scores.
+    auto wait_loads = [&](uint32_t u) { return u >= units || (wait_v(u) && (u + groups >= units || wait_k(u + groups))); };
+    ok = ok && wait_loads(0);
     for (uint32_t u = 0; u < units && ok; ++u) {
       const uint32_t g = group_of(u), j = tile_of(u), st = j & 1u;
       const uint32_t use = keys_mode ? u >> 1 : j;
       const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
       const bool next = u + groups < units;
       const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
-      // the loads are long done: their waits (about 100 cycles each even then) come before the ones on the critical path
-      if (!mbar_wait_warp(v_full + 8 * st, (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
-      if (next && !wait_k(u + groups)) break;
       if (!mbar_wait_warp(p_part + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
       tc_fence_after();
       if (elect_one()) {
@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
             tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, (use | kk) != 0u);
       }
       __syncwarp();
+      if (!wait_loads(u + 1u)) break;
       if (!mbar_wait_warp(p_full + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
       tc_fence_after();
       if (elect_one()) {
@@ -335,26 +336,34 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       tmem_ld_32x32b_x32(s_addr + 64u, s2);
       tmem_ld_32x32b_x32(s_addr + 96u, s3);
       tmem_ld_wait();
-      auto chunk_max = [&](const uint32_t(&c)[32], uint32_t c4) -> float {
-        float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
-        if (valid >= (c4 + 1u) * 32u) {
+      // keys that do not exist weigh nothing: 2^(-inf). Masked here and not per chunk: the exponentials of a tile then are one
+      // block without branches, which the compiler can interleave
+      auto mask = [&]() {
+        if (valid < kRows) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {  // three-input maxima: 16 instructions for 32 values
-            a = max3(a, __uint_as_float(c[i]), __uint_as_float(c[i + 1]));
-            b = max3(b, __uint_as_float(c[i + 2]), __uint_as_float(c[i + 3]));
-            d = max3(d, __uint_as_float(c[i + 4]), __uint_as_float(c[i + 5]));
-            e = max3(e, __uint_as_float(c[i + 6]), __uint_as_float(c[i + 7]));
+          for (int i = 0; i < 32; ++i) {
+            if (uint32_t(i) >= valid) s0[i] = 0xFF800000u;
+            if (32u + uint32_t(i) >= valid) s1[i] = 0xFF800000u;
+            if (64u + uint32_t(i) >= valid) s2[i] = 0xFF800000u;
+            if (96u + uint32_t(i) >= valid) s3[i] = 0xFF800000u;
           }
-        } else {
+        }
+      };
+      mask();
+      auto chunk_max = [&](const uint32_t(&c)[32]) -> float {
+        float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c4 * 32u + uint32_t(i) < valid) a = fmaxf(a, __uint_as_float(c[i]));
+        for (int i = 0; i < 32; i += 8) {  // three-input maxima: 16 instructions for 32 values
+          a = max3(a, __uint_as_float(c[i]), __uint_as_float(c[i + 1]));
+          b = max3(b, __uint_as_float(c[i + 2]), __uint_as_float(c[i + 3]));
+          d = max3(d, __uint_as_float(c[i + 4]), __uint_as_float(c[i + 5]));
+          e = max3(e, __uint_as_float(c[i + 6]), __uint_as_float(c[i + 7]));
         }
         return fmaxf(fmaxf(a, b), fmaxf(d, e));
       };
       uint64_t l01, l23;
       // p = exp2(s * scale_log2 - m) of 32 keys: row sum in f32, P as bf16 pairs (two per 32-bit column, key 2i in the low half)
-      auto exps = [&](uint32_t(&c)[32], uint32_t c4, uint32_t(&w)[16]) {
+      auto exps = [&](uint32_t(&c)[32], uint32_t(&w)[16]) {
         const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(-m_ref, -m_ref);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {  // the scale and the shift for two scores in one packed FMA
@@ -363,18 +372,14 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           c[i] = __float_as_uint(ex2(x0));
           c[i + 1] = __float_as_uint(ex2(x1));
         }
-        if (valid < (c4 + 1u) * 32u) {  // only the last tile of a ragged s_k: keys that do not exist weigh nothing
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c4 * 32u + uint32_t(i) >= valid) c[i] = 0u;
-        }
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
           l01 = add2(l01, pack2u(c[i], c[i + 1]));
           l23 = add2(l23, pack2u(c[i + 2], c[i + 3]));
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
+        for (int i = 0; i < 16; ++i)
+          w[i] = pack_bf16x2(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
       };
       auto sum4 = [&]() -> float {
         float a, b, c, d;
@@ -383,13 +388,13 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         return (a + b) + (c + d);
       };
       uint32_t w0[16], w1[16], w2[16];
-      const float top3 = chunk_max(s3, 3) * p.scale_log2;  // scale > 0: the maximum commutes with it
+      const float top3 = chunk_max(s3) * p.scale_log2;  // scale > 0: the maximum commutes with it
       bool bad = use == 0;     // this row's m has to be taken from the scores
       bool redo = use == 0;    // ... or some row's of this warp
 #pragma unroll 1
       while (true) {
         if (redo) {
-          const float mx = fmaxf(fmaxf(fmaxf(chunk_max(s0, 0), chunk_max(s1, 1)), chunk_max(s2, 2)) * p.scale_log2, top3);
+          const float mx = fmaxf(fmaxf(fmaxf(chunk_max(s0), chunk_max(s1)), chunk_max(s2)) * p.scale_log2, top3);
           float alpha = 1.0f;
           if (bad && mx > m_ref) {
             alpha = ex2(m_ref - mx);
@@ -409,9 +414,9 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           }
         }
         l01 = l23 = pack2(0.0f, 0.0f);
-        exps(s0, 0, w0);
-        exps(s1, 1, w1);
-        exps(s2, 2, w2);
+        exps(s0, w0);
+        exps(s1, w1);
+        exps(s2, w2);
         if (redo) break;
         bad = !(sum4() <= kLazySum) || !(top3 - m_ref <= kLazy);  // NaN counts as too large
         redo = __any_sync(0xFFFFFFFFu, bad);
@@ -420,6 +425,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         tmem_ld_32x32b_x32(s_addr + 32u, s1);
         tmem_ld_32x32b_x32(s_addr + 64u, s2);
         tmem_ld_wait();
+        mask();
       }
       tmem_st_32x32b_x16(s_addr, w0);
       tmem_st_32x32b_x16(s_addr + 16u, w1);
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       tc_fence_before();  // this thread's TMEM reads and writes are ordered before the arrival below
       __syncwarp();
       if (lane == 0) mbar_arrive(p_part + 8 * g);
-      exps(s3, 3, w0);
+      exps(s3, w0);
       tmem_st_32x32b_x16(s_addr + 48u, w0);
       tmem_st_wait();
       tc_fence_before();
