@@ -525,6 +525,7 @@ int32_t tnf_destroy(tnf_ctx* ctx) {
   }
   cudaFree(ctx->dwords);
   cudaFreeHost(ctx->scale_host);
+  if (ctx->write_stage) cudaFreeHost(ctx->write_stage);
   cudaStreamDestroy(ctx->compute);
   cudaStreamDestroy(ctx->copy);
   cudaStreamDestroy(ctx->readback);
@@ -569,6 +570,59 @@ static int32_t raw_range(tnf_ctx* ctx, uint64_t id, uint64_t off, uint64_t n, co
   return TNF_OK;
 }
 
+// Large writes from pageable memory. The driver stages those through one thread (6-8 GB/s); here up to kWriteThreads
+// threads copy into pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the
+// chunks on the compute stream. The slots (kWriteStageBytes in all) are made on first use and freed with the context.
+// Below kWriteStagedMin the threads cost more than they save. Returns false when the caller has to copy the plain way
+// (slots in use by another thread's write, no pinned memory to be had); *err is a failed copy.
+constexpr uint32_t kWriteThreads = 8;
+constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 8u << 20;
+static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n, cudaError_t* err) {
+  std::unique_lock<std::mutex> lk(ctx->write_mu, std::try_to_lock);
+  if (!lk.owns_lock()) return false;
+  if (!ctx->write_stage && cudaHostAlloc(&ctx->write_stage, kWriteStageBytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->write_stage = nullptr;
+    return false;
+  }
+  const uint64_t chunks = (n + kWriteChunk - 1) / kWriteChunk;
+  const uint32_t cores = std::thread::hardware_concurrency();
+  const uint32_t workers = uint32_t(std::min<uint64_t>(chunks, std::max(1u, std::min(kWriteThreads, cores / 2u))));
+  cudaError_t status[kWriteThreads] = {};
+  auto work = [&](uint32_t t) {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    cudaEvent_t read[2] = {nullptr, nullptr};
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&read[i], cudaEventDisableTiming);
+    uint32_t use = 0;
+    for (uint64_t c = t; c < chunks && e == cudaSuccess; c += workers, ++use) {
+      uint8_t* slot = static_cast<uint8_t*>(ctx->write_stage) + (2u * t + (use & 1u)) * kWriteChunk;
+      if (use >= 2u) e = cudaEventSynchronize(read[use & 1u]);  // the copy that last read this slot
+      if (e != cudaSuccess) break;
+      const uint64_t off = c * kWriteChunk, bytes = std::min(kWriteChunk, n - off);
+      std::memcpy(slot, src + off, bytes);
+      e = cudaMemcpyAsync(dst + off, slot, bytes, cudaMemcpyHostToDevice, ctx->compute);
+      if (e == cudaSuccess) e = cudaEventRecord(read[use & 1u], ctx->compute);
+    }
+    for (cudaEvent_t ev : read)
+      if (ev) cudaEventDestroy(ev);
+    status[t] = e;
+  };
+  std::thread pool[kWriteThreads];
+  uint32_t started = 1;
+  try {
+    for (; started < workers; ++started) pool[started] = std::thread(work, started);
+  } catch (...) {  // no thread to be had: this one takes the remaining shares below
+  }
+  work(0);
+  for (uint32_t t = 1; t < started; ++t) pool[t].join();
+  for (uint32_t t = started; t < workers; ++t) work(t);
+  const cudaError_t done = cudaStreamSynchronize(ctx->compute);  // the slots are free again
+  for (uint32_t t = 0; t < workers; ++t)
+    if (status[t] != cudaSuccess) *err = status[t];
+  if (*err == cudaSuccess) *err = done;
+  return true;
+}
+
 int32_t tnf_write(tnf_ctx* ctx, uint64_t id, uint64_t dst_off, const void* src, uint64_t n) {
   TNF_CHECK_CTX(ctx);
   if (dst_off % 4 || n % 4) {  // same rule as Backend::write_buffer
@@ -580,6 +634,14 @@ int32_t tnf_write(tnf_ctx* ctx, uint64_t id, uint64_t dst_off, const void* src, 
   uint8_t* p = nullptr;
   int32_t st = raw_range(ctx, id, dst_off, n, "tnf_write", &p);
   if (st != TNF_OK) return st;
+  cudaPointerAttributes attr;
+  if (n >= kWriteStagedMin && cudaPointerGetAttributes(&attr, src) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered) {
+    cudaError_t e = cudaSuccess;
+    if (staged_write(ctx, p, static_cast<const uint8_t*>(src), n, &e)) {
+      if (e != cudaSuccess) return cuda_fail(e, "tnf_write staged copy");
+      return TNF_OK;
+    }
+  }
   TNF_CUDA(cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, ctx->compute), "tnf_write copy");
   // pageable sources are staged before the call returns; pinned ones are not, so wait
   TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_write sync");

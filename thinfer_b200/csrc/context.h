@@ -91,6 +91,9 @@ struct tnf_ctx {
   void* stage_host[2] = {nullptr, nullptr};
   cudaEvent_t stage_done[2] = {nullptr, nullptr};
   uint64_t stage_bytes = 0;
+  // large writes from pageable memory: pinned slots of the copying threads, one such write at a time
+  std::mutex write_mu;
+  void* write_stage = nullptr;
 };
 
 void tnf_comm_teardown(tnf_ctx* ctx);  // comm.cu
