@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder + 8 - smem_base));
   volatile uint32_t* tmem_holder_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder - smem_base));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform: see gemm_nvfp4_pair.cu
   const uint32_t num_tiles = p.tiles_m * p.tiles_n;
   const bool ktr = kDiag && (p.diag & 16u) && blockIdx.x == 0;
 
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder_gen;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();
   pdl_wait();  // before any access to global memory
   if (ktr && threadIdx.x == 0) p.trace[1201] = clock64();

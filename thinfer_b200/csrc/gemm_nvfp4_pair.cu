@@ -255,7 +255,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
   // staged NVFP4 multicast output: the CTA's eight epilogue warps meet on these ("tile staged" / "staging free")
   const uint32_t bar_qs_full = tmem_holder + 16, bar_qs_free = tmem_holder + 24;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp index as a warp-uniform value: the role branches, stage addresses and MMA descriptors then live in uniform registers
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool ktr = kDiag && (p.diag & 16u) && blockIdx.x == 0 && threadIdx.x == 0;
   if (ktr) p.trace[1200] = clock64();
@@ -292,7 +293,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
   cluster_arrive();
   cluster_wait();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder_gen;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();  // the next kernel's CTAs may be scheduled as ours retire
   pdl_wait();               // operands written by the previous kernel are complete and visible
   if (ktr) p.trace[1201] = clock64();

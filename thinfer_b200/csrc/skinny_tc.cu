@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   uint8_t* a_gen = smem_gen + (sA - smem_base);
   uint8_t* sfa_gen = smem_gen + (sSfa - smem_base);
   float* inv_d_lut = reinterpret_cast<float*>(smem_gen + (sBar + 1024u - smem_base));  // the barriers take < 1 KB
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+  const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;  // warp-uniform: see gemm_nvfp4_pair.cu
   const uint32_t row0 = blockIdx.x * 128u;  // first W row (output column) of this CTA
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder_gen;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();
   pdl_wait();  // before any access to global memory: A may be the previous kernel's output
 
