@@ -68,16 +68,15 @@ __device__ __forceinline__ uint32_t quant_block16(const float (&x)[16], const fl
 template <bool kDirect>
 __device__ __forceinline__ uint32_t quant_block16_bf16_impl(const uint32_t (&w)[8], const float* inv_d_lut, float g, float inv_t,
                                                             uint32_t& lo, uint32_t& hi) {
-  __nv_bfloat162 m2[8];
+  uint32_t m2[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    m2[i] = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-  }
+  for (int i = 0; i < 8; ++i) m2[i] = w[i];
 #pragma unroll
   for (int s = 4; s >= 1; s >>= 1)
 #pragma unroll
-    for (int i = 0; i < s; ++i) m2[i] = __hmax2(m2[i], m2[i + s]);
-  const uint32_t mm = *reinterpret_cast<const uint32_t*>(&m2[0]);
+    for (int i = 0; i < s; ++i)  // the larger magnitude of each half; the sign it carries is dropped below
+      asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(m2[i]) : "r"(m2[i]), "r"(m2[i + s]));
+  const uint32_t mm = m2[0] & 0x7FFF7FFFu;
   const float bmax = fmaxf(fmaxf(0.0f, __uint_as_float(mm << 16)), __uint_as_float(mm & 0xFFFF0000u));
   float s_raw = __fmul_rn(bmax, inv_t);
   uint32_t sc = (uint32_t)__nv_cvt_float_to_fp8(s_raw, __NV_SATFINITE, __NV_E4M3) & 0xFFu;
@@ -88,10 +87,13 @@ __device__ __forceinline__ uint32_t quant_block16_bf16_impl(const uint32_t (&w)[
   if (sc != 0) {
     const float inv_d = kDirect ? __fdiv_rn(1.0f, __fmul_rn(e4m3_decode_dev(sc), g)) : inv_d_lut[sc];
     float y[16];
+    uint64_t d2;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d2) : "f"(inv_d));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      y[2 * i] = __fmul_rn(__uint_as_float(w[i] << 16), inv_d);
-      y[2 * i + 1] = __fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), inv_d);
+    for (int i = 0; i < 8; ++i) {  // two products per instruction, each rounded as __fmul_rn rounds it
+      uint64_t y2;
+      asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tmul.rn.f32x2 %0, t, %3;\n\t}" : "=l"(y2) : "r"(w[i] << 16), "r"(w[i] & 0xFFFF0000u), "l"(d2));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(y[2 * i]), "=f"(y[2 * i + 1]) : "l"(y2));
     }
     lo = e2m1x8(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]);
     hi = e2m1x8(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]);
