@@ -5,11 +5,12 @@
 // Flash-attention tiling, 128 query rows x 128 keys a tile, both products on the tensor cores (tcgen05.mma kind::f16),
 // scores, probabilities and running outputs in TMEM, TWO softmax groups per CTA with nothing between them: each has a score
 // tile S_g, a running output O_g and a reference maximum of its own, so that one group's exponentials run under the
-// other's two products. A CTA's work is one of two shapes:
+// other's two products. One persistent CTA per SM; an item of its work is one of two shapes:
 //   rows mode   256 query rows of one (head, batch): group g has rows 128g .. 128g+127 and all key tiles
 //   keys mode   128 query rows: group g has the key tiles of parity g; the two outputs are joined at the end
-// Rows mode reads K and V once for 256 rows; keys mode halves a CTA's time, which fills the chip when there are few rows
-// and shortens the last wave (see the rule at the launch).
+// Rows mode reads K and V once for 256 rows; keys mode halves an item's time, which fills the chip when there are few rows
+// and shortens the last wave (see the rule at the launch). The loads and the first scores of an item run under the
+// previous one's last products and output.
 //   TMEM columns 0-127 S_0, 128-255 S_1 (f32), 256-383 O_0, 384-511 O_1 (f32). P_g (bf16 pairs, 64 columns) takes the place
 //   of S_g: a thread has its score row in registers before it writes the first probability.
 //   warp 0      TMA: the Q tiles once, then K tiles into a two-stage ring ([128 rows x 64 bf16] boxes with 128-byte swizzle
@@ -68,7 +69,8 @@ struct SdpaParams {
   long long wait_limit;
   uint32_t s_q, s_k, h_q, h_kv;
   uint32_t q_tiles;     // 256-row query tiles per (head, batch)
-  uint32_t full_items;  // query tiles (over all heads and batches) that run in rows mode; each later one as two keys-mode CTAs
+  uint32_t full_items;  // query tiles (over all heads and batches) that run in rows mode; each later one as two keys-mode items
+  uint32_t items;       // work items in all
   float scale_log2;     // scale * log2(e)
 };
 
@@ -141,6 +143,27 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return d;
 }
 
+// Work item `it` of the persistent loop: 256 query rows of one head and batch, or 128 rows of them (keys mode).
+struct SdpaItem {
+  bool keys_mode, work;  // work: the item has rows (the second half of a ragged tile may be empty)
+  uint32_t bb, hq, hkv, q_first, groups, tiles, units;
+  __device__ __forceinline__ SdpaItem(const SdpaParams& p, uint32_t it) {
+    using namespace at;
+    keys_mode = it >= p.full_items;
+    const uint32_t over = keys_mode ? it - p.full_items : 0u;
+    const uint32_t item = keys_mode ? p.full_items + (over >> 1) : it;
+    const uint32_t hb = item / p.q_tiles, qt = item - hb * p.q_tiles;
+    bb = hb / p.h_q;
+    hq = hb - bb * p.h_q;
+    hkv = (hq * p.h_kv) / p.h_q;
+    q_first = qt * 256u + (over & 1u) * kRows;  // first query row within the sequence
+    work = q_first < p.s_q;
+    groups = keys_mode || q_first + kRows < p.s_q ? 2u : 1u;  // rows mode: group 1 may have no rows
+    tiles = work ? (p.s_k + kRows - 1u) / kRows : 0u;
+    units = keys_mode ? tiles : tiles * groups;  // (key tile, group) pairs in the order the MMAs are issued
+  }
+};
+
 __global__ void __launch_bounds__(at::kThreads, 1)
     sdpa_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const SdpaParams p) {
@@ -151,7 +174,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   const uint32_t sQ = smem_base, sK = sQ + 2 * kTile, sV = sK + 2 * kTile, sBar = sV + 2 * kTile;
   const uint32_t q_full = sBar, k_full = sBar + 8, k_empty = sBar + 24, v_full = sBar + 40, v_empty = sBar + 56;
   const uint32_t s_full = sBar + 72, p_part = sBar + 88, p_full = sBar + 104, o_full = sBar + 120;
-  const uint32_t tmem_holder = sBar + 136;
+  const uint32_t q_empty = sBar + 136, tmem_holder = sBar + 144;
   volatile uint32_t* tmem_holder_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder - smem_base));
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder + 8u - smem_base));
   float* inv_d_lut = reinterpret_cast<float*>(smem_gen + (sBar + 512u - smem_base));  // the activation quantiser's table
@@ -161,24 +184,13 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   // the warp index as a warp-uniform value: the role branches and the MMA descriptors then live in uniform registers
   // (score MMAs alone: 593 cycles a tile against 617)
   const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;
-  // this CTA's work: query tile `item` (256 rows of one head and batch), or 128 rows of it
-  const bool keys_mode = blockIdx.x >= p.full_items;
-  const uint32_t over = keys_mode ? blockIdx.x - p.full_items : 0u;
-  const uint32_t item = keys_mode ? p.full_items + (over >> 1) : blockIdx.x;
-  const uint32_t hb = item / p.q_tiles, qt = item - hb * p.q_tiles;
-  const uint32_t bb = hb / p.h_q, hq = hb - bb * p.h_q;
-  const uint32_t hkv = (hq * p.h_kv) / p.h_q;
-  const uint32_t q_first = qt * 256u + (over & 1u) * kRows;  // first query row within the sequence
-  const uint32_t q_row0 = bb * p.s_q + q_first, k_row0 = bb * p.s_k;
-  const bool work = q_first < p.s_q;                                       // the second half of a ragged tile may be empty
-  const uint32_t groups = keys_mode || q_first + kRows < p.s_q ? 2u : 1u;  // rows mode: group 1 may have no rows
-  const uint32_t tiles = work ? (p.s_k + kRows - 1u) / kRows : 0u;
-  const uint32_t units = keys_mode ? tiles : tiles * groups;           // (key tile, group) pairs in the order the MMAs are issued
+  const SdpaItem first(p, blockIdx.x);  // before the wait for the previous kernel: its divisions cost nothing there
   const uint32_t last_valid = p.s_k - ((p.s_k - 1u) / kRows) * kRows;  // keys of the last tile
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
   if (tid == 0) {
     mbar_init(q_full, 1);
+    mbar_init(q_empty, 1);
     for (uint32_t i = 0; i < 2; ++i) {
       mbar_init(k_full + 8 * i, 1);
       mbar_init(k_empty + 8 * i, 1);
@@ -207,39 +219,60 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   pdl_launch_dependents();
   pdl_wait();  // Q, K and V are the previous kernels' outputs
 
-  // Key tile j travels through ring stage j % 2 of K and V.
+  // The CTA's key tiles, counted over all its items, travel through ring stage n % 2 of K and V.
   if (warp == 0) {
     // ---------------- Q and K loader ----------------
-    if (work && elect_one()) {
-      const uint32_t q_tiles = keys_mode ? 1u : groups;
-      mbar_arrive_expect_tx(q_full, q_tiles * kTile);
-      for (uint32_t g = 0; g < q_tiles; ++g) {
-        tma_load_2d(sQ + g * kTile, &map_q, q_full, int32_t(hq * kD), int32_t(q_row0 + g * kRows));
-        tma_load_2d(sQ + g * kTile + kSub, &map_q, q_full, int32_t(hq * kD + 64), int32_t(q_row0 + g * kRows));
-      }
-    }
-    __syncwarp();
-    for (uint32_t j = 0; j < tiles; ++j) {
-      const uint32_t st = j & 1u, use = j >> 1;
-      if (use > 0 && !mbar_wait_warp(k_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
+    uint32_t n = 0, q_use = 0;
+    bool ok = true;
+    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
+      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
+      if (!w.work) continue;
+      if (q_use > 0 && !mbar_wait_warp(q_empty, (q_use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
+      ++q_use;
+      const uint32_t q_row0 = w.bb * p.s_q + w.q_first, k_row0 = w.bb * p.s_k;
       if (elect_one()) {
-        mbar_arrive_expect_tx(k_full + 8 * st, kTile);
-        tma_load_2d(sK + st * kTile, &map_k, k_full + 8 * st, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
-        tma_load_2d(sK + st * kTile + kSub, &map_k, k_full + 8 * st, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
+        const uint32_t q_tiles = w.keys_mode ? 1u : w.groups;
+        mbar_arrive_expect_tx(q_full, q_tiles * kTile);
+        for (uint32_t g = 0; g < q_tiles; ++g) {
+          tma_load_2d(sQ + g * kTile, &map_q, q_full, int32_t(w.hq * kD), int32_t(q_row0 + g * kRows));
+          tma_load_2d(sQ + g * kTile + kSub, &map_q, q_full, int32_t(w.hq * kD + 64), int32_t(q_row0 + g * kRows));
+        }
       }
       __syncwarp();
+      for (uint32_t j = 0; j < w.tiles; ++j, ++n) {
+        const uint32_t st = n & 1u, use = n >> 1;
+        if (use > 0 && !mbar_wait_warp(k_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(k_full + 8 * st, kTile);
+          tma_load_2d(sK + st * kTile, &map_k, k_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + j * kRows));
+          tma_load_2d(sK + st * kTile + kSub, &map_k, k_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + j * kRows));
+        }
+        __syncwarp();
+      }
     }
   } else if (warp == 2) {
     // ---------------- V loader (its ring frees later than K's: a warp of its own, so that K never waits behind V) ----------------
-    for (uint32_t j = 0; j < tiles; ++j) {
-      const uint32_t st = j & 1u, use = j >> 1;
-      if (use > 0 && !mbar_wait_warp(v_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
-      if (elect_one()) {
-        mbar_arrive_expect_tx(v_full + 8 * st, kTile);
-        tma_load_2d(sV + st * kTile, &map_v, v_full + 8 * st, int32_t(hkv * kD), int32_t(k_row0 + j * kRows));
-        tma_load_2d(sV + st * kTile + kSub, &map_v, v_full + 8 * st, int32_t(hkv * kD + 64), int32_t(k_row0 + j * kRows));
+    uint32_t n = 0;
+    bool ok = true;
+    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
+      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
+      const uint32_t k_row0 = w.bb * p.s_k;
+      for (uint32_t j = 0; j < w.tiles; ++j, ++n) {
+        const uint32_t st = n & 1u, use = n >> 1;
+        if (use > 0 && !mbar_wait_warp(v_empty + 8 * st, (use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(v_full + 8 * st, kTile);
+          tma_load_2d(sV + st * kTile, &map_v, v_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + j * kRows));
+          tma_load_2d(sV + st * kTile + kSub, &map_v, v_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + j * kRows));
+        }
+        __syncwarp();
       }
-      __syncwarp();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -249,271 +282,295 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     const uint64_t k_desc = make_desc_sw128(sK), v_desc = make_desc_mn_sw128(sV, kSub);
     const uint32_t k_hi = uint32_t(k_desc >> 32), v_hi = uint32_t(v_desc >> 32);
     const uint32_t q_lo0 = uint32_t(make_desc_sw128(sQ)), k_lo0 = uint32_t(k_desc), v_lo0 = uint32_t(v_desc);
-    const bool by_rows2 = !keys_mode && groups == 2u;
-    // unit u = (key tile, group)
-    auto tile_of = [&](uint32_t u) { return by_rows2 ? u >> 1 : u; };
-    auto group_of = [&](uint32_t u) { return groups == 2u ? u & 1u : 0u; };
-    auto wait_k = [&](uint32_t u) -> bool {
-      const uint32_t j = tile_of(u);
-      return mbar_wait_warp(k_full + 8 * (j & 1u), (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
-    };
-    auto issue_s = [&](uint32_t u) {  // one elected lane
-      const uint32_t g = group_of(u), st = tile_of(u) & 1u;
-      const uint32_t q_lo = q_lo0 + (keys_mode ? 0u : g) * (kTile >> 4), k_lo = k_lo0 + st * (kTile >> 4);
+    uint32_t n0 = 0, q_use = 0, used0 = 0, used1 = 0;  // key tiles, items and each group's tiles of the items before
+    bool ok = true;
+    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
+      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
+      if (!w.work) continue;
+      const uint32_t groups = w.groups, tiles = w.tiles, units = w.units;
+      const bool by_rows2 = !w.keys_mode && groups == 2u;
+      // unit u = (key tile, group)
+      auto tile_of = [&](uint32_t u) { return by_rows2 ? u >> 1 : u; };
+      auto group_of = [&](uint32_t u) { return groups == 2u ? u & 1u : 0u; };
+      auto wait_k = [&](uint32_t u) -> bool {
+        const uint32_t n = n0 + tile_of(u);
+        return mbar_wait_warp(k_full + 8 * (n & 1u), (n >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
+      };
+      auto wait_v = [&](uint32_t u) -> bool {
+        const uint32_t n = n0 + tile_of(u);
+        return mbar_wait_warp(v_full + 8 * (n & 1u), (n >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
+      };
+      auto issue_s = [&](uint32_t u) {  // one elected lane
+        const uint32_t g = group_of(u), st = (n0 + tile_of(u)) & 1u;
+        const uint32_t q_lo = q_lo0 + (w.keys_mode ? 0u : g) * (kTile >> 4), k_lo = k_lo0 + st * (kTile >> 4);
 #pragma unroll
-      for (uint32_t kk = 0; kk < 8; ++kk) {
-        const uint32_t off = ((kk >> 2) * kSub + (kk & 3u) * 32u) >> 4;
-        tc_mma_bf16(tmem_base + g * 128u, (uint64_t(k_hi) << 32) | (q_lo + off), (uint64_t(k_hi) << 32) | (k_lo + off), idesc_qk, kk != 0u);
+        for (uint32_t kk = 0; kk < 8; ++kk) {
+          const uint32_t off = ((kk >> 2) * kSub + (kk & 3u) * 32u) >> 4;
+          tc_mma_bf16(tmem_base + g * 128u, (uint64_t(k_hi) << 32) | (q_lo + off), (uint64_t(k_hi) << 32) | (k_lo + off), idesc_qk, kk != 0u);
+        }
+        tc_commit(s_full + 8 * g);
+        if (w.keys_mode || g + 1u == groups) tc_commit(k_empty + 8 * st);  // the tile's last reader
+        if (u + 1u == units) tc_commit(q_empty);                           // the item's last scores
+      };
+      // Waits take about 100 cycles each even when their phase is long over: those for the loads of the NEXT unit stand where
+      // this warp is idle, between the two parts of a unit's P V, not on the way from a finished P to the next scores.
+      auto wait_loads = [&](uint32_t u) { return u >= units || (wait_v(u) && (u + groups >= units || wait_k(u + groups))); };
+      ok = mbar_wait_warp(q_full, q_use & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
+      ++q_use;
+      for (uint32_t u = 0; u < groups && u < units && ok; ++u) {
+        ok = wait_k(u);
+        tc_fence_after();
+        if (ok && elect_one()) issue_s(u);
+        __syncwarp();
       }
-      tc_commit(s_full + 8 * g);
-      if (keys_mode || g + 1u == groups) tc_commit(k_empty + 8 * st);  // the tile's last reader
-    };
-    bool ok = work && mbar_wait_warp(q_full, 0, abort_flag, kStatusMmaTimeout, wait_limit);
-    for (uint32_t u = 0; u < groups && u < units && ok; ++u) {
-      ok = wait_k(u);
-      tc_fence_after();
-      if (ok && elect_one()) issue_s(u);
-      __syncwarp();
-    }
-    auto wait_v = [&](uint32_t u) -> bool {
-      const uint32_t j = tile_of(u);
-      return mbar_wait_warp(v_full + 8 * (j & 1u), (j >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
-    };
-    // Waits take about 100 cycles each even when their phase is long over: those for the loads of the NEXT unit stand where
-    // this warp is idle, between the two parts of a unit's P V, not on the way from a finished P to the next scores.
-    auto wait_loads = [&](uint32_t u) { return u >= units || (wait_v(u) && (u + groups >= units || wait_k(u + groups))); };
-    ok = ok && wait_loads(0);
-    for (uint32_t u = 0; u < units && ok; ++u) {
-      const uint32_t g = group_of(u), j = tile_of(u), st = j & 1u;
-      const uint32_t use = keys_mode ? u >> 1 : j;
-      const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
-      const bool next = u + groups < units;
-      const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
-      if (!mbar_wait_warp(p_part + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
-      tc_fence_after();
-      if (elect_one()) {
+      ok = ok && wait_loads(0);
+      for (uint32_t u = 0; u < units && ok; ++u) {
+        const uint32_t g = group_of(u), j = tile_of(u), st = (n0 + j) & 1u;
+        const uint32_t use = w.keys_mode ? u >> 1 : j, parity = ((g ? used1 : used0) + use) & 1u;
+        const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
+        const bool next = u + groups < units;
+        const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
+        ok = mbar_wait_warp(p_part + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (uint32_t kk = 0; kk < kSplitK; ++kk)  // P's packed columns 8kk.. in TMEM, V rows 16kk..
-          if (kk < k_steps)
-            tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, (use | kk) != 0u);
-      }
-      __syncwarp();
-      if (!wait_loads(u + 1u)) break;
-      if (!mbar_wait_warp(p_full + 8 * g, use & 1u, abort_flag, kStatusMmaTimeout, wait_limit)) break;
-      tc_fence_after();
-      if (elect_one()) {
+          for (uint32_t kk = 0; kk < kSplitK; ++kk)  // P's packed columns 8kk.. in TMEM, V rows 16kk..
+            if (kk < k_steps)
+              tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, (use | kk) != 0u);
+        }
+        __syncwarp();
+        ok = wait_loads(u + 1u) && mbar_wait_warp(p_full + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (uint32_t kk = kSplitK; kk < 8; ++kk)
-          if (kk < k_steps)
-            tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, 1u);
-        if (keys_mode || g + 1u == groups) tc_commit(v_empty + 8 * st);
-        if (next) issue_s(u + groups);
-        else tc_commit(o_full + 8 * g);  // the group's last product
+          for (uint32_t kk = kSplitK; kk < 8; ++kk)
+            if (kk < k_steps)
+              tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, 1u);
+          if (w.keys_mode || g + 1u == groups) tc_commit(v_empty + 8 * st);
+          if (next) issue_s(u + groups);
+          else tc_commit(o_full + 8 * g);  // the group's last product
+        }
+        __syncwarp();
       }
-      __syncwarp();
+      n0 += tiles;
+      used0 += w.keys_mode ? (tiles + 1u) >> 1 : tiles;
+      used1 += w.keys_mode ? tiles >> 1 : (groups == 2u ? tiles : 0u);
     }
   } else if (warp >= 4) {
     // ---------------- softmax: two groups, one query row per thread ----------------
     const uint32_t g = (warp - 4u) >> 2, quarter = warp & 3u, row = quarter * 32u + lane;
     const uint32_t lane_addr = tmem_base + ((quarter * 32u) << 16);
     const uint32_t s_addr = lane_addr + g * 128u, o_addr = lane_addr + kOCol + g * 128u;
-    float m_ref = -INFINITY, l = 0.0f;
-    bool ok = true;
     uint32_t s0[32], s1[32], s2[32], s3[32];
-    uint32_t use = 0;
-    const uint32_t j_step = keys_mode ? 2u : 1u;
-    for (uint32_t j = keys_mode ? g : 0u; j < tiles && g < groups; j += j_step, ++use) {
-      const uint32_t valid = j + 1u == tiles ? last_valid : kRows;  // keys of this tile that exist
-      // S_g complete; the pipe ran O_g += P_g V of the tile before in front of it, so O_g is complete too
-      if (!mbar_wait_warp(s_full + 8 * g, use & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      // the whole score row goes to registers in one round trip (four loads in flight, one wait)
-      tmem_ld_32x32b_x32(s_addr, s0);
-      tmem_ld_32x32b_x32(s_addr + 32u, s1);
-      tmem_ld_32x32b_x32(s_addr + 64u, s2);
-      tmem_ld_32x32b_x32(s_addr + 96u, s3);
-      tmem_ld_wait();
-      // keys that do not exist weigh nothing: 2^(-inf). Masked here and not per chunk: the exponentials of a tile then are one
-      // block without branches, which the compiler can interleave
-      auto mask = [&]() {
-        if (valid < kRows) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (uint32_t(i) >= valid) s0[i] = 0xFF800000u;
-            if (32u + uint32_t(i) >= valid) s1[i] = 0xFF800000u;
-            if (64u + uint32_t(i) >= valid) s2[i] = 0xFF800000u;
-            if (96u + uint32_t(i) >= valid) s3[i] = 0xFF800000u;
-          }
+    uint32_t seen = 0, done = 0;  // key tiles and items of this group so far
+    bool ok = true;               // once a wait has given up every later one does at once; the barriers of all items are still met
+    for (uint32_t it = blockIdx.x; it < p.items; it += gridDim.x) {
+      const SdpaItem item = it == blockIdx.x ? first : SdpaItem(p, it);
+      const bool keys_mode = item.keys_mode;
+      const uint32_t tiles = item.tiles, groups = item.groups;
+      float m_ref = -INFINITY, l = 0.0f;
+      uint32_t use = 0;
+      const uint32_t j_step = keys_mode ? 2u : 1u;
+      for (uint32_t j = keys_mode ? g : 0u; j < tiles && g < groups && ok; j += j_step, ++use, ++seen) {
+        const uint32_t valid = j + 1u == tiles ? last_valid : kRows;  // keys of this tile that exist
+        // S_g complete; the pipe ran O_g += P_g V of the tile before in front of it, so O_g is complete too
+        if (!mbar_wait_warp(s_full + 8 * g, seen & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
+          ok = false;
+          break;
         }
-      };
-      mask();
-      auto chunk_max = [&](const uint32_t(&c)[32]) -> float {
-        float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 32; i += 8) {  // three-input maxima: 16 instructions for 32 values
-          a = max3(a, __uint_as_float(c[i]), __uint_as_float(c[i + 1]));
-          b = max3(b, __uint_as_float(c[i + 2]), __uint_as_float(c[i + 3]));
-          d = max3(d, __uint_as_float(c[i + 4]), __uint_as_float(c[i + 5]));
-          e = max3(e, __uint_as_float(c[i + 6]), __uint_as_float(c[i + 7]));
-        }
-        return fmaxf(fmaxf(a, b), fmaxf(d, e));
-      };
-      uint64_t l01, l23;
-      // p = exp2(s * scale_log2 - m) of 32 keys: row sum in f32, P as bf16 pairs (two per 32-bit column, key 2i in the low half)
-      auto exps = [&](uint32_t(&c)[32], uint32_t(&w)[16]) {
-        const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(-m_ref, -m_ref);
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {  // the scale and the shift for two scores in one packed FMA
-          float x0, x1;
-          unpack2(fma2(pack2u(c[i], c[i + 1]), sc2, nm2), x0, x1);
-          c[i] = __float_as_uint(ex2(x0));
-          c[i + 1] = __float_as_uint(ex2(x1));
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          l01 = add2(l01, pack2u(c[i], c[i + 1]));
-          l23 = add2(l23, pack2u(c[i + 2], c[i + 3]));
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          w[i] = pack_bf16x2(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
-      };
-      auto sum4 = [&]() -> float {
-        float a, b, c, d;
-        unpack2(l01, a, b);
-        unpack2(l23, c, d);
-        return (a + b) + (c + d);
-      };
-      uint32_t w0[16], w1[16], w2[16];
-      const float top3 = chunk_max(s3) * p.scale_log2;  // scale > 0: the maximum commutes with it
-      bool bad = use == 0;     // this row's m has to be taken from the scores
-      bool redo = use == 0;    // ... or some row's of this warp
-#pragma unroll 1
-      while (true) {
-        if (redo) {
-          const float mx = fmaxf(fmaxf(fmaxf(chunk_max(s0), chunk_max(s1)), chunk_max(s2)) * p.scale_log2, top3);
-          float alpha = 1.0f;
-          if (bad && mx > m_ref) {
-            alpha = ex2(m_ref - mx);
-            l *= alpha;
-            m_ref = mx;
-          }
-          if (use > 0) {  // O_g is rescaled before this tile's product, which waits for the arrivals below
-            uint32_t o8[8];
-#pragma unroll 1
-            for (uint32_t c = 0; c < kD; c += 8u) {
-              tmem_ld_32x32b_x8(o_addr + c, o8);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
-              tmem_st_32x32b_x8(o_addr + c, o8);
-            }
-          }
-        }
-        l01 = l23 = pack2(0.0f, 0.0f);
-        exps(s0, w0);
-        exps(s1, w1);
-        exps(s2, w2);
-        if (redo) break;
-        bad = !(sum4() <= kLazySum) || !(top3 - m_ref <= kLazy);  // NaN counts as too large
-        redo = __any_sync(0xFFFFFFFFu, bad);
-        if (!redo) break;
-        tmem_ld_32x32b_x32(s_addr, s0);  // rare: the scores again (nothing has been written over them yet)
+        tc_fence_after();
+        // the whole score row goes to registers in one round trip (four loads in flight, one wait)
+        tmem_ld_32x32b_x32(s_addr, s0);
         tmem_ld_32x32b_x32(s_addr + 32u, s1);
         tmem_ld_32x32b_x32(s_addr + 64u, s2);
+        tmem_ld_32x32b_x32(s_addr + 96u, s3);
         tmem_ld_wait();
-        mask();
-      }
-      tmem_st_32x32b_x16(s_addr, w0);
-      tmem_st_32x32b_x16(s_addr + 16u, w1);
-      tmem_st_32x32b_x16(s_addr + 32u, w2);
-      tmem_st_wait();
-      tc_fence_before();  // this thread's TMEM reads and writes are ordered before the arrival below
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_part + 8 * g);
-      exps(s3, w0);
-      tmem_st_32x32b_x16(s_addr + 48u, w0);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full + 8 * g);
-      l += sum4();
-    }
-    // ---------------- O / l -> global ----------------
-    // rows mode: a group stores its own rows, all columns. Keys mode: group g stores columns 64g .. 64g+63 of the joint rows,
-    // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
-    if (ok && use > 0) ok = mbar_wait_warp(o_full + 8 * g, 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
-    float f_own = 1.0f / l, f_other = 0.0f;
-    const bool other = keys_mode && (g == 0 ? tiles > 1u : tiles > 0u);  // the other group has seen a tile
-    if (keys_mode) {
-      m_part[g * 128u + row] = m_ref;
-      l_part[g * 128u + row] = l;
-      asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight softmax warps; every one of them gets here, whatever happened
-      if (other) {
-        if (ok) ok = mbar_wait_warp(o_full + 8 * (g ^ 1u), 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
-        const float m_o = m_part[(g ^ 1u) * 128u + row], l_o = l_part[(g ^ 1u) * 128u + row];
-        const float m = use > 0 ? fmaxf(m_ref, m_o) : m_o;
-        const float e_own = use > 0 ? ex2(m_ref - m) : 0.0f, e_other = ex2(m_o - m);
-        const float inv = 1.0f / (use > 0 ? l * e_own + l_o * e_other : l_o * e_other);
-        f_own = e_own * inv;
-        f_other = e_other * inv;
-      }
-    }
-    tc_fence_after();
-    if (ok && work && g < groups && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
-      const uint32_t q_in_seq = q_first + (keys_mode ? 0u : g * kRows) + row;
-      const bool store = q_in_seq < p.s_q;
-      const uint64_t grow = uint64_t(bb) * p.s_q + q_in_seq;  // row of the [b * s_q, h_q * 128] matrix
-      uint16_t* dst = p.out ? p.out + (grow * p.h_q + hq) * kD : nullptr;
-      const uint32_t c_first = keys_mode ? g * 2u : 0u, c_end = keys_mode ? g * 2u + 2u : 4u;  // 32-column chunks
-      uint32_t sc4 = 0;  // the four block scales of 64 columns: one word of the scale layout
-#pragma unroll 1
-      for (uint32_t c2 = c_first; c2 < c_end; ++c2) {
-        if (use > 0) {
-          tmem_ld_32x32b_x32(o_addr + c2 * 32u, s0);
-          tmem_ld_wait();
+        // keys that do not exist weigh nothing: 2^(-inf). Masked here and not per chunk: the exponentials of a tile then are one
+        // block without branches, which the compiler can interleave
+        auto mask = [&]() {
+          if (valid < kRows) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(__uint_as_float(s0[i]) * f_own);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) s0[i] = 0u;
-        }
-        if (other) {
-          tmem_ld_32x32b_x32(lane_addr + kOCol + (g ^ 1u) * 128u + c2 * 32u, s1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), f_other, __uint_as_float(s0[i])));
-        }
-        if (store) {
-          uint32_t w[16];  // 32 columns as bf16 pairs
-#pragma unroll
-          for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(s0[2 * i]), __uint_as_float(s0[2 * i + 1]));
-          if (dst) {
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q)
-              *reinterpret_cast<uint4*>(dst + c2 * 32u + q * 8u) = make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
-          }
-          if (p.q_codes) {
-            // the out-projection's activation quantiser, on the bf16-rounded values: two 16-column blocks per 32 columns,
-            // 8 code bytes each; the same bits tnf_quantize_act makes of the bf16 output
-            uint32_t codes[4];
-            if ((c2 & 1u) == 0u) sc4 = 0;
-#pragma unroll
-            for (uint32_t blk = 0; blk < 2; ++blk) {
-              const uint32_t w8[8] = {w[blk * 8], w[blk * 8 + 1], w[blk * 8 + 2], w[blk * 8 + 3], w[blk * 8 + 4], w[blk * 8 + 5], w[blk * 8 + 6], w[blk * 8 + 7]};
-              const uint32_t sc = quant_block16_bf16(w8, inv_d_lut, p.q_inv_t, codes[blk * 2], codes[blk * 2 + 1]);
-              sc4 |= sc << (8u * ((c2 & 1u) * 2u + blk));
+            for (int i = 0; i < 32; ++i) {
+              if (uint32_t(i) >= valid) s0[i] = 0xFF800000u;
+              if (32u + uint32_t(i) >= valid) s1[i] = 0xFF800000u;
+              if (64u + uint32_t(i) >= valid) s2[i] = 0xFF800000u;
+              if (96u + uint32_t(i) >= valid) s3[i] = 0xFF800000u;
             }
-            *reinterpret_cast<uint4*>(p.q_codes + grow * (uint64_t(p.h_q) * 64u) + hq * 64u + c2 * 16u) =
-                make_uint4(codes[0], codes[1], codes[2], codes[3]);
-            // blocks hq*8 + 4 * half .. +3 of the row: one 4-byte word of atom hq*2 + half (the launcher has cleared the padding)
-            if (c2 & 1u)
-              *reinterpret_cast<uint32_t*>(p.q_scales + ((grow >> 7) * p.q_k_atoms + hq * 2u + (c2 >> 1)) * 512u + (grow & 31u) * 16u + ((grow & 127u) >> 5) * 4u) = sc4;
+          }
+        };
+        mask();
+        auto chunk_max = [&](const uint32_t(&c)[32]) -> float {
+          float a = -INFINITY, b = -INFINITY, d = -INFINITY, e = -INFINITY;
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {  // three-input maxima: 16 instructions for 32 values
+            a = max3(a, __uint_as_float(c[i]), __uint_as_float(c[i + 1]));
+            b = max3(b, __uint_as_float(c[i + 2]), __uint_as_float(c[i + 3]));
+            d = max3(d, __uint_as_float(c[i + 4]), __uint_as_float(c[i + 5]));
+            e = max3(e, __uint_as_float(c[i + 6]), __uint_as_float(c[i + 7]));
+          }
+          return fmaxf(fmaxf(a, b), fmaxf(d, e));
+        };
+        uint64_t l01, l23;
+        // p = exp2(s * scale_log2 - m) of 32 keys: row sum in f32, P as bf16 pairs (two per 32-bit column, key 2i in the low half)
+        auto exps = [&](uint32_t(&c)[32], uint32_t(&w)[16]) {
+          const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(-m_ref, -m_ref);
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {  // the scale and the shift for two scores in one packed FMA
+            float x0, x1;
+            unpack2(fma2(pack2u(c[i], c[i + 1]), sc2, nm2), x0, x1);
+            c[i] = __float_as_uint(ex2(x0));
+            c[i + 1] = __float_as_uint(ex2(x1));
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            l01 = add2(l01, pack2u(c[i], c[i + 1]));
+            l23 = add2(l23, pack2u(c[i + 2], c[i + 3]));
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            w[i] = pack_bf16x2(__uint_as_float(c[2 * i]), __uint_as_float(c[2 * i + 1]));
+        };
+        auto sum4 = [&]() -> float {
+          float a, b, c, d;
+          unpack2(l01, a, b);
+          unpack2(l23, c, d);
+          return (a + b) + (c + d);
+        };
+        uint32_t w0[16], w1[16], w2[16];
+        const float top3 = chunk_max(s3) * p.scale_log2;  // scale > 0: the maximum commutes with it
+        bool bad = use == 0;     // this row's m has to be taken from the scores
+        bool redo = use == 0;    // ... or some row's of this warp
+#pragma unroll 1
+        while (true) {
+          if (redo) {
+            const float mx = fmaxf(fmaxf(fmaxf(chunk_max(s0), chunk_max(s1)), chunk_max(s2)) * p.scale_log2, top3);
+            float alpha = 1.0f;
+            if (bad && mx > m_ref) {
+              alpha = ex2(m_ref - mx);
+              l *= alpha;
+              m_ref = mx;
+            }
+            if (use > 0) {  // O_g is rescaled before this tile's product, which waits for the arrivals below
+              uint32_t o8[8];
+#pragma unroll 1
+              for (uint32_t c = 0; c < kD; c += 8u) {
+                tmem_ld_32x32b_x8(o_addr + c, o8);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o8[i] = __float_as_uint(__uint_as_float(o8[i]) * alpha);
+                tmem_st_32x32b_x8(o_addr + c, o8);
+              }
+            }
+          }
+          l01 = l23 = pack2(0.0f, 0.0f);
+          exps(s0, w0);
+          exps(s1, w1);
+          exps(s2, w2);
+          if (redo) break;
+          bad = !(sum4() <= kLazySum) || !(top3 - m_ref <= kLazy);  // NaN counts as too large
+          redo = __any_sync(0xFFFFFFFFu, bad);
+          if (!redo) break;
+          tmem_ld_32x32b_x32(s_addr, s0);  // rare: the scores again (nothing has been written over them yet)
+          tmem_ld_32x32b_x32(s_addr + 32u, s1);
+          tmem_ld_32x32b_x32(s_addr + 64u, s2);
+          tmem_ld_wait();
+          mask();
+        }
+        tmem_st_32x32b_x16(s_addr, w0);
+        tmem_st_32x32b_x16(s_addr + 16u, w1);
+        tmem_st_32x32b_x16(s_addr + 32u, w2);
+        tmem_st_wait();
+        tc_fence_before();  // this thread's TMEM reads and writes are ordered before the arrival below
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_part + 8 * g);
+        exps(s3, w0);
+        tmem_st_32x32b_x16(s_addr + 48u, w0);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + 8 * g);
+        l += sum4();
+      }
+      // ---------------- O / l -> global ----------------
+      // rows mode: a group stores its own rows, all columns. Keys mode: group g stores columns 64g .. 64g+63 of the joint rows,
+      // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
+      if (ok && use > 0) ok = mbar_wait_warp(o_full + 8 * g, done++ & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
+      float f_own = 1.0f / l, f_other = 0.0f;
+      const bool other = keys_mode && (g == 0 ? tiles > 1u : tiles > 0u);  // the other group has seen a tile
+      if (keys_mode) {
+        m_part[g * 128u + row] = m_ref;
+        l_part[g * 128u + row] = l;
+        tc_fence_before();
+        // the eight softmax warps; every one of them gets here, whatever happened. Each has waited for its group's O by now.
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (other) {
+          const float m_o = m_part[(g ^ 1u) * 128u + row], l_o = l_part[(g ^ 1u) * 128u + row];
+          const float m = use > 0 ? fmaxf(m_ref, m_o) : m_o;
+          const float e_own = use > 0 ? ex2(m_ref - m) : 0.0f, e_other = ex2(m_o - m);
+          const float inv = 1.0f / (use > 0 ? l * e_own + l_o * e_other : l_o * e_other);
+          f_own = e_own * inv;
+          f_other = e_other * inv;
+        }
+      }
+      tc_fence_after();
+      if (ok && item.work && g < groups && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
+        const uint32_t q_in_seq = item.q_first + (keys_mode ? 0u : g * kRows) + row;
+        const bool store = q_in_seq < p.s_q;
+        const uint64_t grow = uint64_t(item.bb) * p.s_q + q_in_seq;  // row of the [b * s_q, h_q * 128] matrix
+        uint16_t* dst = p.out ? p.out + (grow * p.h_q + item.hq) * kD : nullptr;
+        const uint32_t c_first = keys_mode ? g * 2u : 0u, c_end = keys_mode ? g * 2u + 2u : 4u;  // 32-column chunks
+        uint32_t sc4 = 0;  // the four block scales of 64 columns: one word of the scale layout
+#pragma unroll 1
+        for (uint32_t c2 = c_first; c2 < c_end; ++c2) {
+          if (use > 0) {
+            tmem_ld_32x32b_x32(o_addr + c2 * 32u, s0);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(__uint_as_float(s0[i]) * f_own);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s0[i] = 0u;
+          }
+          if (other) {
+            tmem_ld_32x32b_x32(lane_addr + kOCol + (g ^ 1u) * 128u + c2 * 32u, s1);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s0[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), f_other, __uint_as_float(s0[i])));
+          }
+          if (store) {
+            uint32_t w[16];  // 32 columns as bf16 pairs
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(s0[2 * i]), __uint_as_float(s0[2 * i + 1]));
+            if (dst) {
+#pragma unroll
+              for (uint32_t q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(dst + c2 * 32u + q * 8u) = make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
+            }
+            if (p.q_codes) {
+              // the out-projection's activation quantiser, on the bf16-rounded values: two 16-column blocks per 32 columns,
+              // 8 code bytes each; the same bits tnf_quantize_act makes of the bf16 output
+              uint32_t codes[4];
+              if ((c2 & 1u) == 0u) sc4 = 0;
+#pragma unroll
+              for (uint32_t blk = 0; blk < 2; ++blk) {
+                const uint32_t w8[8] = {w[blk * 8], w[blk * 8 + 1], w[blk * 8 + 2], w[blk * 8 + 3], w[blk * 8 + 4], w[blk * 8 + 5], w[blk * 8 + 6], w[blk * 8 + 7]};
+                const uint32_t sc = quant_block16_bf16(w8, inv_d_lut, p.q_inv_t, codes[blk * 2], codes[blk * 2 + 1]);
+                sc4 |= sc << (8u * ((c2 & 1u) * 2u + blk));
+              }
+              *reinterpret_cast<uint4*>(p.q_codes + grow * (uint64_t(p.h_q) * 64u) + item.hq * 64u + c2 * 16u) =
+                  make_uint4(codes[0], codes[1], codes[2], codes[3]);
+              // blocks hq*8 + 4 * half .. +3 of the row: one 4-byte word of atom hq*2 + half (the launcher has cleared the padding)
+              if (c2 & 1u)
+                *reinterpret_cast<uint32_t*>(p.q_scales + ((grow >> 7) * p.q_k_atoms + item.hq * 2u + (c2 >> 1)) * 512u + (grow & 31u) * 16u + ((grow & 127u) >> 5) * 4u) = sc4;
+            }
           }
         }
+      }
+      if (keys_mode) {  // the other group's rows may be overwritten by its next item: not before this group has read them
+        tc_fence_before();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
       }
     }
   }
@@ -614,9 +671,9 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     cudaError_t e = cudaFuncSetAttribute(sdpa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
   }
-  // One CTA per SM. Whole waves run in rows mode. The query tiles left over for a last wave run as two keys-mode CTAs each
-  // when every one of those then finds an SM of its own: half the time instead of a whole one on half the chip. With fewer
-  // tiles than half the SMs, that is all of them.
+  // One persistent CTA per SM, items in turn. Whole waves run in rows mode. The query tiles left over for a last wave run as
+  // two keys-mode items each when every one of those then finds an SM of its own: half the time instead of a whole one on
+  // half the chip. With fewer tiles than half the SMs, that is all of them.
   p.q_tiles = (a->s_q + 255u) / 256u;
   const uint64_t items = uint64_t(p.q_tiles) * a->h_q * a->b;
   const uint64_t sms = uint64_t(ctx->sm_count), tail = items % sms;
@@ -626,7 +683,8 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     return TNF_ERR_INVALID_ARGUMENT;
   }
   p.full_items = uint32_t(full);
-  cudaError_t e = launch_pdl(sdpa_kernel, dim3(uint32_t(full + 2 * (items - full))), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
+  p.items = uint32_t(full + 2 * (items - full));
+  cudaError_t e = launch_pdl(sdpa_kernel, dim3(std::min(p.items, uint32_t(sms))), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
   if (e != cudaSuccess) return cuda_fail(e, "sdpa launch");
   return TNF_OK;
 }
