@@ -71,3 +71,21 @@ def test_rows_mode_fused_output_quantisation(backend):
     assert np.array_equal(dev_scales_to_canonical(dev, s, cols), want_s) and np.array_equal(dev, want_dev)
     for buf in (qb, kb, vb, codes, scales):
         be.free(buf)
+
+
+@pytest.mark.parametrize("s_q,heads", [(140, 2), (256, 80)])  # keys mode, rows mode
+def test_output_on_a_16_byte_boundary(backend, s_q, heads):
+    """The output rows leave as 32-byte stores when they start on 32 bytes, as 16-byte ones otherwise: the same bits."""
+    from thinfer_b200 import _lib as L
+
+    be, n = backend, s_q * heads * 128 * 2
+    q, k, v = _inputs(1, s_q, 150, heads, heads, 99)
+    want = _run(be, q, k, v, SCALE)
+    qb, kb, vb, out = be.upload(q), be.upload(k), be.upload(v), be.upload(np.full(n // 2 + 16, 0x7FC0, np.uint16))
+    be.scope().sdpa(qb, kb, vb, L.Buf(out.id, 16, n), 1, s_q, 150, heads, heads, SCALE)
+    be.submit(30000)
+    got = be.read_buffer(out, np.uint16)
+    assert np.array_equal(got[8: 8 + n // 2], want.ravel())
+    assert (got[:8] == 0x7FC0).all() and (got[8 + n // 2:] == 0x7FC0).all()
+    for buf in (qb, kb, vb, out):
+        be.free(buf)

@@ -71,6 +71,7 @@ struct SdpaParams {
   uint32_t q_tiles;     // 256-row query tiles per (head, batch)
   uint32_t full_items;  // query tiles (over all heads and batches) that run in rows mode; each later one as two keys-mode items
   uint32_t items;       // work items in all
+  uint32_t wide_out;    // out starts on a 32-byte boundary
   float scale_log2;     // scale * log2(e)
 };
 
@@ -143,6 +144,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return d;
 }
 
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 // Work item `it` of the persistent loop: 256 query rows of one head and batch, or 128 rows of them (keys mode).
 struct SdpaItem {
   bool keys_mode, work;  // work: the item has rows (the second half of a ragged tile may be empty)
@@ -544,9 +550,14 @@ __global__ void __launch_bounds__(at::kThreads, 1)
 #pragma unroll
             for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(s0[2 * i]), __uint_as_float(s0[2 * i + 1]));
             if (dst) {
+              if (p.wide_out) {  // whole 32-byte sectors: the rows of a warp are far apart, half sectors would cost two writes each
+                st_global_v8(dst + c2 * 32u, &w[0]);
+                st_global_v8(dst + c2 * 32u + 16u, &w[8]);
+              } else {
 #pragma unroll
-              for (uint32_t q = 0; q < 4; ++q)
-                *reinterpret_cast<uint4*>(dst + c2 * 32u + q * 8u) = make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
+                for (uint32_t q = 0; q < 4; ++q)
+                  *reinterpret_cast<uint4*>(dst + c2 * 32u + q * 8u) = make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
+              }
             }
             if (p.q_codes) {
               // the out-projection's activation quantiser, on the bf16-rounded values: two 16-column blocks per 32 columns,
@@ -643,6 +654,7 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     return TNF_ERR_INVALID_ARGUMENT;
   SdpaParams p{};
   p.out = reinterpret_cast<uint16_t*>(out);
+  p.wide_out = reinterpret_cast<uintptr_t>(out) % 32u == 0 ? 1u : 0u;
   if (q_codes) {
     p.q_codes = q_codes;
     p.q_scales = q_scales;
