@@ -1,0 +1,93 @@
+"""Which kernel a linear takes must not show in its bits: shapes on both sides of the rules (one wave of 128-wide tiles, two with a
+short K, pairs working on halves of their tiles in the only wave), every epilogue, against the same rows computed about 100 at a time
+(1-CTA kernel, few tiles), and against the oracle."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import dev_scales_to_canonical, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (700, 3072, 512),    # 144 tiles of 128 x 128: one wave
+    (300, 6144, 288),    # 144, ragged rows and K
+    (769, 3072, 2048),   # 168: two waves, short K
+    (769, 3072, 2080),   # the same with K past the limit: 48 tiles of 256 x 256 on pairs
+    (513, 3200, 2112),   # 3 x 13 pair tiles, a ragged column tile: not halved
+    (1280, 2048, 2304),  # 40 pair tiles: not halved (more halves than pairs)
+    (130, 9472, 64),     # 148 tiles: exactly one wave
+    (130, 9600, 2304),   # 150: pairs, 38 tiles, ragged column tile
+])
+@pytest.mark.parametrize("kind", ["plain", "gelu", "gate", "chain"])
+def test_kernel_choice_does_not_show(backend, m, n, k, kind):
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+
+    be, rng, g = backend, np.random.default_rng(m + n + k), 0.002
+    a = O.f32_to_bf16(rng.standard_normal((m, k), np.float32))
+    w, bias = rng.standard_normal((n, k), np.float32) * np.float32(0.02), O.f32_to_bf16(rng.standard_normal(n, np.float32))
+    W = T.Nvfp4Weight.from_dense(be, w, bias)
+    gate, res = O.f32_to_bf16(rng.standard_normal(n, np.float32)), O.f32_to_bf16(rng.standard_normal((m, n), np.float32))
+    gated = kind in ("gate", "chain")
+    ab, gb, rb = be.upload(a), be.upload(gate), be.upload(res)
+    out, part = be.upload(np.full((m, n), 0x7FC0, np.uint16)), be.allocate(m * n * 2)
+    kw = dict(act=L.ACT_GELU_TANH if kind in ("gelu", "chain") else L.ACT_NONE, chain=kind == "chain")
+    sc = be.scope()
+    sc.linear(ab, m, W, g, out, gate=gb if gated else None, residual=rb if gated else None, **kw)
+    # slices of 17 rows and more: the skinny kernel (up to 16) rounds the products with alpha before it adds the bias
+    step = 96 if m % 96 > 16 else 100
+    for r in range(0, m, step):
+        rows = min(step, m - r)
+        assert rows > 16
+        view = lambda buf, cols: L.Buf(buf.id, r * cols * 2, rows * cols * 2)
+        sc.linear(view(ab, k), rows, W, g, view(part, n), gate=gb if gated else None, residual=view(rb, n) if gated else None, **kw)
+    be.submit(30000)
+    got, want = be.read_buffer(out, np.uint16).reshape(m, n), be.read_buffer(part, np.uint16).reshape(m, n)
+    assert np.array_equal(got, want)
+    if kind == "plain":
+        wc, ws, gw = O.quantize_weight(w)
+        rows = np.r_[0:3, m // 2: m // 2 + 3, m - 3: m]
+        ref = O.bf16_to_f32(O.linear(a[rows], g, wc, ws, gw, bias=bias))
+        assert rel_fro(O.bf16_to_f32(got[rows]), ref) <= 1e-3
+    W.free(be)
+    for buf in (ab, gb, rb, out, part):
+        be.free(buf)
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 512, 256), (640, 1024, 544), (257, 2304, 256)])  # 2, 12 and 18 pair tiles, all in halves
+def test_halves_in_the_only_wave(backend, m, n, k):
+    """The pair kernel's own epilogues (SwiGLU, dense arm, NVFP4 output) run on it whatever the size."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+    from thinfer_b200.backend import device_scales_bytes
+
+    be, rng, g = backend, np.random.default_rng(m), 0.002
+    a = O.f32_to_bf16(rng.standard_normal((m, k), np.float32))
+    W = T.Nvfp4Weight.from_dense(be, rng.standard_normal((n, k), np.float32) * np.float32(0.02))
+    W.prepare_dense(be)
+    ab, y, codes, scales = be.upload(a), be.allocate(m * n * 2), be.allocate(m * n // 2), be.allocate(device_scales_bytes(m, n))
+    sw, dense = be.allocate(m * n), be.allocate(m * n * 2)
+    sc = be.scope()
+    sc.linear(ab, m, W, g, y)                                      # 1-CTA kernel: the reference bits
+    y2 = be.allocate(m * n * 2)
+    sc.linear(ab, m, W, g, y2, out_nvfp4=(codes, scales, 0.001))   # pair kernel
+    sc.linear(ab, m, W, g, sw, swiglu=True)
+    sc.linear(ab, m, W, g, dense, dense_act=True)
+    be.submit(30000)
+    yv = be.read_buffer(y, np.uint16).reshape(m, n)
+    assert np.array_equal(be.read_buffer(y2, np.uint16).reshape(m, n), yv)
+    oc, os_ = O.quantize_act(yv, 0.001)
+    assert np.array_equal(be.read_buffer(codes).reshape(m, n // 2), oc)
+    assert np.array_equal(dev_scales_to_canonical(be.read_buffer(scales), m, n), os_)  # the GEMM leaves the rows past m alone
+    f = O.bf16_to_f32(yv).astype(np.float64)
+    want = f[:, 0::2] / (1.0 + np.exp(-f[:, 0::2])) * f[:, 1::2]
+    assert rel_fro(O.bf16_to_f32(be.read_buffer(sw, np.uint16)).reshape(m, n // 2), want) <= 8e-3  # from bf16-rounded inputs: 2 x 2^-9 and the output's
+    d = be.read_buffer(dense, np.uint16)
+    img = O.bf16_to_f32(be.read_buffer(W.dense, np.uint16)).reshape(n, k).astype(np.float64)
+    ref = O.bf16_to_f32(a).astype(np.float64) @ img.T * W.global_scale
+    assert rel_fro(O.bf16_to_f32(d).reshape(m, n), ref) <= 4e-3  # one bf16 rounding: 2^-9 at most
+    W.free(be)
+    for buf in (ab, y, y2, codes, scales, sw, dense):
+        be.free(buf)

@@ -620,12 +620,17 @@ static uint32_t env_u32_pair(const char* name, uint32_t dflt) {
 }
 
 bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k) {
-  (void)k;
   static uint32_t force = env_u32_pair("TNF_GEMM_KERNEL", 0);  // diagnostic builds: 1 = always 1-CTA, 2 = always pair
   if (force == 1) return false;
   if (force == 2) return true;
-  // a pair works on a 256x256 tile; with few tiles (skinny M) the 1-CTA kernel's 128x128 tiles fill more SMs
-  return m > 128 && uint64_t((m + 255u) / 256u) * ((n + 255u) / 256u) >= 32u;
+  if (m <= 128u) return false;
+  // A pair works on a 256 x 256 tile (or a half of it), the 1-CTA kernel on 128 x 128 ones: while those fit one wave of CTAs they
+  // occupy more SMs, each for less time. Measured (us, quantiser included, pair in halves against 1-CTA):
+  // 700 x 3072 x 3072 10.6 / 9.5, 300 x 6144 x 3072 12.2 / 9.2, 256 x 9216 x 9216 18.3 / 16.8, 384 x 6144 x 12288 24.8 / 19.2.
+  // In two waves the 1-CTA kernel reads its operands twice as often: only while K is short and the pairs are not filled
+  // either (1024 x 3072 x 1024 9.4 / 8.6, 2048 x 2048 x 2048 11.9 / 11.1, 2048 x 2048 x 4096 15.8 / 15.8, 900 x 2560 x 8192 19.8 / 21.8).
+  const uint64_t tiles1 = uint64_t((m + 127u) / 128u) * ((n + 127u) / 128u), tiles2 = uint64_t((m + 255u) / 256u) * ((n + 255u) / 256u);
+  return tiles1 > 148u && !(k <= 2048u && tiles2 <= 74u);
 }
 
 uint32_t gemm_pair_kblocks() { return 4u; }
@@ -679,8 +684,9 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
     p.band_m = uint32_t(std::min<uint64_t>(p.tiles_m, std::max<uint64_t>(1u, band_bytes / (row_bytes * 256u))));
   const uint32_t avail = uint32_t(max_pairs[dev] > 0 ? max_pairs[dev] : sm_count / 2);
   const uint32_t tail = tiles % avail;
-  // split the last wave's tiles into halves when every half then finds a pair of its own (and no half is empty)
-  p.full_tiles = (tiles > avail && tail > 0 && 2u * tail <= avail && p.n % 256u == 0u && !(kDiag && (diag & 2048u))) ? tiles - tail : tiles;
+  // split the last (or only) wave's tiles into halves when every half then finds a pair of its own (and no half is empty); alone in
+  // their wave: 700 x 3072 x 3072 12.2 -> 10.6 us, 512 x 4096 x 12288 24.7 -> 21.2
+  p.full_tiles = (tail > 0 && 2u * tail <= avail && p.n % 256u == 0u && !(kDiag && (diag & 2048u))) ? tiles - tail : tiles;
   const uint32_t items = p.full_tiles + (tiles - p.full_tiles) * 2u;
   const uint32_t pairs = std::min<uint32_t>(items, avail);
   PairOutMaps om;
