@@ -58,7 +58,7 @@ def test_kernel_choice_does_not_show(backend, m, n, k, kind):
 
 @pytest.mark.parametrize("m,n,k", [(200, 512, 256), (640, 1024, 544), (257, 2304, 256)])  # 2, 12 and 18 pair tiles, all in halves
 def test_halves_in_the_only_wave(backend, m, n, k):
-    """The pair kernel's own epilogues (SwiGLU, dense arm, NVFP4 output) run on it whatever the size."""
+    """The pair kernel's own epilogues (SwiGLU, dense arm) run on it whatever the size."""
     import thinfer_b200 as T
     from thinfer_b200 import _lib as L
     from thinfer_b200.backend import device_scales_bytes
@@ -72,7 +72,7 @@ def test_halves_in_the_only_wave(backend, m, n, k):
     sc = be.scope()
     sc.linear(ab, m, W, g, y)                                      # 1-CTA kernel: the reference bits
     y2 = be.allocate(m * n * 2)
-    sc.linear(ab, m, W, g, y2, out_nvfp4=(codes, scales, 0.001))   # pair kernel
+    sc.linear(ab, m, W, g, y2, out_nvfp4=(codes, scales, 0.001))
     sc.linear(ab, m, W, g, sw, swiglu=True)
     sc.linear(ab, m, W, g, dense, dense_act=True)
     be.submit(30000)
@@ -90,4 +90,46 @@ def test_halves_in_the_only_wave(backend, m, n, k):
     assert rel_fro(O.bf16_to_f32(d).reshape(m, n), ref) <= 4e-3  # one bf16 rounding: 2^-9 at most
     W.free(be)
     for buf in (ab, y, y2, codes, scales, sw, dense):
+        be.free(buf)
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (1, 512, 256), (200, 512, 256),  # 64-wide tiles
+    (100, 9600, 64),                 # 128-wide: 75 tiles
+    (300, 6144, 288),                # 144 tiles, the last rows ragged
+    (130, 9408, 96),                 # the last tile 64 columns wide
+    (40, 37888, 96),                 # 256-wide: 148 tiles
+])
+@pytest.mark.parametrize("act,chain,keep_bf16", [(0, False, True), (1, False, False), (1, True, True), (0, True, False)])
+def test_nvfp4_output_of_the_one_cta_kernel(backend, m, n, k, act, chain, keep_bf16):
+    """Codes and scales of the fused output quantiser, in a window of a wider operand, against the oracle quantiser on the bf16
+    output of the same linear; nothing else in the operand is touched."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+    from thinfer_b200.backend import device_scales_bytes
+
+    be, rng, g, off, ldo = backend, np.random.default_rng(m + n), 0.002, 64, n + 192
+    ab = be.upload(O.f32_to_bf16(rng.standard_normal((m, k), np.float32)))
+    W = T.Nvfp4Weight.from_dense(be, rng.standard_normal((n, k), np.float32) * np.float32(0.05), O.f32_to_bf16(rng.standard_normal(n, np.float32)))
+    plain, wide = be.allocate(m * n * 2), be.upload(np.full((m, ldo), 0x7FC0, np.uint16))
+    codes, scales = be.upload(np.full((m, ldo // 2), 0xA5, np.uint8)), be.upload(np.full(device_scales_bytes(m, ldo), 0x55, np.uint8))
+    sc, go = be.scope(), 0.0007
+    sc.linear(ab, m, W, g, wide if keep_bf16 else None, act=act, chain=chain, n_offset=off, ldo=ldo, out_nvfp4=(codes, scales, go))
+    if m <= 16:
+        sc.act_quant_shared(ab, m, k, g)  # not the skinny kernel, which rounds alpha and bias apart
+    sc.linear(ab, m, W, g, plain, act=act, chain=chain, flags=L.LINEAR_A_PREQUANTIZED if m <= 16 else 0)
+    be.submit(30000)
+    y = be.read_buffer(plain, np.uint16).reshape(m, n)
+    oc, os_ = O.quantize_act(y, go)
+    c = be.read_buffer(codes).reshape(m, ldo // 2)
+    assert np.array_equal(c[:, off // 2: (off + n) // 2], oc)
+    assert (c[:, : off // 2] == 0xA5).all() and (c[:, (off + n) // 2:] == 0xA5).all()
+    s = dev_scales_to_canonical(be.read_buffer(scales), m, ldo)
+    assert np.array_equal(s[:, off // 16: (off + n) // 16], os_)
+    assert (s[:, : off // 16] == 0x55).all() and (s[:, (off + n) // 16:] == 0x55).all()
+    b = be.read_buffer(wide, np.uint16).reshape(m, ldo)
+    assert np.array_equal(b[:, off: off + n], y) if keep_bf16 else (b == 0x7FC0).all()
+    assert (b[:, :off] == 0x7FC0).all() and (b[:, off + n:] == 0x7FC0).all()
+    W.free(be)
+    for buf in (ab, plain, wide, codes, scales):
         be.free(buf)

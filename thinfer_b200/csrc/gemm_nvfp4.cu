@@ -25,6 +25,7 @@
 #include "epilogue.cuh"
 #include "internal.h"
 #include "ptx.cuh"
+#include "quant_dev.cuh"
 
 namespace tnf {
 
@@ -49,7 +50,8 @@ struct TileCfg {
   static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
   static constexpr int kStages = (BN >= 224) ? 4 : (BN >= 192 ? 5 : (BN >= 128 ? 6 : 7));
   static constexpr int kEpiVecBytes = 4 * 1536;  // per epilogue warp: the tile's bias as f32 (1 KB) and gate as bf16 (512 B)
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kEpiVecBytes;
+  static constexpr int kLutBytes = 512;  // 1/(scale*g) per E4M3 code for the quantising epilogue
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kEpiVecBytes + kLutBytes;
   static constexpr uint32_t kAccCol0 = 0;
   static constexpr uint32_t kSfaCol = kAccStages * BN;
   static constexpr uint32_t kSfbCol = kSfaCol + 16;  // within a slot: 16 columns of A scales, then W's
@@ -121,7 +123,50 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ad
   }
 }
 
-template <int BN>
+// The same with an NVFP4 copy of the output (n % 64 == 0; no gated residual, as the host checks): 64 columns at a time, four
+// 16-column blocks quantised from the bf16-rounded values = 32 code bytes and one word of the scale layout per row. Every lane
+// stores its own row.
+template <int BN, bool kGelu, bool kChain>
+__device__ __forceinline__ void epilogue_tile_quant(const GemmParams& p, uint32_t t_addr, uint32_t row, uint32_t n0, float alpha,
+                                                    const float* bias_smem, const float* lut) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 64; ++c) {
+    const uint32_t nc = n0 + c * 64;
+    if (nc >= p.n) break;  // warp-uniform
+    const uint32_t qcol = p.n_offset + nc;
+    uint32_t sw = 0, codes[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t rc[32];
+      tmem_ld_32x32b_x32(t_addr + c * 64 + h * 32, rc);
+      tmem_ld_wait();
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        uint4 v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          v[i] = epilogue8<kGelu, kChain, false>(rc + blk * 16 + i * 8, alpha, bias_smem + c * 64 + h * 32 + blk * 16 + i * 8,
+                                                make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
+        if (p.store_bf16 && row < p.m) {
+          uint16_t* o = p.out[0] + uint64_t(row) * p.ldo + qcol + h * 32 + blk * 16;
+          *reinterpret_cast<uint4*>(o) = v[0];
+          *reinterpret_cast<uint4*>(o + 8) = v[1];
+        }
+        const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+        sw |= quant_block16_bf16(w, lut, p.q_inv_t, codes[h * 4 + blk * 2], codes[h * 4 + blk * 2 + 1]) << (8 * (h * 2 + blk));
+      }
+    }
+    if (row < p.m) {
+      uint4* q = reinterpret_cast<uint4*>(p.q_codes + uint64_t(row) * (p.ldo >> 1) + (qcol >> 1));
+      q[0] = make_uint4(codes[0], codes[1], codes[2], codes[3]);
+      q[1] = make_uint4(codes[4], codes[5], codes[6], codes[7]);
+      *reinterpret_cast<uint32_t*>(p.q_scales + sf_device_offset(row, qcol >> 4, p.q_k_atoms)) = sw;
+    }
+  }
+}
+
+// kQuant: with the NVFP4 output. A kernel of its own: in one kernel with the others it cost those up to 0.7 %.
+template <int BN, bool kQuant>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       const GemmParams p) {
@@ -167,6 +212,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_w);
   }
+  float* lut = reinterpret_cast<float*>(smem_gen + (sBar + 256 + Cfg::kEpiVecBytes - smem_base));
+  if (kQuant) fill_inv_scale_lut(lut, p.q_global, threadIdx.x, kThreads);
   if (warp == 1) {
     tmem_alloc(tmem_holder, kTmemCols);
     tmem_relinquish();
@@ -289,7 +336,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint4* gate_smem = reinterpret_cast<uint4*>(bias_smem + 256);
     const float bias_mul = (p.act == 1u && !p.chain) ? 0.5f : 1.0f;  // the fused GELU works on x/2
     const float alpha = p.alpha * bias_mul;
-    const uint32_t mode = (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u) | (p.gate ? 4u : 0u);
+    const uint32_t mode = (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u) | (!kQuant && p.gate ? 4u : 0u);
     uint32_t acc = 0, acc_phase = 0;
     bool ok = true;
     for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -319,15 +366,24 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t t_addr = tmem_base + Cfg::kAccCol0 + acc * BN + ((quarter * 32u) << 16);
       {
         const bool skip = kDiag && (p.diag & 1u);
-        switch (mode) {  // warp-uniform
-          case 0: epilogue_tile<BN, false, false, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 1: epilogue_tile<BN, true, false, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 2: epilogue_tile<BN, false, true, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 3: epilogue_tile<BN, true, true, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 4: epilogue_tile<BN, false, false, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 5: epilogue_tile<BN, true, false, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          case 6: epilogue_tile<BN, false, true, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
-          default: epilogue_tile<BN, true, true, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+        if constexpr (kQuant) {
+          switch (mode) {  // warp-uniform
+            case 0: epilogue_tile_quant<BN, false, false>(p, t_addr, row, n0, alpha, bias_smem, lut); break;
+            case 1: epilogue_tile_quant<BN, true, false>(p, t_addr, row, n0, alpha, bias_smem, lut); break;
+            case 2: epilogue_tile_quant<BN, false, true>(p, t_addr, row, n0, alpha, bias_smem, lut); break;
+            default: epilogue_tile_quant<BN, true, true>(p, t_addr, row, n0, alpha, bias_smem, lut); break;
+          }
+        } else {
+          switch (mode) {  // warp-uniform
+            case 0: epilogue_tile<BN, false, false, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 1: epilogue_tile<BN, true, false, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 2: epilogue_tile<BN, false, true, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 3: epilogue_tile<BN, true, true, false>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 4: epilogue_tile<BN, false, false, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 5: epilogue_tile<BN, true, false, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            case 6: epilogue_tile<BN, false, true, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+            default: epilogue_tile<BN, true, true, true>(p, t_addr, row, n0, lane, alpha, bias_smem, gate_smem, skip); break;
+          }
         }
       }
       tc_fence_before();
@@ -366,13 +422,13 @@ uint32_t gemm_tile_n(uint32_t m, uint32_t n) {
   return tm * ((n + 127u) / 128u) * 2u <= 148u ? 64u : 128u;
 }
 
-template <int BN>
+template <int BN, bool kQuant>
 static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w, GemmParams p, int sm_count,
                              cudaStream_t s) {
   using Cfg = TileCfg<BN>;
   static PerDeviceOnce once;
   if (once.first_use() >= 0) {  // the shared-memory opt-in is a per-device attribute of the function
-    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, kQuant>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
   }
   static uint32_t diag = env_u32("TNF_GEMM_DIAG", 0);
@@ -382,7 +438,12 @@ static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w,
   uint32_t tiles = p.tiles_m * p.tiles_n;
   if (tiles == 0) return cudaSuccess;
   uint32_t grid = std::min<uint32_t>(tiles, uint32_t(sm_count));
-  return launch_pdl(nvfp4_gemm_kernel<BN>, dim3(grid), dim3(kThreads), Cfg::kSmemBytes, s, map_a, map_w, p);
+  return launch_pdl(nvfp4_gemm_kernel<BN, kQuant>, dim3(grid), dim3(kThreads), Cfg::kSmemBytes, s, map_a, map_w, p);
+}
+
+template <int BN>
+static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w, const GemmParams& p, int sm_count, cudaStream_t s) {
+  return p.q_codes ? launch_bn<BN, true>(map_a, map_w, p, sm_count, s) : launch_bn<BN, false>(map_a, map_w, p, sm_count, s);
 }
 
 cudaError_t launch_gemm_nvfp4(const CUtensorMap& map_a, const CUtensorMap& map_w, const GemmParams& p, int sm_count,
