@@ -133,3 +133,28 @@ def test_nvfp4_output_of_the_one_cta_kernel(backend, m, n, k, act, chain, keep_b
     W.free(be)
     for buf in (ab, plain, wide, codes, scales):
         be.free(buf)
+
+
+@pytest.mark.parametrize("m,n,k,chain", [(1600, 4096, 512, False), (1600, 4112, 96, True), (2048, 9472, 64, False)])
+def test_swiglu_of_either_kernel(backend, m, n, k, chain):
+    """Rows on the pair kernel and the same rows a hundred at a time on the 1-CTA kernel (64-wide and 128-wide tiles, ragged columns)."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+
+    be, rng, g, cols = backend, np.random.default_rng(n), 0.002, n // 2
+    ab = be.upload(O.f32_to_bf16(rng.standard_normal((m, k), np.float32)))
+    W = T.Nvfp4Weight.from_dense(be, rng.standard_normal((n, k), np.float32) * np.float32(0.1), O.f32_to_bf16(rng.standard_normal(n, np.float32)))
+    out, part = be.allocate(m * cols * 2), be.upload(np.full((m, cols + 24), 0x7FC0, np.uint16))
+    sc = be.scope()
+    sc.linear(ab, m, W, g, out, swiglu=True, chain=chain)
+    for r in range(0, m, 100):
+        rows = min(100, m - r)
+        sc.linear(L.Buf(ab.id, r * k * 2, rows * k * 2), rows, W, g, L.Buf(part.id, r * (cols + 24) * 2, rows * (cols + 24) * 2), swiglu=True,
+                  chain=chain, n_offset=8, ldo=cols + 24)
+    be.submit(30000)
+    got, want = be.read_buffer(part, np.uint16).reshape(m, cols + 24), be.read_buffer(out, np.uint16).reshape(m, cols)
+    assert np.array_equal(got[:, 8: 8 + cols], want)
+    assert (got[:, :8] == 0x7FC0).all() and (got[:, 8 + cols:] == 0x7FC0).all()
+    W.free(be)
+    for buf in (ab, out, part):
+        be.free(buf)

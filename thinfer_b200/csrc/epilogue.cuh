@@ -111,4 +111,26 @@ __device__ __forceinline__ uint4 epilogue8(const uint32_t* r, float alpha, const
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// SwiGLU of 8 accumulator columns (a0, b0, a1, b1, ...): four output columns silu(a) * b, silu(v) = v / (1 + exp(-v)). Chain mode
+// rounds a and b to bf16 first, as the reference's two matmul dispatches do.
+template <bool kChain>
+__device__ __forceinline__ uint2 swiglu8(const uint32_t* r, float alpha, const float* bias_smem) {
+  const float4 bl = *reinterpret_cast<const float4*>(bias_smem), bh = *reinterpret_cast<const float4*>(bias_smem + 4);
+  const float bv[8] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
+  float o[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    float a, b;
+    if (kChain) {
+      a = bf16r(bf16r(__uint_as_float(r[2 * h]) * alpha) + bv[2 * h]);
+      b = bf16r(bf16r(__uint_as_float(r[2 * h + 1]) * alpha) + bv[2 * h + 1]);
+    } else {
+      unpack2(fma2(pack2u(r[2 * h], r[2 * h + 1]), pack2(alpha, alpha), pack2(bv[2 * h], bv[2 * h + 1])), a, b);
+    }
+    o[h] = __fdividef(a, 1.0f + __expf(-a)) * b;
+  }
+  const __nv_bfloat162 p0 = __floats2bfloat162_rn(o[0], o[1]), p1 = __floats2bfloat162_rn(o[2], o[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+}
+
 }  // namespace tnf

@@ -158,22 +158,7 @@ __device__ __forceinline__ void epilogue_pair_swiglu(const uint32_t (&r)[64], co
                                                      const float* bias_smem, int lane) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float4 bl = *reinterpret_cast<const float4*>(bias_smem + j * 8), bh = *reinterpret_cast<const float4*>(bias_smem + j * 8 + 4);
-    const float bv[8] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
-    float o[4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      float a, b;
-      if (kChain) {
-        a = bf16r(bf16r(__uint_as_float(r[j * 8 + 2 * h]) * p.alpha) + bv[2 * h]);
-        b = bf16r(bf16r(__uint_as_float(r[j * 8 + 2 * h + 1]) * p.alpha) + bv[2 * h + 1]);
-      } else {
-        unpack2(fma2(pack2u(r[j * 8 + 2 * h], r[j * 8 + 2 * h + 1]), pack2(p.alpha, p.alpha), pack2(bv[2 * h], bv[2 * h + 1])), a, b);
-      }
-      o[h] = __fdividef(a, 1.0f + __expf(-a)) * b;
-    }
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(o[0], o[1]), p1 = __floats2bfloat162_rn(o[2], o[3]);
-    *reinterpret_cast<uint2*>(buf_gen + lane * 64 + j * 8) = make_uint2(*reinterpret_cast<uint32_t*>(&p0), *reinterpret_cast<uint32_t*>(&p1));
+    *reinterpret_cast<uint2*>(buf_gen + lane * 64 + j * 8) = swiglu8<kChain>(&r[j * 8], p.alpha, bias_smem + j * 8);
   }
 }
 
