@@ -570,7 +570,7 @@ static int32_t raw_range(tnf_ctx* ctx, uint64_t id, uint64_t off, uint64_t n, co
   return TNF_OK;
 }
 
-// Large writes from pageable memory. The driver stages those through one thread (6-8 GB/s); here up to kWriteThreads
+// Large writes from pageable memory. A plain copy stages those through one thread (6-8 GB/s); here up to kWriteThreads
 // threads copy into pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the
 // chunks on the compute stream. The slots (kWriteStageBytes in all) are made on first use and freed with the context.
 // Below kWriteStagedMin the threads cost more than they save. Returns false when the caller has to copy the plain way

@@ -660,7 +660,7 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
   // unless it stays in L2 beside the band (kSmallW; then low bands, with 8 MB 1 % faster than with 12 and 6 % than with 24).
   // A W of up to kBandMaxW is worth a second reading only in bands as high as L2 allows (4352 x 12288 x 3072 in bf16:
   // 235.8 -> 232.5 us). Measured (us), one column after the other against bands: 26520 x 14336 x 3072 790-835 -> 612,
-  // 26520 x 3072 x 14336 with GELU 608 -> 557, 6630 x 14336 x 3072 172 -> 162 (part of which is the box).
+  // 26520 x 3072 x 14336 with GELU 608 -> 557, 6630 x 14336 x 3072 172 -> 164.
   const uint64_t row_bytes = kDense ? uint64_t(p.k) * 2u : uint64_t(p.k) * 9u / 16u;
   const uint64_t a_bytes = row_bytes * p.m, w_bytes = row_bytes * p.n;
   const uint64_t band_bytes = w_bytes <= kSmallW ? kBandSmallW : kBandLargeW;

@@ -318,9 +318,11 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         if (w.keys_mode || g + 1u == groups) tc_commit(k_empty + 8 * st);  // the tile's last reader
         if (u + 1u == units) tc_commit(q_empty);                           // the item's last scores
       };
-      // Waits take about 100 cycles each even when their phase is long over: those for the loads of the NEXT unit stand where
-      // this warp is idle, between the two parts of a unit's P V, not on the way from a finished P to the next scores.
-      auto wait_loads = [&](uint32_t u) { return u >= units || (wait_v(u) && (u + groups >= units || wait_k(u + groups))); };
+      // Waits take about 100 cycles each even when their phase is long over: V of the next unit and K of the scores that this
+      // unit issues at its end are waited for where this warp is idle, between the two parts of a unit's P V, not on the way
+      // from a finished P to the next scores. (K of the unit after that would be too early: in keys mode its stage has only
+      // just been freed. 414 x 15764 x 8 heads: 122 us.)
+      auto wait_loads = [&](uint32_t u) { return (u + 1u >= units || wait_v(u + 1u)) && (u + groups >= units || wait_k(u + groups)); };
       ok = mbar_wait_warp(q_full, q_use & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
       ++q_use;
       for (uint32_t u = 0; u < groups && u < units && ok; ++u) {
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         if (ok && elect_one()) issue_s(u);
         __syncwarp();
       }
-      ok = ok && wait_loads(0);
+      ok = ok && wait_v(0);
       for (uint32_t u = 0; u < units && ok; ++u) {
         const uint32_t g = group_of(u), j = tile_of(u), st = (n0 + j) & 1u;
         const uint32_t use = w.keys_mode ? u >> 1 : j, parity = ((g ? used1 : used0) + use) & 1u;
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
               tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, (use | kk) != 0u);
         }
         __syncwarp();
-        ok = wait_loads(u + 1u) && mbar_wait_warp(p_full + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
+        ok = wait_loads(u) && mbar_wait_warp(p_full + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
