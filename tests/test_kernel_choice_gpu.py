@@ -158,3 +158,60 @@ def test_swiglu_of_either_kernel(backend, m, n, k, chain):
     W.free(be)
     for buf in (ab, out, part):
         be.free(buf)
+
+
+@pytest.mark.parametrize("m,n,k,forms", [
+    (18944, 64, 96, ("plain", "quant", "swiglu")),   # 148 row tiles of a W of less than one scale block
+    (18817, 128, 64, ("plain", "quant", "swiglu")),  # the same, a whole block
+    (256, 18704, 96, ("plain", "swiglu")),           # 256-wide tiles, the last with 16 columns
+    (129, 18816, 288, ("plain", "quant")),           # ... with 128: one whole scale block of two
+    (512, 9280, 96, ("plain", "quant")),
+    (40, 37760, 96, ("plain", "quant", "swiglu")),
+])
+def test_last_tile_of_less_than_one_scale_block(backend, m, n, k, forms):
+    """256-wide tiles of the 1-CTA kernel whose last one needs one of two blocks of W's scales: the same rows in slices, and the
+    oracle."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+    from thinfer_b200.backend import device_scales_bytes
+
+    be, rng, g, go = backend, np.random.default_rng(m + n), 0.002, 0.0007
+    a = O.f32_to_bf16(rng.standard_normal((m, k), np.float32))
+    w, bias = rng.standard_normal((n, k), np.float32) * np.float32(0.1), O.f32_to_bf16(rng.standard_normal(n, np.float32))
+    W = T.Nvfp4Weight.from_dense(be, w, bias)
+    ab, out, part = be.upload(a), be.allocate(m * n * 2), be.allocate(m * n * 2)
+    sc = be.scope()
+    sc.linear(ab, m, W, g, out)
+    step = 1024 if n < 256 else 24 if m < 100 else 96
+    for r in range(0, m, step):  # 64- and 128-wide tiles
+        rows = min(step, m - r)
+        if rows <= 16:
+            continue  # the skinny kernel rounds the products with alpha before it adds the bias
+        sc.linear(L.Buf(ab.id, r * k * 2, rows * k * 2), rows, W, g, L.Buf(part.id, r * n * 2, rows * n * 2))
+    be.submit(30000)
+    y, want = be.read_buffer(out, np.uint16).reshape(m, n), be.read_buffer(part, np.uint16).reshape(m, n)
+    whole = m - (m % step if m % step <= 16 else 0)
+    assert np.array_equal(y[:whole], want[:whole])
+    rows = np.r_[0:3, m - 3: m]
+    wc, ws, gw = O.quantize_weight(w)
+    assert rel_fro(O.bf16_to_f32(y[rows]), O.bf16_to_f32(O.linear(a[rows], g, wc, ws, gw, bias=bias))) <= 1e-3
+    bufs = [ab, out, part]
+    if "quant" in forms:
+        codes, scales = be.allocate(m * n // 2), be.allocate(device_scales_bytes(m, n))
+        sc.linear(ab, m, W, g, None, out_nvfp4=(codes, scales, go))
+        be.submit(30000)
+        oc, os_ = O.quantize_act(y, go)
+        assert np.array_equal(be.read_buffer(codes).reshape(m, n // 2), oc)
+        assert np.array_equal(dev_scales_to_canonical(be.read_buffer(scales), m, n), os_)
+        bufs += [codes, scales]
+    if "swiglu" in forms:
+        sw = be.allocate(m * n)
+        sc.linear(ab, m, W, g, sw, swiglu=True)
+        be.submit(30000)
+        f = O.bf16_to_f32(y).astype(np.float64)
+        want = f[:, 0::2] / (1.0 + np.exp(-f[:, 0::2])) * f[:, 1::2]
+        assert rel_fro(O.bf16_to_f32(be.read_buffer(sw, np.uint16)).reshape(m, n // 2), want) <= 8e-3  # from bf16-rounded inputs: 2 x 2^-9 and the output's
+        bufs.append(sw)
+    W.free(be)
+    for buf in bufs:
+        be.free(buf)

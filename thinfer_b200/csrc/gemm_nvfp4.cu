@@ -258,7 +258,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t tm = tile % p.tiles_m, tn = tile / p.tiles_m;
         const uint32_t m0 = tm * kBlockM, n0 = tn * BN;
         const uint8_t* sfa_src = p.sfa + uint64_t(tm) * p.k_atoms * 512u;
-        const uint8_t* sfb_src = p.sfb + uint64_t(n0 >> 7) * p.k_atoms * 512u;
+        const uint8_t* sfb_src[Cfg::kSfbAtoms];
+#pragma unroll
+        for (int j = 0; j < Cfg::kSfbAtoms; ++j) sfb_src[j] = p.sfb + uint64_t(sf_row_block(n0 + uint32_t(j) * 128u, p.n)) * p.k_atoms * 512u;
         for (uint32_t kt = 0; kt < num_k_tiles; ++kt) {
           if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, kStatusProducerTimeout, wait_limit)) {
             ok = false;
@@ -277,8 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           bulk_load_1d(sSfa + stage * Cfg::kSfaBytes, sfa_src + uint64_t(kt) * 2048u, 2048u, full);
 #pragma unroll
           for (int j = 0; j < Cfg::kSfbAtoms; ++j)
-            bulk_load_1d(sSfb + stage * Cfg::kSfbBytes + j * 2048, sfb_src + (uint64_t(j) * p.k_atoms + kt * 4u) * 512u,
-                         2048u, full);
+            bulk_load_1d(sSfb + stage * Cfg::kSfbBytes + j * 2048, sfb_src[j] + uint64_t(kt) * 2048u, 2048u, full);
           }
           __syncwarp();
           if (++stage == S) { stage = 0; phase ^= 1u; }
@@ -439,12 +440,7 @@ static uint32_t env_u32(const char* name, uint32_t dflt) {
 uint32_t gemm_tile_n(uint32_t m, uint32_t n) {
   static uint32_t forced = env_u32("TNF_GEMM_TILE_N", 0);  // tuning knob: 64, 128 or 256
   if (forced == 64 || forced == 128 || forced == 256) return forced;
-  // 256-wide tiles only when they still fill the SMs; 128-wide tiles also double-buffer the accumulator; with so
-  // few tiles that half the SMs would idle, 64-wide ones: a CTA's time is what it has to pull in (its A tile
-  // and its share of W) and what it writes out, and both shrink with the tile
-  const uint64_t tm = (m + 127u) / 128u;
-  if (tm * ((n + 255u) / 256u) >= 148u) return 256u;
-  return tm * ((n + 127u) / 128u) * 2u <= 148u ? 64u : 128u;
+  return tile_n_rule(m, n, 148u);
 }
 
 template <int BN, bool kQuant>

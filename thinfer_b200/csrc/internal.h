@@ -7,6 +7,8 @@
 #include <tuple>
 #include <utility>
 
+#include "rules.h"
+
 namespace tnf {
 
 // Launch with programmatic dependent launch allowed: the kernel's prologue and CTA scheduling may
