@@ -61,3 +61,45 @@ def test_large_writes_from_several_threads(backend):
     for b, d in zip(bufs, datas):
         assert np.array_equal(backend.read_buffer(b), d)
         backend.free(b)
+
+
+@pytest.mark.parametrize("n_threads", [8, 72])  # 72: more calls wait for a scale than there are words to report it in
+def test_own_scales_of_several_threads(backend, n_threads):
+    """Threads that share a context quantise tensors of very different magnitude, each with its own scale: codes, block scales and
+    the reported scale belong to the same tensor, in every interleaving of the calls' launches."""
+    import ctypes as C
+
+    from thinfer_b200 import _lib as L
+
+    be, m, k = backend, 96, 256
+    a = [O.f32_to_bf16(np.random.default_rng(i).standard_normal((m, k)).astype(np.float32) * np.float32(4.0 ** (i % 9 - 4))) for i in range(n_threads)]
+    g = [O.global_scale(O.amax_bf16(x)) for x in a]
+    bufs = [(be.upload(x), be.allocate(m * k // 2), be.allocate(m * k // 16)) for x in a]
+    wrong = []
+
+    def work(i):
+        src, codes, scales = bufs[i]
+        used = C.c_float()
+        for _ in range(300 if n_threads == 8 else 40):
+            st = be.lib.tnf_quantize_act(be._ctx, src, m, k, 0.0, L.SCALES_CANONICAL, codes, scales, C.byref(used))
+            if st != 0 or used.value != np.float32(g[i]):
+                wrong.append((i, st, used.value))
+        # without asking for the scale: the launches of the threads run into one another
+        for _ in range(50):
+            be.lib.tnf_quantize_act(be._ctx, src, m, k, 0.0, L.SCALES_CANONICAL, codes, scales, None)
+
+    for _ in range(6):  # the codes are looked at after each round: the last call of each thread
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(n_threads)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        be.submit(30000)
+        for i in range(n_threads):
+            oc, os_ = O.quantize_act(a[i], g[i])
+            assert np.array_equal(be.read_buffer(bufs[i][1]).reshape(m, k // 2), oc), i
+            assert np.array_equal(be.read_buffer(bufs[i][2]).reshape(m, k // 16), os_), i
+    assert not wrong
+    for group in bufs:
+        for b in group:
+            be.free(b)

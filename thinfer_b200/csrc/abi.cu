@@ -904,6 +904,42 @@ int32_t tnf_selftest_stalled_wait(tnf_ctx* ctx) {
 
 uint64_t tnf_device_scales_bytes(uint32_t rows, uint32_t k) { return sf_device_bytes(rows, k); }
 
+// Quantises with the scale of the tensor itself. The quantiser reads the words that the maximum has left: with another thread's
+// maximum between the two launches it would take that tensor's scale.
+static int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout,
+                                  uint8_t* codes, uint8_t* scales, float* g_used) {
+  const float* g = reinterpret_cast<const float*>(ctx->dwords + 2);
+  const char* what = "amax launch";
+  int slot = -1;
+  cudaError_t e;
+  {
+    std::lock_guard<std::mutex> lk(ctx->scale_mu);
+    if (g_used && ctx->scale_free) {
+      slot = __builtin_ctzll(ctx->scale_free);
+      ctx->scale_free &= ctx->scale_free - 1u;
+    }
+    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->compute);
+    if (e == cudaSuccess) {
+      what = "quantise launch";
+      e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute);
+    }
+    if (e == cudaSuccess && g_used && slot < 0) {  // every word is a waiting call's
+      what = "global scale read";
+      e = cudaMemcpyAsync(g_used, g, 4, cudaMemcpyDeviceToHost, ctx->compute);
+    }
+  }
+  if (e == cudaSuccess && g_used) {
+    what = "quantise sync";
+    e = cudaStreamSynchronize(ctx->compute);
+    if (e == cudaSuccess && slot >= 0) *g_used = *static_cast<volatile float*>(ctx->scale_host + slot);
+  }
+  if (slot >= 0) {
+    std::lock_guard<std::mutex> lk(ctx->scale_mu);
+    ctx->scale_free |= 1ull << slot;
+  }
+  return e == cudaSuccess ? TNF_OK : cuda_fail(e, what);
+}
+
 int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint32_t n, uint32_t k, tnf_buf codes,
                             tnf_buf scales, float* global_scale) {
   TNF_CHECK_CTX(ctx);
@@ -919,15 +955,7 @@ int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint
   if (!c) return st;
   uint8_t* s = resolve(ctx, scales, uint64_t(n) * (k / 16), "scales", &st);
   if (!s) return st;
-  float* g = reinterpret_cast<float*>(ctx->dwords + 2);
-  float* host_g = global_scale ? ctx->scale_host + ctx->scale_next.fetch_add(1) % tnf_ctx::kScaleSlots : nullptr;
-  TNF_CUDA(launch_amax_scale(src, src_dtype, uint64_t(n) * k, ctx->dwords + 1, host_g, ctx->compute), "amax launch");
-  TNF_CUDA(launch_quantize(src, src_dtype, n, k, g, 0.0f, c, s, false, ctx->compute), "weight quantise launch");
-  if (global_scale) {
-    TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_quantize_weight sync");
-    *global_scale = *static_cast<volatile float*>(host_g);
-  }
-  return TNF_OK;
+  return quantize_own_scale(ctx, src, src_dtype, n, k, false, c, s, global_scale);
 }
 
 int32_t tnf_prepare_scales(tnf_ctx* ctx, tnf_buf scales_canonical, uint32_t rows, uint32_t k, tnf_buf scales_device) {
@@ -947,23 +975,9 @@ int32_t tnf_prepare_scales(tnf_ctx* ctx, tnf_buf scales_canonical, uint32_t rows
 
 static int32_t quantize_act_impl(tnf_ctx* ctx, const uint8_t* a, uint32_t m, uint32_t k, float g, bool device_layout,
                                  uint8_t* codes, uint8_t* scales, float* g_used) {
-  const float* g_ptr = nullptr;
-  float* host_g = nullptr;
-  if (!(g > 0.0f)) {
-    if (g_used) host_g = ctx->scale_host + ctx->scale_next.fetch_add(1) % tnf_ctx::kScaleSlots;
-    TNF_CUDA(launch_amax_scale(a, TNF_DTYPE_BF16, uint64_t(m) * k, ctx->dwords + 1, host_g, ctx->compute), "amax launch");
-    g_ptr = reinterpret_cast<float*>(ctx->dwords + 2);
-  }
-  TNF_CUDA(launch_quantize(a, TNF_DTYPE_BF16, m, k, g_ptr, g, codes, scales, device_layout, ctx->compute),
-           "activation quantise launch");
-  if (g_used) {
-    if (g_ptr) {
-      TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_quantize_act sync");
-      *g_used = *static_cast<volatile float*>(host_g);
-    } else {
-      *g_used = g;
-    }
-  }
+  if (!(g > 0.0f)) return quantize_own_scale(ctx, a, TNF_DTYPE_BF16, m, k, device_layout, codes, scales, g_used);
+  TNF_CUDA(launch_quantize(a, TNF_DTYPE_BF16, m, k, nullptr, g, codes, scales, device_layout, ctx->compute), "activation quantise launch");
+  if (g_used) *g_used = g;
   return TNF_OK;
 }
 

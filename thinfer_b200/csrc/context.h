@@ -1,7 +1,6 @@
 // The per-device context behind the C ABI: buffer table with category accounting, streams,
 // scratch, tensor-map cache, pinned host arenas, upload events. Internal to the library.
 #pragma once
-#include <atomic>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -71,11 +70,12 @@ struct tnf_ctx {
   long long wait_limit_cycles = tnf::kDefaultWaitLimitCycles;  // bound of every device-side mbarrier wait
   // small device words: [0] kernel status, [1..4] amax bits, scale g, 1/(6g), block counter of amax_scale_kernel
   uint32_t* dwords = nullptr;
-  // Scales the device reports to a waiting host call: a mapped pinned word per call, taken in turn, so that calls of
-  // several threads do not read each other's.
+  // dwords[1..4] belong to one quantisation at a time: its two launches go out under scale_mu. The scale that the device reports
+  // to a waiting host call has a mapped pinned word that is that call's until it has read it (bit i of scale_free: word i is free).
   static constexpr uint32_t kScaleSlots = 64;
+  std::mutex scale_mu;
   float* scale_host = nullptr;
-  std::atomic<uint32_t> scale_next{0};
+  uint64_t scale_free = ~0ull;
   std::map<tnf::MapSpec, CUtensorMap> maps;
   // fused-scatter peer windows (opened CUDA IPC mappings), index 0 unused
   static constexpr int kPeerSets = 4;
