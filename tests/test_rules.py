@@ -3,6 +3,7 @@ import ctypes as C
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -11,6 +12,19 @@ SHIM = r"""
 extern "C" {
 uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, rows); }
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
+// items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
+int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
+  tnf::SdpaPlan p{};
+  *n = 0;
+  if (!tnf::sdpa_plan(s_q, pairs, sms, &p)) return -1;
+  for (uint32_t c = 0; c < p.ctas; ++c)
+    for (uint32_t it = tnf::sdpa_first(p, c); it < p.items && *n < room; it = tnf::sdpa_next(p, c, it)) {
+      const tnf::SdpaSlot s = tnf::sdpa_slot(p, it);
+      uint32_t* o = out + 4 * (*n)++;
+      o[0] = c; o[1] = s.pair; o[2] = s.q_first; o[3] = s.keys_mode;
+    }
+  return p.ctas;
+}
 }
 """
 
@@ -44,3 +58,35 @@ def test_no_tile_copies_scales_past_the_weight(rules):
                         assert block == row // 128
                     past += row // 128 >= blocks
     assert past > 0  # there are shapes here whose last tile hangs over by a whole block
+
+
+@pytest.mark.parametrize("sms", [148, 7])
+@pytest.mark.parametrize("s_q", [1, 17, 128, 129, 256, 257, 300, 384, 385, 512, 640, 1111, 2000, 4352])
+def test_attention_items(rules, s_q, sms):
+    """Every block of 128 query rows of every (head, batch) pair is in exactly one item, no item is empty, every CTA has one, and
+    the slowest CTA takes the least number of half waves that the blocks allow."""
+    rules.sdpa_items.restype = C.c_int64
+    blocks = -(-s_q // 128)
+    for pairs in (1, 2, 3, 8, 12, 16, 24, 37, 48, 80, 147, 148, 149, 300, 500):
+        room = pairs * blocks
+        out, n = np.zeros((room + 1, 4), np.uint32), C.c_uint64()
+        ctas = rules.sdpa_items(C.c_uint32(s_q), C.c_uint64(pairs), C.c_uint32(sms), out.ctypes.data_as(C.c_void_p), C.byref(n), C.c_uint64(room + 1))
+        assert 0 < ctas <= sms and n.value <= room
+        items = out[: n.value].astype(np.int64)
+        seen = np.zeros((pairs, blocks), np.int64)
+        for half in (0, 1):  # a tile is two blocks
+            rows = items[(items[:, 3] == 0) | (half == 0)]
+            assert (rows[:, 2] % 128 == 0).all()
+            np.add.at(seen, (rows[:, 1], rows[:, 2] // 128 + half), 1)  # raises on a block that does not exist
+        assert (seen == 1).all(), (pairs, s_q)
+        halves = np.bincount(items[:, 0], weights=np.where(items[:, 3] == 0, 2, 1), minlength=ctas)
+        assert (halves > 0).all()
+        best = -(-pairs * blocks // sms)
+        assert halves.max() == best, (pairs, halves.max(), best)
+
+
+def test_attention_items_are_numbered_in_31_bits(rules):
+    rules.sdpa_items.restype = C.c_int64
+    n = C.c_uint64()
+    assert rules.sdpa_items(C.c_uint32((1 << 31) - 1), C.c_uint64(256), C.c_uint32(148), None, C.byref(n), C.c_uint64(0)) == -1
+    assert rules.sdpa_items(C.c_uint32(1 << 20), C.c_uint64(65535), C.c_uint32(148), None, C.byref(n), C.c_uint64(0)) == 148

@@ -1,5 +1,5 @@
-"""Attention with more query tiles than half the SMs: CTAs of 256 query rows (one softmax group per 128), the tiles left over
-for a last wave as two 128-row CTAs whose groups share the keys. Against the restated reference, same tolerance and reason as
+"""Attention with more blocks of 128 query rows than SMs: items of 256 rows (one softmax group per 128) and of 128 rows whose groups
+share the keys, several a CTA, in the mixtures that sdpa_plan (csrc/rules.h; its own test is test_rules.py) makes. Against the restated reference, same tolerance and reason as
 test_sdpa_gpu.py (bf16 probabilities in the second product, bf16 inputs and outputs)."""
 import numpy as np
 import pytest
@@ -13,11 +13,17 @@ SCALE = float(1.0 / np.sqrt(128.0))
 
 
 @pytest.mark.parametrize("b,s_q,s_k,h_q,h_kv,spread", [
-    (1, 300, 200, 80, 80, 1.0),    # 148 whole tiles (every second one with 44 rows: one group), 12 as two key-sharing CTAs (the second empty)
-    (2, 520, 330, 30, 10, 1.0),    # three tiles a sequence, the last with 8 rows; grouped heads; two batches
-    (1, 129, 700, 100, 100, 1.0),  # the second group has one row
-    (1, 100, 17, 100, 50, 1.0),    # one group, one ragged key tile
+    (1, 300, 200, 80, 80, 1.0),    # 80 tiles, and 80 blocks of 44 rows on the other 68 CTAs: two on twelve of them
+    (2, 520, 330, 30, 10, 1.0),    # 120 tiles, 60 blocks of 8 rows: two on each of the other 28 CTAs, four after tiles; grouped heads; two batches
+    (1, 129, 700, 100, 100, 1.0),  # tiles only; the second group has one row
+    (1, 100, 17, 100, 50, 1.0),    # one ragged key tile: the second group has none
     (1, 256, 1024, 76, 76, 6.0),   # peaked rows: the running output of both groups is rescaled from tile to tile
+    (1, 100, 17, 310, 310, 1.0),   # blocks only, three a CTA, the second group without a key tile
+    (1, 100, 130, 150, 150, 6.0),  # blocks only, two a CTA on two of them; two keys more than one tile
+    (1, 1111, 150, 60, 20, 1.0),   # a wave of tiles, 92 more, and 60 blocks of 87 rows on the other 56 CTAs
+    (1, 1111, 400, 37, 37, 1.0),   # a whole wave of tiles, then 37 blocks
+    (1, 300, 64, 140, 70, 1.0),    # 140 tiles and as many blocks of 44 rows: 16 on the idle CTAs, the others after tiles
+    (1, 300, 150, 300, 300, 1.0),  # two waves of tiles and four; 300 blocks: two on 144 CTAs, 12 more on the first
 ])
 def test_rows_mode_matches_reference_recurrence(backend, b, s_q, s_k, h_q, h_kv, spread):
     q, k, v = _inputs(b, s_q, s_k, h_q, h_kv, 31 * s_q + s_k, spread)

@@ -9,7 +9,7 @@
 //   rows mode   256 query rows of one (head, batch): group g has rows 128g .. 128g+127 and all key tiles
 //   keys mode   128 query rows: group g has the key tiles of parity g; the two outputs are joined at the end
 // Rows mode reads K and V once for 256 rows; keys mode halves an item's time, which fills the chip when there are few rows
-// and shortens the last wave (see the rule at the launch). The loads and the first scores of an item run under the
+// and shortens the last wave (sdpa_plan in rules.h says which item is which). The loads and the first scores of an item run under the
 // previous one's last products and output.
 //   TMEM columns 0-127 S_0, 128-255 S_1 (f32), 256-383 O_0, 384-511 O_1 (f32). P_g (bf16 pairs, 64 columns) takes the place
 //   of S_g: a thread has its score row in registers before it writes the first probability.
@@ -68,9 +68,7 @@ struct SdpaParams {
   uint32_t* status;
   long long wait_limit;
   uint32_t s_q, s_k, h_q, h_kv;
-  uint32_t q_tiles;     // 256-row query tiles per (head, batch)
-  uint32_t full_items;  // query tiles (over all heads and batches) that run in rows mode; each later one as two keys-mode items
-  uint32_t items;       // work items in all
+  SdpaPlan plan;
   uint32_t wide_out;    // out starts on a 32-byte boundary
   float scale_log2;     // scale * log2(e)
 };
@@ -149,24 +147,19 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
                "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
 }
-// Work item `it` of the persistent loop: 256 query rows of one head and batch, or 128 rows of them (keys mode).
+// Work item `it` of the persistent loop.
 struct SdpaItem {
-  bool keys_mode, work;  // work: the item has rows (the second half of a ragged tile may be empty)
-  uint32_t bb, hq, hkv, q_first, groups, tiles, units;
+  bool keys_mode;
+  uint32_t bb, hq, hkv, q_first, tiles, units;
   __device__ __forceinline__ SdpaItem(const SdpaParams& p, uint32_t it) {
-    using namespace at;
-    keys_mode = it >= p.full_items;
-    const uint32_t over = keys_mode ? it - p.full_items : 0u;
-    const uint32_t item = keys_mode ? p.full_items + (over >> 1) : it;
-    const uint32_t hb = item / p.q_tiles, qt = item - hb * p.q_tiles;
-    bb = hb / p.h_q;
-    hq = hb - bb * p.h_q;
+    const SdpaSlot slot = sdpa_slot(p.plan, it);
+    keys_mode = slot.keys_mode != 0u;
+    bb = slot.pair / p.h_q;
+    hq = slot.pair - bb * p.h_q;
     hkv = (hq * p.h_kv) / p.h_q;
-    q_first = qt * 256u + (over & 1u) * kRows;  // first query row within the sequence
-    work = q_first < p.s_q;
-    groups = keys_mode || q_first + kRows < p.s_q ? 2u : 1u;  // rows mode: group 1 may have no rows
-    tiles = work ? (p.s_k + kRows - 1u) / kRows : 0u;
-    units = keys_mode ? tiles : tiles * groups;  // (key tile, group) pairs in the order the MMAs are issued
+    q_first = slot.q_first;  // first query row within the sequence
+    tiles = (p.s_k + at::kRows - 1u) / at::kRows;
+    units = keys_mode ? tiles : tiles * 2u;  // (key tile, group) pairs in the order the MMAs are issued
   }
 };
 
@@ -190,7 +183,8 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   // the warp index as a warp-uniform value: the role branches and the MMA descriptors then live in uniform registers
   // (score MMAs alone: 593 cycles a tile against 617)
   const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;
-  const SdpaItem first(p, blockIdx.x);  // before the wait for the previous kernel: its divisions cost nothing there
+  const uint32_t it_first = sdpa_first(p.plan, blockIdx.x);
+  const SdpaItem first(p, it_first);  // before the wait for the previous kernel: its divisions cost nothing there
   const uint32_t last_valid = p.s_k - ((p.s_k - 1u) / kRows) * kRows;  // keys of the last tile
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
@@ -230,14 +224,13 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     // ---------------- Q and K loader ----------------
     uint32_t n = 0, q_use = 0;
     bool ok = true;
-    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
-      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
-      if (!w.work) continue;
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+      const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
       if (q_use > 0 && !mbar_wait_warp(q_empty, (q_use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
       ++q_use;
       const uint32_t q_row0 = w.bb * p.s_q + w.q_first, k_row0 = w.bb * p.s_k;
       if (elect_one()) {
-        const uint32_t q_tiles = w.keys_mode ? 1u : w.groups;
+        const uint32_t q_tiles = w.keys_mode ? 1u : 2u;
         mbar_arrive_expect_tx(q_full, q_tiles * kTile);
         for (uint32_t g = 0; g < q_tiles; ++g) {
           tma_load_2d(sQ + g * kTile, &map_q, q_full, int32_t(w.hq * kD), int32_t(q_row0 + g * kRows));
@@ -263,8 +256,8 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     // ---------------- V loader (its ring frees later than K's: a warp of its own, so that K never waits behind V) ----------------
     uint32_t n = 0;
     bool ok = true;
-    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
-      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+      const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
       const uint32_t k_row0 = w.bb * p.s_k;
       for (uint32_t j = 0; j < w.tiles; ++j, ++n) {
         const uint32_t st = n & 1u, use = n >> 1;
@@ -290,14 +283,10 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     const uint32_t q_lo0 = uint32_t(make_desc_sw128(sQ)), k_lo0 = uint32_t(k_desc), v_lo0 = uint32_t(v_desc);
     uint32_t n0 = 0, q_use = 0, used0 = 0, used1 = 0;  // key tiles, items and each group's tiles of the items before
     bool ok = true;
-    for (uint32_t it = blockIdx.x; it < p.items && ok; it += gridDim.x) {
-      const SdpaItem w = it == blockIdx.x ? first : SdpaItem(p, it);
-      if (!w.work) continue;
-      const uint32_t groups = w.groups, tiles = w.tiles, units = w.units;
-      const bool by_rows2 = !w.keys_mode && groups == 2u;
-      // unit u = (key tile, group)
-      auto tile_of = [&](uint32_t u) { return by_rows2 ? u >> 1 : u; };
-      auto group_of = [&](uint32_t u) { return groups == 2u ? u & 1u : 0u; };
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+      const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
+      const uint32_t tiles = w.tiles, units = w.units;
+      auto tile_of = [&](uint32_t u) { return w.keys_mode ? u : u >> 1; };  // unit u = (key tile, group u & 1)
       auto wait_k = [&](uint32_t u) -> bool {
         const uint32_t n = n0 + tile_of(u);
         return mbar_wait_warp(k_full + 8 * (n & 1u), (n >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
@@ -307,7 +296,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         return mbar_wait_warp(v_full + 8 * (n & 1u), (n >> 1) & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
       };
       auto issue_s = [&](uint32_t u) {  // one elected lane
-        const uint32_t g = group_of(u), st = (n0 + tile_of(u)) & 1u;
+        const uint32_t g = u & 1u, st = (n0 + tile_of(u)) & 1u;
         const uint32_t q_lo = q_lo0 + (w.keys_mode ? 0u : g) * (kTile >> 4), k_lo = k_lo0 + st * (kTile >> 4);
 #pragma unroll
         for (uint32_t kk = 0; kk < 8; ++kk) {
@@ -315,17 +304,17 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           tc_mma_bf16(tmem_base + g * 128u, (uint64_t(k_hi) << 32) | (q_lo + off), (uint64_t(k_hi) << 32) | (k_lo + off), idesc_qk, kk != 0u);
         }
         tc_commit(s_full + 8 * g);
-        if (w.keys_mode || g + 1u == groups) tc_commit(k_empty + 8 * st);  // the tile's last reader
+        if (w.keys_mode || g) tc_commit(k_empty + 8 * st);  // the tile's last reader
         if (u + 1u == units) tc_commit(q_empty);                           // the item's last scores
       };
       // Waits take about 100 cycles each even when their phase is long over: V of the next unit and K of the scores that this
       // unit issues at its end are waited for where this warp is idle, between the two parts of a unit's P V, not on the way
       // from a finished P to the next scores. (K of the unit after that would be too early: in keys mode its stage has only
       // just been freed. 414 x 15764 x 8 heads: 122 us.)
-      auto wait_loads = [&](uint32_t u) { return (u + 1u >= units || wait_v(u + 1u)) && (u + groups >= units || wait_k(u + groups)); };
+      auto wait_loads = [&](uint32_t u) { return (u + 1u >= units || wait_v(u + 1u)) && (u + 2u >= units || wait_k(u + 2u)); };
       ok = mbar_wait_warp(q_full, q_use & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
       ++q_use;
-      for (uint32_t u = 0; u < groups && u < units && ok; ++u) {
+      for (uint32_t u = 0; u < 2u && u < units && ok; ++u) {
         ok = wait_k(u);
         tc_fence_after();
         if (ok && elect_one()) issue_s(u);
@@ -333,10 +322,10 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       }
       ok = ok && wait_v(0);
       for (uint32_t u = 0; u < units && ok; ++u) {
-        const uint32_t g = group_of(u), j = tile_of(u), st = (n0 + j) & 1u;
+        const uint32_t g = u & 1u, j = tile_of(u), st = (n0 + j) & 1u;
         const uint32_t use = w.keys_mode ? u >> 1 : j, parity = ((g ? used1 : used0) + use) & 1u;
         const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
-        const bool next = u + groups < units;
+        const bool next = u + 2u < units;
         const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
         ok = mbar_wait_warp(p_part + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
         if (!ok) break;
@@ -356,15 +345,15 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           for (uint32_t kk = kSplitK; kk < 8; ++kk)
             if (kk < k_steps)
               tc_mma_bf16_ts(d_o, a_p + kk * 8u, (uint64_t(v_hi) << 32) | (v_lo + kk * (2048u >> 4)), idesc_pv, 1u);
-          if (w.keys_mode || g + 1u == groups) tc_commit(v_empty + 8 * st);
-          if (next) issue_s(u + groups);
+          if (w.keys_mode || g) tc_commit(v_empty + 8 * st);
+          if (next) issue_s(u + 2u);
           else tc_commit(o_full + 8 * g);  // the group's last product
         }
         __syncwarp();
       }
       n0 += tiles;
       used0 += w.keys_mode ? (tiles + 1u) >> 1 : tiles;
-      used1 += w.keys_mode ? tiles >> 1 : (groups == 2u ? tiles : 0u);
+      used1 += w.keys_mode ? tiles >> 1 : tiles;
     }
   } else if (warp >= 4) {
     // ---------------- softmax: two groups, one query row per thread ----------------
@@ -374,15 +363,14 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     uint32_t s0[32], s1[32], s2[32], s3[32];
     uint32_t seen = 0, done = 0;  // key tiles and items of this group so far
     bool ok = true;               // once a wait has given up every later one does at once; the barriers of all items are still met
-    for (uint32_t it = blockIdx.x; it < p.items; it += gridDim.x) {
-      const SdpaItem item = it == blockIdx.x ? first : SdpaItem(p, it);
+    for (uint32_t it = it_first; it < p.plan.items; it = sdpa_next(p.plan, blockIdx.x, it)) {
+      const SdpaItem item(p, it);  // its divisions run while the first scores are on their way
       const bool keys_mode = item.keys_mode;
-      const uint32_t tiles = item.tiles, groups = item.groups;
       float m_ref = -INFINITY, l = 0.0f;
       uint32_t use = 0;
       const uint32_t j_step = keys_mode ? 2u : 1u;
-      for (uint32_t j = keys_mode ? g : 0u; j < tiles && g < groups && ok; j += j_step, ++use, ++seen) {
-        const uint32_t valid = j + 1u == tiles ? last_valid : kRows;  // keys of this tile that exist
+      for (uint32_t j = keys_mode ? g : 0u; j * kRows < p.s_k && ok; j += j_step, ++use, ++seen) {
+        const uint32_t valid = min(kRows, p.s_k - j * kRows);  // keys of this tile that exist
         // S_g complete; the pipe ran O_g += P_g V of the tile before in front of it, so O_g is complete too
         if (!mbar_wait_warp(s_full + 8 * g, seen & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
           ok = false;
@@ -506,7 +494,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
       if (ok && use > 0) ok = mbar_wait_warp(o_full + 8 * g, done++ & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
       float f_own = 1.0f / l, f_other = 0.0f;
-      const bool other = keys_mode && (g == 0 ? tiles > 1u : tiles > 0u);  // the other group has seen a tile
+      const bool other = keys_mode && (g == 1u || p.s_k > kRows);  // the other group has seen a tile
       if (keys_mode) {
         m_part[g * 128u + row] = m_ref;
         l_part[g * 128u + row] = l;
@@ -523,7 +511,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         }
       }
       tc_fence_after();
-      if (ok && item.work && g < groups && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
+      if (ok && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
         const uint32_t q_in_seq = item.q_first + (keys_mode ? 0u : g * kRows) + row;
         const bool store = q_in_seq < p.s_q;
         const uint64_t grow = uint64_t(item.bb) * p.s_q + q_in_seq;  // row of the [b * s_q, h_q * 128] matrix
@@ -685,20 +673,11 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     cudaError_t e = cudaFuncSetAttribute(sdpa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
   }
-  // One persistent CTA per SM, items in turn. Whole waves run in rows mode. The query tiles left over for a last wave run as
-  // two keys-mode items each when every one of those then finds an SM of its own: half the time instead of a whole one on
-  // half the chip. With fewer tiles than half the SMs, that is all of them.
-  p.q_tiles = (a->s_q + 255u) / 256u;
-  const uint64_t items = uint64_t(p.q_tiles) * a->h_q * a->b;
-  const uint64_t sms = uint64_t(ctx->sm_count), tail = items % sms;
-  const uint64_t full = 2 * tail <= sms ? items - tail : items;
-  if (full + 2 * (items - full) > 0x7FFFFFFFull) {
-    set_error("tnf_sdpa: problem too large for the grid (%llu query tiles)", (unsigned long long)items);
+  if (!sdpa_plan(a->s_q, uint64_t(a->h_q) * a->b, uint32_t(ctx->sm_count), &p.plan)) {
+    set_error("tnf_sdpa: problem too large for the grid (b=%u s_q=%u h_q=%u)", a->b, a->s_q, a->h_q);
     return TNF_ERR_INVALID_ARGUMENT;
   }
-  p.full_items = uint32_t(full);
-  p.items = uint32_t(full + 2 * (items - full));
-  cudaError_t e = launch_pdl(sdpa_kernel, dim3(std::min(p.items, uint32_t(sms))), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
+  cudaError_t e = launch_pdl(sdpa_kernel, dim3(p.plan.ctas), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
   if (e != cudaSuccess) return cuda_fail(e, "sdpa launch");
   return TNF_OK;
 }
