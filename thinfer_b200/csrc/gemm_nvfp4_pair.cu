@@ -197,9 +197,15 @@ __device__ __forceinline__ void decode_item(const GemmParams& p, uint32_t tiles_
     sub = t & 1u;
     width = 128u;
   }
-  // row tiles in bands of band_m: all column tiles of a band before the next one (see the launcher)
-  const uint32_t band = tile / (p.band_m * p.tiles_n), first = band * p.band_m;
-  const uint32_t in_band = tile - first * p.tiles_n, height = min(p.band_m, tiles_m2 - first);
+  // Row tiles in bands of band_m: all column tiles of a band before the next one (see the launcher). Without bands the order is
+  // found with one division: every role of every item waits for it, and with a short K that shows (GELU, 6630 x 14336 x 1024
+  // 79.5 us with three divisions, 3602 x 8272 x 512 29.0).
+  uint32_t first = 0u, in_band = tile, height = tiles_m2;
+  if (p.band_m < tiles_m2) {  // uniform
+    first = tile / (p.band_m * p.tiles_n) * p.band_m;
+    in_band = tile - first * p.tiles_n;
+    height = min(p.band_m, tiles_m2 - first);
+  }
   const uint32_t tn = in_band / height;
   tm2 = first + in_band - tn * height;
   n0 = tn * 256u + sub * 128u;
