@@ -20,6 +20,7 @@ SCALE = float(1.0 / np.sqrt(128.0))
     (1, 256, 1024, 76, 76, 6.0),   # peaked rows: the running output of both groups is rescaled from tile to tile
     (1, 100, 17, 310, 310, 1.0),   # blocks only, three a CTA, the second group without a key tile
     (1, 100, 130, 150, 150, 6.0),  # blocks only, two a CTA on two of them; two keys more than one tile
+    (1, 70, 1300, 150, 50, 1.0),   # ... with eleven key tiles: both rings go round several times in the second item, too
     (1, 1111, 150, 60, 20, 1.0),   # a wave of tiles, 92 more, and 60 blocks of 87 rows on the other 56 CTAs
     (1, 1111, 400, 37, 37, 1.0),   # a whole wave of tiles, then 37 blocks
     (1, 300, 64, 140, 70, 1.0),    # 140 tiles and as many blocks of 44 rows: 16 on the idle CTAs, the others after tiles

@@ -309,9 +309,11 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       };
       // Waits take about 100 cycles each even when their phase is long over: V of the next unit and K of the scores that this
       // unit issues at its end are waited for where this warp is idle, between the two parts of a unit's P V, not on the way
-      // from a finished P to the next scores. (K of the unit after that would be too early: in keys mode its stage has only
-      // just been freed. 414 x 15764 x 8 heads: 122 us.)
-      auto wait_loads = [&](uint32_t u) { return (u + 1u >= units || wait_v(u + 1u)) && (u + 2u >= units || wait_k(u + 2u)); };
+      // from a finished P to the next scores. K of the unit after that would be too early: in keys mode its stage has only just
+      // been freed. So has V's of the next unit there: keys mode waits for V when its unit begins, after this unit's scores
+      // have been issued (us, waiting here against there, K and V of 16 heads from HBM: 414 x 15764 x 16 135 / 104; from L2:
+      // 700 x 8000 x 24 74 / 62, 700 x 2000 x 24 19.6 / 19.8).
+      auto wait_loads = [&](uint32_t u) { return (w.keys_mode || u + 1u >= units || wait_v(u + 1u)) && (u + 2u >= units || wait_k(u + 2u)); };
       ok = mbar_wait_warp(q_full, q_use & 1u, abort_flag, kStatusMmaTimeout, wait_limit);
       ++q_use;
       for (uint32_t u = 0; u < 2u && u < units && ok; ++u) {
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
         const bool next = u + 2u < units;
         const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
-        ok = mbar_wait_warp(p_part + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
+        ok = (!w.keys_mode || u == 0u || wait_v(u)) && mbar_wait_warp(p_part + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
