@@ -12,6 +12,7 @@ SHIM = r"""
 extern "C" {
 uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, rows); }
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
+int pair(uint32_t m, uint32_t n, uint32_t k, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, peers != 0, sms); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
 int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
   tnf::SdpaPlan p{};
@@ -58,6 +59,19 @@ def test_no_tile_copies_scales_past_the_weight(rules):
                         assert block == row // 128
                     past += row // 128 >= blocks
     assert past > 0  # there are shapes here whose last tile hangs over by a whole block
+
+
+def test_outputs_to_peers_take_the_pair_kernel(rules):
+    """The pair kernel stores to peers in 128-byte row segments: such calls take it from 32 of its tiles on, whatever is the better
+    kernel for a local output."""
+    differ = 0
+    for m in (1, 128, 129, 256, 300, 700, 1024, 4352):
+        for n in (256, 3072, 6144, 9472, 18432):
+            for k in (256, 2048, 12288):
+                tiles = -(-m // 256) * -(-n // 256)
+                assert rules.pair(m, n, k, 1, 148) == (m > 128 and tiles >= 32), (m, n, k)
+                differ += rules.pair(m, n, k, 1, 148) != rules.pair(m, n, k, 0, 148)
+    assert differ > 0
 
 
 @pytest.mark.parametrize("sms", [148, 7])

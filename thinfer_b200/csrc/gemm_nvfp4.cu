@@ -437,10 +437,10 @@ static uint32_t env_u32(const char* name, uint32_t dflt) {
   return v ? uint32_t(strtoul(v, nullptr, 0)) : dflt;
 }
 
-uint32_t gemm_tile_n(uint32_t m, uint32_t n) {
+uint32_t gemm_tile_n(uint32_t m, uint32_t n, int sm_count) {
   static uint32_t forced = env_u32("TNF_GEMM_TILE_N", 0);  // tuning knob: 64, 128 or 256
   if (forced == 64 || forced == 128 || forced == 256) return forced;
-  return tile_n_rule(m, n, 148u);
+  return tile_n_rule(m, n, uint32_t(sm_count));
 }
 
 template <int BN, bool kQuant>
@@ -469,7 +469,7 @@ static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w,
 
 cudaError_t launch_gemm_nvfp4(const CUtensorMap& map_a, const CUtensorMap& map_w, const GemmParams& p, int sm_count,
                               cudaStream_t s) {
-  switch (gemm_tile_n(p.m, p.n)) {
+  switch (gemm_tile_n(p.m, p.n, sm_count)) {
     case 64: return launch_bn<64>(map_a, map_w, p, sm_count, s);
     case 128: return launch_bn<128>(map_a, map_w, p, sm_count, s);
     default: return launch_bn<256>(map_a, map_w, p, sm_count, s);

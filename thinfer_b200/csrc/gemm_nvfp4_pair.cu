@@ -610,18 +610,11 @@ static uint32_t env_u32_pair(const char* name, uint32_t dflt) {
   return v ? uint32_t(strtoul(v, nullptr, 0)) : dflt;
 }
 
-bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k) {
+bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool peers, int sm_count) {
   static uint32_t force = env_u32_pair("TNF_GEMM_KERNEL", 0);  // diagnostic builds: 1 = always 1-CTA, 2 = always pair
   if (force == 1) return false;
   if (force == 2) return true;
-  if (m <= 128u) return false;
-  // A pair works on a 256 x 256 tile (or a half of it), the 1-CTA kernel on 128 x 128 ones: while those fit one wave of CTAs they
-  // occupy more SMs, each for less time. Measured (us, quantiser included, pair in halves against 1-CTA):
-  // 700 x 3072 x 3072 10.6 / 9.5, 300 x 6144 x 3072 12.2 / 9.2, 256 x 9216 x 9216 18.3 / 16.8, 384 x 6144 x 12288 24.8 / 19.2.
-  // In two waves the 1-CTA kernel reads its operands twice as often: only while K is short and the pairs are not filled
-  // either (1024 x 3072 x 1024 9.4 / 8.6, 2048 x 2048 x 2048 11.9 / 11.1, 2048 x 2048 x 4096 15.8 / 15.8, 900 x 2560 x 8192 19.8 / 21.8).
-  const uint64_t tiles1 = uint64_t((m + 127u) / 128u) * ((n + 127u) / 128u), tiles2 = uint64_t((m + 255u) / 256u) * ((n + 255u) / 256u);
-  return tiles1 > 148u && !(k <= 2048u && tiles2 <= 74u);
+  return pair_rule(m, n, k, peers, uint32_t(sm_count));
 }
 
 uint32_t gemm_pair_kblocks() { return 4u; }

@@ -137,12 +137,12 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
   ce = launch_quantize(src, TNF_DTYPE_BF16, a->m, a->k, nullptr, a->a_global, a_codes, a_scales, true, ctx->compute);
   if (ce != cudaSuccess) return cuda_fail(ce, "activation quantise launch");
 
-  const bool pair = gemm_use_pair(a->m, a->n, a->k);
+  const bool pair = gemm_use_pair(a->m, a->n, a->k, false, ctx->sm_count);
   CUtensorMap ma, mw;
   const uint32_t kb = gemm_pair_kblocks();
   const uint32_t box_bytes = pair ? kb * 32 : 128, swz = box_bytes;  // the pair kernel's stage width sets the box
   if (make_tensor_map(&ma, MapSpec{a_codes, 1, a->k / 2, a->m, a->k / 2, box_bytes, 128, swz}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
-  if (make_tensor_map(&mw, MapSpec{w_codes, 1, a->k / 2, a->n, a->k / 2, box_bytes, pair ? 128u : gemm_tile_n(a->m, a->n), swz}) != TNF_OK)
+  if (make_tensor_map(&mw, MapSpec{w_codes, 1, a->k / 2, a->n, a->k / 2, box_bytes, pair ? 128u : gemm_tile_n(a->m, a->n, ctx->sm_count), swz}) != TNF_OK)
     return TNF_ERR_INVALID_ARGUMENT;
   if (pair) {
     CUtensorMap msa, msb, outs[kMaxPeers];

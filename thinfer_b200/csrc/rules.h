@@ -26,6 +26,23 @@ TNF_HD inline uint32_t tile_n_rule(uint32_t m, uint32_t n, uint32_t sms) {
   return tm * ((uint64_t(n) + 127u) / 128u) * 2u <= sms ? 64u : 128u;
 }
 
+// CTA pairs or single CTAs for an NVFP4 linear. A pair works on a 256 x 256 tile (or a half of it), the 1-CTA kernel on 128 x 128
+// ones: while those fit one wave of CTAs they occupy more SMs, each for less time. Measured (us, quantiser included, pair against
+// 1-CTA): 700 x 3072 x 3072 12.2 / 9.5, 300 x 6144 x 3072 12.2 / 9.2, 384 x 6144 x 12288 24.8 / 19.2; 130 shapes of all epilogues
+// 1.42 times as fast in the geometric mean.
+// In two waves the 1-CTA kernel reads its operands twice as often: only while K is short and the pairs are not filled either
+// (1024 x 3072 x 1024 9.4 / 8.6, 2048 x 2048 x 2048 11.9 / 11.1, 2048 x 2048 x 4096 15.8 / 15.8, 900 x 2560 x 8192 19.8 / 21.8).
+// Outputs that are also stored to peers go out in the pair kernel's 128-byte row segments, which NVLink packs well, whenever there
+// are pair tiles for most of the chip.
+TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool peers, uint32_t sms) {
+  if (m <= 128u) return false;
+  const uint64_t tiles1 = ((uint64_t(m) + 127u) / 128u) * ((uint64_t(n) + 127u) / 128u);
+  const uint64_t tiles2 = ((uint64_t(m) + 255u) / 256u) * ((uint64_t(n) + 255u) / 256u);
+  if (peers) return tiles2 >= 32u;
+  if (tiles1 <= sms) return false;
+  return !(tiles2 <= sms / 2u && k <= 2048u);
+}
+
 // Work items of the attention kernel. A (head, batch) pair has ceil(s_q / 128) blocks of 128 query rows; two of them make a tile.
 // An item is a tile (rows mode: one softmax group per block, all keys each) or one block (keys mode: the groups share the keys),
 // which takes about half as long. Items [0, full_items) are tiles, the others the blocks of the tiles that are left and then, where
