@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [
     (700, 3072, 512),    # 144 tiles of 128 x 128: one wave
     (300, 6144, 288),    # 144, ragged rows and K
-    (769, 3072, 2048),   # 168: two waves, short K
+    (769, 3072, 2048),   # 168: two waves, single CTAs where there is no gated residual
+    (513, 4096, 800),    # 160 tiles, the same
+    (513, 4096, 768),    # ... and pairs for a shorter K
     (769, 3072, 2080),   # the same with K past the limit: 48 tiles of 256 x 256 on pairs
     (513, 3200, 2112),   # 3 x 13 pair tiles, a ragged column tile: not halved
     (1280, 2048, 2304),  # 40 pair tiles: not halved (more halves than pairs)

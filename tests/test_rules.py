@@ -12,7 +12,7 @@ SHIM = r"""
 extern "C" {
 uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, rows); }
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
-int pair(uint32_t m, uint32_t n, uint32_t k, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, peers != 0, sms); }
+int pair(uint32_t m, uint32_t n, uint32_t k, int gated, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, gated != 0, peers != 0, sms); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
 int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
   tnf::SdpaPlan p{};
@@ -69,9 +69,20 @@ def test_outputs_to_peers_take_the_pair_kernel(rules):
         for n in (256, 3072, 6144, 9472, 18432):
             for k in (256, 2048, 12288):
                 tiles = -(-m // 256) * -(-n // 256)
-                assert rules.pair(m, n, k, 1, 148) == (m > 128 and tiles >= 32), (m, n, k)
-                differ += rules.pair(m, n, k, 1, 148) != rules.pair(m, n, k, 0, 148)
+                assert rules.pair(m, n, k, 0, 1, 148) == (m > 128 and tiles >= 32), (m, n, k)
+                differ += rules.pair(m, n, k, 0, 1, 148) != rules.pair(m, n, k, 0, 0, 148)
     assert differ > 0
+
+
+@pytest.mark.parametrize("m,n,k,gated,pair", [
+    (700, 3072, 12288, 0, 0), (700, 3072, 12288, 1, 0), (130, 9472, 64, 0, 0),  # one wave of 128 x 128 tiles: single CTAs
+    (893, 3472, 1024, 0, 0), (447, 9408, 2048, 0, 0), (2111, 1520, 1536, 0, 0),  # two waves, K neither short nor long
+    (893, 3472, 1024, 1, 1),                                                     # ... with a gated residual
+    (148, 14608, 288, 0, 1), (2331, 1248, 608, 0, 1), (900, 2560, 8192, 0, 1),   # K short or long
+    (199, 11120, 1024, 0, 1), (4352, 3072, 1024, 0, 1),                          # two rows of tiles; the pairs are filled
+])
+def test_kernel_of_measured_shapes(rules, m, n, k, gated, pair):
+    assert rules.pair(m, n, k, gated, 0, 148) == pair
 
 
 @pytest.mark.parametrize("sms", [148, 7])

@@ -431,7 +431,7 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     return TNF_OK;
   }
   CUtensorMap ma, mw;
-  if (dense || mc_out || gemm_use_pair(a->m, a->n, a->k, p.n_out > 1u, ctx->sm_count)) {  // only the CTA-pair kernel has the dense arm and the multicast epilogue
+  if (dense || mc_out || gemm_use_pair(a->m, a->n, a->k, p.gate != nullptr, p.n_out > 1u, ctx->sm_count)) {  // only the CTA-pair kernel has the dense arm and the multicast epilogue
     const uint32_t kb = gemm_pair_kblocks();
     CUtensorMap msa, msb, outs[kMaxPeers];
     if (dense) {  // bf16 [rows, k]: boxes of 64 elements (128 bytes) x 128 rows, 128-byte swizzle; no scale maps

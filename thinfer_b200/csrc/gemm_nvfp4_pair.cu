@@ -610,11 +610,11 @@ static uint32_t env_u32_pair(const char* name, uint32_t dflt) {
   return v ? uint32_t(strtoul(v, nullptr, 0)) : dflt;
 }
 
-bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool peers, int sm_count) {
+bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool gated, bool peers, int sm_count) {
   static uint32_t force = env_u32_pair("TNF_GEMM_KERNEL", 0);  // diagnostic builds: 1 = always 1-CTA, 2 = always pair
   if (force == 1) return false;
   if (force == 2) return true;
-  return pair_rule(m, n, k, peers, uint32_t(sm_count));
+  return pair_rule(m, n, k, gated, peers, uint32_t(sm_count));
 }
 
 uint32_t gemm_pair_kblocks() { return 4u; }

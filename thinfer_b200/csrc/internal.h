@@ -134,7 +134,7 @@ bool skinny_tc_applies(uint32_t m, uint32_t n, uint32_t k);  // ... and is the f
 cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& p, cudaStream_t s);
 bool gemv_applies(uint32_t m, uint32_t n, uint32_t k);
 cudaError_t launch_gemv_nvfp4(const void* a_bf16, float a_global, const uint8_t* w_codes, const GemmParams& p, cudaStream_t s);
-bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool peers, int sm_count);  // pair_rule in rules.h
+bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool gated, bool peers, int sm_count);  // pair_rule in rules.h
 uint32_t gemm_pair_kblocks();  // 64-element K blocks per pipeline stage of the pair kernel (2 or 4): sets the TMA boxes
 
 // 2-D tensor map description (dim0 is the contiguous one); all maps are built through this.

@@ -137,7 +137,7 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
   ce = launch_quantize(src, TNF_DTYPE_BF16, a->m, a->k, nullptr, a->a_global, a_codes, a_scales, true, ctx->compute);
   if (ce != cudaSuccess) return cuda_fail(ce, "activation quantise launch");
 
-  const bool pair = gemm_use_pair(a->m, a->n, a->k, false, ctx->sm_count);
+  const bool pair = gemm_use_pair(a->m, a->n, a->k, p.gate != nullptr, false, ctx->sm_count);
   CUtensorMap ma, mw;
   const uint32_t kb = gemm_pair_kblocks();
   const uint32_t box_bytes = pair ? kb * 32 : 128, swz = box_bytes;  // the pair kernel's stage width sets the box

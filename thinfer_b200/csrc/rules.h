@@ -30,17 +30,19 @@ TNF_HD inline uint32_t tile_n_rule(uint32_t m, uint32_t n, uint32_t sms) {
 // ones: while those fit one wave of CTAs they occupy more SMs, each for less time. Measured (us, quantiser included, pair against
 // 1-CTA): 700 x 3072 x 3072 12.2 / 9.5, 300 x 6144 x 3072 12.2 / 9.2, 384 x 6144 x 12288 24.8 / 19.2; 130 shapes of all epilogues
 // 1.42 times as fast in the geometric mean.
-// In two waves the 1-CTA kernel reads its operands twice as often: only while K is short and the pairs are not filled either
-// (1024 x 3072 x 1024 9.4 / 8.6, 2048 x 2048 x 2048 11.9 / 11.1, 2048 x 2048 x 4096 15.8 / 15.8, 900 x 2560 x 8192 19.8 / 21.8).
+// In two waves the 1-CTA kernel reads its operands twice as often, and wins only while the pairs are not filled either, K is
+// neither long (900 x 2560 x 8192 19.8 / 21.8) nor short (there a CTA's two epilogues are most of its time: 148 x 14608 x 288
+// 8.1 / 9.2, 2331 x 1248 x 608 9.9 / 10.4), the epilogue reads no residual (186 x 10592 x 1024 10.7 / 11.6) and there are more than
+// two rows of tiles (199 x 11120 x 1024 8.1 / 8.5). Then: 893 x 3472 x 1024 9.4 / 8.4, 447 x 9408 x 2048 with GELU 12.2 / 10.7.
 // Outputs that are also stored to peers go out in the pair kernel's 128-byte row segments, which NVLink packs well, whenever there
 // are pair tiles for most of the chip.
-TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool peers, uint32_t sms) {
+TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool gated, bool peers, uint32_t sms) {
   if (m <= 128u) return false;
   const uint64_t tiles1 = ((uint64_t(m) + 127u) / 128u) * ((uint64_t(n) + 127u) / 128u);
   const uint64_t tiles2 = ((uint64_t(m) + 255u) / 256u) * ((uint64_t(n) + 255u) / 256u);
   if (peers) return tiles2 >= 32u;
   if (tiles1 <= sms) return false;
-  return !(tiles2 <= sms / 2u && k <= 2048u);
+  return !(tiles2 <= sms / 2u && k > 768u && k <= 2048u && m > 256u && !gated);
 }
 
 // Work items of the attention kernel. A (head, batch) pair has ceil(s_q / 128) blocks of 128 query rows; two of them make a tile.
