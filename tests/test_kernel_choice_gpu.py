@@ -217,3 +217,52 @@ def test_last_tile_of_less_than_one_scale_block(backend, m, n, k, forms):
     W.free(be)
     for buf in bufs:
         be.free(buf)
+
+
+@pytest.mark.parametrize("budget", [False, True])
+@pytest.mark.parametrize("n,k", [(2048, 8192), (2112, 2080), (4096, 96)])
+def test_few_rows_in_a_scratch_full_of_others(n, k, budget):
+    """Few rows of activations whose tensor map reaches over the scratch behind them: what an earlier call has left there must not
+    show. With a budget that has no byte to spare the scratch is as large as the operand and the map ends with it."""
+    import thinfer_b200 as T
+    from thinfer_b200.backend import device_scales_bytes
+
+    rng, g, go = np.random.default_rng(k), 0.002, 0.0007
+    big, few = 120, (17, 20, 31)
+    a = O.f32_to_bf16(rng.standard_normal((big, k), np.float32))
+    w = rng.standard_normal((n, k), np.float32) * np.float32(0.05)
+    size = lambda m: m * n * 2
+    fixed = 4 * size(big) + (160 << 20)  # room for the f32 weight while it is quantised
+    be = T.Backend(0, fixed if budget else 0)
+    try:
+        W = T.Nvfp4Weight.from_dense(be, w, O.f32_to_bf16(rng.standard_normal(n, np.float32)))
+        ab, sc = be.upload(a), be.scope()
+        outs = [be.upload(np.full((big, n), 0x7FC0, np.uint16)) for _ in range(2)]
+        sw, codes, scales = be.allocate(size(big) // 2), be.allocate(big * n // 2), be.allocate(device_scales_bytes(big, n))
+        if budget:  # the scratch of 17 rows is the last that fits
+            live = sum(v for key, v in be.mem_snapshot().items() if key.startswith("live"))
+            filler = be.allocate(fixed - live - (17 * k // 2 + device_scales_bytes(17, k)))
+            sc.linear(ab, 17, W, g, outs[0])
+            be.submit(30000)
+            be.free(filler)
+            be.write_buffer(outs[0], np.full((big, n), 0x7FC0, np.uint16))
+        sc.linear(ab, big, W, g, outs[1])
+        be.submit(30000)
+        want = be.read_buffer(outs[1], np.uint16).reshape(big, n)
+        for m in few:
+            sc.linear(ab, m, W, g, outs[0])
+            sc.linear(ab, m, W, g, sw, swiglu=True)
+            sc.linear(ab, m, W, g, None, out_nvfp4=(codes, scales, go))
+            be.submit(30000)
+            got = be.read_buffer(outs[0], np.uint16).reshape(big, n)
+            assert np.array_equal(got[:m], want[:m])
+            assert (got[m:] == 0x7FC0).all()
+            oc, os_ = O.quantize_act(want[:m], go)
+            assert np.array_equal(be.read_buffer(codes)[: m * n // 2].reshape(m, n // 2), oc)
+            assert np.array_equal(dev_scales_to_canonical(be.read_buffer(scales), m, n), os_)
+            f = O.bf16_to_f32(want[:m]).astype(np.float64)
+            ref = f[:, 0::2] / (1.0 + np.exp(-f[:, 0::2])) * f[:, 1::2]
+            assert rel_fro(O.bf16_to_f32(be.read_buffer(sw, np.uint16))[: m * n // 2].reshape(m, n // 2), ref) <= 8e-3  # from bf16-rounded inputs
+            be.write_buffer(outs[0], np.full((big, n), 0x7FC0, np.uint16))
+    finally:
+        be.close()

@@ -13,6 +13,7 @@ extern "C" {
 uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, rows); }
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
 int pair(uint32_t m, uint32_t n, uint32_t k, int gated, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, gated != 0, peers != 0, sms); }
+uint32_t map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) { return tnf::map_rows_rule(m, n, k, room); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
 int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
   tnf::SdpaPlan p{};
@@ -59,6 +60,20 @@ def test_no_tile_copies_scales_past_the_weight(rules):
                         assert block == row // 128
                     past += row // 128 >= blocks
     assert past > 0  # there are shapes here whose last tile hangs over by a whole block
+
+
+def test_map_over_few_rows_stays_inside_the_buffer(rules):
+    for k in (32, 96, 256, 3072, 8192, 8992, 14336, 65536, 262144 + 32, 1 << 20):
+        for m in (1, 16, 17, 31, 32, 100, 128, 5000):
+            need = m * k // 2
+            for room in (0, need, need + k // 2, (128 << 10) + k // 2, 16 << 20, 1 << 40):
+                rows = rules.map_rows(m, 3072, k, C.c_uint64(room))
+                assert rules.map_rows(m, 1024, k, C.c_uint64(room)) == m
+                assert rows >= m
+                assert rows == m or rows * k // 2 <= room
+                assert rows == m or (rows - 1) * k // 2 < 128 << 10  # no taller than it has to be
+                if room >= (128 << 10) + k // 2:
+                    assert rows * k // 2 >= 128 << 10
 
 
 def test_outputs_to_peers_take_the_pair_kernel(rules):

@@ -248,9 +248,11 @@ static int32_t ensure_scratch(tnf_ctx* ctx, uint32_t m, uint32_t k) {
     if (ctx->scratch_codes_id) free_locked(ctx, ctx->scratch_codes_id);
     ctx->scratch_codes_id = 0;
     ctx->scratch_codes_bytes = 0;
-    int32_t st = alloc_locked(ctx, need_codes, TNF_CAT_WORKSPACE, &ctx->scratch_codes_id);
+    // room for a map of full size (map_rows_rule), but not out of a budget that may be planned to the byte
+    const uint64_t bytes = ctx->budget ? need_codes : std::max(need_codes, kSmallMapBytes + k / 2u);
+    int32_t st = alloc_locked(ctx, bytes, TNF_CAT_WORKSPACE, &ctx->scratch_codes_id);
     if (st != TNF_OK) return st;
-    ctx->scratch_codes_bytes = need_codes;
+    ctx->scratch_codes_bytes = bytes;
   }
   if (need_scales > ctx->scratch_scales_bytes) {
     if (ctx->scratch_scales_id) free_locked(ctx, ctx->scratch_scales_id);
@@ -280,7 +282,7 @@ static int32_t ensure_wide(tnf_ctx* ctx, uint64_t bytes) {
 // FP4 x bf16 form, so the activations are widened to bf16 first -- exact: a code times its block scale has at
 // most 6 significant bits -- and the bf16 GEMM applies a_global * w_global in its epilogue.
 static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a_codes, const uint8_t* a_scales,
-                        const uint8_t* a_raw, bool widened);
+                        const uint8_t* a_raw, bool widened, uint64_t a_room = 0);
 static int32_t run_mixed(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a_codes, const uint8_t* a_scales) {
   int32_t st = ensure_wide(ctx, uint64_t(a->m) * a->k * 2);
   if (st != TNF_OK) return st;
@@ -308,10 +310,11 @@ static int32_t check_dims(uint32_t m, uint32_t n, uint32_t k) {
 
 // shared tail of tnf_linear_nvfp4 / tnf_gemm_nvfp4
 // `a_raw` non-null: the skinny-M kernel takes the bf16 activations themselves (its prologue is the quantiser).
+// `a_room`: bytes that may be read from `a_codes` on, where that is more than the operand.
 // `widened`: the dense arm's bf16 activations are the exact image (code x block scale) of NVFP4 activations, so
 // the per-tensor activation scale still has to be applied.
 static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a_codes, const uint8_t* a_scales,
-                        const uint8_t* a_raw, bool widened) {
+                        const uint8_t* a_raw, bool widened, uint64_t a_room) {
   int32_t st = TNF_OK;
   const bool swiglu = (a->flags & TNF_LINEAR_SWIGLU) != 0;
   const uint32_t n_out_cols = swiglu ? a->n / 2 : a->n;  // columns this call writes
@@ -453,7 +456,7 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     TNF_CUDA(launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute), "nvfp4 pair gemm launch");
     return TNF_OK;
   }
-  if (!get_map(ctx, codes_spec(a_codes, a->m, a->k, 128), &ma) ||
+  if (!get_map(ctx, codes_spec(a_codes, map_rows_rule(a->m, a->n, a->k, a_room), a->k, 128), &ma) ||
       !get_map(ctx, codes_spec(w_codes, a->n, a->k, gemm_tile_n(a->m, a->n, ctx->sm_count)), &mw))
     return TNF_ERR_INVALID_ARGUMENT;
   TNF_CUDA(launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute), "nvfp4 gemm launch");
@@ -1103,7 +1106,7 @@ int32_t tnf_linear_nvfp4(tnf_ctx* ctx, const tnf_linear_args* a) {
     return TNF_ERR_INVALID_ARGUMENT;
   }
   return run_gemm(ctx, a, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
-                  static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr, false);
+                  static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr, false, ctx->scratch_codes_bytes);
 }
 
 int32_t tnf_gemm_nvfp4(tnf_ctx* ctx, const tnf_linear_args* a, tnf_buf a_codes, tnf_buf a_scales_device) {

@@ -16,8 +16,8 @@
 //   * the first call on a device looks the array's device address up (cudaGetSymbolAddress with
 //     that device current). Make that first call before any stream capture;
 //   * all calls share the one array and it keeps the previous call's contents. Nothing in it has
-//     to start at zero: the quantiser rewrites every byte the GEMM will read, including the zero
-//     padding of the scale layout, and rows past m are zero-filled by the TMA loads. Two calls
+//     to start at zero: the quantiser rewrites every byte that reaches an output, including the zero
+//     padding of the scale layout; what the TMA loads find in rows past m is not stored. Two calls
 //     whose kernels overlap on the GPU (different streams, different contexts of one device)
 //     race on the array: keep them stream-ordered;
 //   * no cudaMalloc / cudaFree / allocating library routine is called; tensor maps are built on
@@ -141,7 +141,8 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
   CUtensorMap ma, mw;
   const uint32_t kb = gemm_pair_kblocks();
   const uint32_t box_bytes = pair ? kb * 32 : 128, swz = box_bytes;  // the pair kernel's stage width sets the box
-  if (make_tensor_map(&ma, MapSpec{a_codes, 1, a->k / 2, a->m, a->k / 2, box_bytes, 128, swz}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
+  const uint32_t a_rows = pair ? a->m : map_rows_rule(a->m, a->n, a->k, kScratchBytes);
+  if (make_tensor_map(&ma, MapSpec{a_codes, 1, a->k / 2, a_rows, a->k / 2, box_bytes, 128, swz}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
   if (make_tensor_map(&mw, MapSpec{w_codes, 1, a->k / 2, a->n, a->k / 2, box_bytes, pair ? 128u : gemm_tile_n(a->m, a->n, ctx->sm_count), swz}) != TNF_OK)
     return TNF_ERR_INVALID_ARGUMENT;
   if (pair) {
