@@ -38,7 +38,7 @@ def test_scale_of_infinite_and_zero_tensors(backend):
             backend.free(x)
 
 
-@pytest.mark.parametrize("nbytes", [(8 << 20) - 4, 8 << 20, (8 << 20) + 4, (33 << 20) + 12, 100 << 20])
+@pytest.mark.parametrize("nbytes", [(8 << 20) + 4, (24 << 20) - 4, 24 << 20, (24 << 20) + 4, (33 << 20) + 12, 100 << 20])
 def test_large_pageable_writes(backend, nbytes):
     data = np.random.default_rng(nbytes).integers(0, 256, nbytes, np.uint8)
     buf = backend.allocate(nbytes + 64)
@@ -51,7 +51,8 @@ def test_large_pageable_writes(backend, nbytes):
 
 
 def test_large_writes_from_several_threads(backend):
-    datas = [np.random.default_rng(i).integers(0, 256, (12 << 20) + 4 * i, np.uint8) for i in range(4)]
+    """One of them has the pinned slots, the others copy the plain way."""
+    datas = [np.random.default_rng(i).integers(0, 256, (26 << 20) + 4 * i, np.uint8) for i in range(4)]
     bufs = [backend.allocate(d.nbytes) for d in datas]
     threads = [threading.Thread(target=backend.write_buffer, args=(b, d)) for b, d in zip(bufs, datas)]
     for t in threads:

@@ -573,13 +573,15 @@ static int32_t raw_range(tnf_ctx* ctx, uint64_t id, uint64_t off, uint64_t n, co
   return TNF_OK;
 }
 
-// Large writes from pageable memory. A plain copy stages those through one thread (6-8 GB/s); here up to kWriteThreads
-// threads copy into pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the
-// chunks on the compute stream. The slots (kWriteStageBytes in all) are made on first use and freed with the context.
-// Below kWriteStagedMin the threads cost more than they save. Returns false when the caller has to copy the plain way
-// (slots in use by another thread's write, no pinned memory to be had); *err is a failed copy.
-constexpr uint32_t kWriteThreads = 8;
-constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 8u << 20;
+// Large writes from pageable memory. A plain copy stages those through one thread; here up to kWriteThreads threads copy into
+// pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the chunks on the compute
+// stream. Measured (ms, plain / four threads / eight; source in the CPU's caches, then not): 16 MB 0.83 / 0.94 / 1.2 and
+// 1.2 / 1.06 / 1.4; 24 MB 1.24 / 1.15 / 1.65 and 2.1 / 1.25 / 1.9; 48 MB 2.5 / 1.7 / 2.3 and 4.5 / 2.0 / 2.4; 96 MB 8.1 / 2.9 / 3.6
+// and 8.9 / 3.1 / 3.6. Hence four, from kWriteStagedMin on. The slots (kWriteStageBytes in all) are made on first use and freed
+// with the context. Returns false when the caller has to copy the plain way (slots in use by another thread's write, no pinned
+// memory to be had); *err is a failed copy.
+constexpr uint32_t kWriteThreads = 4;
+constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 24u << 20;
 static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n, cudaError_t* err) {
   std::unique_lock<std::mutex> lk(ctx->write_mu, std::try_to_lock);
   if (!lk.owns_lock()) return false;
@@ -637,12 +639,13 @@ int32_t tnf_write(tnf_ctx* ctx, uint64_t id, uint64_t dst_off, const void* src, 
   uint8_t* p = nullptr;
   int32_t st = raw_range(ctx, id, dst_off, n, "tnf_write", &p);
   if (st != TNF_OK) return st;
-  cudaPointerAttributes attr;
-  if (n >= kWriteStagedMin && cudaPointerGetAttributes(&attr, src) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered) {
-    cudaError_t e = cudaSuccess;
-    if (staged_write(ctx, p, static_cast<const uint8_t*>(src), n, &e)) {
-      if (e != cudaSuccess) return cuda_fail(e, "tnf_write staged copy");
-      return TNF_OK;
+  if (n >= kWriteStagedMin) {
+    cudaPointerAttributes attr;
+    cudaError_t e = cudaPointerGetAttributes(&attr, src);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // not the next launch's error
+    } else if (attr.type == cudaMemoryTypeUnregistered && staged_write(ctx, p, static_cast<const uint8_t*>(src), n, &e)) {
+      return e == cudaSuccess ? TNF_OK : cuda_fail(e, "tnf_write staged copy");
     }
   }
   TNF_CUDA(cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, ctx->compute), "tnf_write copy");
