@@ -60,7 +60,8 @@ def test_kernel_choice_does_not_show(backend, m, n, k, kind):
 
 @pytest.mark.parametrize("m,n,k", [(200, 512, 256), (640, 1024, 544), (257, 2304, 256)])  # 2, 12 and 18 pair tiles, all in halves
 def test_halves_in_the_only_wave(backend, m, n, k):
-    """The pair kernel's own epilogues (SwiGLU, dense arm) run on it whatever the size."""
+    """The dense arm runs on the pair kernel whatever the size: its only wave in halves. Beside it, on the 1-CTA kernel: the NVFP4
+    output, the bf16 output of the kernel that makes it, and SwiGLU."""
     import thinfer_b200 as T
     from thinfer_b200 import _lib as L
     from thinfer_b200.backend import device_scales_bytes
@@ -72,7 +73,7 @@ def test_halves_in_the_only_wave(backend, m, n, k):
     ab, y, codes, scales = be.upload(a), be.allocate(m * n * 2), be.allocate(m * n // 2), be.allocate(device_scales_bytes(m, n))
     sw, dense = be.allocate(m * n), be.allocate(m * n * 2)
     sc = be.scope()
-    sc.linear(ab, m, W, g, y)                                      # 1-CTA kernel: the reference bits
+    sc.linear(ab, m, W, g, y)
     y2 = be.allocate(m * n * 2)
     sc.linear(ab, m, W, g, y2, out_nvfp4=(codes, scales, 0.001))
     sc.linear(ab, m, W, g, sw, swiglu=True)

@@ -14,6 +14,7 @@ uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, 
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
 int pair(uint32_t m, uint32_t n, uint32_t k, int gated, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, gated != 0, peers != 0, sms); }
 uint32_t map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) { return tnf::map_rows_rule(m, n, k, room); }
+uint32_t whole_tiles(uint32_t tiles, uint32_t n, uint32_t pairs, int remote) { return tnf::pair_whole_tiles(tiles, n, pairs, remote != 0); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
 int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
   tnf::SdpaPlan p{};
@@ -74,6 +75,19 @@ def test_map_over_few_rows_stays_inside_the_buffer(rules):
                 assert rows == m or (rows - 1) * k // 2 < 128 << 10  # no taller than it has to be
                 if room >= (128 << 10) + k // 2:
                     assert rows * k // 2 >= 128 << 10
+
+
+def test_halves_of_pair_tiles(rules):
+    """No more items than pairs in the last wave, no empty half, and no halves in the only wave of an output that goes to other GPUs."""
+    for pairs in (74, 3):
+        for tiles in range(1, 4 * pairs + 1):
+            for n in (256, 3072, 3080):
+                for remote in (0, 1):
+                    whole = rules.whole_tiles(tiles, n, pairs, remote)
+                    halves = 2 * (tiles - whole)
+                    assert whole == tiles or (n % 256 == 0 and whole % pairs == 0 and 0 < halves <= pairs)
+                    if tiles <= pairs:
+                        assert (whole == tiles) == (bool(remote) or n % 256 != 0 or 2 * tiles > pairs)
 
 
 def test_outputs_to_peers_take_the_pair_kernel(rules):

@@ -667,10 +667,8 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
   if (a_bytes > band_bytes && w_bytes <= kBandMaxW)
     p.band_m = uint32_t(std::min<uint64_t>(p.tiles_m, std::max<uint64_t>(1u, band_bytes / (row_bytes * 256u))));
   const uint32_t avail = uint32_t(max_pairs[dev] > 0 ? max_pairs[dev] : sm_count / 2);
-  const uint32_t tail = tiles % avail;
-  // split the last (or only) wave's tiles into halves when every half then finds a pair of its own (and no half is empty); alone in
-  // their wave: 700 x 3072 x 3072 12.2 -> 10.6 us, 512 x 4096 x 12288 24.7 -> 21.2
-  p.full_tiles = (tail > 0 && 2u * tail <= avail && p.n % 256u == 0u && !(kDiag && (diag & 2048u))) ? tiles - tail : tiles;
+  const bool remote = p.n_out > 1u || p.out_mc || p.q_codes_mc;
+  p.full_tiles = kDiag && (diag & 2048u) ? tiles : pair_whole_tiles(tiles, p.n, avail, remote);
   const uint32_t items = p.full_tiles + (tiles - p.full_tiles) * 2u;
   const uint32_t pairs = std::min<uint32_t>(items, avail);
   PairOutMaps om;

@@ -58,6 +58,16 @@ TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool gated, boo
   return !(tiles2 <= sms / 2u && k > 768u && k <= 2048u && m > 256u && !gated);
 }
 
+// Tiles that the pair kernel takes whole; each later one runs as two halves of 128 columns. The last wave's are split when every half
+// then finds a pair of its own (and none is empty). An only wave is split as well: the dense arm (FP4 calls of so few tiles take
+// the 1-CTA kernel) 256 x 3072 x 3072 18.7 -> 11.7 us, 700 x 3072 x 3072 19.0 -> 14.6, 512 x 4096 x 12288 61.4 -> 50.3,
+// 2048 x 1024 x 4096 23.6 -> 17.1. Not with stores to other GPUs, whose row segments a half would shorten (not measured).
+TNF_HD inline uint32_t pair_whole_tiles(uint32_t tiles, uint32_t n, uint32_t pairs, bool remote) {
+  const uint32_t tail = tiles % pairs;
+  const bool split = tail > 0u && 2u * tail <= pairs && n % 256u == 0u && !(remote && tiles <= pairs);
+  return split ? tiles - tail : tiles;
+}
+
 // Work items of the attention kernel. A (head, batch) pair has ceil(s_q / 128) blocks of 128 query rows; two of them make a tile.
 // An item is a tile (rows mode: one softmax group per block, all keys each) or one block (keys mode: the groups share the keys),
 // which takes about half as long. Items [0, full_items) are tiles, the others the blocks of the tiles that are left and then, where
