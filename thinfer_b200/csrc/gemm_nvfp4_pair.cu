@@ -654,12 +654,13 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
   const uint32_t tiles = p.tiles_m * p.tiles_n;
   if (tiles == 0) return cudaSuccess;
   // Order of the tiles. Down a column of row tiles, then the next column: W is read once, and A once per wave or column from L2
-  // while A stays there. An A that does not comes from HBM every time: 26520 x 14336 x 3072 read 214 MB twelve times, 4.4 TB/s
-  // under the GEMM, which also costs clock at the power limit. So the rows go in bands: A is read once, W once per band
-  // unless it stays in L2 beside the band (kSmallW; then low bands, with 8 MB 1 % faster than with 12 and 6 % than with 24).
-  // A W of up to kBandMaxW is worth a second reading only in bands as high as L2 allows (4352 x 12288 x 3072 in bf16:
-  // 235.8 -> 232.5 us). Measured (us), one column after the other against bands: 26520 x 14336 x 3072 790-835 -> 612,
-  // 26520 x 3072 x 14336 with GELU 608 -> 557, 6630 x 14336 x 3072 172 -> 164.
+  // while A stays there. An A that does not comes from HBM every time: M x N x K = 26520 x 3072 x 14336 reads its 214 MB twelve
+  // times, 3.3 TB/s under the GEMM, which also costs clock at the power limit. So the rows go in bands: A is read once, W once per
+  // band unless it stays in L2 beside the band (kSmallW; then low bands, with 8 MB 1 % faster than with 12 and 6 % than with 24).
+  // A W of up to kBandMaxW is worth a second reading only in bands as high as L2 allows. Measured (us), one column after the
+  // other against bands: W in L2 26520 x 3072 x 14336 790-835 -> 612, 26520 x 14336 x 3072 with GELU 608 -> 557, 6630 x 3072 x 14336
+  // 172 -> 164; high bands 26520 x 8192 x 12288 1310-1430 -> 1155-1205, 16384 x 9216 x 12288 860-950 -> 775-815, in bf16
+  // 8192 x 3072 x 9216 321 -> 300, 8192 x 4096 x 8192 360 -> 339, 4352 x 3072 x 12288 213 -> 210.
   const uint64_t row_bytes = kDense ? uint64_t(p.k) * 2u : uint64_t(p.k) * 9u / 16u;
   const uint64_t a_bytes = row_bytes * p.m, w_bytes = row_bytes * p.n;
   const uint64_t band_bytes = w_bytes <= kSmallW ? kBandSmallW : kBandLargeW;
