@@ -924,7 +924,8 @@ static int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, u
       slot = __builtin_ctzll(ctx->scale_free);
       ctx->scale_free &= ctx->scale_free - 1u;
     }
-    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->compute);
+    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->sm_count,
+                          ctx->compute);
     if (e == cudaSuccess) {
       what = "quantise launch";
       e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute);

@@ -111,7 +111,7 @@ struct GemmParams {
 };
 
 // words: {amax bits (0 between launches), scale g, 1/(6g), block counter (0 between launches)}; host_g: mapped host word or null
-cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, cudaStream_t s);
+cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, int sm_count, cudaStream_t s);
 cudaError_t launch_quantize(const void* src, int dtype, uint32_t rows, uint32_t k, const float* g_ptr, float g_val,
                             uint8_t* codes, uint8_t* scales, bool device_layout, cudaStream_t s);
 cudaError_t launch_multicast_copy(const uint8_t* src, uint8_t* dst_mc, uint64_t bytes, int sm_count, cudaStream_t s);

@@ -218,9 +218,10 @@ cudaError_t launch_dequant_dense(const uint8_t* codes, const uint8_t* scales_dev
   return cudaGetLastError();
 }
 
-cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, cudaStream_t s) {
+cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, int sm_count, cudaStream_t s) {
   const uint64_t n_vec = n / (dtype == 1 ? 8 : 4);  // rows are whole 32-element groups
-  const unsigned blocks = unsigned(std::min<uint64_t>(std::max<uint64_t>(1, (n_vec + kAmaxThreads * kAmaxLoads - 1) / (kAmaxThreads * kAmaxLoads)), 148ull * 4));
+  const uint64_t per_block = kAmaxThreads * kAmaxLoads, resident = uint64_t(sm_count) * 4u;
+  const unsigned blocks = unsigned(std::min(std::max<uint64_t>(1, (n_vec + per_block - 1) / per_block), resident));
   const uint4* v = static_cast<const uint4*>(x);
   return dtype == 1 ? launch_pdl(amax_scale_kernel<__nv_bfloat16>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g)
                     : launch_pdl(amax_scale_kernel<float>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g);
