@@ -603,8 +603,8 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     return TNF_ERR_INVALID_ARGUMENT;
   }
   const uint64_t q_rows = uint64_t(a->b) * a->s_q, k_rows = uint64_t(a->b) * a->s_k;
-  if (q_rows >= (1ull << 31) || k_rows >= (1ull << 31) || uint64_t(a->s_q + 127u) / 128u > 0x7FFFFFFFull || a->h_q > 65535u || a->b > 65535u) {
-    set_error("tnf_sdpa: problem too large for the grid (b*s < 2^31, h_q and b <= 65535)");
+  if (q_rows >= (1ull << 31) || k_rows >= (1ull << 31) || a->h_q > 65535u || a->b > 65535u) {
+    set_error("tnf_sdpa: problem too large (b * s_q and b * s_k below 2^31, h_q and b up to 65535)");
     return TNF_ERR_INVALID_ARGUMENT;
   }
   int32_t st = TNF_OK;
@@ -676,7 +676,7 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
   }
   if (!sdpa_plan(a->s_q, uint64_t(a->h_q) * a->b, uint32_t(ctx->sm_count), &p.plan)) {
-    set_error("tnf_sdpa: problem too large for the grid (b=%u s_q=%u h_q=%u)", a->b, a->s_q, a->h_q);
+    set_error("tnf_sdpa: problem too large (b=%u s_q=%u h_q=%u: more than 2^31 work items)", a->b, a->s_q, a->h_q);
     return TNF_ERR_INVALID_ARGUMENT;
   }
   cudaError_t e = launch_pdl(sdpa_kernel, dim3(p.plan.ctas), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
