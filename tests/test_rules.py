@@ -68,7 +68,7 @@ def test_map_over_few_rows_stays_inside_the_buffer(rules):
         for m in (1, 16, 17, 31, 32, 100, 128, 5000):
             need = m * k // 2
             for room in (0, need, need + k // 2, (128 << 10) + k // 2, 16 << 20, 1 << 40):
-                rows = rules.map_rows(m, 3072, k, C.c_uint64(room))
+                rows = rules.map_rows(m, 4096, k, C.c_uint64(room))
                 assert rules.map_rows(m, 1024, k, C.c_uint64(room)) == m
                 assert rows >= m
                 assert rows == m or rows * k // 2 <= room

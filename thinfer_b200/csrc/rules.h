@@ -29,11 +29,12 @@ TNF_HD inline uint32_t tile_n_rule(uint32_t m, uint32_t n, uint32_t sms) {
 // Rows of the 1-CTA GEMM's tensor map over its packed activations ([m, k / 2] bytes). When many CTAs load through a map of less
 // than 128 KB the loads are slow (K = 8192, N = 9216: 18.1 us for 31 rows, 11.3 for 32). Where there is `room` behind the operand
 // the map reaches over it up to that size; the rows past m are loaded, multiplied and not stored. Measured (us, without / with):
-// 16 x 9216 x 14336 SwiGLU 28.3 / 15.6, 1 x 16384 x 8192 22.0 / 13.3, 20 x 4096 x 12288 19.1 / 13.9. A few CTAs only have the more
-// rows to load: 38 x 304 x 2272 6.5 / 7.0, 1 x 1024 x 8992 11.7 / 12.4.
+// 16 x 9216 x 14336 SwiGLU 28.3 / 15.6, 1 x 16384 x 8192 22.0 / 13.3, 11 x 4096 x 4096 9.6 / 7.6, 11 x 2048 x 3072 7.0 / 6.8. A few
+// CTAs only have the more rows to load, which cost more when they do not start on 128-byte lines: 38 x 304 x 2272 6.5 / 7.0,
+// 11 x 2560 x 3168 7.5 / 8.2, 11 x 3584 x 3168 8.8 / 8.3.
 constexpr uint64_t kSmallMapBytes = 128u << 10;
 TNF_HD inline uint32_t map_rows_rule(uint32_t m, uint32_t n, uint32_t k, uint64_t room) {
-  if (n < 2048u) return m;
+  if (n < (k % 256u ? 3584u : 2048u)) return m;
   const uint64_t row = k / 2u, want = (kSmallMapBytes + row - 1u) / row, fit = room / row;
   const uint64_t rows = want < fit ? want : fit;
   return rows > m ? uint32_t(rows) : m;
