@@ -1,5 +1,5 @@
-"""The warp-per-row form of tnf_norm_modulate_quantize (ten rows per SM and more, up to 3072 columns), on the checks of
-test_norm_quant_gpu.py: the bf16 result against the CPU restatement (row sums in another order), the NVFP4 copy bit for bit
+"""The warp-per-row form of tnf_norm_modulate_quantize (about ten rows per SM and more, up to 3072 columns; the shape (2369, 2048)
+is just past it, in a second round of rows that is nearly empty), on the checks of test_norm_quant_gpu.py: the bf16 result against the CPU restatement (row sums in another order), the NVFP4 copy bit for bit
 against the oracle quantiser on the kernel's own bf16 output."""
 import numpy as np
 import pytest
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 # one block per row; a lane short of a warp, a warp, one more; every count of blocks per lane; 1, 2 and 3 rows per warp
 @pytest.mark.parametrize("m,k", [(1480, 16), (1481, 496), (1500, 512), (1487, 528), (1600, 1040), (2369, 2048), (2400, 2064),
-                                 (1999, 2576), (4737, 3056), (4352, 3072)])
+                                 (1999, 2576), (4737, 3056), (4352, 3072), (1554, 3072), (2724, 2048), (2800, 2064)])
 @pytest.mark.parametrize("mod", [True, False])
 def test_warp_per_row(backend, m, k, mod):
     x, s, t = _inputs(m, k, m + k)

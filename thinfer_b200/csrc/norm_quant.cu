@@ -317,13 +317,20 @@ extern "C" int32_t tnf_norm_modulate_quantize(tnf_ctx* ctx, const tnf_norm_quant
     e = cudaMemsetAsync(scales + full, 0, sbytes - full, ctx->compute);
     if (e != cudaSuccess) return cuda_fail(e, "out_scales clear");
   }
-  // A warp per row once every SM has about ten rows to itself, for rows that a lane can hold (k <= 3072; at 4096 it spills).
+  // A warp per row once every SM has about ten rows to itself, for rows that a lane can hold (k <= 3072; at 4096 it spills). Not for
+  // a second round of rows that is less than 15 % full: the warps then have two rows each at half the occupancy. (Up to 1024
+  // columns, and at five blocks a lane, where a fifth of the other kernel's threads idle, they are the faster ones all the same.)
   // Measured (us, CTA per row against warp per row), k = 3072: 500 rows 7.5 / 8.2, 1000 rows 8.2 / 8.2, 2000 rows 12.3 / 10.3,
   // 4352 rows 16.1 / 12.4, 26520 rows 92 / 62; k = 1024: 1000 rows 7.4 / 7.7, 4352 rows 7.1 / 5.5; k = 4096: 4352 rows 19.8 / 21.0.
+  // At the edges, k = 3072: 1480 rows 7.9 / 8.15, 1550 8.3 / 8.1, 2368 10.9 / 9.6, 2500 11.2 / 11.6, 2800 12.5 / 11.7; k = 2304: 2500 rows
+  // 10.3 / 9.8; k = 512: 1480 rows 8.05 / 6.3, 2500 8.4 / 7.8.
   const uint32_t warp_blocks = (nb_grid + 31u) / 32u;  // 16-element blocks per lane
-  if (!a->parity_mode && warp_blocks <= 6u && a->m >= 10u * uint32_t(ctx->sm_count)) {
+  const uint32_t per_cta = kWarpRowThreads / 32, resident = uint32_t(ctx->sm_count) * kWarpRowCtas * per_cta;
+  const uint64_t rows = a->m;
+  const bool wide = warp_blocks > 2u, few = 2u * rows < (wide ? 21u : 20u) * uint32_t(ctx->sm_count);
+  const bool thin_round = wide && warp_blocks != 5u && rows > resident && 20u * rows < 23u * uint64_t(resident);
+  if (!a->parity_mode && warp_blocks <= 6u && !few && !thin_round) {
     const float inv_t = 1.0f / (6.0f * a->out_global);
-    const uint32_t per_cta = kWarpRowThreads / 32, resident = uint32_t(ctx->sm_count) * kWarpRowCtas * per_cta;
     const uint32_t rounds = (a->m + resident - 1u) / resident, warps = (a->m + rounds - 1u) / rounds;
     auto launch = [&](auto kernel) {
       return launch_pdl(kernel, dim3((warps + per_cta - 1u) / per_cta), dim3(kWarpRowThreads), sc ? size_t(a->k) * 8u : 0, ctx->compute,
