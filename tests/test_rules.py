@@ -13,6 +13,7 @@ extern "C" {
 uint32_t row_block(uint32_t row, uint32_t rows) { return tnf::sf_row_block(row, rows); }
 uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(m, n, sms); }
 int pair(uint32_t m, uint32_t n, uint32_t k, int gated, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, gated != 0, peers != 0, sms); }
+int own_epilogue(uint32_t k, int dense, int gelu, int q, uint32_t tiles, uint32_t pairs) { return tnf::pair_epilogue_rule(k, dense != 0, gelu != 0, q != 0, tiles, pairs); }
 uint32_t map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) { return tnf::map_rows_rule(m, n, k, room); }
 uint32_t whole_tiles(uint32_t tiles, uint32_t n, uint32_t pairs, int remote) { return tnf::pair_whole_tiles(tiles, n, pairs, remote != 0); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
@@ -75,6 +76,14 @@ def test_map_over_few_rows_stays_inside_the_buffer(rules):
                 assert rows == m or (rows - 1) * k // 2 < 128 << 10  # no taller than it has to be
                 if room >= (128 << 10) + k // 2:
                     assert rows * k // 2 >= 128 << 10
+
+
+def test_epilogue_of_the_pair_kernel(rules):
+    own = lambda k, dense=0, gelu=0, q=0, tiles=148, pairs=74: bool(rules.own_epilogue(k, dense, gelu, q, tiles, pairs))
+    assert own(2047) and not own(2048) and own(511, dense=1) and not own(512, dense=1)
+    assert own(3583, gelu=1) and not own(3584, gelu=1) and own(895, dense=1, gelu=1) and not own(896, dense=1, gelu=1)
+    assert own(3071, q=1) and not own(3072, q=1) and own(1 << 20, gelu=1, q=1)
+    assert own(1 << 30, dense=1, tiles=147)  # less than two waves: the last epilogue shows whatever K is
 
 
 def test_halves_of_pair_tiles(rules):

@@ -235,10 +235,6 @@ static MapSpec scales_spec(const void* base, uint32_t rows, uint32_t k, uint32_t
 static MapSpec pair_codes_spec(const void* base, uint32_t rows, uint32_t k, uint32_t kb) {
   return MapSpec{base, 1, k / 2, rows, k / 2, kb * 32, 128, kb * 32};
 }
-// bf16 output window [m, n] with leading dimension ldo: box {64 columns, 32 rows}, 128-byte swizzle
-static MapSpec out_spec(const void* base, uint32_t m, uint32_t n, uint32_t ldo) {
-  return MapSpec{base, 2, n, m, uint64_t(ldo) * 2, 64, 32, 1};
-}
 
 static int32_t ensure_scratch(tnf_ctx* ctx, uint32_t m, uint32_t k) {
   uint64_t need_codes = uint64_t(m) * (k / 2), need_scales = sf_device_bytes(m, k);
@@ -448,11 +444,11 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     for (uint32_t d = 0; d < p.n_out; ++d) {
       // without a bf16 destination the map is never used; any valid one fills the slot
       if (!store_bf16) outs[d] = ma;
-      else if (swiglu) {  // n/2 output columns; boxes of 32 columns x 32 rows, dense 64-byte rows in shared memory
-        if (!get_map(ctx, MapSpec{p.out[d] + a->n_offset, 2, n_out_cols, a->m, uint64_t(ldo) * 2, 32, 32, 0}, &outs[d])) return TNF_ERR_INVALID_ARGUMENT;
-      } else if (!get_map(ctx, out_spec(p.out[d] + a->n_offset, a->m, a->n, ldo), &outs[d])) return TNF_ERR_INVALID_ARGUMENT;
+      else if (!get_map(ctx, pair_out_spec(p.out[d] + a->n_offset, a->m, n_out_cols, ldo, swiglu), &outs[d])) return TNF_ERR_INVALID_ARGUMENT;
     }
     for (uint32_t d = p.n_out; d < kMaxPeers; ++d) outs[d] = outs[0];
+    // the kernel of a local output reads the residual as it writes the output; the map takes the slot of the first peer
+    if (p.n_out == 1u && p.gate && !get_map(ctx, pair_out_spec(p.residual, a->m, a->n, a->n), &outs[1])) return TNF_ERR_INVALID_ARGUMENT;
     TNF_CUDA(launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute), "nvfp4 pair gemm launch");
     return TNF_OK;
   }
@@ -891,7 +887,7 @@ int32_t tnf_selftest_stalled_wait(tnf_ctx* ctx) {
             make_tensor_map(&mw, pair_codes_spec(base + codes, n, k, kb)) == TNF_OK &&
             make_tensor_map(&msa, scales_spec(p.sfa, m, k, kb)) == TNF_OK &&
             make_tensor_map(&msb, scales_spec(p.sfb, n, k, kb)) == TNF_OK &&
-            make_tensor_map(&outs[0], out_spec(p.out[0], m, n, n)) == TNF_OK;
+            make_tensor_map(&outs[0], pair_out_spec(p.out[0], m, n, n)) == TNF_OK;
   if (ok) {
     for (int d = 1; d < kMaxPeers; ++d) outs[d] = outs[0];
     e = launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute);

@@ -8,13 +8,13 @@
 // 38 KB, which is what lets five stages cover the load latency. No TMA multicast is used:
 // the only cluster-wide operations are tcgen05.commit arrivals and remote mbarrier arrivals.
 //
-// Per CTA, 320 threads:
+// Per CTA, 320 threads (576 with the NVFP4 output):
 //   warp 0     TMA producer (tensor-map loads of A, W-half, the CTA's scale atoms of A and the
 //              scale atoms of the whole W tile; bytes are counted on the LEADER's stage barrier)
 //   warp 1     TMEM owner; in the leader one lane issues scale copies smem->TMEM and MMAs for
 //              both CTAs, frees stages in both CTAs with a multicast commit
-//   warps 2-9  epilogue: TMEM -> registers -> alpha/bias/GELU/gated residual -> bf16 -> swizzled
-//              shared staging -> TMA store (one store per destination: local output and peers)
+//   the others epilogue (8 warps, 16 for the NVFP4 output): TMEM -> registers -> alpha/bias/GELU/gated
+//              residual/SwiGLU -> bf16 -> swizzled shared staging -> TMA store; NVFP4 codes and scales from registers
 // TMEM (512 columns): two 256-column accumulators at columns 0 and 192 that overlap in
 // [192,256); the epilogue reads the overlapping 64 columns first and then releases the next
 // tile's MMA, so the drain of tile i runs under the main loop of tile i+1. Scale factors sit
@@ -33,15 +33,17 @@
 namespace tnf {
 
 namespace pair {
-constexpr int kThreads = 320;  // producer warp, MMA warp, 8 epilogue warps
-// Which warps take which role. The epilogue warp with index e reads TMEM lane quarter (warp id & 3).
-#ifdef TNF_ROLES_LAST  // experiment: producer and MMA issuer in the last two warps instead of the first two
-constexpr int kProducerWarp = 8, kMmaWarp = 9, kFirstEpilogueWarp = 0;
-#else
 constexpr int kProducerWarp = 0, kMmaWarp = 1, kFirstEpilogueWarp = 2;
-#endif
+// What a kernel does with the results. The first four have one local output each (all four in one kernel: 440 bytes of spilled
+// registers); kGeneral covers every combination: peer windows, the multicast alias, bf16 and NVFP4 at once, and the calls that
+// pair_epilogue_rule leaves to it.
+enum Epilogue : int { kPlain, kGated, kQuantised, kSwiglu, kGeneral };
+// Epilogue warps: the quantiser's long chains of dependent operations need sixteen to overlap (GELU + NVFP4 output, 9472 x 4096 x 512:
+// 39.1 us with eight, 30.0 with sixteen), the others are as fast with eight.
+constexpr int epilogue_warps(int epi) { return epi == kQuantised ? 16 : 8; }
+constexpr int threads(int epi) { return 64 + 32 * epilogue_warps(epi); }  // producer warp, MMA warp, epilogue warps
 constexpr int kStagingBytes = 8 * 4096;  // 8 epilogue warps x (32 rows x 128 B)
-constexpr int kBiasBytes = 8 * 256;      // 8 epilogue warps x 64 f32 bias values (the column group being processed)
+constexpr int kBiasBytes = 8 * 384;      // 8 epilogue warps x 64 f32 bias and 64 bf16 gate values (the column group being processed)
 constexpr int kLutBytes = 512;           // 1/(scale*g) per E4M3 code for the quantising epilogue
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kAccStride = 192;  // accumulator b starts at column b * 192
@@ -148,20 +150,6 @@ __device__ __forceinline__ void epilogue_pair_math(const uint32_t (&r)[64], cons
   }
 }
 
-// SwiGLU pairwise gating (thinfer-core/src/ops/silu_mul.rs: out = silu(a) * b, silu(v) = v / (1 + exp(-v))) on a
-// GEMM over the row-interleaved weight [W1 row 0, W3 row 0, W1 row 1, ...]: accumulator columns 2j and 2j+1 are
-// a[j] and b[j], one output column. One warp's 32 rows x 64 accumulator columns -> 32 bf16 per row, staged as
-// dense 64-byte rows (no swizzle) for a 32-column TMA store. Chain mode rounds a and b to bf16 first, as the
-// reference's two matmul dispatches do.
-template <bool kChain>
-__device__ __forceinline__ void epilogue_pair_swiglu(const uint32_t (&r)[64], const GemmParams& p, uint8_t* buf_gen,
-                                                     const float* bias_smem, int lane) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    *reinterpret_cast<uint2*>(buf_gen + lane * 64 + j * 8) = swiglu8<kChain>(&r[j * 8], p.alpha, bias_smem + j * 8);
-  }
-}
-
 __device__ __forceinline__ void epilogue_pair_dispatch(uint32_t mode, const uint32_t (&r)[64], const GemmParams& p,
                                                        uint32_t row, uint32_t ncol0, uint8_t* buf_gen, const float* bias_smem,
                                                        const float* lut, int lane, uint8_t* stage_q, uint32_t gq) {
@@ -178,10 +166,147 @@ __device__ __forceinline__ void epilogue_pair_dispatch(uint32_t mode, const uint
     case 8: epilogue_pair_math<false, false, false, true>(r, p, row, ncol0, buf_gen, bias_smem, lut, lane, stage_q, gq); break;
     case 9: epilogue_pair_math<true, false, false, true>(r, p, row, ncol0, buf_gen, bias_smem, lut, lane, stage_q, gq); break;
     case 10: epilogue_pair_math<false, true, false, true>(r, p, row, ncol0, buf_gen, bias_smem, lut, lane, stage_q, gq); break;
-    case 12: epilogue_pair_swiglu<false>(r, p, buf_gen, bias_smem, lane); break;
-    case 13: epilogue_pair_swiglu<true>(r, p, buf_gen, bias_smem, lane); break;
     default: epilogue_pair_math<true, true, false, true>(r, p, row, ncol0, buf_gen, bias_smem, lut, lane, stage_q, gq); break;
   }
+}
+
+// ---- epilogue of a single local output -------------------------------------------------------------------------------------
+// A tile with a short K is bound by its epilogue, and that by latency: accumulator -> registers -> arithmetic -> staging -> store,
+// one after the other. So a warp takes its 32 rows (a lane each) 32 columns at a time: while one chunk's arithmetic runs, the next
+// one's accumulator is on its way to registers and the group before leaves by TMA; bias, gate and residual are asked for a tile ahead.
+// The residual comes by TMA into the buffer that the result then takes (a lane's own loads touch 32 rows an instruction:
+// 10 000 of a tile's 11 000 cycles). 32-byte stores from registers instead of TMA stores, for the same reason: 19.8 -> 26.8 us.
+// Measured, kGeneral's epilogue -> this one (us, 9472 x 4096 x K): gated residual K = 512 53.7 -> 39.2, 3072 65 -> 56, 4096 73 -> 70;
+// GELU + NVFP4 512 37.7 -> 28.9, 2048 43.6 -> 36.9; NVFP4 512 29.5 -> 22.6; SwiGLU 512 32.0 -> 22.2, 3072 44.5 -> 42.9; GELU 512
+// 30.1 -> 25.9; plain 256 19.9 -> 17.9.
+struct PairShare {
+  uint32_t t_addr;   // TMEM address of the warp's lanes, column 0 of the accumulator
+  uint32_t g[2];     // its groups in drain order
+  uint32_t n0, row0; // first output column of the tile, first row of the warp
+  uint32_t live[2];  // the group has rows and columns that exist
+  uint32_t acc_free; // barrier to arrive on when the first group is in registers; 0: arrived before
+  uint32_t bias[2], gate[2];  // bf16 pairs: columns 2 lane, 2 lane + 1 of either group
+};
+
+// Accumulator registers of 32 columns -> bf16 vectors o[] (with SwiGLU 16 columns: o[0], o[1]); `cw` / return: the chunk's NVFP4
+// codes and its two scale bytes.
+// SwiGLU (thinfer-core/src/ops/silu_mul.rs: out = silu(a) * b) is a GEMM over the row-interleaved weight [W1 row 0, W3 row 0, W1 row
+// 1, ...]: accumulator columns 2j and 2j+1 are a[j] and b[j], one output column.
+template <bool kGelu, bool kChain, bool kGate, bool kQuant, bool kSwiglu>
+__device__ __forceinline__ uint32_t epilogue_chunk(const uint32_t (&r)[32], const GemmParams& p, const float* bias, const uint4* gate,
+                                                   const uint4 (&res)[4], const float* lut, uint4 (&o)[4], uint32_t* cw) {
+  const float alpha = (kGelu && !kChain) ? 0.5f * p.alpha : p.alpha;  // the fused GELU works on x/2
+  uint32_t sw = 0;
+  if constexpr (kSwiglu) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint2 a = swiglu8<kChain>(&r[j * 16], alpha, bias + j * 16), b = swiglu8<kChain>(&r[j * 16 + 8], alpha, bias + j * 16 + 8);
+      o[j] = make_uint4(a.x, a.y, b.x, b.y);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = epilogue8<kGelu, kChain, kGate>(&r[j * 8], alpha, bias + j * 8, kGate ? gate[j] : make_uint4(0, 0, 0, 0),
+                                             kGate ? res[j] : make_uint4(0, 0, 0, 0));
+    if constexpr (kQuant) {  // the bf16-rounded values, two blocks of 16
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const uint32_t w[8] = {o[2 * b].x, o[2 * b].y, o[2 * b].z, o[2 * b].w, o[2 * b + 1].x, o[2 * b + 1].y, o[2 * b + 1].z, o[2 * b + 1].w};
+        sw |= quant_block16_bf16(w, lut, p.q_inv_t, cw[2 * b], cw[2 * b + 1]) << (8 * b);
+      }
+    }
+  }
+  return sw;
+}
+
+// `load_residual` (lane 0; gated residual) asks for a group's residual: this tile's second, then (`more`) the next tile's first.
+template <int kGroups, bool kGelu, bool kChain, bool kGate, bool kQuant, bool kSwiglu, typename LoadResidual>
+__device__ __forceinline__ bool epilogue_pair_local(const GemmParams& p, const PairShare& t, const CUtensorMap* out_map, uint32_t buf,
+                                                    uint8_t* buf_gen, float* bias_smem, const float* lut, int lane, uint32_t bar_res,
+                                                    uint32_t& res_uses, volatile uint32_t* abort_flag, long long wait_limit,
+                                                    LoadResidual&& load_residual, bool more) {
+  const float bias_mul = (kGelu && !kChain) ? 0.5f : 1.0f;  // the fused GELU works on x/2
+  uint4* gate_smem = reinterpret_cast<uint4*>(bias_smem + 64);
+  uint32_t r0[32], r1[32];
+  tmem_ld_32x32b_x32(t.t_addr + t.g[0] * 64u, r0);
+  tmem_ld_32x32b_x32(t.t_addr + t.g[0] * 64u + 32u, r1);
+  tmem_ld_wait();
+  if (t.acc_free) {  // the columns that overlap the other accumulator are in registers: the next tile's MMA may start
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(t.acc_free);
+  }
+#pragma unroll (kGate ? 2 : 1)
+  for (uint32_t half = 0; half < uint32_t(kGroups); ++half) {
+    const uint32_t nc = t.n0 + (half ? t.g[1] : t.g[0]) * 64u;
+    const bool live = (half ? t.live[1] : t.live[0]) != 0u;  // warp-uniform
+    uint4 o[4];
+    uint32_t cw[8], sw = 0;
+    auto vec = [&](int j) { return reinterpret_cast<uint4*>(buf_gen + (kSwiglu ? lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4) : lane * 128 + ((j ^ (lane & 7)) << 4))); };
+    auto chunk = [&](const uint32_t(&r)[32], int c) {
+      uint4 res[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) res[j] = kGate ? *vec(c * 4 + j) : make_uint4(0, 0, 0, 0);
+      const uint32_t s2 = epilogue_chunk<kGelu, kChain, kGate, kQuant, kSwiglu>(r, p, bias_smem + c * 32, gate_smem + c * 4, res, lut, o, &cw[c * 4]);
+      if (kQuant) sw |= s2 << (16 * c);
+    };
+    auto stage = [&](int c) {
+      if (kQuant) return;
+#pragma unroll
+      for (int j = 0; j < (kSwiglu ? 2 : 4); ++j) *vec(c * (kSwiglu ? 2 : 4) + j) = o[j];
+    };
+    if (live) {
+      const uint32_t b2 = half ? t.bias[1] : t.bias[0];
+      *reinterpret_cast<float2*>(bias_smem + lane * 2) = make_float2(bf16_lo(b2) * bias_mul, bf16_hi(b2) * bias_mul);
+      if (kGate) reinterpret_cast<uint32_t*>(gate_smem)[lane] = half ? t.gate[1] : t.gate[0];
+      __syncwarp();
+      if (kGate && !mbar_wait_bounded(bar_res, res_uses++ & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) return false;
+      chunk(r0, 0);
+    }
+    if (half + 1u < uint32_t(kGroups)) tmem_ld_32x32b_x32(t.t_addr + t.g[1] * 64u, r0);
+    if (live) {
+      if (!kGate && !kQuant) {
+        if (lane == 0) bulk_wait_group_read<0>();  // the previous store has finished reading the staging buffer
+        __syncwarp();
+      }
+      stage(0);
+      chunk(r1, 1);
+    }
+    if (half + 1u < uint32_t(kGroups)) tmem_ld_32x32b_x32(t.t_addr + t.g[1] * 64u + 32u, r1);
+    if (live) {
+      stage(1);
+      if (!kQuant) {
+        fence_proxy_async();  // generic-proxy writes to smem -> visible to the TMA store
+        __syncwarp();         // ... and every lane has read this group's bias and gate
+        if (lane == 0) {
+          // SwiGLU halves the columns: the 64 accumulator columns of this group are output columns nc/2 .. +32
+          if (!(kDiag && (p.diag & 1u))) tma_store_2d(out_map, buf, int32_t(kSwiglu ? nc >> 1 : nc), int32_t(t.row0));
+          bulk_commit_group();
+        }
+      } else {
+        __syncwarp();
+      }
+      const uint32_t row = t.row0 + uint32_t(lane);
+      if (kQuant && row < p.m) {  // n % 64 == 0: the group is whole
+        const uint32_t qcol = p.n_offset + nc;
+        uint8_t* q = p.q_codes + uint64_t(row) * (p.ldo >> 1) + (qcol >> 1);
+        if (p.wide_q) {
+          st_global_v8(q, cw);
+        } else {
+          reinterpret_cast<uint4*>(q)[0] = make_uint4(cw[0], cw[1], cw[2], cw[3]);
+          reinterpret_cast<uint4*>(q)[1] = make_uint4(cw[4], cw[5], cw[6], cw[7]);
+        }
+        *reinterpret_cast<uint32_t*>(p.q_scales + sf_device_offset(row, qcol >> 4, p.q_k_atoms)) = sw;
+      }
+    }
+    if (kGate && lane == 0) {  // the buffer's next residual: this tile's second group, then the next tile's first
+      bulk_wait_group_read<0>();
+      if (half == 0u) load_residual(t.n0 + t.g[1] * 64u, t.row0, t.live[1]);
+      else if (more) load_residual(0u, 0u, 2u);
+    }
+    if (half + 1u < uint32_t(kGroups)) tmem_ld_wait();
+  }
+  return true;
 }
 
 // Work item w of the persistent loop -> row tile, first column and MMA width. Tiles [0, full_tiles) run whole
@@ -215,8 +340,8 @@ __device__ __forceinline__ void decode_item(const GemmParams& p, uint32_t tiles_
 // kDense: the dense-activation arm of the same kernel. A is bf16 [m,k] (not quantised), W the exact bf16 image of
 // code x block scale [n,k] made once per weight; a stage holds 64 K elements of each (the same 128-byte swizzled
 // rows), there are no scale factors, and the MMAs are kind::f16 with K = 16. Pipeline and epilogue are shared.
-template <int KB, bool kDense>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
+template <int KB, bool kDense, int kEpi>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::threads(kEpi), 1)
     nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                            const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
                            const __grid_constant__ PairOutMaps out_maps, const GemmParams p) {
@@ -249,6 +374,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder + 8 - smem_base));
   // staged NVFP4 multicast output: the CTA's eight epilogue warps meet on these ("tile staged" / "staging free")
   const uint32_t bar_qs_full = tmem_holder + 16, bar_qs_free = tmem_holder + 24;
+  const uint32_t bar_res0 = tmem_holder + 32;  // gated residual: one per epilogue warp, "a group's residual is loaded"
 
   // the warp index as a warp-uniform value: the role branches, stage addresses and MMA descriptors then live in uniform registers
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -267,9 +393,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
       mbar_init(bar_empty + 8 * i, 1);
     }
     mbar_init(bar_acc_full, 1);
-    mbar_init(bar_acc_free, 16);  // every epilogue warp of both CTAs arrives once per tile
+    mbar_init(bar_acc_free, 2 * epilogue_warps(kEpi));  // every epilogue warp of both CTAs arrives once per tile
     mbar_init(bar_qs_full, 8);
     mbar_init(bar_qs_free, 8);
+    for (int i = 0; i < 8; ++i) mbar_init(bar_res0 + 8 * i, 1);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tensormap(&map_a);
@@ -439,15 +566,87 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
     // other accumulator), h == 1 the last two.
     const uint32_t ew = uint32_t(warp - kFirstEpilogueWarp);  // 0..7
     const uint32_t q = warp & 3, h = ew >> 2;
-    const uint32_t buf = sStaging + ew * 4096u;
+    constexpr uint32_t kShare = uint32_t(kStagingBytes) / uint32_t(epilogue_warps(kEpi));
+    const uint32_t buf = sStaging + ew * kShare;
     uint8_t* buf_gen = smem_gen + (buf - smem_base);
-    float* bias_gen = reinterpret_cast<float*>(smem_gen + (sBias - smem_base) + ew * 256u);  // 64 f32: the current group's bias
-    const float bias_mul = (p.act == 1u && !p.chain) ? 0.5f : 1.0f;                          // the fused GELU works on x/2
+    // 64 f32: the current group's bias; 64 bf16: its gate. Nothing is staged on the way to an NVFP4 copy.
+    float* bias_gen = reinterpret_cast<float*>(kEpi == kQuantised ? buf_gen : smem_gen + (sBias - smem_base) + ew * 384u);
     const uint32_t acc_free_leader = mapa_cluster(bar_acc_free, 0);
+    if constexpr (kEpi != kGeneral) {
+      constexpr int kGroups = 16 / epilogue_warps(kEpi);  // 64-column groups of a warp
+      const uint32_t bar_res = bar_res0 + ew * 8u;
+      const uint32_t mode = (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u);
+      // The item that `fetch` saw last: its place, and this lane's bias and gate columns of it, which are asked for an item ahead.
+      PairShare next{};
+      auto fetch = [&](uint32_t item, uint32_t slot) {
+        uint32_t tm2, n_eff;
+        decode_item(p, tiles_m2, item, tm2, next.n0, n_eff);
+        next.row0 = tm2 * 256u + rank * 128u + q * 32u;
+        next.t_addr = tmem_base + slot * kAccStride + ((q * 32u) << 16);
+        const uint32_t first = slot ? 0u : 3u;  // 64-column group that overlaps the other accumulator
+#pragma unroll
+        for (uint32_t i = 0; i < uint32_t(kGroups); ++i) {
+          next.g[i] = (uint32_t(kGroups) * h + i + first) & 3u;
+          const uint32_t nc = next.n0 + next.g[i] * 64u, col = nc + uint32_t(lane) * 2u;
+          next.live[i] = next.g[i] * 64u < n_eff && nc < p.n && next.row0 < p.m ? 1u : 0u;
+          next.bias[i] = p.bias && col < p.n ? __ldg(reinterpret_cast<const uint32_t*>(p.bias + col)) : 0u;
+          if (kEpi == kGated) next.gate[i] = col < p.n ? __ldg(reinterpret_cast<const uint32_t*>(p.gate + col)) : 0u;
+        }
+      };
+      auto load_residual = [&](uint32_t nc, uint32_t row0, uint32_t live) {  // lane 0; live == 2: the first group of the item fetched last
+        if (live == 2u) {
+          nc = next.n0 + next.g[0] * 64u;
+          row0 = next.row0;
+          live = next.live[0];
+        }
+        if (!live) return;
+        mbar_arrive_expect_tx(bar_res, 4096u);
+        tma_load_2d(buf, &out_maps.m[1], bar_res, int32_t(nc), int32_t(row0));
+      };
+      uint32_t it = 0, res_uses = 0;
+      if (pair_id < num_tiles) {
+        fetch(pair_id, 0u);
+        if (kEpi == kGated && lane == 0) load_residual(0u, 0u, 2u);
+      }
+      for (uint32_t tile = pair_id; tile < num_tiles; tile += num_pairs, ++it) {
+        PairShare t = next;
+        t.acc_free = h == 0u ? acc_free_leader : 0u;
+        const bool more = tile + num_pairs < num_tiles;
+        if (more) fetch(tile + num_pairs, (it + 1u) & 1u);
+        const bool ttr = kDiag && (p.diag & 16u) && pair_id == 0 && rank == 0 && it < 16u && lane == 0 && warp == kFirstEpilogueWarp;
+        if (ttr) p.trace[1024 + it * 8 + 3] = clock64();
+        if (!mbar_wait_bounded(bar_acc_full, it & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) break;
+        tc_fence_after();
+        if (ttr) p.trace[1024 + it * 8 + 4] = clock64();
+        // The next tile's MMA overwrites the accumulator of tile it-1 and this tile's overlapping columns. h == 0 warps arrive once
+        // those columns are in registers; the others never touch them and arrive here: having passed this wait they are done
+        // reading tile it-1.
+        if (h != 0u) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_free_leader);
+        }
+        bool ok = true;
+#define TNF_EPILOGUE(gelu, chain)                                                                                                   \
+  ok = epilogue_pair_local<kGroups, gelu, chain, kEpi == kGated, kEpi == kQuantised, kEpi == kSwiglu>(p, t, &out_maps.m[0], buf, buf_gen, bias_gen, \
+                                                                                                lut_gen, lane, bar_res, res_uses, abort_flag, \
+                                                                                                wait_limit, load_residual, more)
+        switch (mode) {  // warp-uniform
+          case 0: TNF_EPILOGUE(false, false); break;
+          case 1: TNF_EPILOGUE(kEpi != kSwiglu, false); break;
+          case 2: TNF_EPILOGUE(false, true); break;
+          default: TNF_EPILOGUE(kEpi != kSwiglu, true); break;
+        }
+#undef TNF_EPILOGUE
+        if (!ok) break;
+        if (ttr) p.trace[1024 + it * 8 + 6] = clock64();
+      }
+      if (lane == 0) bulk_wait_group_read<0>();
+    } else {
+    const float bias_mul = (p.act == 1u && !p.chain) ? 0.5f : 1.0f;                          // the fused GELU works on x/2
     uint32_t it = 0;
     bool ok = true;
-    const uint32_t mode = p.swiglu ? (p.chain ? 13u : 12u)
-                                   : (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u) | (p.q_codes ? 8u : (p.gate ? 4u : 0u));
+    const uint32_t mode = (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u) | (p.q_codes ? 8u : (p.gate ? 4u : 0u));
     // NVFP4 output through the multicast alias with no bf16 store: the (then idle) bf16 staging area collects the
     // CTA's whole tile of codes and scale atoms, and all eight warps write it out in 128-byte row segments and whole
     // 16-byte atom rows. Scattered 16- and 4-byte multimem stores straight from the registers ran at a fifth of the link rate.
@@ -526,9 +725,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
         fence_proxy_async();  // generic-proxy writes to smem -> visible to the TMA store
         __syncwarp();
         if (lane == 0) {
-          // SwiGLU halves the columns: the 64 accumulator columns of this group are output columns ncol0/2 .. +32
-          if (!(kDiag && (p.diag & 1u)) && p.store_bf16 && !p.out_mc)
-            tma_store_2d(&out_maps.m[0], buf, int32_t(p.swiglu ? ncol0 >> 1 : ncol0), int32_t(row0));
+          if (!(kDiag && (p.diag & 1u)) && p.store_bf16 && !p.out_mc) tma_store_2d(&out_maps.m[0], buf, int32_t(ncol0), int32_t(row0));
           bulk_commit_group();
         }
         // Multicast output: the staging rows leave as 16-byte multimem stores (8 lanes cover one 128-byte row
@@ -585,6 +782,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
     }
     if (lane == 0) bulk_wait_group_read<0>();
     if (p.out_mc || p.q_codes_mc) __threadfence_system();  // multicast stores are performed before the kernel ends
+    }
   }
 
   // ---------------- tear-down ----------------
@@ -621,7 +819,7 @@ uint32_t gemm_pair_kblocks() { return 4u; }
 
 constexpr uint64_t kSmallW = 32u << 20, kBandMaxW = 96u << 20, kBandSmallW = 8u << 20, kBandLargeW = 54u << 20;
 
-template <int KB, bool kDense>
+template <int KB, bool kDense, int kEpi>
 static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& map_w, const CUtensorMap& map_sfa,
                                   const CUtensorMap& map_sfb, const CUtensorMap* out_maps, const GemmParams& p_in,
                                   int sm_count, cudaStream_t s) {
@@ -632,14 +830,14 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= kMaxDevices) dev = 0;
   if (once.first_use() >= 0) {  // the shared-memory opt-in is a per-device attribute of the function
-    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_pair_kernel<KB, kDense>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_pair_kernel<KB, kDense, kEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(sm_count & ~1), 1, 1);
-    cfg.blockDim = dim3(pair::kThreads, 1, 1);
+    cfg.blockDim = dim3(pair::threads(kEpi), 1, 1);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, nvfp4_gemm_pair_kernel<KB, kDense>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&clusters, nvfp4_gemm_pair_kernel<KB, kDense, kEpi>, &cfg);
     if (e != cudaSuccess || clusters <= 0) {
       cudaGetLastError();
       clusters = sm_count / 2;
@@ -647,6 +845,7 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
     max_pairs[dev] = std::min(clusters, sm_count / 2);
   }
   GemmParams p = p_in;
+  p.wide_q = reinterpret_cast<uintptr_t>(p.q_codes) % 32u == 0 ? 1u : 0u;  // ldo and n_offset are multiples of 64
   static uint32_t diag = env_u32_pair("TNF_GEMM_DIAG", 0);
   p.diag = diag;
   p.tiles_m = (p.m + 255u) / 256u;
@@ -667,22 +866,34 @@ static cudaError_t launch_pair_kb(const CUtensorMap& map_a, const CUtensorMap& m
   p.band_m = p.tiles_m;
   if (a_bytes > band_bytes && w_bytes <= kBandMaxW)
     p.band_m = uint32_t(std::min<uint64_t>(p.tiles_m, std::max<uint64_t>(1u, band_bytes / (row_bytes * 256u))));
-  const uint32_t avail = uint32_t(max_pairs[dev] > 0 ? max_pairs[dev] : sm_count / 2);
   const bool remote = p.n_out > 1u || p.out_mc || p.q_codes_mc;
+  const uint32_t avail = uint32_t(max_pairs[dev] > 0 ? max_pairs[dev] : sm_count / 2);
   p.full_tiles = kDiag && (diag & 2048u) ? tiles : pair_whole_tiles(tiles, p.n, avail, remote);
   const uint32_t items = p.full_tiles + (tiles - p.full_tiles) * 2u;
   const uint32_t pairs = std::min<uint32_t>(items, avail);
   PairOutMaps om;
   for (int i = 0; i < kMaxPeers; ++i) om.m[i] = out_maps[i];
-  return launch_pdl(nvfp4_gemm_pair_kernel<KB, kDense>, dim3(pairs * 2), dim3(pair::kThreads), Cfg::kSmemBytes, s, map_a, map_w, map_sfa,
+  return launch_pdl(nvfp4_gemm_pair_kernel<KB, kDense, kEpi>, dim3(pairs * 2), dim3(pair::threads(kEpi)), Cfg::kSmemBytes, s, map_a, map_w, map_sfa,
                     map_sfb, om, p);
 }
 
 cudaError_t launch_gemm_nvfp4_pair(const CUtensorMap& map_a, const CUtensorMap& map_w, const CUtensorMap& map_sfa,
                                    const CUtensorMap& map_sfb, const CUtensorMap* out_maps, const GemmParams& p,
                                    int sm_count, cudaStream_t s) {
-  return p.dense ? launch_pair_kb<4, true>(map_a, map_w, map_sfa, map_sfb, out_maps, p, sm_count, s)
-                 : launch_pair_kb<4, false>(map_a, map_w, map_sfa, map_sfb, out_maps, p, sm_count, s);
+  decltype(&launch_pair_kb<4, false, pair::kPlain>) launch;
+  const uint32_t tiles = ((p.m + 255u) / 256u) * ((p.n + 255u) / 256u);
+  const bool one_output = p.n_out == 1u && !p.out_mc && !p.q_codes_mc && !(p.q_codes && p.store_bf16);
+  const int epilogue = !one_output ? pair::kGeneral : p.gate ? pair::kGated : p.swiglu ? pair::kSwiglu
+                       : !pair_epilogue_rule(p.k, p.dense != 0u, p.act == 1u, p.q_codes != nullptr, tiles, uint32_t(sm_count) / 2u) ? pair::kGeneral
+                       : p.q_codes ? pair::kQuantised : pair::kPlain;
+  switch (epilogue) {
+    case pair::kGated: launch = p.dense ? launch_pair_kb<4, true, pair::kGated> : launch_pair_kb<4, false, pair::kGated>; break;
+    case pair::kQuantised: launch = p.dense ? launch_pair_kb<4, true, pair::kQuantised> : launch_pair_kb<4, false, pair::kQuantised>; break;
+    case pair::kSwiglu: launch = p.dense ? launch_pair_kb<4, true, pair::kSwiglu> : launch_pair_kb<4, false, pair::kSwiglu>; break;
+    case pair::kPlain: launch = p.dense ? launch_pair_kb<4, true, pair::kPlain> : launch_pair_kb<4, false, pair::kPlain>; break;
+    default: launch = p.dense ? launch_pair_kb<4, true, pair::kGeneral> : launch_pair_kb<4, false, pair::kGeneral>;
+  }
+  return launch(map_a, map_w, map_sfa, map_sfb, out_maps, p, sm_count, s);
 }
 
 }  // namespace tnf

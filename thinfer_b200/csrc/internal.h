@@ -101,6 +101,7 @@ struct GemmParams {
                                // [n,k]; no scale factors, tcgen05.mma kind::f16 (pair kernel only)
   uint32_t swiglu;             // pairwise gating epilogue: out[m, j] = silu(v[2j]) * v[2j+1], n/2 output columns
   uint32_t store_bf16;         // 0: skip the bf16 store
+  uint32_t wide_q;             // pair kernel: the 32 code bytes of 64 columns start on a 32-byte boundary
   uint32_t* status;            // device status word
   long long wait_limit;        // SM cycles after which a device-side wait gives up (0 = kDefaultWaitLimitCycles)
   uint32_t stall;              // self-test: the producer issues no loads, so the first wait on a loaded stage runs out
@@ -151,6 +152,11 @@ struct MapSpec {
   }
 };
 int make_tensor_map(CUtensorMap* out, const MapSpec& spec);
+// bf16 rows [m, n] that the pair kernel stores (output) or loads (residual) by 64 columns x 32 rows, 128-byte swizzle; with SwiGLU
+// by the 32 columns that 64 accumulator columns make, 64-byte swizzle
+inline MapSpec pair_out_spec(const void* base, uint32_t m, uint32_t n, uint32_t ld, bool swiglu = false) {
+  return MapSpec{base, 2, n, m, uint64_t(ld) * 2, swiglu ? 32u : 64u, 32, swiglu ? 64u : 128u};
+}
 uint32_t gemm_tile_n(uint32_t m, uint32_t n, int sm_count);  // tile width the 1-CTA launcher will pick (for the map of W)
 
 }  // namespace tnf

@@ -150,9 +150,9 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
     if (make_tensor_map(&msa, MapSpec{a_scales, 1, 128, scales_bytes / 128, 128, 128, kb * 4, 0}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
     if (make_tensor_map(&msb, MapSpec{w_scales, 1, 128, sf_device_bytes(a->n, a->k) / 128, 128, 128, kb * 4, 0}) != TNF_OK)
       return TNF_ERR_INVALID_ARGUMENT;
-    if (make_tensor_map(&outs[0], MapSpec{p.out[0] + a->n_offset, 2, a->n, a->m, uint64_t(ldo) * 2, 64, 32, 1}) != TNF_OK)
-      return TNF_ERR_INVALID_ARGUMENT;
+    if (make_tensor_map(&outs[0], pair_out_spec(p.out[0] + a->n_offset, a->m, a->n, ldo)) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
     for (int d = 1; d < kMaxPeers; ++d) outs[d] = outs[0];
+    if (p.gate && make_tensor_map(&outs[1], pair_out_spec(p.residual, a->m, a->n, a->n)) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
     ce = launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute);
   } else {
     ce = launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute);

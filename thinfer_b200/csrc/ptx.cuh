@@ -210,6 +210,12 @@ __device__ __forceinline__ void bulk_wait_group_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 
+// One whole 32-byte sector; `p` on a 32-byte boundary.
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 // ---- NVSwitch multicast stores -----------------------------------------------------------------------
 // A store to the multicast alias of a symmetric allocation is replicated by the switch into every
 // rank's copy at the same offset (bits are moved unchanged; the .f32 type only names the width). Weak stores:

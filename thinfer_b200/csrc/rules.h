@@ -69,6 +69,19 @@ TNF_HD inline uint32_t pair_whole_tiles(uint32_t tiles, uint32_t n, uint32_t pai
   return split ? tiles - tail : tiles;
 }
 
+// Whether a plain or an NVFP4 output (local, no residual) takes its own epilogue, which shortens a tile that the epilogue bounds, or the
+// general one. With a long K the tile is bound by its main loop, and the general one, whose stores are spread over more of it,
+// disturbs the loop less. Measured (us, general / own): plain 4257 x 1120 x 768 10.9 / 10.2, 3352 x 2992 x 1280 15.8 / 15.3, 4137 x 7280 x 2048
+// 35.5 / 36.3; GELU 5394 x 10640 x 1280 54.8 / 48.2, 5434 x 4144 x 2048 32.5 / 30.2, 6013 x 4416 x 4096 59.1 / 59.7; NVFP4 4601 x 7168 x 1792
+// 35.3 / 31.5, 3716 x 12096 x 3072 60.6 / 61.6; GELU + NVFP4 3228 x 18176 x 3584 91.4 / 89.3, 8456 x 11968 x 6144 248.7 / 248.2. In less than two
+// waves the last epilogue is not hidden at all: plain 1612 x 1520 x 2560 12.1 / 11.7, GELU 4129 x 944 x 9216 37.0 / 36.4. The dense arm takes
+// four times as long for a K.
+TNF_HD inline bool pair_epilogue_rule(uint32_t k, bool dense, bool gelu, bool quantised, uint32_t tiles, uint32_t pairs) {
+  if (tiles < 2u * pairs || (quantised && gelu)) return true;
+  const uint64_t k4 = dense ? uint64_t(k) * 4u : k;
+  return k4 < (quantised ? 3072u : gelu ? 3584u : 2048u);
+}
+
 // Work items of the attention kernel. A (head, batch) pair has ceil(s_q / 128) blocks of 128 query rows; two of them make a tile.
 // An item is a tile (rows mode: one softmax group per block, all keys each) or one block (keys mode: the groups share the keys),
 // which takes about half as long. Items [0, full_items) are tiles, the others the blocks of the tiles that are left and then, where

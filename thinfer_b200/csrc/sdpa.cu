@@ -142,11 +142,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return d;
 }
 
-__device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
-               "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
-}
 // Work item `it` of the persistent loop.
 struct SdpaItem {
   bool keys_mode;
