@@ -481,14 +481,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::threads(kEpi),
       for (uint32_t tile = pair_id; tile < num_tiles && ok; tile += num_pairs, ++it) {
         const bool ttr = kDiag && (p.diag & 16u) && pair_id == 0 && it < 16u && lane == 0;
         if (ttr) p.trace[1024 + it * 8 + 0] = clock64();
-        if (it > 0) {  // the previous tile's epilogues (both CTAs) have read the overlapping columns
-          if (!mbar_wait_warp(bar_acc_free, (it - 1u) & 1u, abort_flag, kStatusAccEmptyTimeout, wait_limit)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-        }
-        if (ttr) p.trace[1024 + it * 8 + 1] = clock64();
         const uint32_t d_tmem = tmem_base + (it & 1u) * kAccStride;
         uint32_t tm2_, n0_, n_eff;
         decode_item(p, tiles_m2, tile, tm2_, n0_, n_eff);  // as in the producer
@@ -506,8 +498,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::threads(kEpi),
           const uint32_t nstage = stage + 1u == uint32_t(S) ? 0u : stage + 1u;
           const bool probe = mbar_test_wait(bar_full + 8 * nstage, nstage == 0u ? phase ^ 1u : phase);
           const bool tr = kDiag && (p.diag & 16u) && pair_id == 0 && titer < 256u;
-          if (elect_one()) {
-          if (tr) p.trace[titer * 4 + 2] = clock64();
           // Descriptors of this stage: the constant high words were built before the loop, a stage only moves the
           // 14-bit start-address field (shared addresses are below 256 KB, so the add never carries out of it).
           const uint32_t a_lo = a_lo0 + stage * uint32_t(kABytes >> 4), b_lo = b_lo0 + stage * uint32_t(kBBytes >> 4);
@@ -517,6 +507,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::threads(kEpi),
           const uint32_t sf_slot = Cfg::kSfSlots == 2 ? (kt & 1u) : 0u;
           const uint32_t t_sfa = tmem_base + kSfaCol + sf_slot * (KB * 4), t_sfb = tmem_base + kSfbCol + sf_slot * (KB * 8);
           const bool do_cp = !(kDiag && (p.diag & 2u)) || kt == 0, do_mma = !(kDiag && (p.diag & 4u));
+          if (kt == 0u && it > 0u) {  // warp-uniform
+            // The previous tile's epilogues (both CTAs) have to have read the overlapping columns. What does not need them is done by
+            // now, the item's place (its divisions stood behind this wait: GELU + NVFP4 output 9472 x 4096 x 1024 30.5 -> 28.0 us,
+            // 3072 44.0 -> 42.2, dense 768 43.5 -> 42.1) and the stage's arrival; with its scale copies before the wait as well the
+            // gains were smaller (plain 1536 31.1 -> 32.4).
+            if (!mbar_wait_warp(bar_acc_free, (it - 1u) & 1u, abort_flag, kStatusAccEmptyTimeout, wait_limit)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            if (ttr) p.trace[1024 + it * 8 + 1] = clock64();
+          }
+          if (elect_one()) {
+          if (tr) p.trace[titer * 4 + 2] = clock64();
           if (kDense) {
 #pragma unroll
             for (int kb = 0; kb < KB; ++kb)
