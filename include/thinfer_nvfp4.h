@@ -147,6 +147,12 @@ int32_t tnf_streams(tnf_ctx* ctx, void** compute_stream, void** copy_stream);
  * [n,k/2], scales [n,k/16] canonical. *global_scale receives amax/(6*448). Blocking. */
 int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint32_t n, uint32_t k,
                             tnf_buf codes, tnf_buf scales, float* global_scale);
+/* The same from host memory (f32 or bf16 [n,k], pageable or pinned) in one call: makes the buffers (codes [n,k/2], DEVICE-layout
+ * scales, and with bias_host the bf16 bias [n]; free each with tnf_free) and fills them. Without a budget the context keeps the
+ * staging for the next load (up to 160 MB, given back when an allocation fails) and lets weights share allocations of 64 MB, which
+ * go back with their last buffer. bias_host and bias_id may be null. Blocking. */
+int32_t tnf_load_weight(tnf_ctx* ctx, const void* w_host, int32_t src_dtype, uint32_t n, uint32_t k, const uint16_t* bias_host,
+                        uint64_t* codes_id, uint64_t* scales_id, uint64_t* bias_id, float* global_scale);
 /* Bytes of the DEVICE scale layout for a [rows,k] operand. */
 uint64_t tnf_device_scales_bytes(uint32_t rows, uint32_t k);
 /* Canonical scales -> DEVICE layout (weights: once at load; PreparedWeight idea,

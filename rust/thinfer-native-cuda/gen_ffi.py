@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 HEADER = os.path.join(HERE, "..", "..", "include", "thinfer_nvfp4.h")
 
 TYPES = {
-    "int32_t": "i32", "uint32_t": "u32", "uint64_t": "u64", "int": "i32", "float": "f32", "void": "c_void",
+    "int32_t": "i32", "uint32_t": "u32", "uint64_t": "u64", "int": "i32", "float": "f32", "uint16_t": "u16", "void": "c_void",
     "tnf_ctx": "TnfCtx", "tnf_buf": "TnfBuf", "tnf_linear_args": "TnfLinearArgs", "tnf_norm_quant_args": "TnfNormQuantArgs",
     "tnf_stack": "TnfStack", "tnf_stack_linear": "TnfStackLinear", "tnf_gguf": "TnfGguf",
     "tnf_gguf_tensor_info": "TnfGgufTensorInfo", "tnf_dense_act_sites": "TnfDenseActSites", "char": "c_char",

@@ -107,6 +107,7 @@ extern "C" {
     pub fn tnf_selftest_stalled_wait(ctx: *mut TnfCtx) -> i32;
     pub fn tnf_streams(ctx: *mut TnfCtx, compute_stream: *mut *mut c_void, copy_stream: *mut *mut c_void) -> i32;
     pub fn tnf_quantize_weight(ctx: *mut TnfCtx, w_src: TnfBuf, src_dtype: i32, n: u32, k: u32, codes: TnfBuf, scales: TnfBuf, global_scale: *mut f32) -> i32;
+    pub fn tnf_load_weight(ctx: *mut TnfCtx, w_host: *const c_void, src_dtype: i32, n: u32, k: u32, bias_host: *const u16, codes_id: *mut u64, scales_id: *mut u64, bias_id: *mut u64, global_scale: *mut f32) -> i32;
     pub fn tnf_device_scales_bytes(rows: u32, k: u32) -> u64;
     pub fn tnf_prepare_scales(ctx: *mut TnfCtx, scales_canonical: TnfBuf, rows: u32, k: u32, scales_device: TnfBuf) -> i32;
     pub fn tnf_quantize_act(ctx: *mut TnfCtx, a_bf16: TnfBuf, m: u32, k: u32, global_scale: f32, scales_layout: i32, codes: TnfBuf, scales: TnfBuf, global_scale_used: *mut f32) -> i32;

@@ -1,0 +1,109 @@
+"""Loading a dense weight in one call: the same bytes as upload + quantise + scale layout, from several threads, through slabs that fill
+up and go, and with a budget; and pageable writes around the sizes where the staged copy changes its chunks."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _weight(n, k, bf16, seed):
+    w = np.random.default_rng(seed).standard_normal((n, k), np.float32) * np.float32(0.02)
+    return O.f32_to_bf16(w) if bf16 else w
+
+
+def _check(be, W, w, bias):
+    import thinfer_b200 as T
+
+    V = T.Nvfp4Weight.from_dense(be, w, bias, keep_canonical=True)  # upload, quantise, scale layout: a call each
+    assert W.global_scale == V.global_scale
+    assert np.array_equal(be.read_buffer(W.codes), be.read_buffer(V.codes))
+    assert np.array_equal(be.read_buffer(W.scales_device), be.read_buffer(V.scales_device))
+    if bias is None:
+        assert W.bias is None
+    else:
+        assert np.array_equal(be.read_buffer(W.bias, np.uint16), bias)
+    V.free(be)
+
+
+@pytest.mark.parametrize("n,k,bf16", [(2, 32, True), (130, 96, False), (1000, 2080, True), (4104, 3072, True), (12288, 3072, False)])
+@pytest.mark.parametrize("budget", [0, 1 << 30])
+def test_load_equals_its_parts(n, k, bf16, budget):
+    import thinfer_b200 as T
+
+    with T.Backend(0, budget) as be:
+        w, bias = _weight(n, k, bf16, n + k), O.f32_to_bf16(np.random.default_rng(n).standard_normal(n, np.float32))
+        for b in (bias, None):
+            W = T.Nvfp4Weight.from_dense(be, w, b)
+            _check(be, W, w, b)
+            W.free(be)
+        live = be.mem_snapshot()
+        assert live["live_weights"] == 0
+        assert not budget or live["live_staging"] == 0  # nothing stays where memory is planned
+
+
+def test_slabs_fill_up_and_go(backend):
+    """Weights of 9 MB in slabs of 64: dozens of them, freed in another order, every other one read back after its neighbours went."""
+    import thinfer_b200 as T
+
+    be, before = backend, backend.mem_snapshot()["live_weights"]
+    w = [_weight(4096, 4096, True, i) for i in range(3)]
+    W = [T.Nvfp4Weight.from_dense(be, w[i % 3]) for i in range(24)]
+    ref = [be.read_buffer(W[i].codes) for i in range(3)]
+    for i in range(0, 24, 2):
+        W[i].free(be)
+    for i in range(1, 24, 2):
+        assert np.array_equal(be.read_buffer(W[i].codes), ref[i % 3])
+        W[i].free(be)
+    assert be.mem_snapshot()["live_weights"] == before
+
+
+def test_loads_of_several_threads(backend):
+    import thinfer_b200 as T
+
+    w, out = [_weight(2048 + 128 * i, 1024, i % 2 == 0, i) for i in range(4)], [None] * 4
+    def load(i):
+        for _ in range(3):
+            if out[i]:
+                out[i].free(backend)
+            out[i] = T.Nvfp4Weight.from_dense(backend, w[i])
+    threads = [threading.Thread(target=load, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for W, x in zip(out, w):
+        _check(backend, W, x, None)
+        W.free(backend)
+
+
+def test_exported_weight_leaves_its_slab(backend):
+    """An IPC handle covers an allocation: the buffer gets one of its own, with its contents."""
+    import thinfer_b200 as T
+    from thinfer_b200.backend import _check as check
+
+    w = _weight(1024, 1024, True, 7)
+    W, V = T.Nvfp4Weight.from_dense(backend, w), T.Nvfp4Weight.from_dense(backend, w)
+    handle, p = C.create_string_buffer(64), backend.device_ptr(V.codes)
+    check(backend.lib.tnf_ipc_export(backend._ctx, V.codes.id, handle))
+    assert backend.device_ptr(V.codes) != p
+    _check(backend, V, w, None)
+    _check(backend, W, w, None)
+    V.free(backend)
+    W.free(backend)
+
+
+@pytest.mark.parametrize("nbytes", [(1 << 20) - 4, 1 << 20, (2 << 20) - 4, (2 << 20) + 4, (3 << 20) + 8, 8 << 20, (11 << 20) + 12])
+def test_pageable_writes(backend, nbytes):
+    data = np.random.default_rng(nbytes).integers(0, 256, nbytes + 3, np.uint8)[3:]  # not aligned
+    buf = backend.allocate(nbytes + 64)
+    backend.write_buffer(buf, np.full(nbytes + 64, 0xA5, np.uint8))
+    backend.write_buffer(buf, data, offset=16)
+    got = backend.read_buffer(buf)
+    assert np.array_equal(got[16: 16 + nbytes], data)
+    assert (got[:16] == 0xA5).all() and (got[16 + nbytes:] == 0xA5).all()
+    backend.free(buf)

@@ -110,6 +110,7 @@ SIGNATURES = {
     "tnf_set_device_wait_limit": (C.c_int32, [_ctx, C.c_uint64]),
     "tnf_selftest_stalled_wait": (C.c_int32, [_ctx]),
     "tnf_quantize_weight": (C.c_int32, [_ctx, Buf, C.c_int32, C.c_uint32, C.c_uint32, Buf, Buf, C.POINTER(C.c_float)]),
+    "tnf_load_weight": (C.c_int32, [_ctx, C.c_void_p, C.c_int32, C.c_uint32, C.c_uint32, C.c_void_p, _u64p, _u64p, _u64p, C.POINTER(C.c_float)]),
     "tnf_device_scales_bytes": (C.c_uint64, [C.c_uint32, C.c_uint32]),
     "tnf_prepare_scales": (C.c_int32, [_ctx, Buf, C.c_uint32, C.c_uint32, Buf]),
     "tnf_quantize_act": (C.c_int32, [_ctx, Buf, C.c_uint32, C.c_uint32, C.c_float, C.c_int32, Buf, Buf, C.POINTER(C.c_float)]),

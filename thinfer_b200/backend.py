@@ -242,6 +242,13 @@ class Nvfp4Weight:
         dtype = L.DTYPE_BF16 if w.dtype == np.uint16 else L.DTYPE_F32
         if dtype == L.DTYPE_F32:
             w = w.astype(np.float32, copy=False)
+        bias_bf16 = None if bias_bf16 is None else _host(bias_bf16.astype(np.uint16, copy=False))
+        if not keep_canonical and n * k and (bias_bf16 is None or (bias_bf16.size == n and n % 2 == 0)):  # an odd bias is refused by the write
+            w, ids, g = _host(w), [C.c_uint64() for _ in range(3)], C.c_float()
+            _check(be.lib.tnf_load_weight(be._ctx, w.ctypes.data, dtype, n, k, None if bias_bf16 is None else bias_bf16.ctypes.data,
+                                          C.byref(ids[0]), C.byref(ids[1]), C.byref(ids[2]), C.byref(g)))
+            return Nvfp4Weight(n, k, Buf(ids[0].value, 0, n * k // 2), Buf(ids[1].value, 0, device_scales_bytes(n, k)), float(g.value),
+                               None if bias_bf16 is None else Buf(ids[2].value, 0, n * 2), None)
         src = be.upload(w, L.CAT_STAGING)
         codes = be.allocate_in(n * k // 2, L.CAT_WEIGHTS)
         canon = be.allocate_in(max(n * k // 16, 16), L.CAT_WEIGHTS if keep_canonical else L.CAT_STAGING)
@@ -254,7 +261,7 @@ class Nvfp4Weight:
         if not keep_canonical:
             be.free(canon)
             canon = None
-        bias = be.upload(bias_bf16.astype(np.uint16, copy=False), L.CAT_WEIGHTS) if bias_bf16 is not None else None
+        bias = be.upload(bias_bf16, L.CAT_WEIGHTS) if bias_bf16 is not None else None
         return Nvfp4Weight(n, k, codes, dev, float(g.value), bias, canon)
 
     @staticmethod

@@ -1,5 +1,9 @@
 // C ABI of the NVFP4 linear path: context, buffers, quantisers, the linear, uploads.
 // See include/thinfer_nvfp4.h for the reference interface each entry point replaces.
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
+
 #include <algorithm>
 #include <chrono>
 #include <cstdarg>
@@ -75,7 +79,60 @@ uint8_t* resolve_multicast(tnf_ctx* ctx, const tnf_buf& b, const char* name, int
   return static_cast<uint8_t*>(it->second.mc) + b.offset;
 }
 
-int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id) {
+// A block of the open slab, or of a new one; null when there is no memory for a slab. An allocation of its own costs about 330 us and
+// its cudaFree 280, a slab the same: the codes and scales of a loaded weight were half of the time of loading it.
+constexpr uint64_t kSlabBytes = 64u << 20, kSlabMaxBlock = kSlabBytes / 2;
+static void* slab_block(tnf_ctx* ctx, uint64_t bytes, uint64_t* slab_id) {
+  bytes = (bytes + 511u) & ~uint64_t(511);
+  auto open = ctx->slabs.find(ctx->open_slab);
+  if (open == ctx->slabs.end() || open->second.used + bytes > kSlabBytes) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, kSlabBytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (open != ctx->slabs.end() && open->second.live == 0) {
+      cudaFree(open->second.ptr);
+      ctx->slabs.erase(open);
+    }
+    ctx->open_slab = ctx->next_slab++;
+    open = ctx->slabs.emplace(ctx->open_slab, tnf_slab{p}).first;
+  }
+  void* p = static_cast<uint8_t*>(open->second.ptr) + open->second.used;
+  open->second.used += bytes;
+  open->second.live++;
+  *slab_id = ctx->open_slab;
+  return p;
+}
+
+// The block's slab loses it; cudaFree with the last one, unless further blocks can still come from it.
+static cudaError_t slab_release(tnf_ctx* ctx, uint64_t slab_id) {
+  auto s = ctx->slabs.find(slab_id);
+  if (--s->second.live > 0 || slab_id == ctx->open_slab) return cudaSuccess;
+  const cudaError_t e = cudaFree(s->second.ptr);
+  ctx->slabs.erase(s);
+  return e;
+}
+
+// What this library holds and nobody uses: the idle staging of loads and an open slab without blocks. True when there was some.
+static bool give_back_idle(tnf_ctx* ctx) {
+  bool any = false;
+  if (ctx->load_stage_id && !ctx->load_busy) {
+    const uint64_t id = ctx->load_stage_id;
+    ctx->load_stage_id = ctx->load_stage_bytes = 0;
+    any = free_locked(ctx, id) == TNF_OK;
+  }
+  auto open = ctx->slabs.find(ctx->open_slab);
+  if (open != ctx->slabs.end() && open->second.live == 0) {
+    cudaFree(open->second.ptr);
+    ctx->slabs.erase(open);
+    ctx->open_slab = 0;
+    any = true;
+  }
+  return any;
+}
+
+int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id, bool slab) {
   if (category < 0 || category > 2 || bytes == 0) {
     set_error("tnf_alloc: bad category %d or zero size", category);
     return TNF_ERR_INVALID_ARGUMENT;
@@ -101,19 +158,57 @@ int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id) {
               (unsigned long long)bytes, (unsigned long long)ctx->budget);
     return TNF_ERR_BUDGET_EXCEEDED;
   }
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return cuda_fail(e, "cudaMalloc");
+  uint64_t slab_id = 0;
+  void* p = slab && bytes <= kSlabMaxBlock ? slab_block(ctx, bytes, &slab_id) : nullptr;
+  if (!p) {
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back_idle(ctx)) {
+      cudaGetLastError();
+      e = cudaMalloc(&p, bytes);
+      total = ctx->live[0] + ctx->live[1] + ctx->live[2];
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return cuda_fail(e, "cudaMalloc");
+    }
   }
   uint64_t nid = ctx->next_id++;
   ctx->bufs[nid] = tnf_buffer_rec{p, bytes, category};
+  ctx->bufs[nid].slab = slab_id;
   ctx->live[category] += bytes;
   ctx->peak[category] = std::max(ctx->peak[category], ctx->live[category]);
   ctx->true_peak = std::max(ctx->true_peak, total + bytes);
   *id = nid;
   return TNF_OK;
+}
+
+// tensor maps over a range that is freed are dropped (a later buffer may reuse the address)
+static void drop_maps(tnf_ctx* ctx, const void* ptr, uint64_t bytes) {
+  const uint8_t* lo = static_cast<const uint8_t*>(ptr);
+  for (auto m = ctx->maps.begin(); m != ctx->maps.end();) {
+    const uint8_t* b = static_cast<const uint8_t*>(m->first.base);
+    if (b >= lo && b < lo + bytes) m = ctx->maps.erase(m);
+    else ++m;
+  }
+}
+
+int32_t leave_slab_locked(tnf_ctx* ctx, uint64_t id) {
+  tnf_buffer_rec& r = ctx->bufs.at(id);
+  if (!r.slab) return TNF_OK;
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, r.bytes);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // work that still writes the buffer
+  if (e == cudaSuccess) e = cudaMemcpy(p, r.ptr, r.bytes, cudaMemcpyDeviceToDevice);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (p) cudaFree(p);
+    return cuda_fail(e, "buffer move");
+  }
+  drop_maps(ctx, r.ptr, r.bytes);
+  e = slab_release(ctx, r.slab);
+  r.ptr = p;
+  r.slab = 0;
+  return e == cudaSuccess ? TNF_OK : cuda_fail(e, "cudaFree");
 }
 
 int32_t free_locked(tnf_ctx* ctx, uint64_t id) {
@@ -123,15 +218,9 @@ int32_t free_locked(tnf_ctx* ctx, uint64_t id) {
     return TNF_ERR_UNKNOWN_BUFFER;
   }
   // cudaFree waits for work that may still use the memory; an imported range is only forgotten
-  cudaError_t e = it->second.owned ? cudaFree(it->second.ptr) : cudaSuccess;
+  cudaError_t e = it->second.slab ? slab_release(ctx, it->second.slab) : it->second.owned ? cudaFree(it->second.ptr) : cudaSuccess;
   ctx->live[it->second.category] -= it->second.bytes;
-  // tensor maps over the freed range are dropped (a later buffer may reuse the address)
-  for (auto m = ctx->maps.begin(); m != ctx->maps.end();) {
-    const uint8_t* b = static_cast<const uint8_t*>(m->first.base);
-    const uint8_t* lo = static_cast<const uint8_t*>(it->second.ptr);
-    if (b >= lo && b < lo + it->second.bytes) m = ctx->maps.erase(m);
-    else ++m;
-  }
+  drop_maps(ctx, it->second.ptr, it->second.bytes);
   ctx->bufs.erase(it);
   // a pool buffer freed directly leaves the pool's books too
   auto rented = ctx->ws_rented.find(id);
@@ -459,6 +548,126 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
   return TNF_OK;
 }
 
+// Large writes from pageable memory. A plain copy stages those through one thread; here up to kWriteThreads threads copy into
+// pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the chunks on the compute
+// stream. The slots are written past the caches: they are read next by the DMA engine, and ordinary stores fetch every line first and
+// leave it dirty where the engine has to ask for it. Measured (us, plain copy / ordinary stores with four threads / these): 1 MB
+// 108 / - / 60, 3 MB 311 / - / 125, 6 MB 488 / 661 / 210, 12 MB 896 / 952 / 370, 24 MB 1860 / 1220 / 670, 72 MB 6490 / 2310 / 1800 (PCIe
+// alone 1305). Two threads are enough for a few MB (two against six at 4 MB: 147 / 180), six are best from 24 MB on. The slots
+// (kWriteStageBytes in all) are made on first use and freed with the context. Returns false when the caller has to copy the plain way
+// (slots in use by another thread's write, no pinned memory to be had); *err is a failed copy.
+constexpr uint32_t kWriteThreads = 6;
+constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 1u << 20;
+// `dst` on a 16-byte boundary
+static void copy_past_caches(uint8_t* dst, const uint8_t* src, uint64_t n) {
+  uint64_t i = 0;
+#if defined(__SSE2__)
+  for (; i + 64u <= n; i += 64u) {
+    __m128i v[4];
+    for (int j = 0; j < 4; ++j) v[j] = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i) + j);
+    for (int j = 0; j < 4; ++j) _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i) + j, v[j]);
+  }
+  _mm_sfence();
+#endif
+  std::memcpy(dst + i, src + i, n - i);
+}
+static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n, cudaError_t* err) {
+  std::unique_lock<std::mutex> lk(ctx->write_mu, std::try_to_lock);
+  if (!lk.owns_lock()) return false;
+  if (!ctx->write_stage && cudaHostAlloc(&ctx->write_stage, kWriteStageBytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->write_stage = nullptr;
+    return false;
+  }
+  const uint64_t chunk = n >= (8u << 20) ? kWriteChunk : n >= (2u << 20) ? kWriteChunk / 2 : kWriteChunk / 4;
+  const uint64_t chunks = (n + chunk - 1) / chunk;
+  const uint32_t cores = std::thread::hardware_concurrency();
+  const uint32_t wanted = uint32_t(std::min<uint64_t>(kWriteThreads, std::max<uint64_t>(2u, n >> 21)));
+  const uint32_t workers = uint32_t(std::min<uint64_t>(chunks, std::max(1u, std::min(wanted, cores / 2u))));
+  cudaError_t status[kWriteThreads] = {};
+  auto work = [&](uint32_t t) {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    cudaEvent_t read[2] = {nullptr, nullptr};
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&read[i], cudaEventDisableTiming);
+    uint32_t use = 0;
+    for (uint64_t c = t; c < chunks && e == cudaSuccess; c += workers, ++use) {
+      uint8_t* slot = static_cast<uint8_t*>(ctx->write_stage) + (2u * t + (use & 1u)) * kWriteChunk;
+      if (use >= 2u) e = cudaEventSynchronize(read[use & 1u]);  // the copy that last read this slot
+      if (e != cudaSuccess) break;
+      const uint64_t off = c * chunk, bytes = std::min(chunk, n - off);
+      copy_past_caches(slot, src + off, bytes);
+      e = cudaMemcpyAsync(dst + off, slot, bytes, cudaMemcpyHostToDevice, ctx->compute);
+      if (e == cudaSuccess) e = cudaEventRecord(read[use & 1u], ctx->compute);
+    }
+    for (cudaEvent_t ev : read)
+      if (ev) cudaEventDestroy(ev);
+    status[t] = e;
+  };
+  std::thread pool[kWriteThreads];
+  uint32_t started = 1;
+  try {
+    for (; started < workers; ++started) pool[started] = std::thread(work, started);
+  } catch (...) {  // no thread to be had: this one takes the remaining shares below
+  }
+  work(0);
+  for (uint32_t t = 1; t < started; ++t) pool[t].join();
+  for (uint32_t t = started; t < workers; ++t) work(t);
+  const cudaError_t done = cudaStreamSynchronize(ctx->compute);  // the slots are free again
+  for (uint32_t t = 0; t < workers; ++t)
+    if (status[t] != cudaSuccess) *err = status[t];
+  if (*err == cudaSuccess) *err = done;
+  return true;
+}
+
+cudaError_t write_host(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n) {
+  cudaError_t e = cudaSuccess;
+  if (n >= kWriteStagedMin) {
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, src) != cudaSuccess) cudaGetLastError();  // not the next launch's error
+    else if (attr.type == cudaMemoryTypeUnregistered && staged_write(ctx, dst, src, n, &e)) return e;
+  }
+  e = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, ctx->compute);
+  // pageable sources are staged before the call returns; pinned ones are not, so wait
+  return e == cudaSuccess ? cudaStreamSynchronize(ctx->compute) : e;
+}
+
+// Quantises with the scale of the tensor itself. The quantiser reads the words that the maximum has left: with another thread's
+// maximum between the two launches it would take that tensor's scale.
+int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout,
+                                  uint8_t* codes, uint8_t* scales, float* g_used) {
+  const float* g = reinterpret_cast<const float*>(ctx->dwords + 2);
+  const char* what = "amax launch";
+  int slot = -1;
+  cudaError_t e;
+  {
+    std::lock_guard<std::mutex> lk(ctx->scale_mu);
+    if (g_used && ctx->scale_free) {
+      slot = __builtin_ctzll(ctx->scale_free);
+      ctx->scale_free &= ctx->scale_free - 1u;
+    }
+    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->sm_count,
+                          ctx->compute);
+    if (e == cudaSuccess) {
+      what = "quantise launch";
+      e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute);
+    }
+    if (e == cudaSuccess && g_used && slot < 0) {  // every word is a waiting call's
+      what = "global scale read";
+      e = cudaMemcpyAsync(g_used, g, 4, cudaMemcpyDeviceToHost, ctx->compute);
+    }
+  }
+  if (e == cudaSuccess && g_used) {
+    what = "quantise sync";
+    e = cudaStreamSynchronize(ctx->compute);
+    if (e == cudaSuccess && slot >= 0) *g_used = *static_cast<volatile float*>(ctx->scale_host + slot);
+  }
+  if (slot >= 0) {
+    std::lock_guard<std::mutex> lk(ctx->scale_mu);
+    ctx->scale_free |= 1ull << slot;
+  }
+  return e == cudaSuccess ? TNF_OK : cuda_fail(e, what);
+}
+
 }  // namespace tnf
 
 using namespace tnf;
@@ -511,7 +720,8 @@ int32_t tnf_destroy(tnf_ctx* ctx) {
   cudaDeviceSynchronize();
   tnf_comm_teardown(ctx);
   for (auto& kv : ctx->bufs)
-    if (kv.second.owned) cudaFree(kv.second.ptr);
+    if (kv.second.owned && !kv.second.slab) cudaFree(kv.second.ptr);
+  for (auto& kv : ctx->slabs) cudaFree(kv.second.ptr);
   for (auto& kv : ctx->hosts) {
     if (kv.second.owned) cudaFreeHost(kv.second.ptr);
     else cudaHostUnregister(kv.second.ptr);
@@ -569,61 +779,6 @@ static int32_t raw_range(tnf_ctx* ctx, uint64_t id, uint64_t off, uint64_t n, co
   return TNF_OK;
 }
 
-// Large writes from pageable memory. A plain copy stages those through one thread; here up to kWriteThreads threads copy into
-// pinned slots of their own (two each, so that a slot's DMA runs under the other's copy) and put the chunks on the compute
-// stream. Measured (ms, plain / four threads / eight; source in the CPU's caches, then not): 16 MB 0.83 / 0.94 / 1.2 and
-// 1.2 / 1.06 / 1.4; 24 MB 1.24 / 1.15 / 1.65 and 2.1 / 1.25 / 1.9; 48 MB 2.5 / 1.7 / 2.3 and 4.5 / 2.0 / 2.4; 96 MB 8.1 / 2.9 / 3.6
-// and 8.9 / 3.1 / 3.6. Hence four, from kWriteStagedMin on. The slots (kWriteStageBytes in all) are made on first use and freed
-// with the context. Returns false when the caller has to copy the plain way (slots in use by another thread's write, no pinned
-// memory to be had); *err is a failed copy.
-constexpr uint32_t kWriteThreads = 4;
-constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 24u << 20;
-static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n, cudaError_t* err) {
-  std::unique_lock<std::mutex> lk(ctx->write_mu, std::try_to_lock);
-  if (!lk.owns_lock()) return false;
-  if (!ctx->write_stage && cudaHostAlloc(&ctx->write_stage, kWriteStageBytes, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->write_stage = nullptr;
-    return false;
-  }
-  const uint64_t chunks = (n + kWriteChunk - 1) / kWriteChunk;
-  const uint32_t cores = std::thread::hardware_concurrency();
-  const uint32_t workers = uint32_t(std::min<uint64_t>(chunks, std::max(1u, std::min(kWriteThreads, cores / 2u))));
-  cudaError_t status[kWriteThreads] = {};
-  auto work = [&](uint32_t t) {
-    cudaError_t e = cudaSetDevice(ctx->device);
-    cudaEvent_t read[2] = {nullptr, nullptr};
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&read[i], cudaEventDisableTiming);
-    uint32_t use = 0;
-    for (uint64_t c = t; c < chunks && e == cudaSuccess; c += workers, ++use) {
-      uint8_t* slot = static_cast<uint8_t*>(ctx->write_stage) + (2u * t + (use & 1u)) * kWriteChunk;
-      if (use >= 2u) e = cudaEventSynchronize(read[use & 1u]);  // the copy that last read this slot
-      if (e != cudaSuccess) break;
-      const uint64_t off = c * kWriteChunk, bytes = std::min(kWriteChunk, n - off);
-      std::memcpy(slot, src + off, bytes);
-      e = cudaMemcpyAsync(dst + off, slot, bytes, cudaMemcpyHostToDevice, ctx->compute);
-      if (e == cudaSuccess) e = cudaEventRecord(read[use & 1u], ctx->compute);
-    }
-    for (cudaEvent_t ev : read)
-      if (ev) cudaEventDestroy(ev);
-    status[t] = e;
-  };
-  std::thread pool[kWriteThreads];
-  uint32_t started = 1;
-  try {
-    for (; started < workers; ++started) pool[started] = std::thread(work, started);
-  } catch (...) {  // no thread to be had: this one takes the remaining shares below
-  }
-  work(0);
-  for (uint32_t t = 1; t < started; ++t) pool[t].join();
-  for (uint32_t t = started; t < workers; ++t) work(t);
-  const cudaError_t done = cudaStreamSynchronize(ctx->compute);  // the slots are free again
-  for (uint32_t t = 0; t < workers; ++t)
-    if (status[t] != cudaSuccess) *err = status[t];
-  if (*err == cudaSuccess) *err = done;
-  return true;
-}
-
 int32_t tnf_write(tnf_ctx* ctx, uint64_t id, uint64_t dst_off, const void* src, uint64_t n) {
   TNF_CHECK_CTX(ctx);
   if (dst_off % 4 || n % 4) {  // same rule as Backend::write_buffer
@@ -635,18 +790,7 @@ int32_t tnf_write(tnf_ctx* ctx, uint64_t id, uint64_t dst_off, const void* src, 
   uint8_t* p = nullptr;
   int32_t st = raw_range(ctx, id, dst_off, n, "tnf_write", &p);
   if (st != TNF_OK) return st;
-  if (n >= kWriteStagedMin) {
-    cudaPointerAttributes attr;
-    cudaError_t e = cudaPointerGetAttributes(&attr, src);
-    if (e != cudaSuccess) {
-      cudaGetLastError();  // not the next launch's error
-    } else if (attr.type == cudaMemoryTypeUnregistered && staged_write(ctx, p, static_cast<const uint8_t*>(src), n, &e)) {
-      return e == cudaSuccess ? TNF_OK : cuda_fail(e, "tnf_write staged copy");
-    }
-  }
-  TNF_CUDA(cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, ctx->compute), "tnf_write copy");
-  // pageable sources are staged before the call returns; pinned ones are not, so wait
-  TNF_CUDA(cudaStreamSynchronize(ctx->compute), "tnf_write sync");
+  TNF_CUDA(write_host(ctx, p, static_cast<const uint8_t*>(src), n), "tnf_write copy");
   return TNF_OK;
 }
 
@@ -905,43 +1049,6 @@ int32_t tnf_selftest_stalled_wait(tnf_ctx* ctx) {
 // ---- quantisers ----------------------------------------------------------------------------------
 
 uint64_t tnf_device_scales_bytes(uint32_t rows, uint32_t k) { return sf_device_bytes(rows, k); }
-
-// Quantises with the scale of the tensor itself. The quantiser reads the words that the maximum has left: with another thread's
-// maximum between the two launches it would take that tensor's scale.
-static int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout,
-                                  uint8_t* codes, uint8_t* scales, float* g_used) {
-  const float* g = reinterpret_cast<const float*>(ctx->dwords + 2);
-  const char* what = "amax launch";
-  int slot = -1;
-  cudaError_t e;
-  {
-    std::lock_guard<std::mutex> lk(ctx->scale_mu);
-    if (g_used && ctx->scale_free) {
-      slot = __builtin_ctzll(ctx->scale_free);
-      ctx->scale_free &= ctx->scale_free - 1u;
-    }
-    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->sm_count,
-                          ctx->compute);
-    if (e == cudaSuccess) {
-      what = "quantise launch";
-      e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute);
-    }
-    if (e == cudaSuccess && g_used && slot < 0) {  // every word is a waiting call's
-      what = "global scale read";
-      e = cudaMemcpyAsync(g_used, g, 4, cudaMemcpyDeviceToHost, ctx->compute);
-    }
-  }
-  if (e == cudaSuccess && g_used) {
-    what = "quantise sync";
-    e = cudaStreamSynchronize(ctx->compute);
-    if (e == cudaSuccess && slot >= 0) *g_used = *static_cast<volatile float*>(ctx->scale_host + slot);
-  }
-  if (slot >= 0) {
-    std::lock_guard<std::mutex> lk(ctx->scale_mu);
-    ctx->scale_free |= 1ull << slot;
-  }
-  return e == cudaSuccess ? TNF_OK : cuda_fail(e, what);
-}
 
 int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint32_t n, uint32_t k, tnf_buf codes,
                             tnf_buf scales, float* global_scale) {

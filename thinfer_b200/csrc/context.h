@@ -19,7 +19,16 @@ struct tnf_buffer_rec {
   uint64_t bytes = 0;
   int category = 0;
   bool owned = true;   // false: registered with tnf_import_symmetric, never freed here
+  uint64_t slab = 0;   // id of the slab that holds it; 0: an allocation of its own
   void* mc = nullptr;  // NVSwitch multicast alias of the same range (imported symmetric buffers only)
+};
+
+// Device memory that loaded weights share. Blocks are handed out one after the other and no byte is handed out twice: a slab goes
+// back to the driver with its last block, by cudaFree, which waits for work that may still use any of them.
+struct tnf_slab {
+  void* ptr = nullptr;
+  uint64_t used = 0;  // bytes handed out
+  uint32_t live = 0;  // blocks that have not been freed
 };
 
 struct tnf_host_rec {
@@ -91,6 +100,11 @@ struct tnf_ctx {
   void* stage_host[2] = {nullptr, nullptr};
   cudaEvent_t stage_done[2] = {nullptr, nullptr};
   uint64_t stage_bytes = 0;
+  // tnf_load_weight: the slabs, the one that takes further blocks, and the staging that the loads use in turn
+  std::unordered_map<uint64_t, tnf_slab> slabs;
+  uint64_t next_slab = 1, open_slab = 0;
+  uint64_t load_stage_id = 0, load_stage_bytes = 0;
+  bool load_busy = false;
   // large writes from pageable memory: pinned slots of the copying threads, one such write at a time
   std::mutex write_mu;
   void* write_stage = nullptr;
@@ -105,8 +119,15 @@ int32_t cuda_fail(cudaError_t e, const char* what);
 uint8_t* resolve(tnf_ctx* ctx, const tnf_buf& b, uint64_t need_bytes, const char* name, int32_t* status);
 // Multicast alias of a view already validated by resolve(); null (error set) if its buffer has none.
 uint8_t* resolve_multicast(tnf_ctx* ctx, const tnf_buf& b, const char* name, int32_t* status);
-int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id);
+int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id, bool slab = false);
 int32_t free_locked(tnf_ctx* ctx, uint64_t id);
+// Gives a buffer of a slab an allocation of its own (same contents), for uses that reach past it: an IPC handle covers an allocation.
+int32_t leave_slab_locked(tnf_ctx* ctx, uint64_t id);
+// Host -> device copy on the compute stream; the source may be reused when it returns.
+cudaError_t write_host(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n);
+// Quantises with the scale of the tensor itself, which g_used (may be null) waits for.
+int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout, uint8_t* codes,
+                           uint8_t* scales, float* g_used);
 // Frees idle pool buffers, smallest class first, until `at_least` bytes are back; returns the bytes freed.
 uint64_t ws_spill_locked(tnf_ctx* ctx, uint64_t at_least);
 bool get_map(tnf_ctx* ctx, const MapSpec& spec, CUtensorMap* out);  // copies the (cached) map out under the lock
