@@ -633,23 +633,27 @@ cudaError_t write_host(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t 
 
 // Quantises with the scale of the tensor itself. The quantiser reads the words that the maximum has left: with another thread's
 // maximum between the two launches it would take that tensor's scale.
-int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout,
-                                  uint8_t* codes, uint8_t* scales, float* g_used) {
+int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t rows, uint32_t k, bool device_layout, uint8_t* codes,
+                           uint8_t* scales, float* g_used) {
   const float* g = reinterpret_cast<const float*>(ctx->dwords + 2);
   const char* what = "amax launch";
   int slot = -1;
+  volatile uint32_t* word = nullptr;
+  constexpr uint32_t kPending = 0xFFFFFFFFu;  // no scale has these bits
   cudaError_t e;
   {
     std::lock_guard<std::mutex> lk(ctx->scale_mu);
     if (g_used && ctx->scale_free) {
       slot = __builtin_ctzll(ctx->scale_free);
       ctx->scale_free &= ctx->scale_free - 1u;
+      word = reinterpret_cast<volatile uint32_t*>(ctx->scale_host + slot);
+      *word = kPending;
     }
-    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, slot >= 0 ? ctx->scale_host + slot : nullptr, ctx->sm_count,
-                          ctx->compute);
+    e = launch_amax_scale(src, dtype, uint64_t(rows) * k, ctx->dwords + 1, ctx->sm_count, ctx->compute);
     if (e == cudaSuccess) {
       what = "quantise launch";
-      e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute);
+      e = launch_quantize(src, dtype, rows, k, g, 0.0f, codes, scales, device_layout, ctx->compute, ctx->dwords + 5,
+                          slot >= 0 ? ctx->scale_host + slot : nullptr);
     }
     if (e == cudaSuccess && g_used && slot < 0) {  // every word is a waiting call's
       what = "global scale read";
@@ -658,8 +662,18 @@ int32_t quantize_own_scale(tnf_ctx* ctx, const uint8_t* src, int dtype, uint32_t
   }
   if (e == cudaSuccess && g_used) {
     what = "quantise sync";
-    e = cudaStreamSynchronize(ctx->compute);
-    if (e == cudaSuccess && slot >= 0) *g_used = *static_cast<volatile float*>(ctx->scale_host + slot);
+    // The quantiser's last block writes the word: reading it saves the way through the driver (4352 x 3072 26.2 -> 24.7 us, 100 x 3072 20.5 -> 18.8). A word that does
+    // not come within two milliseconds is waited for there, which also tells why it did not.
+    bool ready = false;
+    if (slot >= 0)
+      for (const auto t0 = std::chrono::steady_clock::now(); !(ready = *word != kPending);) {
+#if defined(__SSE2__)
+        _mm_pause();
+#endif
+        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2)) break;
+      }
+    if (!ready) e = cudaStreamSynchronize(ctx->compute);
+    if (e == cudaSuccess && slot >= 0) *g_used = *reinterpret_cast<volatile float*>(ctx->scale_host + slot);
   }
   if (slot >= 0) {
     std::lock_guard<std::mutex> lk(ctx->scale_mu);

@@ -77,9 +77,9 @@ struct tnf_ctx {
   uint32_t scratch_m = 0, scratch_k = 0;  // shape the scratch was last filled for (0 = never)
   uint64_t wide_id = 0, wide_bytes = 0;   // bf16 image of NVFP4 activations for the mixed arm (workspace category)
   long long wait_limit_cycles = tnf::kDefaultWaitLimitCycles;  // bound of every device-side mbarrier wait
-  // small device words: [0] kernel status, [1..4] amax bits, scale g, 1/(6g), block counter of amax_scale_kernel
+  // small device words: [0] kernel status, [1..4] amax bits, scale g, 1/(6g), block counter of amax_scale_kernel, [5] of quantize_kernel
   uint32_t* dwords = nullptr;
-  // dwords[1..4] belong to one quantisation at a time: its two launches go out under scale_mu. The scale that the device reports
+  // dwords[1..5] belong to one quantisation at a time: its two launches go out under scale_mu. The scale that the device reports
   // to a waiting host call has a mapped pinned word that is that call's until it has read it (bit i of scale_free: word i is free).
   static constexpr uint32_t kScaleSlots = 64;
   std::mutex scale_mu;

@@ -111,10 +111,12 @@ struct GemmParams {
   unsigned long long* trace;   // 4 stamps per K tile (diag bit 16), 256 K tiles
 };
 
-// words: {amax bits (0 between launches), scale g, 1/(6g), block counter (0 between launches)}; host_g: mapped host word or null
-cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, int sm_count, cudaStream_t s);
+// words: {amax bits (0 between launches), scale g, 1/(6g), block counter (0 between launches)}
+cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, int sm_count, cudaStream_t s);
+// host_g: mapped host word that gets the scale when codes and scales are complete, counted in *done (0 between launches); or null
 cudaError_t launch_quantize(const void* src, int dtype, uint32_t rows, uint32_t k, const float* g_ptr, float g_val,
-                            uint8_t* codes, uint8_t* scales, bool device_layout, cudaStream_t s);
+                            uint8_t* codes, uint8_t* scales, bool device_layout, cudaStream_t s, uint32_t* done = nullptr,
+                            float* host_g = nullptr);
 cudaError_t launch_multicast_copy(const uint8_t* src, uint8_t* dst_mc, uint64_t bytes, int sm_count, cudaStream_t s);
 cudaError_t launch_dequant_dense(const uint8_t* codes, const uint8_t* scales_device, uint32_t n, uint32_t k, uint16_t* out_bf16,
                                  cudaStream_t s);

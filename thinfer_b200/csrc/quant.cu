@@ -22,11 +22,11 @@ namespace tnf {
 // the result into the scale amax / (6 * 448) (1.0 for an all-zero tensor) and leaves words[0] and the block counter at
 // zero for the next launch on the stream. HBM-bound: a thread has four 16-byte loads in flight, 2048 threads per SM;
 // bf16 maxima are taken on packed pairs (exact, NaNs dropped as fmaxf drops them).
-// words: {amax bits, scale g, 1/(6g), blocks done}; host_g (mapped host memory, may be null) receives g as well.
+// words: {amax bits, scale g, 1/(6g), blocks done}.
 constexpr uint32_t kAmaxThreads = 512, kAmaxLoads = 4;
 template <typename T>
 __global__ void __launch_bounds__(kAmaxThreads, 4)
-    amax_scale_kernel(const uint4* __restrict__ x, uint64_t n_vec, uint32_t* __restrict__ words, float* host_g) {
+    amax_scale_kernel(const uint4* __restrict__ x, uint64_t n_vec, uint32_t* __restrict__ words) {
   __shared__ float part[kAmaxThreads / 32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with programmatic dependent launch: see internal.h
@@ -66,10 +66,6 @@ __global__ void __launch_bounds__(kAmaxThreads, 4)
   const float gv = a > 0.0f ? __fdiv_rn(a, 2688.0f) : 1.0f;
   words[1] = __float_as_uint(gv);
   words[2] = __float_as_uint(__fdiv_rn(1.0f, __fmul_rn(6.0f, gv)));  // 1/(6g), shared by every block
-  if (host_g) {
-    *reinterpret_cast<volatile float*>(host_g) = gv;
-    __threadfence_system();
-  }
 }
 
 // ---- block quantiser --------------------------------------------------------------------------
@@ -80,12 +76,14 @@ __global__ void __launch_bounds__(kAmaxThreads, 4)
 // there is no half-empty last wave. With the device scale layout the block grid is PADDED (rows up
 // to a multiple of 128, blocks up to k_atoms*4), each aligned group of 4 lanes owns one 4-byte
 // scale word (row r, blocks 4i..4i+3), assembled with shuffles; padding words are written as zero.
-// g_ptr (device: {g, 1/(6g)}) wins over g_val when not null. The launcher guarantees
-// rows_grid*nb_grid < 2^32.
+// g_ptr (device: {g, 1/(6g)}) wins over g_val when not null. With host_g (mapped host memory) the block that
+// finishes last, by the counter *done, which it leaves at zero, writes g there: whoever polls that word knows
+// that codes and scales are complete. The launcher guarantees rows_grid*nb_grid < 2^32.
 template <typename T, bool kDeviceLayout>
 __global__ void __launch_bounds__(256, 6)
     quantize_kernel(const T* __restrict__ src, uint32_t rows, uint32_t k, const float* __restrict__ g_ptr, float g_val,
-                    float inv_t_val, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, uint32_t k_atoms) {
+                    float inv_t_val, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, uint32_t k_atoms, uint32_t* done,
+                    float* host_g) {
   constexpr int kVec = sizeof(T) == 2 ? 2 : 4;  // 16-byte loads per block
   const uint32_t nb = k >> 4;
   const uint32_t nb_grid = kDeviceLayout ? k_atoms * 4u : nb;
@@ -169,6 +167,14 @@ __global__ void __launch_bounds__(256, 6)
 #pragma unroll
     for (int i = 0; i < kVec; ++i) cur[i] = nxt[i];
   }
+  if (host_g) {  // uniform
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicInc(done, gridDim.x - 1u) == gridDim.x - 1u) {
+      __threadfence_system();
+      *reinterpret_cast<volatile float*>(host_g) = g;
+    }
+  }
 }
 
 // canonical [rows, k/16] -> device layout, padding written as zero
@@ -218,17 +224,17 @@ cudaError_t launch_dequant_dense(const uint8_t* codes, const uint8_t* scales_dev
   return cudaGetLastError();
 }
 
-cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, float* host_g, int sm_count, cudaStream_t s) {
+cudaError_t launch_amax_scale(const void* x, int dtype, uint64_t n, uint32_t* words, int sm_count, cudaStream_t s) {
   const uint64_t n_vec = n / (dtype == 1 ? 8 : 4);  // rows are whole 32-element groups
   const uint64_t per_block = kAmaxThreads * kAmaxLoads, resident = uint64_t(sm_count) * 4u;
   const unsigned blocks = unsigned(std::min(std::max<uint64_t>(1, (n_vec + per_block - 1) / per_block), resident));
   const uint4* v = static_cast<const uint4*>(x);
-  return dtype == 1 ? launch_pdl(amax_scale_kernel<__nv_bfloat16>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g)
-                    : launch_pdl(amax_scale_kernel<float>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words, host_g);
+  return dtype == 1 ? launch_pdl(amax_scale_kernel<__nv_bfloat16>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words)
+                    : launch_pdl(amax_scale_kernel<float>, dim3(blocks), dim3(kAmaxThreads), 0, s, v, n_vec, words);
 }
 
 cudaError_t launch_quantize(const void* src, int dtype, uint32_t rows, uint32_t k, const float* g_ptr, float g_val,
-                            uint8_t* codes, uint8_t* scales, bool device_layout, cudaStream_t s) {
+                            uint8_t* codes, uint8_t* scales, bool device_layout, cudaStream_t s, uint32_t* done, float* host_g) {
   const uint32_t k_atoms = sf_k_atoms(k);
   const float inv_t_val = 1.0f / (6.0f * g_val);  // same f32 operations as the device and the oracle
   uint64_t threads = device_layout ? uint64_t((rows + 127u) & ~127u) * (k_atoms * 4u) : uint64_t(rows) * (k >> 4);
@@ -255,12 +261,12 @@ cudaError_t launch_quantize(const void* src, int dtype, uint32_t rows, uint32_t 
   }
   if (dtype == 1) {
     auto* p = (const __nv_bfloat16*)src;
-    if (device_layout) return launch_pdl(quantize_kernel<__nv_bfloat16, true>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms);
-    return launch_pdl(quantize_kernel<__nv_bfloat16, false>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms);
+    if (device_layout) return launch_pdl(quantize_kernel<__nv_bfloat16, true>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms, done, host_g);
+    return launch_pdl(quantize_kernel<__nv_bfloat16, false>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms, done, host_g);
   } else {
     auto* p = (const float*)src;
-    if (device_layout) return launch_pdl(quantize_kernel<float, true>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms);
-    return launch_pdl(quantize_kernel<float, false>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms);
+    if (device_layout) return launch_pdl(quantize_kernel<float, true>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms, done, host_g);
+    return launch_pdl(quantize_kernel<float, false>, dim3(blocks), dim3(256), 0, s, p, rows, k, g_ptr, g_val, inv_t_val, codes, scales, k_atoms, done, host_g);
   }
   return cudaGetLastError();
 }
