@@ -29,6 +29,15 @@ int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, ui
     }
   return p.ctas;
 }
+uint32_t split(uint64_t blocks, uint32_t s_k, const int* clusters) { return tnf::sdpa_split(blocks, s_k, clusters); }
+void split_items(uint32_t s_q, uint64_t pairs, uint32_t* out) {  // {pair, q_first, keys_mode} of every item
+  tnf::SdpaPlan p{};
+  tnf::sdpa_split_plan(s_q, pairs, &p);
+  for (uint32_t it = 0; it < p.items; ++it) {
+    const tnf::SdpaSlot s = tnf::sdpa_slot(p, it);
+    out[3 * it] = s.pair; out[3 * it + 1] = s.q_first; out[3 * it + 2] = s.keys_mode;
+  }
+}
 }
 """
 
@@ -153,3 +162,30 @@ def test_attention_items_are_numbered_in_31_bits(rules):
     n = C.c_uint64()
     assert rules.sdpa_items(C.c_uint32((1 << 31) - 1), C.c_uint64(256), C.c_uint32(148), None, C.byref(n), C.c_uint64(0)) == -1
     assert rules.sdpa_items(C.c_uint32(1 << 20), C.c_uint64(65535), C.c_uint32(148), None, C.byref(n), C.c_uint64(0)) == 148
+
+
+def test_shares_of_the_keys(rules):
+    """Clusters only where all of them fit the chip at once, with two key tiles at least for every CTA, and a cheaper share."""
+    fit = (C.c_int * 9)(0, 0, 74, 45, 36, 27, 20, 14, 14)
+    split = lambda blocks, s_k: rules.split(C.c_uint64(blocks), C.c_uint32(s_k), fit)
+    for blocks in (1, 7, 14, 15, 20, 21, 36, 37, 45, 46, 74, 75, 148, 1 << 40):
+        for tiles in range(1, 140):
+            n = split(blocks, tiles * 128 - 5)
+            assert n == split(blocks, tiles * 128) and 1 <= n <= 8
+            if n > 1:
+                assert blocks <= fit[n] and tiles >= 2 * n and -(-tiles // n) + 4 <= tiles
+            if blocks > 74 or tiles < 8:
+                assert n == 1
+    assert split(1, 1024) == 4 and split(64, 1024) == 1 and split(14, 4096) == 8 and split(48, 2048) == 2 and split(45, 4096) == 3
+    none = (C.c_int * 9)()
+    assert rules.split(C.c_uint64(1), C.c_uint32(1 << 20), none) == 1
+
+
+def test_every_block_has_a_cluster(rules):
+    for s_q in (1, 128, 129, 256, 300, 520, 1111):
+        for pairs in (1, 3, 10):
+            blocks = (s_q + 127) // 128
+            out = np.zeros((pairs * blocks, 3), np.uint32)
+            rules.split_items(C.c_uint32(s_q), C.c_uint64(pairs), out.ctypes.data_as(C.c_void_p))
+            assert sorted((int(p), int(q)) for p, q, _ in out) == [(p, 128 * b) for p in range(pairs) for b in range(blocks)]
+            assert (out[:, 2] == 1).all()

@@ -111,6 +111,27 @@ inline bool sdpa_plan(uint32_t s_q, uint64_t pairs, uint32_t sms, SdpaPlan* p) {
   p->skip = p->full_items % p->ctas;
   return true;
 }
+// CTAs of a cluster that share the keys of one block, 1 for none; `clusters[n]`: clusters of n CTAs that are on the device at once. Few
+// blocks leave SMs idle: all blocks have to be on the chip at once, and of the sizes that allow it the one with the fewest key
+// tiles a CTA wins, the two groups' tiles counted in pairs. Joining the outputs costs about what four tiles take (2.6 us). Measured
+// (us, blocks x key tiles, one CTA / so many): 1 x 8 11.5 / 9.3 (4), 16 x 8 12.0 / 10.0 (4), 64 x 8 12.7 / 13.0 (2, not taken), 8 x 32 30.7 / 13.4 (8),
+// 24 x 32 31.3 / 16.6 (5), 48 x 16 19.0 / 16.7 (2), 48 x 128 108 / 74 (2). More CTAs than fit at once never won.
+inline uint32_t sdpa_split(uint64_t blocks, uint32_t s_k, const int* clusters) {
+  const uint32_t tiles = (s_k + 127u) / 128u;
+  uint32_t best = 1u, cost = tiles;
+  for (uint32_t n = 2; n <= 8u && tiles >= 2u * n; ++n) {
+    const uint32_t share = (tiles + n - 1u) / n, c = (share + 1u) / 2u * 2u + 4u;
+    if (clusters[n] < 0 || blocks > uint64_t(clusters[n]) || c >= cost) continue;
+    best = n;
+    cost = c;
+  }
+  return best;
+}
+// Its plan: every block an item, a cluster each.
+inline void sdpa_split_plan(uint32_t s_q, uint64_t pairs, SdpaPlan* p) {
+  const uint64_t blocks = (uint64_t(s_q) + 127u) / 128u, items = pairs * blocks;
+  *p = SdpaPlan{uint32_t(blocks / 2u), 0u, uint32_t(items - pairs * (blocks & 1u)), uint32_t(items), uint32_t(items), 0u};
+}
 // The items of a CTA: sdpa_first, then sdpa_next until it is not below `items`.
 TNF_HD inline uint32_t sdpa_first_block(const SdpaPlan& p, uint32_t cta) {
   return p.full_items + (cta >= p.skip ? cta - p.skip : 2u * (p.ctas - p.skip) + cta);

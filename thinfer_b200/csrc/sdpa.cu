@@ -8,6 +8,8 @@
 // other's two products. One persistent CTA per SM; an item of its work is one of two shapes:
 //   rows mode   256 query rows of one (head, batch): group g has rows 128g .. 128g+127 and all key tiles
 //   keys mode   128 query rows: group g has the key tiles of parity g; the two outputs are joined at the end
+// With so few blocks of 128 query rows that SMs would idle, a cluster of CTAs takes a block in keys mode, a share of the key tiles
+// each, and joins the outputs through distributed shared memory (kSplit; sdpa_split in rules.h).
 // Rows mode reads K and V once for 256 rows; keys mode halves an item's time, which fills the chip when there are few rows
 // and shortens the last wave (sdpa_plan in rules.h says which item is which). The loads and the first scores of an item run under the
 // previous one's last products and output.
@@ -69,6 +71,7 @@ struct SdpaParams {
   long long wait_limit;
   uint32_t s_q, s_k, h_q, h_kv;
   SdpaPlan plan;
+  uint32_t split;       // CTAs of a cluster that share an item's keys (kSplit)
   uint32_t wide_out;    // out starts on a 32-byte boundary
   float scale_log2;     // scale * log2(e)
 };
@@ -125,6 +128,14 @@ __device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem,
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
@@ -146,18 +157,132 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 struct SdpaItem {
   bool keys_mode;
   uint32_t bb, hq, hkv, q_first, tiles, units;
-  __device__ __forceinline__ SdpaItem(const SdpaParams& p, uint32_t it) {
+  uint32_t tile0 = 0, end;  // first key tile of this CTA, key tiles of the sequence
+  // rank, split: this CTA's share of the keys
+  __device__ __forceinline__ SdpaItem(const SdpaParams& p, uint32_t it, uint32_t rank = 0u, uint32_t split = 1u) {
     const SdpaSlot slot = sdpa_slot(p.plan, it);
     keys_mode = slot.keys_mode != 0u;
     bb = slot.pair / p.h_q;
     hq = slot.pair - bb * p.h_q;
     hkv = (hq * p.h_kv) / p.h_q;
     q_first = slot.q_first;  // first query row within the sequence
-    tiles = (p.s_k + at::kRows - 1u) / at::kRows;
+    end = tiles = (p.s_k + at::kRows - 1u) / at::kRows;
+    if (split > 1u) {
+      tile0 = rank * tiles / split;
+      tiles = (rank + 1u) * tiles / split - tile0;
+    }
     units = keys_mode ? tiles : tiles * 2u;  // (key tile, group) pairs in the order the MMAs are issued
   }
 };
 
+// Joins the outputs of a cluster. Every CTA has its rows' joint O of its two groups, as factor-free sums for its own reference maximum;
+// 16-column unit u goes to CTA u * split / 8, which gets it from all CTAs with their maxima and sums of probabilities, adds them up in
+// the order of the ranks and stores. The units travel as f32 into the K and V stages, whose last reader is done once every CTA has
+// passed the first barrier; [unit][4 columns][row] keeps the accesses of a warp contiguous.
+__device__ __forceinline__ uint32_t split_owner(uint32_t unit, uint32_t split) { return unit * split / 8u; }
+__device__ __forceinline__ uint32_t split_first(uint32_t rank, uint32_t split) { return (rank * 8u + split - 1u) / split; }  // first unit
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void st_cluster_v2(uint32_t addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_shared_v2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __noinline__ void split_output(const SdpaParams& p, const SdpaItem& item, uint32_t rank, uint32_t split, uint32_t sQ, uint32_t sK,
+                                          const float* lut, uint32_t lane_addr, uint32_t g, uint32_t row, bool own, bool other, float m_own, float l_own,
+                                          float m_o, float l_o) {
+  using namespace at;
+  constexpr uint32_t kUnit = 16u * kRows * 4u;  // bytes of a unit
+  const uint32_t per = (8u + split - 1u) / split;  // units of a CTA, at most
+  const float m = fmaxf(own ? m_own : -INFINITY, other ? m_o : -INFINITY);
+  const float e_own = own ? ex2(m_own - m) : 0.0f, e_other = other ? ex2(m_o - m) : 0.0f;
+  const float l = (own ? l_own * e_own : 0.0f) + (other ? l_o * e_other : 0.0f);
+  tc_fence_before();
+  cluster_arrive();
+  cluster_wait();  // every CTA's products are complete: K, V and Q may be overwritten
+  tc_fence_after();
+  for (uint32_t u = g * 4u; u < g * 4u + 4u; ++u) {
+    uint32_t a[16], b[16];
+    if (own) tmem_ld_32x32b_x16(lane_addr + kOCol + g * 128u + u * 16u, a);
+    if (other) tmem_ld_32x32b_x16(lane_addr + kOCol + (g ^ 1u) * 128u + u * 16u, b);
+    tmem_ld_wait();
+    const uint32_t to = split_owner(u, split);
+    const uint32_t dst = mapa_cluster(sK + ((rank * per + u - split_first(to, split)) * kUnit) + row * 16u, to);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      float v[4];
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        v[i] = (own ? __uint_as_float(a[q * 4 + i]) * e_own : 0.0f) + (other ? __uint_as_float(b[q * 4 + i]) * e_other : 0.0f);
+      st_cluster_v4(dst + q * kRows * 16u, v[0], v[1], v[2], v[3]);
+    }
+  }
+  for (uint32_t to = g; to < split; to += 2u) st_cluster_v2(mapa_cluster(sQ + (rank * kRows + row) * 8u, to), m, l);
+  cluster_arrive();
+  cluster_wait();
+  const uint32_t q_in_seq = item.q_first + row;
+  if (q_in_seq >= p.s_q) return;
+  float m_all = -INFINITY, l_all = 0.0f, f[8];
+  for (uint32_t r = 0; r < split; ++r) m_all = fmaxf(m_all, ld_shared_v2(sQ + (r * kRows + row) * 8u).x);
+#pragma unroll
+  for (uint32_t r = 0; r < 8; ++r)
+    if (r < split) {
+      const float2 s = ld_shared_v2(sQ + (r * kRows + row) * 8u);
+      f[r] = ex2(s.x - m_all);
+      l_all += s.y * f[r];
+    }
+  const float inv = 1.0f / l_all;
+  const uint64_t grow = uint64_t(item.bb) * p.s_q + q_in_seq;  // row of the [b * s_q, h_q * 128] matrix
+  const uint32_t first = split_first(rank, split), units = split_first(rank + 1u, split) - first;
+  for (uint32_t i = g; i < units; i += 2u) {
+    float o[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) o[c] = 0.0f;
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r)
+      if (r < split)
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          const float4 v = ld_shared_v4(sK + (r * per + i) * kUnit + q * kRows * 16u + row * 16u);
+          o[q * 4] = fmaf(v.x, f[r], o[q * 4]);
+          o[q * 4 + 1] = fmaf(v.y, f[r], o[q * 4 + 1]);
+          o[q * 4 + 2] = fmaf(v.z, f[r], o[q * 4 + 2]);
+          o[q * 4 + 3] = fmaf(v.w, f[r], o[q * 4 + 3]);
+        }
+    uint32_t w[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = pack_bf16x2(o[2 * c] * inv, o[2 * c + 1] * inv);
+    const uint32_t u = first + i;
+    if (p.out) {
+      uint16_t* dst = p.out + (grow * p.h_q + item.hq) * kD + u * 16u;
+      if (p.wide_out) {
+        st_global_v8(dst, w);
+      } else {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    }
+    if (p.q_codes) {  // as in the kernel's own output, a block at a time
+      uint32_t lo, hi;
+      const uint32_t sc = quant_block16_bf16(w, lut, p.q_inv_t, lo, hi);
+      *reinterpret_cast<uint2*>(p.q_codes + grow * (uint64_t(p.h_q) * 64u) + item.hq * 64u + u * 8u) = make_uint2(lo, hi);
+      p.q_scales[((grow >> 7) * p.q_k_atoms + item.hq * 2u + (u >> 2)) * 512u + (grow & 31u) * 16u + ((grow & 127u) >> 5) * 4u + (u & 3u)] = uint8_t(sc);
+    }
+  }
+}
+
+// kSplit: a cluster of p.split CTAs takes one item, 128 query rows in keys mode, a share of the key tiles each, and joins the outputs
+// through distributed shared memory: for calls whose blocks of query rows leave SMs idle.
+template <bool kSplit>
 __global__ void __launch_bounds__(at::kThreads, 1)
     sdpa_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const SdpaParams p) {
@@ -178,8 +303,10 @@ __global__ void __launch_bounds__(at::kThreads, 1)
   // the warp index as a warp-uniform value: the role branches and the MMA descriptors then live in uniform registers
   // (score MMAs alone: 593 cycles a tile against 617)
   const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;
-  const uint32_t it_first = sdpa_first(p.plan, blockIdx.x);
-  const SdpaItem first(p, it_first);  // before the wait for the previous kernel: its divisions cost nothing there
+  const uint32_t rank = kSplit ? cluster_ctarank() : 0u, split = kSplit ? p.split : 1u;
+  const uint32_t it_first = kSplit ? blockIdx.x / split : sdpa_first(p.plan, blockIdx.x);
+  auto next_item = [&](uint32_t it) { return kSplit ? p.plan.items : sdpa_next(p.plan, blockIdx.x, it); };
+  const SdpaItem first(p, it_first, rank, split);  // before the wait for the previous kernel: its divisions cost nothing there
   const uint32_t last_valid = p.s_k - ((p.s_k - 1u) / kRows) * kRows;  // keys of the last tile
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
@@ -219,7 +346,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     // ---------------- Q and K loader ----------------
     uint32_t n = 0, q_use = 0;
     bool ok = true;
-    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = next_item(it)) {
       const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
       if (q_use > 0 && !mbar_wait_warp(q_empty, (q_use - 1u) & 1u, abort_flag, kStatusProducerTimeout, wait_limit)) break;
       ++q_use;
@@ -241,8 +368,8 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         }
         if (elect_one()) {
           mbar_arrive_expect_tx(k_full + 8 * st, kTile);
-          tma_load_2d(sK + st * kTile, &map_k, k_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + j * kRows));
-          tma_load_2d(sK + st * kTile + kSub, &map_k, k_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + j * kRows));
+          tma_load_2d(sK + st * kTile, &map_k, k_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + (w.tile0 + j) * kRows));
+          tma_load_2d(sK + st * kTile + kSub, &map_k, k_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + (w.tile0 + j) * kRows));
         }
         __syncwarp();
       }
@@ -251,7 +378,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     // ---------------- V loader (its ring frees later than K's: a warp of its own, so that K never waits behind V) ----------------
     uint32_t n = 0;
     bool ok = true;
-    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = next_item(it)) {
       const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
       const uint32_t k_row0 = w.bb * p.s_k;
       for (uint32_t j = 0; j < w.tiles; ++j, ++n) {
@@ -262,8 +389,8 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         }
         if (elect_one()) {
           mbar_arrive_expect_tx(v_full + 8 * st, kTile);
-          tma_load_2d(sV + st * kTile, &map_v, v_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + j * kRows));
-          tma_load_2d(sV + st * kTile + kSub, &map_v, v_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + j * kRows));
+          tma_load_2d(sV + st * kTile, &map_v, v_full + 8 * st, int32_t(w.hkv * kD), int32_t(k_row0 + (w.tile0 + j) * kRows));
+          tma_load_2d(sV + st * kTile + kSub, &map_v, v_full + 8 * st, int32_t(w.hkv * kD + 64), int32_t(k_row0 + (w.tile0 + j) * kRows));
         }
         __syncwarp();
       }
@@ -278,7 +405,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     const uint32_t q_lo0 = uint32_t(make_desc_sw128(sQ)), k_lo0 = uint32_t(k_desc), v_lo0 = uint32_t(v_desc);
     uint32_t n0 = 0, q_use = 0, used0 = 0, used1 = 0;  // key tiles, items and each group's tiles of the items before
     bool ok = true;
-    for (uint32_t it = it_first; it < p.plan.items && ok; it = sdpa_next(p.plan, blockIdx.x, it)) {
+    for (uint32_t it = it_first; it < p.plan.items && ok; it = next_item(it)) {
       const SdpaItem w = it == it_first ? first : SdpaItem(p, it);
       const uint32_t tiles = w.tiles, units = w.units;
       auto tile_of = [&](uint32_t u) { return w.keys_mode ? u : u >> 1; };  // unit u = (key tile, group u & 1)
@@ -321,7 +448,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       for (uint32_t u = 0; u < units && ok; ++u) {
         const uint32_t g = u & 1u, j = tile_of(u), st = (n0 + j) & 1u;
         const uint32_t use = w.keys_mode ? u >> 1 : j, parity = ((g ? used1 : used0) + use) & 1u;
-        const uint32_t k_steps = j + 1u == tiles ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
+        const uint32_t k_steps = w.tile0 + j + 1u == w.end ? (last_valid + 15u) >> 4 : 8u;  // 16 keys each: those past s_k are left out
         const bool next = u + 2u < units;
         const uint32_t v_lo = v_lo0 + st * (kTile >> 4), d_o = tmem_base + kOCol + g * 128u, a_p = tmem_base + g * 128u;
         ok = (!w.keys_mode || u == 0u || wait_v(u)) && mbar_wait_warp(p_part + 8 * g, parity, abort_flag, kStatusMmaTimeout, wait_limit);
@@ -348,6 +475,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         }
         __syncwarp();
       }
+      if (kSplit) break;
       n0 += tiles;
       used0 += w.keys_mode ? (tiles + 1u) >> 1 : tiles;
       used1 += w.keys_mode ? tiles >> 1 : tiles;
@@ -360,13 +488,15 @@ __global__ void __launch_bounds__(at::kThreads, 1)
     uint32_t s0[32], s1[32], s2[32], s3[32];
     uint32_t seen = 0, done = 0;  // key tiles and items of this group so far
     bool ok = true;               // once a wait has given up every later one does at once; the barriers of all items are still met
-    for (uint32_t it = it_first; it < p.plan.items; it = sdpa_next(p.plan, blockIdx.x, it)) {
-      const SdpaItem item(p, it);  // its divisions run while the first scores are on their way
-      const bool keys_mode = item.keys_mode;
-      float m_ref = -INFINITY, l = 0.0f;
+    for (uint32_t it = it_first; it < p.plan.items; it = next_item(it)) {
+      const SdpaItem item(p, it, rank, split);  // its divisions run while the first scores are on their way
+      const bool keys_mode = kSplit || item.keys_mode;
+      // below every finite score, so that a first tile of scores of -inf weighs nothing and a later tile moves m
+      float m_ref = -3.402823466e38f, l = 0.0f;
       uint32_t use = 0;
       const uint32_t j_step = keys_mode ? 2u : 1u;
-      for (uint32_t j = keys_mode ? g : 0u; j * kRows < p.s_k && ok; j += j_step, ++use, ++seen) {
+      for (uint32_t j = (keys_mode ? g : 0u) + (kSplit ? item.tile0 : 0u); (kSplit ? j < item.tile0 + item.tiles : j * kRows < p.s_k) && ok;
+           j += j_step, ++use, ++seen) {
         const uint32_t valid = min(kRows, p.s_k - j * kRows);  // keys of this tile that exist
         // S_g complete; the pipe ran O_g += P_g V of the tile before in front of it, so O_g is complete too
         if (!mbar_wait_warp(s_full + 8 * g, seen & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
@@ -491,7 +621,7 @@ __global__ void __launch_bounds__(at::kThreads, 1)
       // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
       if (ok && use > 0) ok = mbar_wait_warp(o_full + 8 * g, done++ & 1u, abort_flag, kStatusEpilogueTimeout, wait_limit);
       float f_own = 1.0f / l, f_other = 0.0f;
-      const bool other = keys_mode && (g == 1u || p.s_k > kRows);  // the other group has seen a tile
+      const bool other = keys_mode && (g == 1u || (kSplit ? item.tiles > 1u : p.s_k > kRows));  // the other group has seen a tile
       if (keys_mode) {
         m_part[g * 128u + row] = m_ref;
         l_part[g * 128u + row] = l;
@@ -506,6 +636,11 @@ __global__ void __launch_bounds__(at::kThreads, 1)
           f_own = e_own * inv;
           f_other = e_other * inv;
         }
+      }
+      if constexpr (kSplit) {
+        split_output(p, item, rank, split, sQ, sK, inv_d_lut, lane_addr, g, row, use > 0, other, m_ref, l, m_part[(g ^ 1u) * 128u + row],
+                     l_part[(g ^ 1u) * 128u + row]);
+        break;
       }
       tc_fence_after();
       if (ok && __all_sync(0xFFFFFFFFu, *abort_flag == 0u)) {
@@ -571,6 +706,12 @@ __global__ void __launch_bounds__(at::kThreads, 1)
         asm volatile("bar.sync 1, 256;" ::: "memory");
       }
     }
+  }
+  if (kSplit && warp < 4u) {  // the warps without rows: split_output has the others'
+    cluster_arrive();
+    cluster_wait();
+    cluster_arrive();
+    cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -666,15 +807,40 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
   p.s_q = a->s_q; p.s_k = a->s_k; p.h_q = a->h_q; p.h_kv = a->h_kv;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   static PerDeviceOnce once;
+  static int clusters[kMaxDevices][9] = {};  // clusters of 2 .. 8 CTAs that fit the device at once
+  int dev = ctx->device < kMaxDevices ? ctx->device : 0;
   if (once.first_use() >= 0) {
-    cudaError_t e = cudaFuncSetAttribute(sdpa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
+    cudaError_t e = cudaFuncSetAttribute(sdpa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sdpa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
+    for (int n = 2; n <= 8; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(unsigned(ctx->sm_count / n * n));
+      cfg.blockDim = dim3(at::kThreads);
+      cfg.dynamicSmemBytes = at::kSmemBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = unsigned(n);
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters[dev][n], sdpa_kernel<true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters[dev][n] = 0;
+      }
+    }
   }
-  if (!sdpa_plan(a->s_q, uint64_t(a->h_q) * a->b, uint32_t(ctx->sm_count), &p.plan)) {
+  const uint64_t pairs = uint64_t(a->h_q) * a->b;
+  const uint32_t split = sdpa_split(pairs * ((uint64_t(a->s_q) + 127u) / 128u), a->s_k, clusters[dev]);
+  if (split > 1u) {
+    sdpa_split_plan(a->s_q, pairs, &p.plan);
+  } else if (!sdpa_plan(a->s_q, pairs, uint32_t(ctx->sm_count), &p.plan)) {
     set_error("tnf_sdpa: problem too large (b=%u s_q=%u h_q=%u: more than 2^31 work items)", a->b, a->s_q, a->h_q);
     return TNF_ERR_INVALID_ARGUMENT;
   }
-  cudaError_t e = launch_pdl(sdpa_kernel, dim3(p.plan.ctas), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
+  p.split = split;
+  cudaError_t e = split > 1u ? launch_pdl_cluster(sdpa_kernel<true>, dim3(p.plan.items * split), dim3(at::kThreads), split, at::kSmemBytes, ctx->compute, mq, mk, mv, p)
+                             : launch_pdl(sdpa_kernel<false>, dim3(p.plan.ctas), dim3(at::kThreads), at::kSmemBytes, ctx->compute, mq, mk, mv, p);
   if (e != cudaSuccess) return cuda_fail(e, "sdpa launch");
   return TNF_OK;
 }
