@@ -29,6 +29,10 @@ int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, ui
     }
   return p.ctas;
 }
+void skinny(uint32_t m, uint32_t n, uint32_t k, int one, const int* clusters, uint32_t* out) {
+  const tnf::SkinnySplit s = tnf::skinny_split_rule(m, n, k, one != 0, clusters);
+  out[0] = s.ctas; out[1] = s.share;
+}
 uint32_t split(uint64_t blocks, uint32_t s_k, const int* clusters) { return tnf::sdpa_split(blocks, s_k, clusters); }
 void split_items(uint32_t s_q, uint64_t pairs, uint32_t* out) {  // {pair, q_first, keys_mode} of every item
   tnf::SdpaPlan p{};
@@ -189,3 +193,27 @@ def test_every_block_has_a_cluster(rules):
             rules.split_items(C.c_uint32(s_q), C.c_uint64(pairs), out.ctypes.data_as(C.c_void_p))
             assert sorted((int(p), int(q)) for p, q, _ in out) == [(p, 128 * b) for p in range(pairs) for b in range(blocks)]
             assert (out[:, 2] == 1).all()
+
+
+def test_shares_of_k(rules):
+    """Clusters for a few rows: all of them on the chip at once, every CTA with a K tile, all K tiles covered, and no more CTAs than that."""
+    fit = (C.c_int * 9)(0, 0, 74, 45, 36, 27, 20, 14, 14)
+    out = (C.c_uint32 * 2)()
+
+    def split(m, n, k, one, counts=fit):
+        rules.skinny(C.c_uint32(m), C.c_uint32(n), C.c_uint32(k), int(one), counts, out)
+        return out[0], out[1]
+    seen = set()
+    for m in range(1, 17):
+        for n in (8, 128, 136, 1024, 3072, 4736, 4744, 6144, 9472, 9480, 18432, 1 << 20):
+            for k in (32, 256, 288, 1024, 1312, 2048, 3072, 4128, 9216, 14336, 1 << 20):
+                for one in (False, True):
+                    ctas, share = split(m, n, k, one)
+                    seen.add(ctas)
+                    nkt, tiles = -(-k // 256), -(-n // 128)
+                    if ctas > 1:
+                        assert tiles <= fit[ctas] and ctas * share >= nkt > (ctas - 1) * share
+                    assert split(m, n, k, one, (C.c_int * 9)())[0] == 1
+    assert seen >= {1, 2, 3, 4, 5, 6, 8}
+    assert split(1, 3072, 3072, True) == (4, 3) and split(4, 9216, 9216, False) == (2, 18)  # measured choices ...
+    assert split(4, 6144, 1024, True)[0] == 1 and split(1, 4736, 512, True)[0] == 1         # ... and what lost

@@ -377,6 +377,14 @@ static int32_t run_mixed(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* 
   return run_gemm(ctx, a, wide, nullptr, nullptr, true);
 }
 
+static bool overlap(tnf_ctx* ctx, const tnf_buf& x, const tnf_buf& y) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  const auto i = ctx->bufs.find(x.id), j = ctx->bufs.find(y.id);
+  if (i == ctx->bufs.end() || j == ctx->bufs.end()) return false;
+  const uint8_t *p = static_cast<const uint8_t*>(i->second.ptr) + x.offset, *q = static_cast<const uint8_t*>(j->second.ptr) + y.offset;
+  return p < q + y.len && q < p + x.len;
+}
+
 static int32_t check_dims(uint32_t m, uint32_t n, uint32_t k) {
   if (m == 0 || n == 0 || k == 0) {
     set_error("empty problem m=%u n=%u k=%u", m, n, k);
@@ -394,7 +402,8 @@ static int32_t check_dims(uint32_t m, uint32_t n, uint32_t k) {
 }
 
 // shared tail of tnf_linear_nvfp4 / tnf_gemm_nvfp4
-// `a_raw` non-null: the skinny-M kernel takes the bf16 activations themselves (its prologue is the quantiser).
+// `a_raw` non-null: the skinny-M kernel takes the bf16 activations themselves (its prologue is the quantiser) and, with `a_codes` and
+// `a_scales`, leaves the quantised ones there.
 // `a_room`: bytes that may be read from `a_codes` on, where that is more than the operand.
 // `widened`: the dense arm's bf16 activations are the exact image (code x block scale) of NVFP4 activations, so
 // the per-tensor activation scale still has to be applied.
@@ -509,10 +518,13 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
   p.wait_limit = ctx->wait_limit_cycles;
   p.trace = reinterpret_cast<unsigned long long*>(ctx->dwords + 64);
   if (a_raw) {
-    if (skinny_tc_applies(a->m, a->n, a->k)) {
+    p.a_codes = const_cast<uint8_t*>(a_codes);
+    p.a_scales = const_cast<uint8_t*>(a_scales);
+    const SkinnySplit split = skinny_split(a->m, a->n, a->k, ctx->sm_count);
+    if (split.ctas > 1u || skinny_tc_applies(a->m, a->n, a->k)) {
       CUtensorMap mw;
       if (!get_map(ctx, codes_spec(w_codes, a->n, a->k, 128), &mw)) return TNF_ERR_INVALID_ARGUMENT;
-      TNF_CUDA(launch_skinny_tc(mw, a_raw, a->a_global, p, ctx->compute), "nvfp4 skinny-M tensor-core launch");
+      TNF_CUDA(launch_skinny_tc(mw, a_raw, a->a_global, p, split, ctx->compute), "nvfp4 skinny-M tensor-core launch");
       return TNF_OK;
     }
     TNF_CUDA(launch_gemv_nvfp4(a_raw, a->a_global, w_codes, p, ctx->compute), "nvfp4 skinny-M launch");
@@ -1215,6 +1227,10 @@ int32_t tnf_linear_nvfp4(tnf_ctx* ctx, const tnf_linear_args* a) {
     if (st != TNF_OK) return st;
     ctx->scratch_m = a->m;
     ctx->scratch_k = a->k;
+    // one launch, which fills the scratch as the quantiser would; not into its own input, which the quantiser has read by then
+    if (a->flags == 0 && skinny_split(a->m, a->n, a->k, ctx->sm_count).ctas > 1u && !overlap(ctx, a->a_bf16, a->out_bf16))
+      return run_gemm(ctx, a, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
+                      static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), src, false);
     st = quantize_act_impl(ctx, src, a->m, a->k, a->a_global, true,
                            static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
                            static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr);

@@ -48,6 +48,27 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// counts[n]: clusters of n = 2 .. 8 CTAs of this kernel that are on the current device at once (0: none, or not to be told).
+template <typename Kernel>
+inline void max_clusters(Kernel kernel, int threads, size_t smem, int sm_count, int* counts) {
+  for (int n = 2; n <= 8; ++n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(sm_count / n * n));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(n);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&counts[n], kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      counts[n] = 0;
+    }
+  }
+}
+
 // 512-byte scale atoms along K per 128-row block: ceil(K/64) rounded up to a multiple of 4,
 // so that a 256-element K tile always reads four whole, contiguous atoms.
 __host__ __device__ inline uint32_t sf_k_atoms(uint32_t k) { return (((k + 63u) / 64u) + 3u) & ~3u; }
@@ -121,6 +142,7 @@ struct GemmParams {
   uint32_t swiglu;             // pairwise gating epilogue: out[m, j] = silu(v[2j]) * v[2j+1], n/2 output columns
   uint32_t store_bf16;         // 0: skip the bf16 store
   uint32_t wide_q;             // pair kernel: the 32 code bytes of 64 columns start on a 32-byte boundary
+  uint8_t *a_codes, *a_scales; // skinny kernel: where the quantised activations are also left; null: nowhere
   uint32_t* status;            // device status word
   long long wait_limit;        // SM cycles after which a device-side wait gives up (0 = kDefaultWaitLimitCycles)
   uint32_t stall;              // self-test: the producer issues no loads, so the first wait on a loaded stage runs out
@@ -153,7 +175,9 @@ cudaError_t launch_gemm_nvfp4_pair(const CUtensorMap& map_a, const CUtensorMap& 
 // weight's codes as [n, k/2] bytes with a {128 B, 128 rows} box and 128-byte swizzle.
 bool skinny_tc_capable(uint32_t m, uint32_t n, uint32_t k);  // the tensor-core skinny kernel can run this shape
 bool skinny_tc_applies(uint32_t m, uint32_t n, uint32_t k);  // ... and is the faster path for it
-cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& p, cudaStream_t s);
+SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, int sm_count);  // clusters for it; ctas == 1: none
+cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& p, const SkinnySplit& split,
+                             cudaStream_t s);
 bool gemv_applies(uint32_t m, uint32_t n, uint32_t k);
 cudaError_t launch_gemv_nvfp4(const void* a_bf16, float a_global, const uint8_t* w_codes, const GemmParams& p, cudaStream_t s);
 bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool gated, bool peers, int sm_count);  // pair_rule in rules.h

@@ -59,6 +59,33 @@ TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool gated, boo
   return !(tiles2 <= sms / 2u && k > 768u && k <= 2048u && m > 256u && !gated);
 }
 
+// CTAs of a cluster that share the K tiles (256 elements) of 128 output columns of a linear of up to 16 rows, 1 for none, and the K tiles
+// of each. `clusters[n]`: clusters of n CTAs that are on the device at once; all have to be. `one_launch`: the call would otherwise take
+// the skinny kernel without clusters, else quantiser and GEMM. The costs are fitted (10 ns) to 400 shapes of 1 to 16 rows, which the
+// split makes 1.27 times as fast in the geometric mean, the best choice for each 1.27: a start, and per K tile of a CTA its weight and the
+// quantisation of its activations (with 256 threads for up to four rows, 512 for more). Measured (us, without / with clusters): 1 x 3072 x 3072 5.6 /
+// 4.2, 16 x 3072 x 3072 6.8 / 6.0, 1 x 256 x 14336 28.6 / 4.7, 4 x 9216 x 9216 19.8 / 9.8, 16 x 9216 x 14336 28.4 / 17.7; not taken: 4 x 6144 x 1024
+// 3.9 / 4.1, 1 x 4736 x 512 3.2 / 3.5, 16 x 6144 x 2048 6.3 / 6.5, 16 x 256 x 512 4.98 / 4.8.
+struct SkinnySplit {
+  uint32_t ctas, share;
+};
+inline uint32_t skinny_split_threads(uint32_t m) { return m <= 4u ? 256u : 512u; }
+inline SkinnySplit skinny_split_rule(uint32_t m, uint32_t n, uint32_t k, bool one_launch, const int* clusters) {
+  const uint32_t tiles = (n + 127u) / 128u, nkt = (k + 255u) / 256u;
+  const uint64_t per_tile = 84u + 12u * m;  // quarter units: 21 + 3 m
+  uint64_t best = 4u * (one_launch ? 290u : 440u) + nkt * (one_launch ? per_tile : tiles >= 32u ? 136u : 72u);
+  SkinnySplit s{1u, 0u};
+  for (uint32_t c = 2; c <= 8u; ++c) {
+    if (clusters[c] < 0 || tiles > uint32_t(clusters[c]) || nkt < (m <= 4u ? 6u : 4u) || nkt < c || (c == 2u && nkt < (m <= 4u ? 8u : 12u))) continue;
+    const uint32_t share = (nkt + c - 1u) / c;
+    const uint64_t cost = m <= 4u ? 4u * 340u + share * per_tile : 4u * (350u + 4u * m) + share * uint64_t(84u + 7u * m);
+    if (cost >= best) continue;
+    best = cost;
+    s = SkinnySplit{(nkt + share - 1u) / share, share};
+  }
+  return s;
+}
+
 // Tiles that the pair kernel takes whole; each later one runs as two halves of 128 columns. The last wave's are split when every half
 // then finds a pair of its own (and none is empty). An only wave is split as well: the dense arm (FP4 calls of so few tiles take
 // the 1-CTA kernel) 256 x 3072 x 3072 18.7 -> 11.7 us, 700 x 3072 x 3072 19.0 -> 14.6, 512 x 4096 x 12288 61.4 -> 50.3,

@@ -813,22 +813,7 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
     cudaError_t e = cudaFuncSetAttribute(sdpa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sdpa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
     if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
-    for (int n = 2; n <= 8; ++n) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(unsigned(ctx->sm_count / n * n));
-      cfg.blockDim = dim3(at::kThreads);
-      cfg.dynamicSmemBytes = at::kSmemBytes;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = unsigned(n);
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&clusters[dev][n], sdpa_kernel<true>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        clusters[dev][n] = 0;
-      }
-    }
+    max_clusters(sdpa_kernel<true>, at::kThreads, at::kSmemBytes, ctx->sm_count, clusters[dev]);
   }
   const uint64_t pairs = uint64_t(a->h_q) * a->b;
   const uint32_t split = sdpa_split(pairs * ((uint64_t(a->s_q) + 127u) / 128u), a->s_k, clusters[dev]);

@@ -20,6 +20,9 @@
 //   * four warps read the accumulator (lane = W row = output column, register i = activation row i) and apply the
 //     usual epilogue (alpha, bias, tanh-GELU, gated residual, bf16 RNE); consecutive lanes store consecutive
 //     output columns.
+// A CTA's time grows with its K tiles and with the activations it quantises, and a narrow weight makes few CTAs: then a cluster of up to
+// eight shares the K tiles of 128 columns, each quantises its own part of K, and the partial sums meet in distributed shared memory
+// (kSplit; skinny_split_rule in rules.h says when).
 // Every mbarrier wait is bounded; a wait that gives up sets the context's status word and the kernel returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -35,7 +38,7 @@
 namespace tnf {
 
 namespace sk {
-constexpr int kThreads = 256;           // warp 0 loads, warp 1 issues MMAs, warps 4-7 read the accumulator; all quantise A
+// kThreads (256; 512 with clusters and more than four rows): warp 0 loads, warp 1 issues MMAs, warps 4-7 read the accumulator; all quantise A
 constexpr uint32_t kMaxM = 16;          // the MMA's N
 constexpr uint32_t kTileK = 256;        // elements per K tile: 128 bytes of codes per row, four scale atoms
 constexpr uint32_t kWBytes = 128 * 128; // W codes of one stage
@@ -45,6 +48,7 @@ constexpr uint32_t kABytes = kMaxM * 128;  // A codes of one K tile
 constexpr uint32_t kTmemCols = 64;
 constexpr uint32_t kAccCol = 0, kSfwCol = 16, kSfaCol = 32;  // accumulator | W scales (M side) | A scales (N side)
 constexpr uint32_t kSmemMax = 227u * 1024u;
+constexpr uint32_t kRecvMax = 512u * (kMaxM + 7u);  // partial sums that a CTA of a cluster receives: 128 columns x at most split * ceil(m / split) rows
 constexpr uint32_t kSmemTail = 1024u /* alignment slack */ + 2048u /* barriers, holder, flag | quantiser table */;
 }  // namespace sk
 
@@ -57,7 +61,9 @@ struct SkinnyParams {
   uint16_t* out;
   uint32_t* status;
   long long wait_limit;
+  uint8_t *a_codes, *a_scales;  // the quantised activations are also left here (codes [m, k/2], device-layout scales); null: nowhere
   uint32_t m, n, k, k_atoms, ldo, n_offset, act, chain, stages;
+  uint32_t split, share;  // CTAs of a cluster that share the K tiles of 128 output columns, K tiles of each (kSplit)
   float a_global, inv_t, alpha;
 };
 
@@ -71,20 +77,26 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "memory");
 }
 
-__global__ void __launch_bounds__(sk::kThreads, 1)
+// kSplit: a cluster of p.split CTAs shares the K tiles of its 128 W rows; every CTA quantises its own part of K only. The partial sums
+// go through distributed shared memory to the CTA that owns the activation row (row i: CTA i % split), which adds them up in
+// the order of the ranks.
+template <bool kSplit, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
     nvfp4_skinny_tc_kernel(const __grid_constant__ CUtensorMap map_w, const SkinnyParams p) {
   using namespace sk;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // the 128-byte swizzle atoms want 1024
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t S = p.stages;
-  const uint32_t nkt = (p.k + kTileK - 1u) / kTileK;
-  const uint32_t nb = p.k >> 4;
+  const uint32_t rank = kSplit ? cluster_ctarank() : 0u, split = kSplit ? p.split : 1u, tile = kSplit ? blockIdx.x / split : blockIdx.x;
+  const uint32_t all_kt = (p.k + kTileK - 1u) / kTileK, kt0 = kSplit ? min(rank * p.share, all_kt) : 0u;  // this CTA's K tiles
+  const uint32_t nkt = kSplit ? min(p.share, all_kt - kt0) : all_kt, room = kSplit ? p.share : all_kt;
+  const uint32_t b0 = kt0 * 16u, nb = kSplit ? min((p.k >> 4) - b0, nkt * 16u) : p.k >> 4;  // 16-element blocks of a row
   const uint32_t sW = smem_base;                // [S][128 rows][128 B], swizzled by the TMA
   const uint32_t sSfw = sW + S * kWBytes;       // [S][4 atoms]
   const uint32_t sA = sSfw + S * kSfBytes;      // [nkt][16 rows][128 B], swizzled by the prologue
-  const uint32_t sSfa = sA + nkt * kABytes;     // [nkt][4 atoms]
-  const uint32_t sBar = sSfa + nkt * kSfBytes;
+  const uint32_t sSfa = sA + room * kABytes;    // [nkt][4 atoms]
+  const uint32_t sBar = sSfa + room * kSfBytes;
   const uint32_t bar_full = sBar, bar_empty = bar_full + 8u * S, bar_acc = bar_empty + 8u * S;
   const uint32_t tmem_holder = bar_acc + 8u;
   volatile uint32_t* tmem_holder_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_holder - smem_base));
@@ -93,7 +105,8 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   uint8_t* sfa_gen = smem_gen + (sSfa - smem_base);
   float* inv_d_lut = reinterpret_cast<float*>(smem_gen + (sBar + 1024u - smem_base));  // the barriers take < 1 KB
   const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31u;  // warp-uniform: see gemm_nvfp4_pair.cu
-  const uint32_t row0 = blockIdx.x * 128u;  // first W row (output column) of this CTA
+  const uint32_t sRecv = sBar + 2048u;  // kSplit: [rank][row of this CTA][128 columns] f32
+  const uint32_t row0 = tile * 128u;  // first W row (output column) of this CTA
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
   if (tid == 0) {
@@ -112,6 +125,7 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
+  if (kSplit) cluster_arrive();  // waited for before the first access to another CTA's memory
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();
@@ -122,16 +136,16 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
   if (tid < total) {
     const uint32_t row = tid / nb, b = tid - row * nb;
-    const uint4* src = reinterpret_cast<const uint4*>(p.a + uint64_t(row) * p.k + b * 16u);
+    const uint4* src = reinterpret_cast<const uint4*>(p.a + uint64_t(row) * p.k + (b0 + b) * 16u);
     v0 = __ldg(src);
     v1 = __ldg(src + 1);
   }
   // ---- every stage of the ring is requested now ----
-  const uint8_t* sfw_src = p.sfw + uint64_t(blockIdx.x) * p.k_atoms * 512u;
+  const uint8_t* sfw_src = p.sfw + uint64_t(tile) * p.k_atoms * 512u + uint64_t(kt0) * kSfBytes;
   auto load_tile = [&](uint32_t kt, uint32_t stage) {  // one elected lane
     const uint32_t full = bar_full + 8u * stage;
     mbar_arrive_expect_tx(full, kStageBytes);
-    tma_load_2d(sW + stage * kWBytes, &map_w, full, int32_t(kt * 128u), int32_t(row0));
+    tma_load_2d(sW + stage * kWBytes, &map_w, full, int32_t((kt0 + kt) * 128u), int32_t(row0));
     bulk_load_1d(sSfw + stage * kSfBytes, sfw_src + uint64_t(kt) * kSfBytes, kSfBytes, full);
   };
   if (warp == 0 && elect_one())
@@ -139,7 +153,7 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   // ---- prologue: zero A's tiles and scale atoms, then quantise the real rows into them ----
   {
     uint4* z = reinterpret_cast<uint4*>(a_gen);  // sA and sSfa are adjacent
-    const uint32_t n16 = nkt * (kABytes + kSfBytes) / 16u;
+    const uint32_t n16 = room * (kABytes + kSfBytes) / 16u;
     for (uint32_t i = tid; i < n16; i += kThreads) z[i] = make_uint4(0, 0, 0, 0);
   }
   fill_inv_scale_lut(inv_d_lut, p.a_global, tid, kThreads);
@@ -147,7 +161,7 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   for (uint32_t i = tid; i < total; i += kThreads) {
     const uint32_t row = i / nb, b = i - row * nb;
     if (i != tid) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.a + uint64_t(row) * p.k + b * 16u);
+      const uint4* src = reinterpret_cast<const uint4*>(p.a + uint64_t(row) * p.k + (b0 + b) * 16u);
       v0 = __ldg(src);
       v1 = __ldg(src + 1);
     }
@@ -158,11 +172,17 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
     // the 128-byte swizzle stores chunk c of row r at chunk position c ^ (r % 8)
     const uint32_t kt = b >> 4, c = (b & 15u) >> 1;
     *reinterpret_cast<uint2*>(a_gen + kt * kABytes + row * 128u + ((c ^ (row & 7u)) << 4) + (b & 1u) * 8u) = make_uint2(lo, hi);
+    if (kSplit && p.a_codes && tile == 0u) *reinterpret_cast<uint2*>(p.a_codes + uint64_t(row) * (p.k >> 1) + (b0 + b) * 8u) = make_uint2(lo, hi);
     // scale atom b/4: row r (< 32) has its four bytes at r*16, block b at byte b % 4
     sfa_gen[(b >> 2) * 512u + row * 16u + (b & 3u)] = uint8_t(sc);
   }
   fence_proxy_async();  // the MMA and the scale copies read what the threads above wrote
   __syncthreads();
+  if (kSplit && p.a_codes && tile == 0u) {  // one 128-row block: the atoms as they are, rows past m zero
+    const uint4* src = reinterpret_cast<const uint4*>(sfa_gen);
+    uint4* dst = reinterpret_cast<uint4*>(p.a_scales + uint64_t(kt0) * kSfBytes);
+    for (uint32_t i = tid; i < nkt * kSfBytes / 16u; i += kThreads) dst[i] = src[i];
+  }
 
   if (warp == 0) {
     // ---------------- loader: the tiles that did not fit the ring at the start ----------------
@@ -216,36 +236,68 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
     __syncwarp();
   } else if (warp >= 4) {
     // ---------------- epilogue: lane = W row = output column; register i = activation row i ----------------
-    const uint32_t quarter = warp & 3u;
-    const uint32_t n = row0 + quarter * 32u + lane;
+    const uint32_t quarter = warp & 3u, col = quarter * 32u + lane;
+    const uint32_t n = row0 + col;
     // the column's bias and gate are requested before the wait: their latency runs under the main loop
     const float bias = (p.bias && n < p.n) ? bf16_lo(uint32_t(__ldg(p.bias + n))) : 0.0f;
     const float gate = (p.gate && n < p.n) ? bf16_lo(uint32_t(__ldg(p.gate + n))) : 0.0f;
-    if (mbar_wait_bounded(bar_acc, 0, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
+    auto finish = [&](uint32_t i, float acc) {  // activation row i
+      float x = acc * p.alpha;
+      if (p.chain) x = bf16r(x);
+      if (p.bias) {
+        x += bias;
+        if (p.chain) x = bf16r(x);
+      }
+      if (p.act == 1u) {
+        x = p.chain ? gelu_tanh_exact(x) : gelu_tanh_fast(x);
+        if (p.chain) x = bf16r(x);
+      }
+      if (p.gate) x = fmaf(gate, x, bf16_lo(uint32_t(p.residual[uint64_t(i) * p.n + n])));
+      p.out[uint64_t(i) * p.ldo + p.n_offset + n] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+    };
+    const bool reader = warp < 8u;  // the others only help to finish
+    const bool done = reader && mbar_wait_bounded(bar_acc, 0, abort_flag, kStatusEpilogueTimeout, wait_limit);
+    uint32_t r[16];
+    if (done) {
       tc_fence_after();
-      uint32_t r[16];
       tmem_ld_32x32b_x16(tmem_base + ((quarter * 32u) << 16) + kAccCol, r);
       tmem_ld_wait();
-      if (n < p.n) {
-#pragma unroll
-        for (uint32_t i = 0; i < kMaxM; ++i) {
-          if (i < p.m) {
-            float x = __uint_as_float(r[i]) * p.alpha;
-            if (p.chain) x = bf16r(x);
-            if (p.bias) {
-              x += bias;
-              if (p.chain) x = bf16r(x);
-            }
-            if (p.act == 1u) {
-              x = p.chain ? gelu_tanh_exact(x) : gelu_tanh_fast(x);
-              if (p.chain) x = bf16r(x);
-            }
-            if (p.gate) x = fmaf(gate, x, bf16_lo(uint32_t(p.residual[uint64_t(i) * p.n + n])));
-            p.out[uint64_t(i) * p.ldo + p.n_offset + n] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
-          }
-        }
-      }
     }
+    if constexpr (kSplit) {
+      const uint32_t rows = (p.m + split - 1u) / split;  // of a CTA, at most
+      cluster_wait();  // every CTA of the cluster runs
+      if (done)
+#pragma unroll
+        for (uint32_t i = 0; i < kMaxM; ++i)
+          if (i < p.m) {
+            const uint32_t to = i % split;
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_cluster(sRecv + ((rank * rows + i / split) * 128u + col) * 4u, to)),
+                         "f"(__uint_as_float(r[i]))
+                         : "memory");
+          }
+      cluster_arrive();
+      cluster_wait();
+      if (n < p.n && *abort_flag == 0u)
+        for (uint32_t i = rank + ((warp - 4u) >> 2) * split; i < p.m; i += uint32_t(kThreads / 128 - 1) * split) {  // a row for every four warps
+          float acc = 0.0f;
+#pragma unroll 4
+          for (uint32_t c = 0; c < split; ++c) {
+            float v;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(sRecv + ((c * rows + i / split) * 128u + col) * 4u) : "memory");
+            acc += v;
+          }
+          finish(i, acc);
+        }
+    } else if (done && n < p.n) {
+#pragma unroll
+      for (uint32_t i = 0; i < kMaxM; ++i)
+        if (i < p.m) finish(i, __uint_as_float(r[i]));
+    }
+  }
+  if (kSplit && warp < 4u) {  // the epilogue warps have met the others' already
+    cluster_wait();
+    cluster_arrive();
+    cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -253,17 +305,16 @@ __global__ void __launch_bounds__(sk::kThreads, 1)
   if (tid == 0 && *abort_flag != 0u) atomicCAS(p.status, 0u, *abort_flag);
 }
 
-// Ring depth for a K: what is left of shared memory beside A's tiles and scale atoms, at most one stage per K tile. (A shallow
+// Ring depth for `nkt` K tiles: what is left of shared memory beside A's tiles and scale atoms, at most one stage per K tile. (A shallow
 // ring, so that two CTAs share an SM, with the weight asked into L2 beforehand: 8.1 -> 9.2 us at N = 18432, K = 3072.)
-static uint32_t skinny_stages(uint32_t k) {
-  const uint32_t nkt = (k + sk::kTileK - 1u) / sk::kTileK;
-  const uint64_t fixed = uint64_t(nkt) * (sk::kABytes + sk::kSfBytes) + sk::kSmemTail;
+static uint32_t skinny_stages(uint32_t nkt, uint32_t tail = sk::kSmemTail) {
+  const uint64_t fixed = uint64_t(nkt) * (sk::kABytes + sk::kSfBytes) + tail;
   if (fixed >= sk::kSmemMax) return 0;
   return uint32_t(std::min<uint64_t>((sk::kSmemMax - fixed) / sk::kStageBytes, nkt));
 }
 
 bool skinny_tc_capable(uint32_t m, uint32_t n, uint32_t k) {
-  return m >= 1 && m <= sk::kMaxM && k % 32 == 0 && n % 8 == 0 && skinny_stages(k) >= std::min(4u, (k + 255u) / 256u);
+  return m >= 1 && m <= sk::kMaxM && k % 32 == 0 && n % 8 == 0 && skinny_stages((k + 255u) / 256u) >= std::min(4u, (k + 255u) / 256u);
 }
 
 // Every CTA quantises all of A in its prologue, so the kernel's time grows with m * k (0.4 us per row at K = 3072,
@@ -274,7 +325,29 @@ bool skinny_tc_applies(uint32_t m, uint32_t n, uint32_t k) {
   return skinny_tc_capable(m, n, k) && uint64_t(m) * k <= (n >= 12288u ? 24576u : 12288u);
 }
 
-cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& g, cudaStream_t s) {
+// Clusters of 2 .. 8 CTAs with all of an SM's shared memory that fit the device at once.
+static const int* cluster_counts(int sm_count) {
+  static PerDeviceOnce once;
+  static int counts[kMaxDevices][9] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= kMaxDevices) dev = 0;
+  if (once.first_use() >= 0) {
+    const auto kernel = nvfp4_skinny_tc_kernel<true, 512>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sk::kSmemMax)) != cudaSuccess) cudaGetLastError();
+    else max_clusters(kernel, 512, sk::kSmemMax, sm_count, counts[dev]);
+  }
+  return counts[dev];
+}
+
+SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, int sm_count) {
+  if (m < 1 || m > sk::kMaxM || k % 32 || n % 8 || (n + 127u) / 128u > uint32_t(sm_count) / 2u) return SkinnySplit{1u, 0u};
+  const SkinnySplit s = skinny_split_rule(m, n, k, skinny_tc_applies(m, n, k), cluster_counts(sm_count));
+  if (s.ctas > 1u && skinny_stages(s.share, sk::kSmemTail + sk::kRecvMax) < std::min(4u, s.share)) return SkinnySplit{1u, 0u};
+  return s;
+}
+
+cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& g, const SkinnySplit& split, cudaStream_t s) {
   SkinnyParams p{};
   p.a = static_cast<const uint16_t*>(a_bf16);
   p.sfw = g.sfb;
@@ -290,19 +363,31 @@ cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float
   p.n_offset = g.n_offset;
   p.act = g.act;
   p.chain = g.chain;
-  p.stages = skinny_stages(g.k);
+  p.a_codes = g.a_codes;
+  p.a_scales = g.a_scales;
+  const uint32_t nkt = split.ctas > 1u ? split.share : (g.k + sk::kTileK - 1u) / sk::kTileK;
+  const uint32_t tail = sk::kSmemTail + (split.ctas > 1u ? 512u * split.ctas * ((g.m + split.ctas - 1u) / split.ctas) : 0u);
+  p.split = split.ctas;
+  p.share = split.share;
+  p.stages = skinny_stages(nkt, tail);
   p.a_global = a_global;
   p.inv_t = 1.0f / (6.0f * a_global);
   p.alpha = g.alpha;
   if (p.stages == 0) return cudaErrorInvalidValue;
-  const uint32_t nkt = (g.k + sk::kTileK - 1u) / sk::kTileK;
-  const size_t smem = size_t(p.stages) * sk::kStageBytes + size_t(nkt) * (sk::kABytes + sk::kSfBytes) + sk::kSmemTail;
+  const size_t smem = size_t(p.stages) * sk::kStageBytes + size_t(nkt) * (sk::kABytes + sk::kSfBytes) + tail;
   static PerDeviceOnce once;
   if (once.first_use() >= 0) {
-    cudaError_t e = cudaFuncSetAttribute(nvfp4_skinny_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sk::kSmemMax));
+    const int most = int(sk::kSmemMax);
+    cudaError_t e = cudaFuncSetAttribute(nvfp4_skinny_tc_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(nvfp4_skinny_tc_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(nvfp4_skinny_tc_kernel<true, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
   }
-  return launch_pdl(nvfp4_skinny_tc_kernel, dim3((g.n + 127u) / 128u), dim3(sk::kThreads), smem, s, map_w, p);
+  const uint32_t tiles = (g.n + 127u) / 128u, threads = skinny_split_threads(g.m);
+  if (split.ctas > 1u)
+    return launch_pdl_cluster(threads == 256u ? nvfp4_skinny_tc_kernel<true, 256> : nvfp4_skinny_tc_kernel<true, 512>, dim3(tiles * split.ctas),
+                              dim3(threads), split.ctas, smem, s, map_w, p);
+  return launch_pdl(nvfp4_skinny_tc_kernel<false, 256>, dim3(tiles), dim3(256), smem, s, map_w, p);
 }
 
 }  // namespace tnf
