@@ -15,6 +15,8 @@ uint32_t tile_n(uint32_t m, uint32_t n, uint32_t sms) { return tnf::tile_n_rule(
 int pair(uint32_t m, uint32_t n, uint32_t k, int gated, int peers, uint32_t sms) { return tnf::pair_rule(m, n, k, gated != 0, peers != 0, sms); }
 int own_epilogue(uint32_t k, int dense, int gelu, int q, uint32_t tiles, uint32_t pairs) { return tnf::pair_epilogue_rule(k, dense != 0, gelu != 0, q != 0, tiles, pairs); }
 uint32_t map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) { return tnf::map_rows_rule(m, n, k, room); }
+uint32_t a_box(uint32_t m) { return tnf::a_box_rule(m); }
+uint32_t a_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) { return tnf::a_map_rows(m, n, k, room); }
 uint32_t whole_tiles(uint32_t tiles, uint32_t n, uint32_t pairs, int remote) { return tnf::pair_whole_tiles(tiles, n, pairs, remote != 0); }
 // items of every CTA in its order, as {cta, pair, q_first, keys_mode}; the number of CTAs, or -1 when there are too many items
 int64_t sdpa_items(uint32_t s_q, uint64_t pairs, uint32_t sms, uint32_t* out, uint64_t* n, uint64_t room) {
@@ -89,6 +91,20 @@ def test_map_over_few_rows_stays_inside_the_buffer(rules):
                 assert rows == m or (rows - 1) * k // 2 < 128 << 10  # no taller than it has to be
                 if room >= (128 << 10) + k // 2:
                     assert rows * k // 2 >= 128 << 10
+
+
+def test_boxes_over_few_rows(rules):
+    """A box holds every row of its tile; the map covers the box where the buffer has room and never more than the buffer."""
+    for k in (32, 96, 3072, 8992, 14336, 1 << 20):
+        for m in (1, 16, 17, 32, 33, 64, 65, 128, 129, 5000):
+            box = rules.a_box(m)
+            assert box in (32, 64, 128) and box >= min(m, 128)
+            for n in (256, 4096):
+                for room in (0, m * k // 2, box * k // 2, (128 << 10) + k // 2, 1 << 40):
+                    rows = rules.a_rows(m, n, k, C.c_uint64(room))
+                    assert rows >= m and (rows == m or rows * k // 2 <= room)
+                    if n == 4096 and m <= 64 and room >= box * k // 2:
+                        assert rows >= box
 
 
 def test_epilogue_of_the_pair_kernel(rules):

@@ -334,7 +334,7 @@ static int32_t ensure_scratch(tnf_ctx* ctx, uint32_t m, uint32_t k) {
     ctx->scratch_codes_id = 0;
     ctx->scratch_codes_bytes = 0;
     // room for a map of full size (map_rows_rule), but not out of a budget that may be planned to the byte
-    const uint64_t bytes = ctx->budget ? need_codes : std::max(need_codes, kSmallMapBytes + k / 2u);
+    const uint64_t bytes = ctx->budget ? need_codes : std::max({need_codes, kSmallMapBytes + k / 2u, m <= 64u ? uint64_t(a_box_rule(m)) * (k / 2u) : 0u});
     int32_t st = alloc_locked(ctx, bytes, TNF_CAT_WORKSPACE, &ctx->scratch_codes_id);
     if (st != TNF_OK) return st;
     ctx->scratch_codes_bytes = bytes;
@@ -553,9 +553,10 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     TNF_CUDA(launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute), "nvfp4 pair gemm launch");
     return TNF_OK;
   }
-  if (!get_map(ctx, codes_spec(a_codes, map_rows_rule(a->m, a->n, a->k, a_room), a->k, 128), &ma) ||
+  if (!get_map(ctx, codes_spec(a_codes, a_map_rows(a->m, a->n, a->k, a_room), a->k, a_box_rule(a->m)), &ma) ||
       !get_map(ctx, codes_spec(w_codes, a->n, a->k, gemm_tile_n(a->m, a->n, ctx->sm_count)), &mw))
     return TNF_ERR_INVALID_ARGUMENT;
+  p.a_box = a_box_rule(a->m);
   TNF_CUDA(launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute), "nvfp4 gemm launch");
   return TNF_OK;
 }

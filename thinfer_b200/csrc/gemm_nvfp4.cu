@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (kDiag && (p.diag & 8u)) {
             mbar_arrive_expect_tx(full, Cfg::kSfaBytes + Cfg::kSfbBytes);
           } else {
-            mbar_arrive_expect_tx(full, Cfg::kStageBytes);
+            mbar_arrive_expect_tx(full, Cfg::kStageBytes - (kBlockM - p.a_box) * kBlockKBytes);
             tma_load_2d(sA + stage * Cfg::kABytes, &map_a, full, int32_t(kt * kBlockKBytes), int32_t(m0));
             tma_load_2d(sB + stage * Cfg::kBBytes, &map_w, full, int32_t(kt * kBlockKBytes), int32_t(n0));
           }

@@ -128,6 +128,7 @@ struct GemmParams {
   uint32_t ldo, n_offset;
   uint32_t act, chain;
   uint32_t tiles_m, tiles_n;
+  uint32_t a_box;              // 1-CTA kernel: rows of A that a tile loads (a_box_rule; the box of map_a)
   uint32_t band_m;             // pair kernel: row tiles per band of the tile order
   uint32_t full_tiles;         // pair kernel: tiles [0, full_tiles) run whole; each later one as two 128-column halves
   uint8_t* q_codes;            // optional NVFP4 copy of the output: codes [m, n/2] ...

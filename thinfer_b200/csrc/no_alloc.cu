@@ -141,8 +141,8 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
   CUtensorMap ma, mw;
   const uint32_t kb = gemm_pair_kblocks();
   const uint32_t box_bytes = pair ? kb * 32 : 128, swz = box_bytes;  // the pair kernel's stage width sets the box
-  const uint32_t a_rows = pair ? a->m : map_rows_rule(a->m, a->n, a->k, kScratchBytes);
-  if (make_tensor_map(&ma, MapSpec{a_codes, 1, a->k / 2, a_rows, a->k / 2, box_bytes, 128, swz}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
+  const uint32_t a_rows = pair ? a->m : a_map_rows(a->m, a->n, a->k, kScratchBytes);
+  if (make_tensor_map(&ma, MapSpec{a_codes, 1, a->k / 2, a_rows, a->k / 2, box_bytes, pair ? 128u : a_box_rule(a->m), swz}) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
   if (make_tensor_map(&mw, MapSpec{w_codes, 1, a->k / 2, a->n, a->k / 2, box_bytes, pair ? 128u : gemm_tile_n(a->m, a->n, ctx->sm_count), swz}) != TNF_OK)
     return TNF_ERR_INVALID_ARGUMENT;
   if (pair) {
@@ -155,6 +155,7 @@ int32_t tnf_linear_nvfp4_noalloc(tnf_ctx* ctx, const tnf_linear_args* a) {
     if (p.gate && make_tensor_map(&outs[1], pair_out_spec(p.residual, a->m, a->n, a->n)) != TNF_OK) return TNF_ERR_INVALID_ARGUMENT;
     ce = launch_gemm_nvfp4_pair(ma, mw, msa, msb, outs, p, ctx->sm_count, ctx->compute);
   } else {
+    p.a_box = a_box_rule(a->m);
     ce = launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute);
   }
   if (ce != cudaSuccess) return cuda_fail(ce, "nvfp4 gemm launch");

@@ -40,6 +40,18 @@ TNF_HD inline uint32_t map_rows_rule(uint32_t m, uint32_t n, uint32_t k, uint64_
   return rows > m ? uint32_t(rows) : m;
 }
 
+// Rows of A that the 1-CTA GEMM's tiles load. The rows behind them in shared memory hold whatever they held: theirs are other rows of the
+// accumulator, which are not stored. With 128 rows always, half of a K tile's bytes were A's whatever m was. Measured (us, 128 rows / these):
+// 32 x 8640 x 8992 16.0 / 14.5, 64 x 9408 x 8992 with SwiGLU 17.1 / 15.8, 32 x 320 x 4768 with SwiGLU 8.6 / 7.85, 24 x 9408 x 12288 14.4 / 14.1.
+TNF_HD inline uint32_t a_box_rule(uint32_t m) { return m <= 32u ? 32u : m <= 64u ? 64u : 128u; }
+// The map's rows for such boxes: where the map may reach past the operand at all it covers a whole box.
+TNF_HD inline uint32_t a_map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) {
+  const uint32_t rows = map_rows_rule(m, n, k, room), box = a_box_rule(m);
+  if (n < (k % 256u ? 3584u : 2048u) || m > 64u || rows >= box) return rows;
+  const uint64_t fit = room / (k / 2u);
+  return fit >= box ? box : fit > rows ? uint32_t(fit) : rows;
+}
+
 // CTA pairs or single CTAs for an NVFP4 linear. A pair works on a 256 x 256 tile (or a half of it), the 1-CTA kernel on 128 x 128
 // ones: while those fit one wave of CTAs they occupy more SMs, each for less time. Measured (us, quantiser included, pair against
 // 1-CTA): 700 x 3072 x 3072 12.2 / 9.5, 300 x 6144 x 3072 12.2 / 9.2, 384 x 6144 x 12288 24.8 / 19.2; 130 shapes of all epilogues
