@@ -531,7 +531,16 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     return TNF_OK;
   }
   CUtensorMap ma, mw;
-  if (dense || mc_out || gemm_use_pair(a->m, a->n, a->k, p.gate != nullptr, p.n_out > 1u, ctx->sm_count)) {  // only the CTA-pair kernel has the dense arm and the multicast epilogue
+  const uint32_t dense_tile = dense && !mc_out && p.n_out == 1u ? dense_tile_rule(a->m, a->n, q_out, uint32_t(ctx->sm_count)) : 0u;
+  if (dense_tile) {
+    p.a_box = a_box_rule(a->m);
+    if (!get_map(ctx, MapSpec{a_codes, 2, a->k, a->m, uint64_t(a->k) * 2, 64, p.a_box, 128}, &ma) ||
+        !get_map(ctx, MapSpec{w_codes, 2, a->k, a->n, uint64_t(a->k) * 2, 64, dense_tile, 128}, &mw))
+      return TNF_ERR_INVALID_ARGUMENT;
+    TNF_CUDA(launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute), "dense gemm launch");
+    return TNF_OK;
+  }
+  if (dense || mc_out || gemm_use_pair(a->m, a->n, a->k, p.gate != nullptr, p.n_out > 1u, ctx->sm_count)) {  // only the CTA-pair kernel has the multicast epilogue
     const uint32_t kb = gemm_pair_kblocks();
     CUtensorMap msa, msb, outs[kMaxPeers];
     if (dense) {  // bf16 [rows, k]: boxes of 64 elements (128 bytes) x 128 rows, 128-byte swizzle; no scale maps

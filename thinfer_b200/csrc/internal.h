@@ -139,7 +139,7 @@ struct GemmParams {
   uint8_t* q_codes_mc;         //   (bf16 rows, NVFP4 codes, scale words) goes out as multimem.st and lands on
   uint8_t* q_scales_mc;        //   every rank of the group, this one included
   uint32_t dense;              // dense-activation arm: A is bf16 [m,k], W the exact bf16 image of code x block scale
-                               // [n,k]; no scale factors, tcgen05.mma kind::f16 (pair kernel only)
+                               // [n,k]; no scale factors, tcgen05.mma kind::f16
   uint32_t swiglu;             // pairwise gating epilogue: out[m, j] = silu(v[2j]) * v[2j+1], n/2 output columns
   uint32_t store_bf16;         // 0: skip the bf16 store
   uint32_t wide_q;             // pair kernel: the 32 code bytes of 64 columns start on a 32-byte boundary

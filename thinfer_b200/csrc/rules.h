@@ -44,6 +44,7 @@ TNF_HD inline uint32_t map_rows_rule(uint32_t m, uint32_t n, uint32_t k, uint64_
 // accumulator, which are not stored. With 128 rows always, half of a K tile's bytes were A's whatever m was. Measured (us, 128 rows / these):
 // 32 x 8640 x 8992 16.0 / 14.5, 64 x 9408 x 8992 with SwiGLU 17.1 / 15.8, 32 x 320 x 4768 with SwiGLU 8.6 / 7.85, 24 x 9408 x 12288 14.4 / 14.1.
 TNF_HD inline uint32_t a_box_rule(uint32_t m) { return m <= 32u ? 32u : m <= 64u ? 64u : 128u; }
+// The map claims no memory that is not there, not even to load nothing from it: one with further planes that were never loaded faulted.
 // The map's rows for such boxes: where the map may reach past the operand at all it covers a whole box.
 TNF_HD inline uint32_t a_map_rows(uint32_t m, uint32_t n, uint32_t k, uint64_t room) {
   const uint32_t rows = map_rows_rule(m, n, k, room), box = a_box_rule(m);
@@ -69,6 +70,18 @@ TNF_HD inline bool pair_rule(uint32_t m, uint32_t n, uint32_t k, bool gated, boo
   if (peers) return tiles2 >= 32u;
   if (tiles1 <= sms) return false;
   return !(tiles2 <= sms / 2u && k > 768u && k <= 2048u && m > 256u && !gated);
+}
+
+// Width of the 1-CTA kernel's tiles for the dense arm, 0 for the pair kernel: the narrowest that leaves one wave. A CTA's time is its K loop,
+// which the issue of small MMAs bounds (55-60 cycles each up to 64 columns, 80-90 with 128), and the weight of few rows comes in faster the more
+// CTAs have loads in flight. In two waves the pair kernel is the better one (300 x 9216 x 3072 20.1 / 22.8, 512 x 9216 x 14336 89 / 114). Measured
+// (us, pair kernel / these): 16 x 3072 x 3072 12.2 / 8.2, 64 x 4736 x 14336 69.9 / 27.8, 128 x 9216 x 3072 14.5 / 10.4, 512 x 4736 x 3072 18.5 / 13.6,
+// 1 x 256 x 512 4.8 / 3.2; 150 shapes 1.8 times as fast in the geometric mean, the least 1.06 (292 x 4096 x 2976 15.2 / 14.3).
+TNF_HD inline uint32_t dense_tile_rule(uint32_t m, uint32_t n, bool quantised, uint32_t sms) {
+  const uint64_t tm = (uint64_t(m) + 127u) / 128u;
+  for (uint32_t bn = quantised ? 64u : 32u; bn <= 128u; bn *= 2u)
+    if (tm * ((uint64_t(n) + bn - 1u) / bn) <= sms) return bn;
+  return 0u;
 }
 
 // CTAs of a cluster that share the K tiles (256 elements) of 128 output columns of a linear of up to 16 rows, 1 for none, and the K tiles
