@@ -61,6 +61,36 @@ def test_epilogues(backend, m, n, k, mode):
         be.free(buf)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 272, 14336), (2, 9216, 3072), (3, 1008, 4128), (5, 3072, 3072), (16, 144, 1024), (16, 6144, 6176)])
+@pytest.mark.parametrize("chain", [False, True])
+def test_swiglu(backend, m, n, k, chain):
+    """Against the GEMM's epilogue, which takes over where the scratch is filled beforehand: the f32 sums differ in their order only, so that
+    few results are another bf16 value (2^-8 of them at most)."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+
+    be = backend
+    a, (wc, ws, gw), b = _problem(m, n, k, m + n)
+    ga = O.global_scale(O.amax_bf16(a))
+    W = T.Nvfp4Weight.from_packed(be, wc, ws, gw, b)
+    ldo, off = n // 2 + 24, 8
+    ab, got = be.upload(a), []
+    for flags in (L.LINEAR_A_PREQUANTIZED, 0):
+        out = be.upload(np.full((m + 1, ldo), 0x7FC0, np.uint16))
+        sc = be.scope()
+        sc.act_quant_shared(ab, m, k, ga)
+        sc.linear(ab if flags == 0 else None, m, W, ga, out, flags=flags, swiglu=True, chain=chain, n_offset=off, ldo=ldo)
+        be.submit(30000)
+        got.append(be.read_buffer(out, np.uint16).reshape(m + 1, ldo))
+        be.free(out)
+    want, have = (O.bf16_to_f32(g[:m, off: off + n // 2]) for g in got)
+    for i in range(m):
+        assert rel_fro(have[i], want[i]) <= (4e-3 if chain else 1e-3)  # chain: halves of the pair rounded to bf16 before, 2^-8 where they fall the other way
+    assert (got[1][m] == 0x7FC0).all() and (got[1][:m, :off] == 0x7FC0).all() and (got[1][:m, off + n // 2:] == 0x7FC0).all()
+    W.free(be)
+    be.free(ab)
+
+
 @pytest.mark.parametrize("m,n,k", [(16, 1024, 4128), (5, 264, 6144)])
 def test_scratch_holds_the_activations(backend, m, n, k):
     """A call that would have run the quantiser leaves what the quantiser leaves: the shared scratch serves the next call."""

@@ -520,7 +520,7 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
   if (a_raw) {
     p.a_codes = const_cast<uint8_t*>(a_codes);
     p.a_scales = const_cast<uint8_t*>(a_scales);
-    const SkinnySplit split = skinny_split(a->m, a->n, a->k, ctx->sm_count, ctx->device);
+    const SkinnySplit split = skinny_split(a->m, a->n, a->k, swiglu, ctx->sm_count, ctx->device);
     if (split.ctas > 1u || skinny_tc_applies(a->m, a->n, a->k)) {
       CUtensorMap mw;
       if (!get_map(ctx, codes_spec(w_codes, a->n, a->k, 128), &mw)) return TNF_ERR_INVALID_ARGUMENT;
@@ -1238,7 +1238,8 @@ int32_t tnf_linear_nvfp4(tnf_ctx* ctx, const tnf_linear_args* a) {
     ctx->scratch_m = a->m;
     ctx->scratch_k = a->k;
     // one launch, which fills the scratch as the quantiser would; not into its own input, which the quantiser has read by then
-    if (a->flags == 0 && skinny_split(a->m, a->n, a->k, ctx->sm_count, ctx->device).ctas > 1u && !overlap(ctx, a->a_bf16, a->out_bf16))
+    if ((a->flags == 0 || a->flags == TNF_LINEAR_SWIGLU) &&
+        skinny_split(a->m, a->n, a->k, a->flags != 0, ctx->sm_count, ctx->device).ctas > 1u && !overlap(ctx, a->a_bf16, a->out_bf16))
       return run_gemm(ctx, a, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
                       static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), src, false);
     st = quantize_act_impl(ctx, src, a->m, a->k, a->a_global, true,

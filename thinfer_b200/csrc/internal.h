@@ -176,7 +176,7 @@ cudaError_t launch_gemm_nvfp4_pair(const CUtensorMap& map_a, const CUtensorMap& 
 // weight's codes as [n, k/2] bytes with a {128 B, 128 rows} box and 128-byte swizzle.
 bool skinny_tc_capable(uint32_t m, uint32_t n, uint32_t k);  // the tensor-core skinny kernel can run this shape
 bool skinny_tc_applies(uint32_t m, uint32_t n, uint32_t k);  // ... and is the faster path for it
-SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, int sm_count, int device);  // clusters for it; ctas == 1: none
+SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, bool swiglu, int sm_count, int device);  // clusters for it; ctas == 1: none
 cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& p, const SkinnySplit& split,
                              cudaStream_t s);
 bool gemv_applies(uint32_t m, uint32_t n, uint32_t k);

@@ -91,6 +91,8 @@ TNF_HD inline uint32_t dense_tile_rule(uint32_t m, uint32_t n, bool quantised, u
 // quantisation of its activations (with 256 threads for up to four rows, 512 for more). Measured (us, without / with clusters): 1 x 3072 x 3072 5.6 /
 // 4.2, 16 x 3072 x 3072 6.8 / 6.0, 1 x 256 x 14336 28.6 / 4.7, 4 x 9216 x 9216 19.8 / 9.8, 16 x 9216 x 14336 28.4 / 17.7; not taken: 4 x 6144 x 1024
 // 3.9 / 4.1, 1 x 4736 x 512 3.2 / 3.5, 16 x 6144 x 2048 6.3 / 6.5, 16 x 256 x 512 4.98 / 4.8.
+// SwiGLU, which would otherwise always take two launches: 150 shapes 1.44 times as fast, none slower (1 x 3072 x 3072 6.8 / 4.0, 8 x 9216 x 3072 8.2 /
+// 6.5, 1 x 9216 x 14336 28.8 / 10.2, 16 x 9216 x 14336 28.8 / 17.7).
 struct SkinnySplit {
   uint32_t ctas, share;
 };
@@ -112,9 +114,8 @@ inline SkinnySplit skinny_split_rule(uint32_t m, uint32_t n, uint32_t k, bool on
 }
 
 // Tiles that the pair kernel takes whole; each later one runs as two halves of 128 columns. The last wave's are split when every half
-// then finds a pair of its own (and none is empty). An only wave is split as well: the dense arm (FP4 calls of so few tiles take
-// the 1-CTA kernel) 256 x 3072 x 3072 18.7 -> 11.7 us, 700 x 3072 x 3072 19.0 -> 14.6, 512 x 4096 x 12288 61.4 -> 50.3,
-// 2048 x 1024 x 4096 23.6 -> 17.1. Not with stores to other GPUs, whose row segments a half would shorten (not measured).
+// then finds a pair of its own (and none is empty). An only wave would be split as well, but calls of so few tiles
+// take the 1-CTA kernel. Not with stores to other GPUs, whose row segments a half would shorten (not measured).
 TNF_HD inline uint32_t pair_whole_tiles(uint32_t tiles, uint32_t n, uint32_t pairs, bool remote) {
   const uint32_t tail = tiles % pairs;
   const bool split = tail > 0u && 2u * tail <= pairs && n % 256u == 0u && !(remote && tiles <= pairs);

@@ -70,6 +70,7 @@ struct SkinnyParams {
 struct SkinnySplitParams : SkinnyParams {
   uint8_t *a_codes, *a_scales;  // the quantised activations are also left here (codes [m, k/2], device-layout scales); null: nowhere
   uint32_t split, share;        // CTAs of a cluster that share the K tiles of 128 output columns, K tiles of each
+  uint32_t swiglu;              // columns 2j and 2j + 1 are one output column, silu(v[2j]) * v[2j + 1]
 };
 template <bool kSplit>
 using SkinnyParamsOf = std::conditional_t<kSplit, SkinnySplitParams, SkinnyParams>;
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
       cluster_arrive();
       cluster_wait();
-      if (n < p.n && *abort_flag == 0u)
+      if (*abort_flag == 0u)
         for (uint32_t i = rank + ((warp - 4u) >> 2) * split; i < p.m; i += uint32_t(kThreads / 128 - 1) * split) {  // a row for every four warps
           float acc = 0.0f;
 #pragma unroll 4
@@ -301,7 +302,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(sRecv + ((c * rows + i / split) * 128u + col) * 4u) : "memory");
             acc += v;
           }
-          finish(i, acc);
+          if (p.swiglu) {  // the column's partner is the neighbouring lane's
+            const float v = p.chain ? bf16r(bf16r(acc * p.alpha) + bias) : fmaf(acc, p.alpha, bias), other = __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+            if ((lane & 1u) == 0u && n < p.n)
+              p.out[uint64_t(i) * p.ldo + p.n_offset + (n >> 1)] = __bfloat16_as_ushort(__float2bfloat16_rn(__fdividef(v, 1.0f + __expf(-v)) * other));
+          } else if (n < p.n) {
+            finish(i, acc);
+          }
         }
     } else if (mbar_wait_bounded(bar_acc, 0, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
       tc_fence_after();
@@ -359,9 +366,9 @@ static const int* cluster_counts(int sm_count, int device) {
   return counts[device];
 }
 
-SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, int sm_count, int device) {
+SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, bool swiglu, int sm_count, int device) {
   if (m < 1 || m > sk::kMaxM || k <= 768u || k % 32 || n % 8 || (n + 127u) / 128u > uint32_t(sm_count) / 2u) return SkinnySplit{1u, 0u};
-  const SkinnySplit s = skinny_split_rule(m, n, k, skinny_tc_applies(m, n, k), cluster_counts(sm_count, device));
+  const SkinnySplit s = skinny_split_rule(m, n, k, !swiglu && skinny_tc_applies(m, n, k), cluster_counts(sm_count, device));
   if (s.ctas > 1u && skinny_stages(s.share, sk::kSmemTail + sk::kRecvMax) < std::min(4u, s.share)) return SkinnySplit{1u, 0u};
   return s;
 }
@@ -388,6 +395,7 @@ cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float
   const uint32_t tail = sk::kSmemTail + (split.ctas > 1u ? 512u * split.ctas * ((g.m + split.ctas - 1u) / split.ctas) : 0u);
   p.split = split.ctas;
   p.share = split.share;
+  p.swiglu = g.swiglu;
   p.stages = skinny_stages(nkt, tail);
   p.a_global = a_global;
   p.inv_t = 1.0f / (6.0f * a_global);
