@@ -1,5 +1,6 @@
 """The dense arm with few rows (the 1-CTA kernel) gives the bits of the CTA-pair kernel, which takes the same rows within a longer operand:
-boxes of 32, 64 and 128 rows, tiles of 32, 64 and 128 columns, K that ends within a box or a stage, every epilogue."""
+boxes of 32, 64 and 128 rows, tiles of 32, 64 and 128 columns, K that ends within a box or a stage, every epilogue. Up to 16 rows
+clusters share K where that pays, and the order of the f32 sums is another one: few results are another bf16 value (2^-8 of them at most)."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 MANY = 1200  # rows: the pair kernel's
 
 
-@pytest.mark.parametrize("n,k", [(256, 32), (1040, 1120), (4736, 96), (4800, 160), (9536, 608), (320, 8992), (19008, 128)])
+@pytest.mark.parametrize("n,k", [(256, 32), (1040, 1120), (4736, 96), (4800, 160), (9536, 608), (320, 8992), (2400, 3104), (3008, 4000), (19008, 128)])
 @pytest.mark.parametrize("form", ["plain", "gelu", "gate", "swiglu", "quantised"])
 def test_few_rows_as_in_a_long_operand(backend, n, k, form):
     import thinfer_b200 as T
@@ -34,7 +35,7 @@ def test_few_rows_as_in_a_long_operand(backend, n, k, form):
     if form == "quantised":
         kw.update(out_nvfp4=(codes, scales, 0.01))
     sc, ref = be.scope(), None
-    for m in (MANY, 128, 100, 65, 64, 33, 32, 17, 1):
+    for m in (MANY, 128, 100, 65, 64, 33, 32, 17, 16, 5, 1):
         be.write_buffer(out, np.full((MANY + 1) * cols, 0x7FC0, np.uint16))
         sc.linear(ab, m, W, 0.0, out, **kw)
         be.submit(30000)
@@ -45,7 +46,12 @@ def test_few_rows_as_in_a_long_operand(backend, n, k, form):
             ref, refq = got, q
             if form == "plain":
                 assert rel_fro(O.bf16_to_f32(got[:16]), O.bf16_to_f32(O.linear(a[:16], 1.0, wc, ws, gw, bias=b, quantize_a=False))) <= 1e-3
-        assert np.array_equal(got[:m], ref[:m]) and np.array_equal(q, refq[:m])
+        if m > 16:
+            assert np.array_equal(got[:m], ref[:m]) and np.array_equal(q, refq[:m])
+        else:
+            for i in range(m):
+                assert rel_fro(O.bf16_to_f32(got[i]), O.bf16_to_f32(ref[i])) <= 1e-3
+            assert (q != refq[:m]).mean() <= 0.01
     W.free(be)
     for buf in (ab, out, codes, scales, gate, res):
         be.free(buf)

@@ -531,11 +531,14 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
     return TNF_OK;
   }
   CUtensorMap ma, mw;
-  const uint32_t dense_tile = dense && !mc_out && p.n_out == 1u ? dense_tile_rule(a->m, a->n, q_out, uint32_t(ctx->sm_count)) : 0u;
-  if (dense_tile) {
+  const DenseTiles tiles = dense && !mc_out && p.n_out == 1u ? dense_tiles(a->m, a->n, a->k, q_out, ctx->sm_count, ctx->device) : DenseTiles{};
+  if (tiles.bn) {
     p.a_box = a_box_rule(a->m);
+    p.tile_n = tiles.bn;
+    p.split = tiles.ctas;
+    p.share = tiles.share;
     if (!get_map(ctx, MapSpec{a_codes, 2, a->k, a->m, uint64_t(a->k) * 2, 64, p.a_box, 128}, &ma) ||
-        !get_map(ctx, MapSpec{w_codes, 2, a->k, a->n, uint64_t(a->k) * 2, 64, dense_tile, 128}, &mw))
+        !get_map(ctx, MapSpec{w_codes, 2, a->k, a->n, uint64_t(a->k) * 2, 64, tiles.bn, 128}, &mw))
       return TNF_ERR_INVALID_ARGUMENT;
     TNF_CUDA(launch_gemm_nvfp4(ma, mw, p, ctx->sm_count, ctx->compute), "dense gemm launch");
     return TNF_OK;

@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 
 #include "epilogue.cuh"
 #include "internal.h"
@@ -39,7 +40,8 @@ constexpr uint32_t kTmemCols = 512;
 // kDense: bf16 activations against the weight's bf16 image. A stage is two or four 128-byte boxes of each operand and no scales, A's boxes
 // of p.a_box rows, and as many stages as fit. Four boxes take off a quarter of the issuing warp's waits where four such stages fit: 69 shapes of
 // up to 64 rows with 32 columns 1.06 times as fast, up to 1.14 with a long K; with fewer stages 0.5-0.98.
-template <int BN, bool kDense>
+// kSplit: a cluster of CTAs shares K (up to 16 rows); the partial sums of the others come into kRecvBytes of the first.
+template <int BN, bool kDense, bool kSplit>
 struct TileCfg {
   // 128-row scale blocks a tile touches: tiles that divide 128 never straddle a block
   static constexpr int kSfbAtoms = (BN % 128 == 0) ? BN / 128 : (128 % BN == 0 ? 1 : (BN + 96 + 127) / 128);
@@ -53,12 +55,13 @@ struct TileCfg {
   static constexpr int kSfbBytes = 2048 * kSfbAtoms;
   static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
   static constexpr int kStages = (BN >= 224) ? 4 : (BN >= 192 ? 5 : (BN >= 128 ? 6 : 7));
-  static constexpr uint32_t kOperandBytes = kDense ? 219u * 1024u : uint32_t(kStages * kStageBytes);
+  static constexpr uint32_t kRecvBytes = kSplit ? 7u * 16u * BN * 4u : 0u;
+  static constexpr uint32_t kOperandBytes = kDense ? 219u * 1024u - kRecvBytes : uint32_t(kStages * kStageBytes);
   static constexpr uint32_t kMaxBoxes = BN == 32 ? 4u : 2u;
   __device__ static uint32_t dense_boxes(uint32_t a_box) { return a_box <= 64u ? kMaxBoxes : 2u; }
   static constexpr int kEpiVecBytes = 4 * 1536;  // per epilogue warp: the tile's bias as f32 (1 KB) and gate as bf16 (512 B)
   static constexpr int kLutBytes = 512;  // 1/(scale*g) per E4M3 code for the quantising epilogue
-  static constexpr int kSmemBytes = kOperandBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kEpiVecBytes + kLutBytes;
+  static constexpr int kSmemBytes = kOperandBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kEpiVecBytes + kLutBytes + kRecvBytes;
   static constexpr uint32_t kAccCol0 = 0;
   static constexpr uint32_t kSfaCol = kAccStages * BN;
   static constexpr uint32_t kSfbCol = kSfaCol + 16;  // within a slot: 16 columns of A scales, then W's
@@ -196,11 +199,11 @@ __device__ __forceinline__ void epilogue_tile_swiglu(const GemmParams& p, uint32
 }
 
 // kQuant: the NVFP4 output and SwiGLU. A kernel of its own: in one kernel with the others the former cost those up to 0.7 %.
-template <int BN, bool kQuant, bool kDense>
+template <int BN, bool kQuant, bool kDense, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       const GemmParams p) {
-  using Cfg = TileCfg<BN, kDense>;
+  using Cfg = TileCfg<BN, kDense, kSplit>;
   const uint32_t stage_boxes = kDense ? Cfg::dense_boxes(p.a_box) : 1u;
   const uint32_t stage_k = kDense ? 64u * stage_boxes : 256u, dense_bytes = stage_boxes * (p.a_box + BN) * kBlockKBytes;
   const uint32_t S = kDense ? min(12u, Cfg::kOperandBytes / dense_bytes) : uint32_t(Cfg::kStages);
@@ -230,7 +233,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t num_tiles = p.tiles_m * p.tiles_n;
   const bool ktr = kDiag && (p.diag & 16u) && blockIdx.x == 0;
 
-  const uint32_t num_k_tiles = (p.k + stage_k - 1) / stage_k;
+  uint32_t num_k_tiles = (p.k + stage_k - 1) / stage_k, kt0 = 0, rank = 0, first_tile = blockIdx.x, tile_step = gridDim.x;
+  if constexpr (kSplit) {  // a CTA has one tile, and of K the stages [kt0, kt0 + num_k_tiles); every CTA of a cluster has some
+    rank = cluster_ctarank();
+    first_tile = blockIdx.x / p.split;
+    tile_step = num_tiles;
+    kt0 = rank * p.share;
+    num_k_tiles = min(p.share, num_k_tiles - kt0);
+  }
   const long long wait_limit = p.wait_limit > 0 ? p.wait_limit : kDefaultWaitLimitCycles;
 
   if (threadIdx.x == 0) {
@@ -255,6 +265,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
+  if (kSplit) cluster_arrive();  // waited for before the first access to another CTA's memory
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder_gen, 0);
   pdl_launch_dependents();
@@ -266,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
         const uint32_t tm = tile % p.tiles_m, tn = tile / p.tiles_m;
         const uint32_t m0 = tm * kBlockM, n0 = tn * BN;
         const uint8_t* sfa_src = p.sfa + uint64_t(tm) * p.k_atoms * 512u;
@@ -282,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (ktr && kt < 16 && lane == 0) p.trace[1240 + kt] = clock64();
           if (kDense) {
             if (elect_one()) {
-              const uint32_t x = kt * stage_k, boxes = min(stage_boxes, (p.k - x + 63u) / 64u);
+              const uint32_t x = (kt0 + kt) * stage_k, boxes = min(stage_boxes, (p.k - x + 63u) / 64u);
               mbar_arrive_expect_tx(full, boxes * (a_box_bytes + Cfg::kBBytes));
               for (uint32_t b = 0; b < boxes; ++b) {
                 tma_load_2d(sB + stage * b_stage + b * Cfg::kBBytes, &map_w, full, int32_t(x + b * 64u), int32_t(n0));
@@ -320,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto d64 = [](uint32_t lo, uint32_t hi) { return (uint64_t(hi) << 32) | lo; };
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, titer = 0;
       bool ok = true, ready = false;
-      for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
         const uint32_t n0 = (tile / p.tiles_m) * BN;
         const uint32_t sfb_shift = (n0 & 127u) >> 5;  // TMEM column shift when the tile starts inside a 128-row scale block
         if (!mbar_wait_warp(bar_acc_empty + 8 * acc, acc_phase ^ 1u, abort_flag, kStatusAccEmptyTimeout, wait_limit)) {
@@ -344,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (elect_one()) {
           const uint32_t a_lo = a_lo0 + stage * (a_stage >> 4), b_lo = b_lo0 + stage * (b_stage >> 4);
           if (kDense) {
-            const uint32_t boxes = min(stage_boxes, (p.k - kt * stage_k + 63u) / 64u);
+            const uint32_t boxes = min(stage_boxes, (p.k - (kt0 + kt) * stage_k + 63u) / 64u);
 #pragma unroll
             for (uint32_t b = 0; b < Cfg::kMaxBoxes; ++b) {
               if (b >= boxes) break;
@@ -396,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t mode = (p.act == 1u ? 1u : 0u) | (p.chain ? 2u : 0u) | (kQuant ? (p.swiglu ? 4u : 0u) : (p.gate ? 4u : 0u));
     uint32_t acc = 0, acc_phase = 0;
     bool ok = true;
-    for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (uint32_t tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
       const uint32_t tm = tile % p.tiles_m, tn = tile / p.tiles_m;
       const uint32_t row = tm * kBlockM + quarter * 32 + lane;
       const uint32_t n0 = tn * BN;
@@ -416,9 +427,55 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!mbar_wait_bounded(bar_acc_full + 8 * acc, acc_phase, abort_flag, kStatusEpilogueTimeout, wait_limit)) {
         ok = false;
-        break;
+        if (!kSplit) break;
       }
       tc_fence_after();
+      if constexpr (kSplit) {
+        // rows 0 .. 15 of the partial sums go to the first CTA, [rank - 1][column / 4][row] float4; its quarter 0 adds them in the order of the
+        // ranks and puts the sum where the accumulator was
+        ok = __all_sync(0xFFFFFFFFu, ok) != 0;
+        const uint32_t recv = sBar + 256 + Cfg::kEpiVecBytes + Cfg::kLutBytes, t0 = tmem_base + Cfg::kAccCol0;
+        cluster_wait();  // every CTA of the cluster runs
+        if (rank != 0u && quarter == 0u && ok) {
+          const uint32_t to = mapa_cluster(recv + ((rank - 1u) * (BN / 4) * 16u + uint32_t(lane)) * 16u, 0u);
+#pragma unroll 1
+          for (uint32_t c = 0; c < BN / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(t0 + c * 32, r);
+            tmem_ld_wait();
+            if (lane < 16)
+#pragma unroll
+              for (uint32_t j = 0; j < 8; ++j)
+                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + (c * 8u + j) * 256u), "r"(r[j * 4]), "r"(r[j * 4 + 1]),
+                             "r"(r[j * 4 + 2]), "r"(r[j * 4 + 3])
+                             : "memory");
+          }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (rank != 0u || quarter != 0u || !ok) break;  // no rows from here on
+#pragma unroll 1
+        for (uint32_t c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t0 + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll 1
+          for (uint32_t q = 1; q < p.split; ++q)
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+              float v[4];
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                           : "r"(recv + (((q - 1u) * (BN / 4) + c * 8u + j) * 16u + uint32_t(lane & 15)) * 16u)
+                           : "memory");
+#pragma unroll
+              for (int e = 0; e < 4; ++e) r[j * 4 + e] = __float_as_uint(__uint_as_float(r[j * 4 + e]) + v[e]);
+            }
+          tmem_st_32x32b_x32(t0 + c * 32, r);
+          tmem_st_wait();
+        }
+      }
       if (ktr && warp == 2 && lane == 0) p.trace[1206] = clock64();
       const uint32_t t_addr = tmem_base + Cfg::kAccCol0 + acc * BN + ((quarter * 32u) << 16);
       {
@@ -453,6 +510,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
 
+  if (kSplit && warp < 2) {  // the epilogue warps have met the others' already
+    __syncwarp();
+    cluster_wait();
+    cluster_arrive();
+    cluster_wait();
+  }
   // ---------------- tear-down ----------------
   tc_fence_before();
   __syncthreads();
@@ -476,13 +539,13 @@ uint32_t gemm_tile_n(uint32_t m, uint32_t n, int sm_count) {
   return tile_n_rule(m, n, uint32_t(sm_count));
 }
 
-template <int BN, bool kQuant, bool kDense>
+template <int BN, bool kQuant, bool kDense, bool kSplit>
 static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w, GemmParams p, int sm_count,
                              cudaStream_t s) {
-  using Cfg = TileCfg<BN, kDense>;
+  using Cfg = TileCfg<BN, kDense, kSplit>;
   static PerDeviceOnce once;
   if (once.first_use() >= 0) {  // the shared-memory opt-in is a per-device attribute of the function
-    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, kQuant, kDense>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, kQuant, kDense, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
   }
   static uint32_t diag = env_u32("TNF_GEMM_DIAG", 0);
@@ -491,23 +554,41 @@ static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w,
   p.tiles_n = (p.n + BN - 1) / BN;
   uint32_t tiles = p.tiles_m * p.tiles_n;
   if (tiles == 0) return cudaSuccess;
+  if constexpr (kSplit)
+    return launch_pdl_cluster(nvfp4_gemm_kernel<BN, kQuant, kDense, kSplit>, dim3(tiles * p.split), dim3(kThreads), p.split, Cfg::kSmemBytes, s, map_a, map_w, p);
   uint32_t grid = std::min<uint32_t>(tiles, uint32_t(sm_count));
-  return launch_pdl(nvfp4_gemm_kernel<BN, kQuant, kDense>, dim3(grid), dim3(kThreads), Cfg::kSmemBytes, s, map_a, map_w, p);
+  return launch_pdl(nvfp4_gemm_kernel<BN, kQuant, kDense, kSplit>, dim3(grid), dim3(kThreads), Cfg::kSmemBytes, s, map_a, map_w, p);
 }
 
-template <int BN, bool kDense>
+template <int BN, bool kDense, bool kSplit = false>
 static cudaError_t launch_bn(const CUtensorMap& map_a, const CUtensorMap& map_w, const GemmParams& p, int sm_count, cudaStream_t s) {
-  return p.q_codes || p.swiglu ? launch_bn<BN, true, kDense>(map_a, map_w, p, sm_count, s)
-                               : launch_bn<BN, false, kDense>(map_a, map_w, p, sm_count, s);
+  return p.q_codes || p.swiglu ? launch_bn<BN, true, kDense, kSplit>(map_a, map_w, p, sm_count, s)
+                               : launch_bn<BN, false, kDense, kSplit>(map_a, map_w, p, sm_count, s);
+}
+
+// Clusters of 2 .. 8 CTAs with all of an SM's shared memory that fit the device at once. The caller's device is the current one.
+DenseTiles dense_tiles(uint32_t m, uint32_t n, uint32_t k, bool quantised, int sm_count, int device) {
+  static std::once_flag once[kMaxDevices];
+  static int counts[kMaxDevices][9] = {};
+  if (device < 0 || device >= kMaxDevices) device = 0;
+  if (m <= 16u)
+    std::call_once(once[device], [&] {
+      const auto kernel = nvfp4_gemm_kernel<128, true, true, true>;
+      constexpr int smem = TileCfg<128, true, true>::kSmemBytes;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) cudaGetLastError();
+      else max_clusters(kernel, kThreads, smem, sm_count, counts[device]);
+    });
+  return dense_tiles_rule(m, n, k, quantised, uint32_t(sm_count), counts[device]);
 }
 
 cudaError_t launch_gemm_nvfp4(const CUtensorMap& map_a, const CUtensorMap& map_w, const GemmParams& p, int sm_count,
                               cudaStream_t s) {
   if (p.dense) {
-    switch (dense_tile_rule(p.m, p.n, p.q_codes != nullptr, uint32_t(sm_count))) {
-      case 32: return launch_bn<32, true>(map_a, map_w, p, sm_count, s);
-      case 64: return launch_bn<64, true>(map_a, map_w, p, sm_count, s);
-      default: return launch_bn<128, true>(map_a, map_w, p, sm_count, s);
+    const bool split = p.split > 1u;
+    switch (p.tile_n) {
+      case 32: return split ? launch_bn<32, true, true>(map_a, map_w, p, sm_count, s) : launch_bn<32, true>(map_a, map_w, p, sm_count, s);
+      case 64: return split ? launch_bn<64, true, true>(map_a, map_w, p, sm_count, s) : launch_bn<64, true>(map_a, map_w, p, sm_count, s);
+      default: return split ? launch_bn<128, true, true>(map_a, map_w, p, sm_count, s) : launch_bn<128, true>(map_a, map_w, p, sm_count, s);
     }
   }
   switch (gemm_tile_n(p.m, p.n, sm_count)) {

@@ -129,6 +129,7 @@ struct GemmParams {
   uint32_t act, chain;
   uint32_t tiles_m, tiles_n;
   uint32_t a_box;              // 1-CTA kernel: rows of A that a tile loads (a_box_rule; the box of map_a)
+  uint32_t tile_n, split, share;  // 1-CTA kernel, dense arm: dense_tiles_rule
   uint32_t band_m;             // pair kernel: row tiles per band of the tile order
   uint32_t full_tiles;         // pair kernel: tiles [0, full_tiles) run whole; each later one as two 128-column halves
   uint8_t* q_codes;            // optional NVFP4 copy of the output: codes [m, n/2] ...
@@ -179,6 +180,7 @@ bool skinny_tc_applies(uint32_t m, uint32_t n, uint32_t k);  // ... and is the f
 SkinnySplit skinny_split(uint32_t m, uint32_t n, uint32_t k, bool swiglu, int sm_count, int device);  // clusters for it; ctas == 1: none
 cudaError_t launch_skinny_tc(const CUtensorMap& map_w, const void* a_bf16, float a_global, const GemmParams& p, const SkinnySplit& split,
                              cudaStream_t s);
+DenseTiles dense_tiles(uint32_t m, uint32_t n, uint32_t k, bool quantised, int sm_count, int device);  // dense_tiles_rule on this device
 bool gemv_applies(uint32_t m, uint32_t n, uint32_t k);
 cudaError_t launch_gemv_nvfp4(const void* a_bf16, float a_global, const uint8_t* w_codes, const GemmParams& p, cudaStream_t s);
 bool gemm_use_pair(uint32_t m, uint32_t n, uint32_t k, bool gated, bool peers, int sm_count);  // pair_rule in rules.h

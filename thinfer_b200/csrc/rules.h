@@ -84,6 +84,36 @@ TNF_HD inline uint32_t dense_tile_rule(uint32_t m, uint32_t n, bool quantised, u
   return 0u;
 }
 
+// With up to 16 rows clusters of CTAs also share K, in stages of 256 elements with 32 columns, else of 128. Cycles: what 64 elements of K take a
+// CTA, or the weight from HBM where that is more, and for the join a start and every further CTA's sums. Only where that leaves four
+// fifths, and in clusters of 2, 4 or 8: of 3, 5 and 6 too few fit beside the launch before (1600 columns in clusters of five, K = 3072: 7.6 us alone,
+// 9.2). Measured (us, alone / clusters): 16 x 256 x 14336 25.2 / 6.8, 1 x 1024 x 3072 7.6 / 5.7, 16 x 1024 x 9216 17.3 / 7.9, 8 x 3072 x 6144 13.6 / 10.9,
+// 16 x 2048 x 14336 25.7 / 12.7; 210 shapes 1.29 times as fast in the geometric mean, the least 0.98; not taken: 16 x 2048 x 1024 4.3 / 5.2,
+// 16 x 9216 x 9216 29.5 / 30.8.
+struct DenseTiles {
+  uint32_t bn, ctas, share;  // bn 0: the pair kernel; ctas 1: no clusters; stages of each CTA
+};
+inline DenseTiles dense_tiles_rule(uint32_t m, uint32_t n, uint32_t k, bool quantised, uint32_t sms, const int* clusters) {
+  DenseTiles t{dense_tile_rule(m, n, quantised, sms), 1u, 0u};
+  if (m > 16u || !t.bn) return t;
+  const uint64_t boxes = (k + 63u) / 64u, hbm = uint64_t(n) * k / 1750u;
+  auto loop = [&](uint32_t bn, uint64_t b) {
+    const uint64_t c = b * (bn == 32u ? 220u : bn == 64u ? 270u : 330u);
+    return c > hbm ? c : hbm;
+  };
+  uint64_t best = loop(t.bn, boxes) * 4u / 5u;
+  for (uint32_t bn = quantised ? 64u : 32u; bn <= 128u; bn *= 2u)
+    for (uint32_t c = 2; c <= 8u; c *= 2u) {
+      const uint32_t per = bn == 32u ? 4u : 2u, stages = (uint32_t(boxes) + per - 1u) / per, share = (stages + c - 1u) / c, ctas = (stages + share - 1u) / share;
+      if (clusters[c] < 0 || (n + bn - 1u) / bn > uint32_t(clusters[c]) || ctas != c) continue;
+      const uint64_t cost = loop(bn, share * per) + 2600u + (c - 1u) * (bn / 32u) * 220u;
+      if (cost >= best) continue;
+      best = cost;
+      t = DenseTiles{bn, c, share};
+    }
+  return t;
+}
+
 // CTAs of a cluster that share the K tiles (256 elements) of 128 output columns of a linear of up to 16 rows, 1 for none, and the K tiles
 // of each. `clusters[n]`: clusters of n CTAs that are on the device at once; all have to be. `one_launch`: the call would otherwise take
 // the skinny kernel without clusters, else quantiser and GEMM. The costs are fitted (10 ns) to 400 shapes of 1 to 16 rows, which the
