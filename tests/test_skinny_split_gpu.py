@@ -17,7 +17,7 @@ def _problem(m, n, k, seed):
 
 
 @pytest.mark.parametrize("m,n,k", [
-    (1, 3072, 3072),    # five CTAs of three K tiles, the last with none left over
+    (1, 3072, 3072),    # four CTAs of three K tiles
     (1, 264, 14336),    # eight CTAs; 8 columns in the last tile; K past what the kernel without clusters can hold
     (3, 1000, 4128),    # 17 K tiles, the last of 32 elements, in uneven shares
     (4, 4736, 6144),    # 37 tiles
@@ -109,6 +109,39 @@ def test_scratch_holds_the_activations(backend, m, n, k):
     sc.act_quant_shared(other, m, k, ga)
     sc.linear(ab, m, W, ga, out)
     sc.linear(None, m, W, ga, out, flags=L.LINEAR_A_PREQUANTIZED)
+    be.submit(30000)
+    assert np.array_equal(be.read_buffer(out, np.uint16), be.read_buffer(ref, np.uint16))
+    W.free(be)
+    for buf in (ab, other, out, ref):
+        be.free(buf)
+
+
+@pytest.mark.parametrize("flaw", ["window", "weight", "bias"])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_refused_call_leaves_its_own_activations(backend, flaw, swiglu):
+    """The quantiser runs ahead of a linear's other checks: after a refused call the scratch holds that call's activations, not an earlier
+    call's under the same shape."""
+    import thinfer_b200 as T
+    from thinfer_b200 import _lib as L
+    from thinfer_b200.backend import InvalidArgument
+
+    be, (m, n, k) = backend, (16, 1024, 4128)
+    a, (wc, ws, gw), b = _problem(m, n, k, 13)
+    ga, cols = O.global_scale(O.amax_bf16(a)), n // 2 if swiglu else n
+    W = T.Nvfp4Weight.from_packed(be, wc, ws, gw, b)
+    ab, other, out, ref = be.upload(a), be.upload(np.roll(a, 1)), be.allocate(m * cols * 2), be.allocate(m * cols * 2)
+    sc = be.scope()
+    sc.act_quant_shared(ab, m, k, ga)
+    sc.linear(None, m, W, ga, ref, flags=L.LINEAR_A_PREQUANTIZED, swiglu=swiglu)
+    sc.act_quant_shared(other, m, k, ga)
+    V = T.Nvfp4Weight(n, k, W.codes, W.scales_device, gw, W.bias)
+    if flaw == "weight":
+        V.codes = L.Buf(W.codes.id, 0, n * k // 2 - 16)
+    if flaw == "bias":
+        V.bias = L.Buf(W.bias.id, 0, 16)
+    with pytest.raises(InvalidArgument):
+        sc.linear(ab, m, V, ga, out, swiglu=swiglu, n_offset=8 if flaw == "window" else 0, ldo=cols)
+    sc.linear(None, m, W, ga, out, flags=L.LINEAR_A_PREQUANTIZED, swiglu=swiglu)
     be.submit(30000)
     assert np.array_equal(be.read_buffer(out, np.uint16), be.read_buffer(ref, np.uint16))
     W.free(be)

@@ -1159,10 +1159,13 @@ int32_t tnf_quantize_act_shared(tnf_ctx* ctx, tnf_buf a_bf16, uint32_t m, uint32
   if (!a) return st;
   st = ensure_scratch(ctx, m, k);
   if (st != TNF_OK) return st;
+  ctx->scratch_m = ctx->scratch_k = 0;
+  st = quantize_act_impl(ctx, a, m, k, global_scale, true, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
+                         static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr);
+  if (st != TNF_OK) return st;
   ctx->scratch_m = m;
   ctx->scratch_k = k;
-  return quantize_act_impl(ctx, a, m, k, global_scale, true, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
-                           static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr);
+  return TNF_OK;
 }
 
 int32_t tnf_prepare_dense(tnf_ctx* ctx, tnf_buf w_codes, tnf_buf w_scales_device, uint32_t n, uint32_t k, tnf_buf out_bf16) {
@@ -1238,17 +1241,22 @@ int32_t tnf_linear_nvfp4(tnf_ctx* ctx, const tnf_linear_args* a) {
     if (!src) return st;
     st = ensure_scratch(ctx, a->m, a->k);
     if (st != TNF_OK) return st;
+    uint8_t* codes = static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr);
+    uint8_t* scales = static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr);
+    ctx->scratch_m = ctx->scratch_k = 0;  // until the launch that fills it has gone out
+    // one launch, which fills the scratch as the quantiser would; not into its own input, which the quantiser has read by then. A call
+    // that is refused there goes on below: the scratch then holds this call's activations, whatever is wrong with its other arguments
+    if ((a->flags == 0 || a->flags == TNF_LINEAR_SWIGLU) &&
+        skinny_split(a->m, a->n, a->k, a->flags != 0, ctx->sm_count, ctx->device).ctas > 1u && !overlap(ctx, a->a_bf16, a->out_bf16) &&
+        run_gemm(ctx, a, codes, scales, src, false) == TNF_OK) {
+      ctx->scratch_m = a->m;
+      ctx->scratch_k = a->k;
+      return TNF_OK;
+    }
+    st = quantize_act_impl(ctx, src, a->m, a->k, a->a_global, true, codes, scales, nullptr);
+    if (st != TNF_OK) return st;
     ctx->scratch_m = a->m;
     ctx->scratch_k = a->k;
-    // one launch, which fills the scratch as the quantiser would; not into its own input, which the quantiser has read by then
-    if ((a->flags == 0 || a->flags == TNF_LINEAR_SWIGLU) &&
-        skinny_split(a->m, a->n, a->k, a->flags != 0, ctx->sm_count, ctx->device).ctas > 1u && !overlap(ctx, a->a_bf16, a->out_bf16))
-      return run_gemm(ctx, a, static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
-                      static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), src, false);
-    st = quantize_act_impl(ctx, src, a->m, a->k, a->a_global, true,
-                           static_cast<uint8_t*>(ctx->bufs[ctx->scratch_codes_id].ptr),
-                           static_cast<uint8_t*>(ctx->bufs[ctx->scratch_scales_id].ptr), nullptr);
-    if (st != TNF_OK) return st;
   } else if (ctx->scratch_m != a->m || ctx->scratch_k != a->k) {
     // the scratch is tagged with the shape it was last filled for: a pre-quantised call for any other shape would
     // multiply stale codes (the scale layout depends on m and k), so it is refused
