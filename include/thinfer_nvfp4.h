@@ -83,7 +83,7 @@ int32_t tnf_read(tnf_ctx* ctx, uint64_t id, uint64_t off, void* dst, uint64_t n)
 /* Backend::copy_buffer_to_buffer (thinfer-core/src/backend/mod.rs:150-160). */
 int32_t tnf_copy(tnf_ctx* ctx, uint64_t src_id, uint64_t src_off, uint64_t dst_id, uint64_t dst_off, uint64_t n);
 /* Raw device address of a buffer, for callers that interoperate with other CUDA code
- * (no reference counterpart: wgpu hides addresses). */
+ * (no reference counterpart: wgpu hides addresses). It is the buffer's for as long as the buffer lives. */
 int32_t tnf_buf_ptr(tnf_ctx* ctx, uint64_t id, void** device_ptr, uint64_t* bytes);
 /* Awaited Backend::submit (thinfer-core/src/backend/wgpu.rs:941-1071): waits for the
  * compute and copy streams, then reports a device-side wait that gave up as
@@ -149,8 +149,7 @@ int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint
                             tnf_buf codes, tnf_buf scales, float* global_scale);
 /* The same from host memory (f32 or bf16 [n,k], pageable or pinned) in one call: makes the buffers (codes [n,k/2], DEVICE-layout
  * scales, and with bias_host the bf16 bias [n]; free each with tnf_free) and fills them. Without a budget the context keeps the
- * staging for the next load (up to 160 MB, given back when an allocation fails) and lets weights share allocations of 64 MB, which
- * go back with their last buffer. bias_host and bias_id may be null. Blocking. */
+ * staging for the next load (up to 160 MB, given back when an allocation fails). bias_host and bias_id may be null. Blocking. */
 int32_t tnf_load_weight(tnf_ctx* ctx, const void* w_host, int32_t src_dtype, uint32_t n, uint32_t k, const uint16_t* bias_host,
                         uint64_t* codes_id, uint64_t* scales_id, uint64_t* bias_id, float* global_scale);
 /* Bytes of the DEVICE scale layout for a [rows,k] operand. */

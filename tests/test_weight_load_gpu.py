@@ -1,5 +1,5 @@
-"""Loading a dense weight in one call: the same bytes as upload + quantise + scale layout, from several threads, through slabs that fill
-up and go, and with a budget; and pageable writes around the sizes where the staged copy changes its chunks."""
+"""Loading a dense weight in one call: the same bytes as upload + quantise + scale layout, from several threads and with a budget, what it
+leaves allocated; and pageable writes around the sizes where the staged copy changes its chunks."""
 import ctypes as C
 import threading
 
@@ -46,8 +46,34 @@ def test_load_equals_its_parts(n, k, bf16, budget):
         assert not budget or live["live_staging"] == 0  # nothing stays where memory is planned
 
 
-def test_slabs_fill_up_and_go(backend):
-    """Weights of 9 MB in slabs of 64: dozens of them, freed in another order, every other one read back after its neighbours went."""
+def test_loads_hold_what_they_account_for(backend):
+    """Device memory in use against the snapshot's live bytes: whole weights, then their biases alone, then nothing."""
+    import torch
+    import thinfer_b200 as T
+
+    be, n, k = backend, 16384, 4096  # codes of 32 MiB, scales of 4
+    w, bias = _weight(n, k, True, 1), O.f32_to_bf16(np.random.default_rng(2).standard_normal(n, np.float32))
+    T.Nvfp4Weight.from_dense(be, w, bias).free(be)
+    be.drain_pool()
+    live = lambda: sum(v for x, v in be.mem_snapshot().items() if x in ("live_weights", "live_workspace", "live_staging"))
+    free0, live0 = torch.cuda.mem_get_info()[0], live()
+    grain = 2 << 20  # the driver's pages: an allocation takes whole ones
+    used = lambda: free0 - torch.cuda.mem_get_info()[0]
+    W = [T.Nvfp4Weight.from_dense(be, w, bias) for _ in range(4)]
+    assert used() <= live() - live0 + 13 * grain  # four times three buffers, and the loads' staging
+    for x in W:
+        be.free(x.codes)
+        be.free(x.scales_device)
+    be.drain_pool()
+    assert live() - live0 == 4 * 2 * n and used() <= live() - live0 + 4 * grain
+    for x in W:
+        assert np.array_equal(be.read_buffer(x.bias, np.uint16), bias)
+        be.free(x.bias)
+    assert live() == live0 and used() <= grain
+
+
+def test_weights_freed_in_another_order(backend):
+    """Two dozen weights of 9 MB: every other one read back after its neighbours went."""
     import thinfer_b200 as T
 
     be, before = backend, backend.mem_snapshot()["live_weights"]
@@ -81,19 +107,18 @@ def test_loads_of_several_threads(backend):
         W.free(backend)
 
 
-def test_exported_weight_leaves_its_slab(backend):
-    """An IPC handle covers an allocation: the buffer gets one of its own, with its contents."""
+def test_exported_weight_stays_where_it_is(backend):
+    """The address of a buffer is the caller's for as long as it lives; every buffer can be exported."""
     import thinfer_b200 as T
     from thinfer_b200.backend import _check as check
 
-    w = _weight(1024, 1024, True, 7)
-    W, V = T.Nvfp4Weight.from_dense(backend, w), T.Nvfp4Weight.from_dense(backend, w)
-    handle, p = C.create_string_buffer(64), backend.device_ptr(V.codes)
-    check(backend.lib.tnf_ipc_export(backend._ctx, V.codes.id, handle))
-    assert backend.device_ptr(V.codes) != p
-    _check(backend, V, w, None)
-    _check(backend, W, w, None)
-    V.free(backend)
+    w, bias = _weight(1024, 1024, True, 7), O.f32_to_bf16(np.ones(1024, np.float32))
+    W = T.Nvfp4Weight.from_dense(backend, w, bias)
+    for buf in (W.codes, W.scales_device, W.bias):
+        handle, p = C.create_string_buffer(64), backend.device_ptr(buf)
+        check(backend.lib.tnf_ipc_export(backend._ctx, buf.id, handle))
+        assert backend.device_ptr(buf) == p
+    _check(backend, W, w, bias)
     W.free(backend)
 
 

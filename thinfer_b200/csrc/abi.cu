@@ -79,60 +79,15 @@ uint8_t* resolve_multicast(tnf_ctx* ctx, const tnf_buf& b, const char* name, int
   return static_cast<uint8_t*>(it->second.mc) + b.offset;
 }
 
-// A block of the open slab, or of a new one; null when there is no memory for a slab. An allocation of its own costs about 330 us and
-// its cudaFree 280, a slab the same: the codes and scales of a loaded weight were half of the time of loading it.
-constexpr uint64_t kSlabBytes = 64u << 20, kSlabMaxBlock = kSlabBytes / 2;
-static void* slab_block(tnf_ctx* ctx, uint64_t bytes, uint64_t* slab_id) {
-  bytes = (bytes + 511u) & ~uint64_t(511);
-  auto open = ctx->slabs.find(ctx->open_slab);
-  if (open == ctx->slabs.end() || open->second.used + bytes > kSlabBytes) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, kSlabBytes) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    if (open != ctx->slabs.end() && open->second.live == 0) {
-      cudaFree(open->second.ptr);
-      ctx->slabs.erase(open);
-    }
-    ctx->open_slab = ctx->next_slab++;
-    open = ctx->slabs.emplace(ctx->open_slab, tnf_slab{p}).first;
-  }
-  void* p = static_cast<uint8_t*>(open->second.ptr) + open->second.used;
-  open->second.used += bytes;
-  open->second.live++;
-  *slab_id = ctx->open_slab;
-  return p;
+// Frees the staging that loads have left, unless one is using it. True when there was some.
+static bool give_back_staging(tnf_ctx* ctx) {
+  const uint64_t id = ctx->load_stage_id;
+  if (!id || ctx->load_busy) return false;
+  ctx->load_stage_id = ctx->load_stage_bytes = 0;
+  return free_locked(ctx, id) == TNF_OK;
 }
 
-// The block's slab loses it; cudaFree with the last one, unless further blocks can still come from it.
-static cudaError_t slab_release(tnf_ctx* ctx, uint64_t slab_id) {
-  auto s = ctx->slabs.find(slab_id);
-  if (--s->second.live > 0 || slab_id == ctx->open_slab) return cudaSuccess;
-  const cudaError_t e = cudaFree(s->second.ptr);
-  ctx->slabs.erase(s);
-  return e;
-}
-
-// What this library holds and nobody uses: the idle staging of loads and an open slab without blocks. True when there was some.
-static bool give_back_idle(tnf_ctx* ctx) {
-  bool any = false;
-  if (ctx->load_stage_id && !ctx->load_busy) {
-    const uint64_t id = ctx->load_stage_id;
-    ctx->load_stage_id = ctx->load_stage_bytes = 0;
-    any = free_locked(ctx, id) == TNF_OK;
-  }
-  auto open = ctx->slabs.find(ctx->open_slab);
-  if (open != ctx->slabs.end() && open->second.live == 0) {
-    cudaFree(open->second.ptr);
-    ctx->slabs.erase(open);
-    ctx->open_slab = 0;
-    any = true;
-  }
-  return any;
-}
-
-int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id, bool slab) {
+int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id) {
   if (category < 0 || category > 2 || bytes == 0) {
     set_error("tnf_alloc: bad category %d or zero size", category);
     return TNF_ERR_INVALID_ARGUMENT;
@@ -158,57 +113,24 @@ int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id, b
               (unsigned long long)bytes, (unsigned long long)ctx->budget);
     return TNF_ERR_BUDGET_EXCEEDED;
   }
-  uint64_t slab_id = 0;
-  void* p = slab && bytes <= kSlabMaxBlock ? slab_block(ctx, bytes, &slab_id) : nullptr;
-  if (!p) {
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && give_back_idle(ctx)) {
-      cudaGetLastError();
-      e = cudaMalloc(&p, bytes);
-      total = ctx->live[0] + ctx->live[1] + ctx->live[2];
-    }
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return cuda_fail(e, "cudaMalloc");
-    }
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && give_back_staging(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+    total = ctx->live[0] + ctx->live[1] + ctx->live[2];
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(e, "cudaMalloc");
   }
   uint64_t nid = ctx->next_id++;
   ctx->bufs[nid] = tnf_buffer_rec{p, bytes, category};
-  ctx->bufs[nid].slab = slab_id;
   ctx->live[category] += bytes;
   ctx->peak[category] = std::max(ctx->peak[category], ctx->live[category]);
   ctx->true_peak = std::max(ctx->true_peak, total + bytes);
   *id = nid;
   return TNF_OK;
-}
-
-// tensor maps over a range that is freed are dropped (a later buffer may reuse the address)
-static void drop_maps(tnf_ctx* ctx, const void* ptr, uint64_t bytes) {
-  const uint8_t* lo = static_cast<const uint8_t*>(ptr);
-  for (auto m = ctx->maps.begin(); m != ctx->maps.end();) {
-    const uint8_t* b = static_cast<const uint8_t*>(m->first.base);
-    if (b >= lo && b < lo + bytes) m = ctx->maps.erase(m);
-    else ++m;
-  }
-}
-
-int32_t leave_slab_locked(tnf_ctx* ctx, uint64_t id) {
-  tnf_buffer_rec& r = ctx->bufs.at(id);
-  if (!r.slab) return TNF_OK;
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, r.bytes);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // work that still writes the buffer
-  if (e == cudaSuccess) e = cudaMemcpy(p, r.ptr, r.bytes, cudaMemcpyDeviceToDevice);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    if (p) cudaFree(p);
-    return cuda_fail(e, "buffer move");
-  }
-  drop_maps(ctx, r.ptr, r.bytes);
-  e = slab_release(ctx, r.slab);
-  r.ptr = p;
-  r.slab = 0;
-  return e == cudaSuccess ? TNF_OK : cuda_fail(e, "cudaFree");
 }
 
 int32_t free_locked(tnf_ctx* ctx, uint64_t id) {
@@ -218,9 +140,15 @@ int32_t free_locked(tnf_ctx* ctx, uint64_t id) {
     return TNF_ERR_UNKNOWN_BUFFER;
   }
   // cudaFree waits for work that may still use the memory; an imported range is only forgotten
-  cudaError_t e = it->second.slab ? slab_release(ctx, it->second.slab) : it->second.owned ? cudaFree(it->second.ptr) : cudaSuccess;
+  cudaError_t e = it->second.owned ? cudaFree(it->second.ptr) : cudaSuccess;
   ctx->live[it->second.category] -= it->second.bytes;
-  drop_maps(ctx, it->second.ptr, it->second.bytes);
+  // tensor maps over the freed range are dropped (a later buffer may reuse the address)
+  for (auto m = ctx->maps.begin(); m != ctx->maps.end();) {
+    const uint8_t* b = static_cast<const uint8_t*>(m->first.base);
+    const uint8_t* lo = static_cast<const uint8_t*>(it->second.ptr);
+    if (b >= lo && b < lo + it->second.bytes) m = ctx->maps.erase(m);
+    else ++m;
+  }
   ctx->bufs.erase(it);
   // a pool buffer freed directly leaves the pool's books too
   auto rented = ctx->ws_rented.find(id);
@@ -759,8 +687,7 @@ int32_t tnf_destroy(tnf_ctx* ctx) {
   cudaDeviceSynchronize();
   tnf_comm_teardown(ctx);
   for (auto& kv : ctx->bufs)
-    if (kv.second.owned && !kv.second.slab) cudaFree(kv.second.ptr);
-  for (auto& kv : ctx->slabs) cudaFree(kv.second.ptr);
+    if (kv.second.owned) cudaFree(kv.second.ptr);
   for (auto& kv : ctx->hosts) {
     if (kv.second.owned) cudaFreeHost(kv.second.ptr);
     else cudaHostUnregister(kv.second.ptr);

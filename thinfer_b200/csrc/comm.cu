@@ -264,8 +264,6 @@ int32_t tnf_ipc_export(tnf_ctx* ctx, uint64_t id, void* handle_64) {
       set_error("tnf_ipc_export: unknown buffer id %llu", (unsigned long long)id);
       return TNF_ERR_UNKNOWN_BUFFER;
     }
-    const int32_t st = leave_slab_locked(ctx, id);
-    if (st != TNF_OK) return st;
     p = it->second.ptr;
   }
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "cudaIpcMemHandle_t is 64 bytes");

@@ -19,16 +19,7 @@ struct tnf_buffer_rec {
   uint64_t bytes = 0;
   int category = 0;
   bool owned = true;   // false: registered with tnf_import_symmetric, never freed here
-  uint64_t slab = 0;   // id of the slab that holds it; 0: an allocation of its own
   void* mc = nullptr;  // NVSwitch multicast alias of the same range (imported symmetric buffers only)
-};
-
-// Device memory that loaded weights share. Blocks are handed out one after the other and no byte is handed out twice: a slab goes
-// back to the driver with its last block, by cudaFree, which waits for work that may still use any of them.
-struct tnf_slab {
-  void* ptr = nullptr;
-  uint64_t used = 0;  // bytes handed out
-  uint32_t live = 0;  // blocks that have not been freed
 };
 
 struct tnf_host_rec {
@@ -100,9 +91,7 @@ struct tnf_ctx {
   void* stage_host[2] = {nullptr, nullptr};
   cudaEvent_t stage_done[2] = {nullptr, nullptr};
   uint64_t stage_bytes = 0;
-  // tnf_load_weight: the slabs, the one that takes further blocks, and the staging that the loads use in turn
-  std::unordered_map<uint64_t, tnf_slab> slabs;
-  uint64_t next_slab = 1, open_slab = 0;
+  // tnf_load_weight: the staging that the loads use in turn
   uint64_t load_stage_id = 0, load_stage_bytes = 0;
   bool load_busy = false;
   // large writes from pageable memory: pinned slots of the copying threads, one such write at a time
@@ -119,10 +108,8 @@ int32_t cuda_fail(cudaError_t e, const char* what);
 uint8_t* resolve(tnf_ctx* ctx, const tnf_buf& b, uint64_t need_bytes, const char* name, int32_t* status);
 // Multicast alias of a view already validated by resolve(); null (error set) if its buffer has none.
 uint8_t* resolve_multicast(tnf_ctx* ctx, const tnf_buf& b, const char* name, int32_t* status);
-int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id, bool slab = false);
+int32_t alloc_locked(tnf_ctx* ctx, uint64_t bytes, int category, uint64_t* id);
 int32_t free_locked(tnf_ctx* ctx, uint64_t id);
-// Gives a buffer of a slab an allocation of its own (same contents), for uses that reach past it: an IPC handle covers an allocation.
-int32_t leave_slab_locked(tnf_ctx* ctx, uint64_t id);
 // Host -> device copy on the compute stream; the source may be reused when it returns.
 cudaError_t write_host(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n);
 // Quantises with the scale of the tensor itself, which g_used (may be null) waits for.

@@ -64,7 +64,7 @@ extern "C" int32_t tnf_load_weight(tnf_ctx* ctx, const void* w_host, int32_t src
     if (st == TNF_OK) {
       std::lock_guard<std::mutex> lk(ctx->mu);
       for (int i = 0; i < made && st == TNF_OK; ++i) {
-        st = alloc_locked(ctx, bytes[i], TNF_CAT_WEIGHTS, &ids[i], ctx->budget == 0);
+        st = alloc_locked(ctx, bytes[i], TNF_CAT_WEIGHTS, &ids[i]);
         if (st == TNF_OK) ptr[i] = static_cast<uint8_t*>(ctx->bufs.at(ids[i]).ptr);
       }
     }
