@@ -108,7 +108,8 @@ int32_t tnf_reclaimed_bytes(tnf_ctx* ctx, uint64_t* bytes);
  *   tnf_ws_release  puts a rented buffer back as idle. Its bytes stay allocated and stay in the
  *                   workspace category of the snapshot; work already enqueued on the compute stream
  *                   that uses it is ordered before whatever the next renter enqueues there.
- *   tnf_ws_drain    frees every idle buffer (the phase boundary call); buffers out on rent stay.
+ *   tnf_ws_drain    frees every idle buffer (the phase boundary call); buffers out on rent stay. The staging that
+ *                   tnf_load_weight keeps goes too; *freed_bytes counts the pool's buffers alone.
  *   tnf_ws_stats    out = {idle bytes, idle buffers, buffers out on rent, hits, misses, bytes freed
  *                   under memory pressure}.
  * The idle pool is the first holder asked when an allocation does not fit the budget
@@ -149,7 +150,8 @@ int32_t tnf_quantize_weight(tnf_ctx* ctx, tnf_buf w_src, int32_t src_dtype, uint
                             tnf_buf codes, tnf_buf scales, float* global_scale);
 /* The same from host memory (f32 or bf16 [n,k], pageable or pinned) in one call: makes the buffers (codes [n,k/2], DEVICE-layout
  * scales, and with bias_host the bf16 bias [n]; free each with tnf_free) and fills them. Without a budget the context keeps the
- * staging for the next load (up to 160 MB, given back when an allocation fails). bias_host and bias_id may be null. Blocking. */
+ * staging for the next load (up to 160 MB, in the snapshot's staging category); tnf_ws_drain gives it back, and so does an allocation of
+ * the context that fails without. bias_host and bias_id may be null. Blocking. */
 int32_t tnf_load_weight(tnf_ctx* ctx, const void* w_host, int32_t src_dtype, uint32_t n, uint32_t k, const uint16_t* bias_host,
                         uint64_t* codes_id, uint64_t* scales_id, uint64_t* bias_id, float* global_scale);
 /* Bytes of the DEVICE scale layout for a [rows,k] operand. */

@@ -88,6 +88,18 @@ def test_weights_freed_in_another_order(backend):
     assert be.mem_snapshot()["live_weights"] == before
 
 
+def test_staging_of_loads_is_given_back(backend):
+    import thinfer_b200 as T
+
+    be, w = backend, _weight(1000, 2080, True, 3)
+    for _ in range(2):
+        W = T.Nvfp4Weight.from_dense(be, w)
+        be.drain_pool()
+        assert be.mem_snapshot()["live_staging"] == 0
+        _check(be, W, w, None)
+        W.free(be)
+
+
 def test_loads_of_several_threads(backend):
     import thinfer_b200 as T
 

@@ -178,7 +178,7 @@ class Backend:
         return WsBuf(self, Buf(bid.value, 0, nbytes))
 
     def drain_pool(self) -> int:
-        """Frees every idle pool buffer (Workspace::drain_pool); returns the bytes freed."""
+        """Frees every idle pool buffer (Workspace::drain_pool) and the staging that weight loads keep; returns the pool's bytes freed."""
         freed = C.c_uint64()
         _check(self.lib.tnf_ws_drain(self._ctx, C.byref(freed)))
         return int(freed.value)

@@ -921,6 +921,7 @@ int32_t tnf_ws_drain(tnf_ctx* ctx, uint64_t* freed_bytes) {
   const uint64_t spilled = ctx->ws_spilled;
   const uint64_t freed = ws_spill_locked(ctx, UINT64_MAX);
   ctx->ws_spilled = spilled;  // a drain is a phase boundary, not memory pressure
+  give_back_staging(ctx);
   if (freed_bytes) *freed_bytes = freed;
   return TNF_OK;
 }
