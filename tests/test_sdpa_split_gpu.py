@@ -1,10 +1,13 @@
 """Attention with few blocks of 128 query rows and many keys: clusters of 2 to 8 CTAs share a block's key tiles (sdpa_split in
 csrc/rules.h; its rule is tested in test_rules.py). Against the restated reference, same tolerance and reason as test_sdpa_gpu.py."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import oracle as O
-from conftest import dev_scales_to_canonical, rel_fro
+from conftest import ROOT, dev_scales_to_canonical, rel_fro
 from test_sdpa_gpu import TOL, _inputs, _run
 
 pytestmark = pytest.mark.gpu
@@ -31,6 +34,35 @@ def test_split_matches_reference_recurrence(backend, b, s_q, s_k, h_q, h_kv, spr
             for r in range(0, s_q, 128):  # per block: an error in one cluster must not hide in the norm over all of them
                 assert rel_fro(got[bi, r: r + 128, h], want[bi, r: r + 128, h]) <= 1.5 * TOL, (bi, h, r)
     assert rel_fro(got, want) <= TOL
+
+
+FIRST_CALLS = """
+import threading
+import numpy as np
+import thinfer_b200 as T
+s_q, s_k, heads, n = 200, 2048, 2, 8
+rng = np.random.default_rng(5)
+q, k, v = (rng.standard_normal((1, s, heads, 128)).astype(np.float32) for s in (s_q, s_k, s_k))
+q, k, v = ((t.view(np.uint32) >> 16).astype(np.uint16) for t in (q, k, v))
+backends = [T.Backend(0) for _ in range(n)]
+bufs = [[be.upload(t) for t in (q, k, v)] + [be.allocate(q.nbytes)] for be in backends]
+gate, got = threading.Barrier(n), [None] * n
+def call(i):
+    gate.wait()
+    backends[i].scope().sdpa(*bufs[i], 1, s_q, s_k, heads, heads, 0.088)
+    backends[i].submit(30000)
+    got[i] = backends[i].read_buffer(bufs[i][3], np.uint16)
+threads = [threading.Thread(target=call, args=(i,)) for i in range(n)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+assert all(g is not None and np.array_equal(g, got[0]) for g in got), [g is not None and int((g != got[0]).sum()) for g in got]
+"""
+
+
+def test_first_calls_of_several_threads():
+    """The first calls of a process, all at once on contexts of their own, take the same kernel: the same bits."""
+    for _ in range(3):
+        subprocess.run([sys.executable, "-c", FIRST_CALLS], check=True, cwd=ROOT, timeout=300)
 
 
 @pytest.mark.parametrize("jumps", [

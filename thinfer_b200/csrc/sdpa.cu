@@ -37,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include <cstdint>
+#include <mutex>
 
 #include "../../include/thinfer_nvfp4.h"
 #include "context.h"
@@ -786,17 +787,25 @@ extern "C" int32_t tnf_sdpa(tnf_ctx* ctx, const tnf_sdpa_args* a) {
   p.wait_limit = ctx->wait_limit_cycles;
   p.s_q = a->s_q; p.s_k = a->s_k; p.h_q = a->h_q; p.h_kv = a->h_kv;
   p.scale_log2 = a->scale * 1.4426950408889634f;
-  static PerDeviceOnce once;
-  static int clusters[kMaxDevices][9] = {};  // clusters of 2 .. 8 CTAs that fit the device at once
-  int dev = ctx->device < kMaxDevices ? ctx->device : 0;
-  if (once.first_use() >= 0) {
-    cudaError_t e = cudaFuncSetAttribute(sdpa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sdpa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
-    if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
-    max_clusters(sdpa_kernel<true>, at::kThreads, at::kSmemBytes, ctx->sm_count, clusters[dev]);
-  }
   const uint64_t pairs = uint64_t(a->h_q) * a->b;
-  const uint32_t split = sdpa_split(pairs * ((uint64_t(a->s_q) + 127u) / 128u), a->s_k, clusters[dev]);
+  uint32_t split = 1u;
+  {
+    // One thread prepares a device; another's first call waits for the attributes and the whole table, so that the same call takes
+    // the same kernel whoever comes first. What failed is tried again by the next call.
+    static std::mutex mu;
+    static bool ready[kMaxDevices + 1] = {};       // the last entry: devices past the table, prepared by every call
+    static int clusters[kMaxDevices + 1][9] = {};  // clusters of 2 .. 8 CTAs that fit the device at once
+    const int dev = ctx->device < kMaxDevices ? ctx->device : kMaxDevices;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!ready[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(sdpa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(sdpa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(at::kSmemBytes));
+      if (e != cudaSuccess) return cuda_fail(e, "sdpa kernel attribute");
+      max_clusters(sdpa_kernel<true>, at::kThreads, at::kSmemBytes, ctx->sm_count, clusters[dev]);
+      ready[dev] = dev < kMaxDevices;
+    }
+    split = sdpa_split(pairs * ((uint64_t(a->s_q) + 127u) / 128u), a->s_k, clusters[dev]);
+  }
   if (split > 1u) {
     sdpa_split_plan(a->s_q, pairs, &p.plan);
   } else if (!sdpa_plan(a->s_q, pairs, uint32_t(ctx->sm_count), &p.plan)) {
