@@ -506,11 +506,13 @@ static int32_t run_gemm(tnf_ctx* ctx, const tnf_linear_args* a, const uint8_t* a
 // stream. The slots are written past the caches: they are read next by the DMA engine, and ordinary stores fetch every line first and
 // leave it dirty where the engine has to ask for it. Measured (us, plain copy / ordinary stores with four threads / these): 1 MB
 // 108 / - / 60, 3 MB 311 / - / 125, 6 MB 488 / 661 / 210, 12 MB 896 / 952 / 370, 24 MB 1860 / 1220 / 670, 72 MB 6490 / 2310 / 1800 (PCIe
-// alone 1305). Two threads are enough for a few MB (two against six at 4 MB: 147 / 180), six are best from 24 MB on. The slots
-// (kWriteStageBytes in all) are made on first use and freed with the context. Returns false when the caller has to copy the plain way
-// (slots in use by another thread's write, no pinned memory to be had); *err is a failed copy.
+// alone 1305). Two threads are enough for a few MB (two against six at 4 MB: 147 / 180), six are best from 24 MB on. The slots are made on
+// first use and freed with the context: 1 MB of them, which takes the driver 25 us, until the context's writes have carried
+// kWriteMany bytes, then 12 MB, which takes it 7 ms (a context's first 1 MB, with these at once: 5400 us, with those 230). Returns false when
+// the caller has to copy the plain way (slots in use by another thread's write, no pinned memory to be had); *err is a failed copy.
 constexpr uint32_t kWriteThreads = 6;
 constexpr uint64_t kWriteChunk = 1u << 20, kWriteStageBytes = 2 * kWriteThreads * kWriteChunk, kWriteStagedMin = 1u << 20;
+constexpr uint64_t kWriteFewBytes = 1u << 20, kWriteMany = 24u << 20;
 // `dst` on a 16-byte boundary
 static void copy_past_caches(uint8_t* dst, const uint8_t* src, uint64_t n) {
   uint64_t i = 0;
@@ -527,15 +529,25 @@ static void copy_past_caches(uint8_t* dst, const uint8_t* src, uint64_t n) {
 static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_t n, cudaError_t* err) {
   std::unique_lock<std::mutex> lk(ctx->write_mu, std::try_to_lock);
   if (!lk.owns_lock()) return false;
-  if (!ctx->write_stage && cudaHostAlloc(&ctx->write_stage, kWriteStageBytes, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->write_stage = nullptr;
-    return false;
+  ctx->write_seen += n;
+  const uint64_t room = ctx->write_seen >= kWriteMany ? kWriteStageBytes : kWriteFewBytes;
+  if (ctx->write_stage_bytes < room) {
+    void* stage = nullptr;
+    if (cudaHostAlloc(&stage, room, cudaHostAllocDefault) == cudaSuccess) {
+      if (ctx->write_stage) cudaFreeHost(ctx->write_stage);
+      ctx->write_stage = stage;
+      ctx->write_stage_bytes = room;
+    } else {  // goes on with those it has
+      cudaGetLastError();
+      if (!ctx->write_stage) return false;
+    }
   }
-  const uint64_t chunk = n >= (8u << 20) ? kWriteChunk : n >= (2u << 20) ? kWriteChunk / 2 : kWriteChunk / 4;
+  const bool few = ctx->write_stage_bytes < kWriteStageBytes;  // four slots, two threads
+  const uint64_t slot_bytes = few ? kWriteFewBytes / 4 : kWriteChunk;
+  const uint64_t chunk = std::min(slot_bytes, n >= (8u << 20) ? kWriteChunk : n >= (2u << 20) ? kWriteChunk / 2 : kWriteChunk / 4);
   const uint64_t chunks = (n + chunk - 1) / chunk;
   const uint32_t cores = std::thread::hardware_concurrency();
-  const uint32_t wanted = uint32_t(std::min<uint64_t>(kWriteThreads, std::max<uint64_t>(2u, n >> 21)));
+  const uint32_t wanted = few ? 2u : uint32_t(std::min<uint64_t>(kWriteThreads, std::max<uint64_t>(2u, n >> 21)));
   const uint32_t workers = uint32_t(std::min<uint64_t>(chunks, std::max(1u, std::min(wanted, cores / 2u))));
   cudaError_t status[kWriteThreads] = {};
   auto work = [&](uint32_t t) {
@@ -544,7 +556,7 @@ static bool staged_write(tnf_ctx* ctx, uint8_t* dst, const uint8_t* src, uint64_
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&read[i], cudaEventDisableTiming);
     uint32_t use = 0;
     for (uint64_t c = t; c < chunks && e == cudaSuccess; c += workers, ++use) {
-      uint8_t* slot = static_cast<uint8_t*>(ctx->write_stage) + (2u * t + (use & 1u)) * kWriteChunk;
+      uint8_t* slot = static_cast<uint8_t*>(ctx->write_stage) + (2u * t + (use & 1u)) * slot_bytes;
       if (use >= 2u) e = cudaEventSynchronize(read[use & 1u]);  // the copy that last read this slot
       if (e != cudaSuccess) break;
       const uint64_t off = c * chunk, bytes = std::min(chunk, n - off);

@@ -97,6 +97,7 @@ struct tnf_ctx {
   // large writes from pageable memory: pinned slots of the copying threads, one such write at a time
   std::mutex write_mu;
   void* write_stage = nullptr;
+  uint64_t write_stage_bytes = 0, write_seen = 0;  // bytes of the slots; bytes of all such writes
 };
 
 void tnf_comm_teardown(tnf_ctx* ctx);  // comm.cu
