@@ -35,6 +35,11 @@ void skinny(uint32_t m, uint32_t n, uint32_t k, int one, const int* clusters, ui
   const tnf::SkinnySplit s = tnf::skinny_split_rule(m, n, k, one != 0, clusters);
   out[0] = s.ctas; out[1] = s.share;
 }
+uint32_t dense_tile(uint32_t m, uint32_t n, int q, uint32_t sms) { return tnf::dense_tile_rule(m, n, q != 0, sms); }
+void dense_tiles(uint32_t m, uint32_t n, uint32_t k, int q, uint32_t sms, const int* clusters, uint32_t* out) {
+  const tnf::DenseTiles t = tnf::dense_tiles_rule(m, n, k, q != 0, sms, clusters);
+  out[0] = t.bn; out[1] = t.ctas; out[2] = t.share;
+}
 uint32_t split(uint64_t blocks, uint32_t s_k, const int* clusters) { return tnf::sdpa_split(blocks, s_k, clusters); }
 void split_items(uint32_t s_q, uint64_t pairs, uint32_t* out) {  // {pair, q_first, keys_mode} of every item
   tnf::SdpaPlan p{};
@@ -233,3 +238,31 @@ def test_shares_of_k(rules):
     assert seen >= {1, 2, 3, 4, 5, 6, 8}
     assert split(1, 3072, 3072, True) == (4, 3) and split(4, 9216, 9216, False) == (2, 18)  # measured choices ...
     assert split(4, 6144, 1024, True)[0] == 1 and split(1, 4736, 512, True)[0] == 1         # ... and what lost
+
+
+def test_dense_tiles(rules):
+    """The 1-CTA kernel takes the dense arm in one wave of its tiles, with 64 columns at least where they are quantised; clusters only for up
+    to 16 rows, all of them on the chip at once, every CTA with a stage of K, all stages covered."""
+    fit, none, out = (C.c_int * 9)(0, 0, 74, 45, 36, 27, 20, 14, 14), (C.c_int * 9)(), (C.c_uint32 * 3)()
+    seen = set()
+    for sms in (148, 7):
+        for m in (1, 5, 16, 17, 64, 128, 129, 512, 1200, 6400, 9600, 1 << 20):
+            for n in (8, 64, 256, 320, 1040, 2048, 3072, 4736, 9216, 18944, 18952, 1 << 20):
+                for q in (0, 1):
+                    bn, wave = rules.dense_tile(m, n, q, sms), lambda width: -(-m // 128) * -(-n // width) <= sms
+                    assert bn in (0, 32, 64, 128) and not (q and bn == 32)
+                    assert wave(bn) if bn else not wave(128)
+                    assert bn in (0, 64 if q else 32) or not wave(bn // 2)  # the narrowest
+                    for k in (32, 96, 512, 1120, 3072, 9216, 14336, 1 << 20):
+                        for counts in (fit, none):
+                            rules.dense_tiles(C.c_uint32(m), C.c_uint32(n), C.c_uint32(k), q, C.c_uint32(sms), counts, out)
+                            width, ctas, share = out
+                            if ctas == 1:
+                                assert width == bn
+                                continue
+                            assert m <= 16 and bn and ctas in (2, 4, 8) and width in (32, 64, 128) and not (q and width == 32)
+                            stages = -(-k // (256 if width == 32 else 128))
+                            assert (ctas - 1) * share < stages <= ctas * share
+                            assert -(-n // width) <= counts[ctas]
+                            seen.add((width, ctas))
+    assert {c for _, c in seen} == {2, 4, 8} and {w for w, _ in seen} == {32, 64, 128}
