@@ -39,7 +39,7 @@ constexpr int kProducerWarp = 0, kMmaWarp = 1, kFirstEpilogueWarp = 2;
 // pair_epilogue_rule leaves to it.
 enum Epilogue : int { kPlain, kGated, kQuantised, kSwiglu, kGeneral };
 // Epilogue warps: the quantiser's long chains of dependent operations need sixteen to overlap (GELU + NVFP4 output, 9472 x 4096 x 512:
-// 39.1 us with eight, 30.0 with sixteen), the others are as fast with eight.
+// 39.1 us with eight, 28.9 with sixteen), the others are as fast with eight.
 constexpr int epilogue_warps(int epi) { return epi == kQuantised ? 16 : 8; }
 constexpr int threads(int epi) { return 64 + 32 * epilogue_warps(epi); }  // producer warp, MMA warp, epilogue warps
 constexpr int kStagingBytes = 8 * 4096;  // 8 epilogue warps x (32 rows x 128 B)
@@ -176,9 +176,10 @@ __device__ __forceinline__ void epilogue_pair_dispatch(uint32_t mode, const uint
 // one's accumulator is on its way to registers and the group before leaves by TMA; bias, gate and residual are asked for a tile ahead.
 // The residual comes by TMA into the buffer that the result then takes (a lane's own loads touch 32 rows an instruction:
 // 10 000 of a tile's 11 000 cycles). 32-byte stores from registers instead of TMA stores, for the same reason: 19.8 -> 26.8 us.
-// Measured, kGeneral's epilogue -> this one (us, 9472 x 4096 x K): gated residual K = 512 53.7 -> 39.2, 3072 65 -> 56, 4096 73 -> 70;
-// GELU + NVFP4 512 37.7 -> 28.9, 2048 43.6 -> 36.9; NVFP4 512 29.5 -> 22.6; SwiGLU 512 32.0 -> 22.2, 3072 44.5 -> 42.9; GELU 512
-// 30.1 -> 25.9; plain 256 19.9 -> 17.9.
+// Measured when it came in, kGeneral's epilogue -> this one (us, 9472 x 4096 x K): gated residual K = 512 53.7 -> 39.2, 3072 65 -> 56,
+// 4096 73 -> 70; GELU + NVFP4 512 37.7 -> 28.9, 2048 43.6 -> 36.9; NVFP4 512 29.5 -> 22.6; SwiGLU 512 32.0 -> 22.2, 3072 44.5 -> 42.9; GELU
+// 512 30.1 -> 25.9; plain 256 19.9 -> 17.9. With the item's place before the accumulator wait as well: gated 512 39.3, 3072 52.9; GELU +
+// NVFP4 512 25.3; NVFP4 512 19.7; SwiGLU 512 21.9, 3072 40.7; GELU 512 26.3.
 struct PairShare {
   uint32_t t_addr;   // TMEM address of the warp's lanes, column 0 of the accumulator
   uint32_t g[2];     // its groups in drain order
